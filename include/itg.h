@@ -124,9 +124,9 @@ ITG_API int itg_fp64_peak(itg_handle* h, double* tflops);
  * reference's per-(mode, dim) algorithm cache (src/cudense.jl:284-326, cache
  * declared at src/ITensorsGPU.jl:55), which sweeps cuTENSOR algorithms on the
  * first use of a shape.  Here the first FP64 contraction of a shape whose
- * 128x128 tiling leaves the GPU under-filled times the tile variants
- * (128x128, 128x64, 64x64) on the call's own operands into a throw-away
- * output, and split contractions time the tcgen05 tile variants;
+ * 128x128 tiling leaves the GPU under-filled times the three most promising of
+ * the tile variants (128x128, 128x64, 64x64, 32x32, 16x16) on the call's own
+ * operands into a throw-away output, and split contractions time the tcgen05 tile variants;
  * grouped launches choose their tile per shape class.  All variants compute
  * bit-identical results (the same k order per output element), so tuning only
  * changes speed.  The choices live in one per-process cache guarded by a
@@ -135,7 +135,7 @@ ITG_API int itg_fp64_peak(itg_handle* h, double* tflops);
  * tune (they use the cached choice or the heuristic).
  * enable: 1 (default unless ITG_AUTOTUNE=0 in the environment) or 0
  * (heuristic choice only). */
-enum { ITG_TILE_128x128 = 0, ITG_TILE_128x64 = 1, ITG_TILE_64x64 = 2 };
+enum { ITG_TILE_128x128 = 0, ITG_TILE_128x64 = 1, ITG_TILE_64x64 = 2, ITG_TILE_32x32 = 3, ITG_TILE_16x16 = 4 };
 /* Split-precision tile variants (split_bn below): 128 and 256 columns per
  * CTA.  Either | ITG_SPLIT_STREAMK: one persistent CTA per resident slot, the
  * launch's work divided evenly between them, a tile shared by consecutive

@@ -34,8 +34,21 @@ constexpr int SPAD = 4;  // shared-memory row padding (doubles)
 // One BM x BN tile of C = alpha * A B + beta * C through the offset tables.
 // 256 threads as 16 x 16, each computing (BM/16) x (BN/16) outputs split in
 // two halves (rows ty*TM/2.. and BM/2 + ty*TM/2..) to keep shared-memory reads
-// conflict-free.  AK / BK: the operand's k offsets are the fast ones (then a
-// thread loads along k, otherwise along m / n).
+// conflict-free (one row / column per thread when the tile has 16 of them).
+// AK / BK: the operand's k offsets are the fast ones (then a thread loads along
+// k, otherwise along m / n).
+//
+// Bound by the FP64 pipe: an SM retires two FMAs a clock, so a 64 x 64 tile
+// spends 2048 clocks on each k, and the operands of even a 16 x 16 tile (32
+// doubles per 128 clocks) cost nothing beside the arithmetic.
+// Hence any tile runs at the same rate and the choice among them (cost_f64)
+// is only about filling the SMs evenly.
+template <int T>
+__device__ __forceinline__ int tile_pos(int lane, int i) {  // T positions per lane of a 16 T wide tile
+  if (T == 1) return lane;
+  return i < T / 2 ? lane * (T / 2) + i : 8 * T + lane * (T / 2) + (i - T / 2);
+}
+
 template <int BM, int BN, bool AK, bool BK>
 __device__ __forceinline__ void gemm_tile_f64(const double* __restrict__ A, const double* __restrict__ B,
                   double* __restrict__ C, const int64_t* __restrict__ offAm,
@@ -143,15 +156,9 @@ __device__ __forceinline__ void gemm_tile_f64(const double* __restrict__ A, cons
       const double* ap = as + kk * (BM + SPAD);
       const double* bp = bs + kk * (BN + SPAD);
 #pragma unroll
-      for (int i = 0; i < TM / 2; ++i) {
-        a[i] = ap[ty * (TM / 2) + i];
-        a[TM / 2 + i] = ap[BM / 2 + ty * (TM / 2) + i];
-      }
+      for (int i = 0; i < TM; ++i) a[i] = ap[tile_pos<TM>(ty, i)];
 #pragma unroll
-      for (int j = 0; j < TN / 2; ++j) {
-        b[j] = bp[tx * (TN / 2) + j];
-        b[TN / 2 + j] = bp[BN / 2 + tx * (TN / 2) + j];
-      }
+      for (int j = 0; j < TN; ++j) b[j] = bp[tile_pos<TN>(tx, j)];
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -164,12 +171,12 @@ __device__ __forceinline__ void gemm_tile_f64(const double* __restrict__ A, cons
   // Epilogue: scatter to C's layout.
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    int64_t m = m0 + (i < TM / 2 ? ty * (TM / 2) + i : BM / 2 + ty * (TM / 2) + (i - TM / 2));
+    int64_t m = m0 + tile_pos<TM>(ty, i);
     if (m >= M) continue;
     int64_t cm = offCm[m];
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      int64_t n = n0 + (j < TN / 2 ? tx * (TN / 2) + j : BN / 2 + tx * (TN / 2) + (j - TN / 2));
+      int64_t n = n0 + tile_pos<TN>(tx, j);
       if (n >= N) continue;
       double* c = C + cm + offCn[n];
       double v = alpha * acc[i][j];
@@ -233,8 +240,10 @@ template <int BM, int BN>
 constexpr size_t gemm_smem() { return sizeof(double) * 2 * GBK * ((BM + SPAD) + (BN + SPAD)); }
 
 // Tile shape of each ITG_TILE_* variant.
-inline int tile_bm(int tile) { return tile == ITG_TILE_64x64 ? 64 : 128; }
-inline int tile_bn(int tile) { return tile == ITG_TILE_128x128 ? 128 : 64; }
+constexpr int TILE_BM[] = {128, 128, 64, 32, 16}, TILE_BN[] = {128, 64, 64, 32, 16};
+constexpr int NTILE = 5;
+inline int tile_bm(int tile) { return TILE_BM[tile >= 0 && tile < NTILE ? tile : 0]; }
+inline int tile_bn(int tile) { return TILE_BN[tile >= 0 && tile < NTILE ? tile : 0]; }
 inline int64_t tile_count(int tile, int64_t M, int64_t N) {
   const int bm = tile_bm(tile), bn = tile_bn(tile);
   return ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
@@ -265,6 +274,8 @@ template <bool AK, bool BK>
 int launch_gemm_v(itg_handle* h, int tile, const ContractPlan& p, const double* A, const double* B, double* C,
                   double alpha, double beta) {
   switch (tile) {
+    case ITG_TILE_16x16: return launch_gemm_t<16, 16, AK, BK>(h, p, A, B, C, alpha, beta);
+    case ITG_TILE_32x32: return launch_gemm_t<32, 32, AK, BK>(h, p, A, B, C, alpha, beta);
     case ITG_TILE_64x64: return launch_gemm_t<64, 64, AK, BK>(h, p, A, B, C, alpha, beta);
     case ITG_TILE_128x64: return launch_gemm_t<128, 64, AK, BK>(h, p, A, B, C, alpha, beta);
     default: return launch_gemm_t<128, 128, AK, BK>(h, p, A, B, C, alpha, beta);
@@ -277,6 +288,20 @@ int launch_gemm(itg_handle* h, int tile, const ContractPlan& p, const double* A,
   if (p.a_kmaj) return launch_gemm_v<true, false>(h, tile, p, A, B, C, alpha, beta);
   if (p.b_kmaj) return launch_gemm_v<false, true>(h, tile, p, A, B, C, alpha, beta);
   return launch_gemm_v<false, false>(h, tile, p, A, B, C, alpha, beta);
+}
+
+template <int BM, int BN>
+int launch_grouped(itg_handle* h, const GroupProb* probs, int count, int64_t tiles, double alpha, double beta) {
+  static bool attr = false;
+  if (!attr) {
+    ITG_CUDA(h, cudaFuncSetAttribute(k_gemm_gather_f64_grouped<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)gemm_smem<BM, BN>()));
+    attr = true;
+  }
+  k_gemm_gather_f64_grouped<BM, BN><<<(unsigned)tiles, GTHREADS, gemm_smem<BM, BN>(), h->stream>>>(probs, count,
+                                                                                                  alpha, beta);
+  ITG_CHECK_LAUNCH(h);
+  return ITG_OK;
 }
 
 __global__ void k_scale_or_zero(int64_t n, double beta, double* __restrict__ C) {
@@ -569,10 +594,35 @@ int time_variant(itg_handle* h, F&& launch, float& best_ms) {
   return st;
 }
 
-int heuristic_tile(itg_handle* h, int64_t M, int64_t N) {
-  if (tile_count(ITG_TILE_128x128, M, N) >= h->num_sms) return ITG_TILE_128x128;
-  if (tile_count(ITG_TILE_128x64, M, N) >= h->num_sms) return ITG_TILE_128x64;
-  return ITG_TILE_64x64;
+// Modelled time of one tile shape, in FP64-pipe clocks: CTAs spread evenly, so
+// the busiest SM computes ceil(tiles / SMs) of them at two FMAs a clock.  The
+// last partial tiles count whole (their padding is computed).  A CTA also
+// spends about TILE_OVERHEAD clocks on its first loads and its epilogue, which
+// other CTAs of the SM hide except for one.  Against 128 / 64-wide tiles alone
+// (chosen by CTA count): the complex 150 x 131 x 143 contraction (600 x 286 x
+// 262 real) 291 -> 96 us, the H_eff chain at chi = 181 x 167 1312 -> 470 us.
+constexpr double TILE_OVERHEAD = 3000.0;
+double cost_f64(itg_handle* h, int tile, double tiles, double K) {
+  const double per = (double)tile_bm(tile) * tile_bn(tile) * std::ceil(K / GBK) * GBK / 2.0;
+  return std::ceil(tiles / h->num_sms) * per + TILE_OVERHEAD;
+}
+
+// All tile shapes, the cheapest by the model first (the wider one where the
+// narrower saves less than 3%: it reads its operands less often).
+void rank_tiles(itg_handle* h, int64_t M, int64_t N, int64_t K, int (&order)[NTILE]) {
+  double c[NTILE];
+  for (int t = 0; t < NTILE; ++t) {
+    c[t] = cost_f64(h, t, (double)tile_count(t, M, N), (double)K) * (1.0 + 0.03 * t);
+    order[t] = t;
+    if ((N + tile_bn(t) - 1) / tile_bn(t) > 65535) c[t] = 1e300 * (1 + t);  // the grid's y limit
+  }
+  std::stable_sort(order, order + NTILE, [&](int a, int b) { return c[a] < c[b]; });
+}
+
+int heuristic_tile(itg_handle* h, int64_t M, int64_t N, int64_t K) {
+  int order[NTILE];
+  rank_tiles(h, M, N, K, order);
+  return order[0];
 }
 
 int choose_f64(itg_handle* h, const ContractPlan& p, const double* A, const double* B, double alpha, int& tile) {
@@ -580,7 +630,7 @@ int choose_f64(itg_handle* h, const ContractPlan& p, const double* A, const doub
     tile = p.tile;
     return ITG_OK;
   }
-  tile = heuristic_tile(h, p.M, p.N);
+  tile = heuristic_tile(h, p.M, p.N, p.K);
   const bool big = tile_count(ITG_TILE_128x128, p.M, p.N) >= 4 * (int64_t)h->num_sms;
   if (p.key.empty() || big) {
     if (!p.key.empty()) p.tile = tile;
@@ -600,7 +650,10 @@ int choose_f64(itg_handle* h, const ContractPlan& p, const double* A, const doub
   float best = 1e30f;
   int best_tile = tile;
   int st = ITG_OK;
-  for (int cand : {ITG_TILE_128x128, ITG_TILE_128x64, ITG_TILE_64x64}) {
+  int order[NTILE];
+  rank_tiles(h, p.M, p.N, p.K, order);
+  for (int q = 0; q < 3; ++q) {  // the three that the model puts first
+    const int cand = order[q];
     float ms = 0.f;
     st = time_variant(h, [&]() { return launch_gemm(h, cand, p, A, B, out, alpha, 0.0); }, ms);
     if (st != ITG_OK) break;
@@ -799,50 +852,31 @@ int contract_grouped_f64(itg_handle* h, int count, double alpha, const double* c
     if (tiles > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "grouped: too many tiles");
     ProfScope prof(h, ITG_KERNEL_GEMM_F64);
     switch (tile) {
-      case ITG_TILE_64x64: {
-        static bool attr = false;
-        if (!attr) {
-          ITG_CUDA(h, cudaFuncSetAttribute(k_gemm_gather_f64_grouped<64, 64>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<64, 64>()));
-          attr = true;
-        }
-        k_gemm_gather_f64_grouped<64, 64><<<(unsigned)tiles, GTHREADS, gemm_smem<64, 64>(), h->stream>>>(
-            dprobs, count, alpha, bta);
-        break;
-      }
-      case ITG_TILE_128x64: {
-        static bool attr = false;
-        if (!attr) {
-          ITG_CUDA(h, cudaFuncSetAttribute(k_gemm_gather_f64_grouped<128, 64>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<128, 64>()));
-          attr = true;
-        }
-        k_gemm_gather_f64_grouped<128, 64><<<(unsigned)tiles, GTHREADS, gemm_smem<128, 64>(), h->stream>>>(
-            dprobs, count, alpha, bta);
-        break;
-      }
-      default: {
-        static bool attr = false;
-        if (!attr) {
-          ITG_CUDA(h, cudaFuncSetAttribute(k_gemm_gather_f64_grouped<128, 128>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)gemm_smem<128, 128>()));
-          attr = true;
-        }
-        k_gemm_gather_f64_grouped<128, 128><<<(unsigned)tiles, GTHREADS, gemm_smem<128, 128>(), h->stream>>>(
-            dprobs, count, alpha, bta);
-        break;
-      }
+      case ITG_TILE_16x16: return launch_grouped<16, 16>(h, dprobs, count, tiles, alpha, bta);
+      case ITG_TILE_32x32: return launch_grouped<32, 32>(h, dprobs, count, tiles, alpha, bta);
+      case ITG_TILE_64x64: return launch_grouped<64, 64>(h, dprobs, count, tiles, alpha, bta);
+      case ITG_TILE_128x64: return launch_grouped<128, 64>(h, dprobs, count, tiles, alpha, bta);
+      default: return launch_grouped<128, 128>(h, dprobs, count, tiles, alpha, bta);
     }
-    ITG_CHECK_LAUNCH(h);
-    return ITG_OK;
   };
-  // tile choice: cached per shape class (mode structure, log2 of the mean
-  // M, N, K and of the count), timed on first use when the GPU is under-filled
+  // tile choice: the cheapest by the model over all the problems' tiles (their
+  // mean depth standing for each one's), cached per shape class (mode structure,
+  // log2 of the mean M, N, K and of the count) and timed on first use when the
+  // GPU is under-filled
   int64_t t128 = 0;
   for (int i = 0; i < count; ++i) t128 += tile_count(ITG_TILE_128x128, plans[i]->M, plans[i]->N);
-  int tile = t128 >= h->num_sms ? ITG_TILE_128x128
-             : (2 * t128 >= h->num_sms ? ITG_TILE_128x64 : ITG_TILE_64x64);
+  int order[NTILE];
+  {
+    double c[NTILE];
+    for (int t = 0; t < NTILE; ++t) {
+      double nt = 0;
+      for (int i = 0; i < count; ++i) nt += (double)tile_count(t, plans[i]->M, plans[i]->N);
+      c[t] = tune::cost_f64(h, t, nt, sumK / count) * (1.0 + 0.03 * t);
+      order[t] = t;
+    }
+    std::stable_sort(order, order + NTILE, [&](int a, int b) { return c[a] < c[b]; });
+  }
+  int tile = order[0];
   std::vector<GroupProb> probs;
   if (t128 < 4 * (int64_t)h->num_sms) {
     std::vector<int64_t> ones(ITG_MAX_RANK, 1);
@@ -864,7 +898,8 @@ int contract_grouped_f64(itg_handle* h, int count, double alpha, const double* c
       h->prof_on = false;
       float best = 1e30f;
       int best_tile = tile, st = ITG_OK;
-      for (int cand : {ITG_TILE_128x128, ITG_TILE_128x64, ITG_TILE_64x64}) {
+      for (int q = 0; q < 3; ++q) {
+        const int cand = order[q];
         const int64_t tiles = build(cand, nullptr, tout, tp);
         if (cudaMemcpy(tdesc, tp.data(), sizeof(GroupProb) * tp.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
           st = itg_fail(h, ITG_ERR_CUDA, "autotune descriptor upload failed");
@@ -967,7 +1002,7 @@ extern "C" int itg_autotune_query(itg_handle* h, int rankA, const int64_t* dimsA
   int v = 0;
   if (p.tile >= 0) *tile = p.tile;
   else if (tune::lookup("f64|" + p.key, v)) *tile = v;
-  else *tile = tune::heuristic_tile(h, p.M, p.N);
+  else *tile = tune::heuristic_tile(h, p.M, p.N, p.K);
   if (p.split_bn) *split_bn = p.split_bn;
   else if (tune::lookup("split|" + p.key, v)) *split_bn = v;
   else *split_bn = p.N <= 128 ? ITG_SPLIT_BN_128 : ITG_SPLIT_BN_256;
@@ -978,7 +1013,7 @@ extern "C" int itg_autotune_force(itg_handle* h, int rankA, const int64_t* dimsA
                                   int rankB, const int64_t* dimsB, const int32_t* modesB, int rankC,
                                   const int64_t* dimsC, const int32_t* modesC, int tile, int split_bn) {
   if (!h) return ITG_ERR_INVALID;
-  if (tile > ITG_TILE_64x64 ||
+  if (tile >= NTILE ||
       (split_bn > 0 && (split_bn & ~ITG_SPLIT_STREAMK) != ITG_SPLIT_BN_128 &&
        (split_bn & ~ITG_SPLIT_STREAMK) != ITG_SPLIT_BN_256))
     return itg_fail(h, ITG_ERR_INVALID, "unknown variant (tile %d, split_bn %d)", tile, split_bn);
