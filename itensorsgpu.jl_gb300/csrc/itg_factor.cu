@@ -487,14 +487,36 @@ __global__ void k_build_rt(const double* __restrict__ A, int64_t m, int n, const
 }
 
 
+}  // namespace
+
+namespace itg {
+int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, double fro, double* ws, float* ws32,
+                   int* flag);
+}
+
+namespace {
 constexpr int JACOBI_MAX_SWEEPS = 60;
 constexpr int JACOBI_AUX_INTS = 8 + JACOBI_MAX_SWEEPS;
 constexpr int64_t ONECTA_MAX_N = 192;
+constexpr int64_t PRECOND_MIN_N = 24;
+constexpr int64_t START32_MIN_N = 192;  // FP64 Jacobi starts from the FP32 rotations above this (jacobi_run)
+// Below this many columns one CTA runs all sweeps in one launch (n = 10: 0.64
+// against 0.75 ms for the queued steps, n = 12: 0.87 against 0.82 ms).
+constexpr int64_t REG_MIN_N = 12;
+
+// Workspace of jacobi_run's FP32 start, 0 where it is not taken.
+bool start32(const itg_handle* h, int64_t m, int64_t n) {
+  return n > START32_MIN_N && h->jacobi_mode == 0 && m <= 2048;
+}
+size_t start32_bytes(const itg_handle* h, int64_t m, int64_t n) {
+  return start32(h, m, n) ? itg_align256(sizeof(double) * (n * n + m * n)) + sizeof(float) * (m * n + n * n) : 0;
+}
 
 // Runs Jacobi on W (m x n, m >= n) with V = I.  Returns ITG_ERR_NOTCONVERGED
 // (results still usable) when the sweep limit is hit.  flag_dev: at least
 // JACOBI_AUX_INTS device ints.
-int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* flag_dev,
+// ws: start32_bytes(m, n).
+int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* flag_dev, char* ws,
                int* sweeps_done) {
   k_identity<<<itg_blocks_for(n * n, 256, h->num_sms * 8), 256, 0, h->stream>>>((int)n, V);
   ITG_CHECK_LAUNCH(h);
@@ -510,7 +532,10 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   ITG_CUDA(h, cudaStreamSynchronize(h->stream));
   const double fro = h->pinned[0];
   const double amin_conv = (10.0 * 2.220446049250313e-16 * fro) * (10.0 * 2.220446049250313e-16 * fro);
-  if (n <= ONECTA_MAX_N) {
+  // one CTA for all sweeps: the smallest problems, and those that the
+  // register-resident steps cannot take (a small n with very long columns) or
+  // where they are switched off
+  if (n <= ONECTA_MAX_N && (h->jacobi_mode != 0 || m > 2048 || n < REG_MIN_N)) {
     k_jacobi_onecta<<<1, 1024, 0, h->stream>>>(W, m, (int)n, V, tol, amin_conv, JACOBI_MAX_SWEEPS, flag_dev);
     ITG_CHECK_LAUNCH(h);
     int* hp = (int*)h->pinned;
@@ -519,6 +544,9 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
     *sweeps_done = hp[0];
     return hp[0] >= JACOBI_MAX_SWEEPS ? ITG_ERR_NOTCONVERGED : ITG_OK;
   }
+  if (start32(h, m, n) && std::isfinite(fro) && fro > 0.0)
+    ITG_TRY(itg::jacobi_start32(h, W, m, n, V, fro, (double*)ws,
+                                (float*)(ws + itg_align256(sizeof(double) * (n * n + m * n))), flag_dev));
   if (h->jacobi_mode == 0 || h->jacobi_mode == 3) {
     const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, JACOBI_MAX_SWEEPS, flag_dev,
                                                sweeps_done, amin_conv);
@@ -621,7 +649,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
   // exactly orthonormal: that side is then Q times the rotations (or the
   // refined eigenvectors), never U_J = J V_J / S, which loses orthogonality
   // in columns whose S is small or rounding noise (rank-deficient inputs)
-  const bool pre = (h->svd_qr_precond && nn > ONECTA_MAX_N) || iso != ISO_NONE;
+  const bool pre = (h->svd_qr_precond && nn > PRECOND_MIN_N) || iso != ISO_NONE;
   const bool two = pre && iso == ISO_RIGHT;
   // the Jacobi problem: W itself (mj = mm rows) or J (nn x nn)
   const int64_t mj = pre ? nn : mm;
@@ -636,6 +664,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     oWs = take(sizeof(double) * itg::svd_mixed_ws_doubles(mj, nn));
     oWs32 = take(sizeof(float) * (mj * nn + nn * nn));
   }
+  const size_t oStart = take(start32_bytes(h, mj, nn));
   size_t oTq = 0, oTq2 = 0, oQws = 0;
   if (pre) {
     oVh = take(sizeof(double) * mm * nn);
@@ -735,7 +764,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     k_gather_cols<<<g2, 256, 0, h->stream>>>(Vw, nn, order, sig, 0, (int)nn, Jr_dst, ld_r);
     ITG_CHECK_LAUNCH(h);
   } else {
-    st = jacobi_run(h, J, mj, nn, Vw, flag, &sweeps);
+    st = jacobi_run(h, J, mj, nn, Vw, flag, base + oStart, &sweeps);
     if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
     k_unit_cols<<<(unsigned)nn, 256, 0, h->stream>>>(Vw, nn);
     k_col_norms<<<(unsigned)nn, 256, 0, h->stream>>>(J, mj, sig);
@@ -846,7 +875,7 @@ extern "C" int itg_eigh_trunc(itg_handle* h, int64_t n, const double* A, int64_t
   size_t oW = take(sizeof(double) * n * n), oV = take(sizeof(double) * n * n),
          oSig = take(sizeof(double) * n), oP = take(sizeof(double) * n),
          oOrd = take(sizeof(int) * n), oOut = take(4 * sizeof(double)), oFlag = take(sizeof(int) * JACOBI_AUX_INTS),
-         oC = take(sizeof(double));
+         oC = take(sizeof(double)), oStart = take(start32_bytes(h, n, n));
   ITG_TRY(itg_scratch_reserve(h, off));
   char* base = (char*)h->scratch;
   double* W = (double*)(base + oW);
@@ -865,7 +894,7 @@ extern "C" int itg_eigh_trunc(itg_handle* h, int64_t n, const double* A, int64_t
   k_copy_matrix<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, n, n, W, shift);
   ITG_CHECK_LAUNCH(h);
   int sweeps = 0;
-  int st = jacobi_run(h, W, n, n, Vw, flag, &sweeps);
+  int st = jacobi_run(h, W, n, n, Vw, flag, base + oStart, &sweeps);
   if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
   k_unit_cols<<<(unsigned)n, 256, 0, h->stream>>>(Vw, n);
   k_col_norms<<<(unsigned)n, 256, 0, h->stream>>>(W, n, sig);

@@ -232,13 +232,6 @@ __host__ __device__ inline T conv_tol(T tol) {
   return sizeof(T) == 8 ? T(4) * tol : tol;
 }
 
-// Short FP64 columns (m <= JB_SMALL_M) run one warp per pair (THREADS =
-// 32 WB): the pair's sums then come from warp shuffles alone, which saves a
-// shared-memory reduction and one of the two barriers of every round
-// (measured at n = 378: 104 -> 82 ms per FP64 split; the FP32 Jacobi of the
-// mixed method was slower that way, 20.4 -> 22.7 ms, and keeps 512 threads).
-constexpr int64_t JB_SMALL_M = 1024;
-
 template <class T, int WB, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 k_jacobi_block_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, T tol, T tol_conv, T amin,
@@ -419,210 +412,333 @@ k_jacobi_block_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, T to
   if (t == 0 && major) *rotated = 1;
 }
 
-// FP32 block step with 16-byte accesses (m and n multiples of 4, n <= m):
-// the rotations of k_jacobi_block_step<float> in the same order, with the
-// pair's columns staged, summed and rotated four rows at a time.  V's columns
-// are staged in shared memory (the column buffer is free after the write-back)
-// and each thread applies Q to four rows x four columns with its four Q
-// columns held in registers; the per-output sums run over d in the same order
-// as the element-wise kernel's.
-template <int WB, int THREADS>
-__global__ void __launch_bounds__(THREADS)
-k_jacobi_block_step_f4(float* __restrict__ W, int64_t m, int n, float* __restrict__ V, float tol, float tol_conv,
-                       float amin, float amin_conv, int step, int first, int* __restrict__ rotated) {
-  constexpr int C2 = 2 * WB;          // local columns
-  constexpr int TP = THREADS / WB;    // threads per pair
-  constexpr int WPG = TP / 32;        // warps per pair group
-  constexpr int NG = C2 / 4;          // output column groups of the V update
-  extern __shared__ __align__(16) unsigned char jb_smem[];
-  float* cols = (float*)jb_smem;       // [C2][m]
-  float* Q = cols + (int64_t)C2 * m;   // [C2][C2], column-major
-  float* red = Q + C2 * C2;            // [WB][WPG][3]
-  __shared__ int any, major;
+// ------------------------------------------- register-resident block step
+// The same block-cyclic step with the pair's columns held in registers: thread
+// t keeps RPT rows of all 2 WB columns (rows t, t + threads, ..., or four
+// consecutive ones with 16-byte accesses, VEC), so a rotation round touches
+// no shared memory but for its sums.  A round's WB dot products are reduced
+// together (a transposing butterfly: 9 shuffles for 8 values instead of 40)
+// and the squared norms are carried along (a' = a - t g, b' = b + t g;
+// computed afresh at the start of a step and whenever one shrank to less than
+// a quarter, where the difference has cancelled).  The rotations of all rounds
+// are kept and replayed on the rows of V afterwards.
+//
+// What bounds it: FP32, the issue of its FMAs (5 a row, pair and round, 4 more
+// for V) and the latency of a round's reduction and angle; FP64,
+// the FP64 pipe (a warp instruction takes 64 clocks of its quarter of the SM),
+// so there the divisions and square roots of the angle are taken in FP32 and
+// corrected by Newton steps in FP64 (15 FP64 instructions instead of several
+// hundred), and a problem runs on few warps with many rows each.  Blocks of 8
+// columns in FP32 and 4 in FP64 (fewer pairs wait for one SM's FP64 pipe).
+// Measured: a step of the FP32 sweeps 27 -> 19 us at n = 2048 and 15.5 -> 9 us
+// at n = 366; FP64, n = 120: 14 us a step where one CTA needed 9 ms a sweep
+// (the 150 x 120 SVD 153 -> 6 ms together with the QR before it), and errors of
+// 6e-16 |W| instead of 2e-14 |W| in the singular values.
+// Sums of NV values over the warp's lanes: afterwards lane l holds the sum of
+// value l >> (5 - log2 NV).
+template <class T, int NV>
+__device__ __forceinline__ T jp_transpose_sum(T (&v)[NV], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int n = NV; n > 1; n >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const T send = up ? v[i] : v[i + n / 2];
+      const T keep = up ? v[i + n / 2] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    o >>= 1;
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// A rotation is applied as w_p -= s (w_q + u w_p), w_q += s (w_p - u w_q) with
+// u = tan(theta / 2) = s / (1 + c): two FMAs a column like the plain form, but
+// its rounding is proportional to s, so the many small rotations of the late
+// sweeps leave no trace in the columns' norms (Rutishauser, "The Jacobi method
+// for real symmetric matrices", Numer. Math. 9 (1966)).  It is orthogonal to
+// rounding for any u as long as s = 2 u / (1 + u^2).
+//
+// jp_angle: the rotation of a pair from its squared norms and dot product;
+// true when the pair is rotated.  t = tan(theta), for the norms' update; major:
+// it counts against convergence.
+__device__ __forceinline__ float jp_sqrt1p2(float x) {  // sqrt(1 + x^2), a few ulp
+  const float y = fmaf(x, x, 1.f);
+  return y * rsqrtf(y);
+}
+__device__ __forceinline__ bool jp_angle(float a, float b, float g, float tol, float tol_conv, float amin,
+                                         float amin_conv, float& t, float& u, float& s, bool& major) {
+  const float cosine = fabsf(g) * rsqrtf(a) * rsqrtf(b);  // NaN for a zero column
+  major = a > amin_conv && b > amin_conv && cosine > tol_conv;
+  t = u = s = 0.f;
+  if (a <= amin || b <= amin || !(cosine > tol)) return false;
+  const float zeta = __fdividef(b - a, 2.f * g);
+  const float az = fabsf(zeta);
+  t = copysignf(__fdividef(az > 1e9f ? 0.5f : 1.f, az > 1e9f ? az : az + jp_sqrt1p2(az)), zeta);
+  u = __fdividef(t, 1.f + jp_sqrt1p2(t));
+  const float x = fmaf(u, u, 1.f);
+  const float r = __fdividef(1.f, x);
+  s = 2.f * u * fmaf(r, fmaf(-x, r, 1.f), r);
+  return true;
+}
+
+// x 2^-(e - 1023) as a float, truncated, and a float as a double, by integer
+// instructions: an FP64 conversion occupies a quarter of an SM for 64 clocks.
+__device__ __forceinline__ float jp_to_float(double x, int e) {
+  const int hi = __double2hiint(x);
+  const int ex = ((hi >> 20) & 0x7FF) - e + 127;
+  const int bits = (ex << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)__double2loint(x) >> 29);
+  return ex <= 0 ? 0.f : __int_as_float((hi & 0x80000000) | (ex >= 255 ? 0x7F800000 : bits));
+}
+__device__ __forceinline__ double jp_to_double(float x) {  // normal numbers; below that zero
+  const int b = __float_as_int(x), ex = (b >> 23) & 0xFF;
+  return ex == 0 ? 0.0 : __hiloint2double((b & 0x80000000) | ((ex + 896) << 20) | ((b & 0x7FFFFF) >> 3), b << 29);
+}
+__device__ __forceinline__ bool jp_less(double x, double y) {  // x < y for non-negative x and y
+  return __double_as_longlong(x) < __double_as_longlong(y);
+}
+__device__ __forceinline__ bool jp_angle(double a, double b, double g, float tol, float tol_conv, double amin,
+                                         double amin_conv, double& t, double& u, double& s, bool& major) {
+  // scaled by a power of two so that max(a, b) is in [1, 2): FP32 then spans
+  // norm ratios to 1e-19
+  const int ea = (__double2hiint(a) >> 20) & 0x7FF, eb = (__double2hiint(b) >> 20) & 0x7FF;
+  const int e = ea > eb ? ea : eb;
+  const double d = b - a;
+  const float fg = jp_to_float(g, e), fa = jp_to_float(a, e), fb = jp_to_float(b, e), fd = jp_to_float(d, e);
+  const float cosine = fabsf(fg) * rsqrtf(fa) * rsqrtf(fb);
+  major = jp_less(amin_conv, a) && jp_less(amin_conv, b) && cosine > tol_conv;
+  const bool rot = jp_less(amin, a) && jp_less(amin, b) && cosine > tol;
+  const float zeta = __fdividef(fd, 2.f * fg);
+  const float az = fabsf(zeta);
+  const float tf = copysignf(__fdividef(az > 1e9f ? 0.5f : 1.f, az > 1e9f ? az : az + jp_sqrt1p2(az)), zeta);
+  t = jp_to_double(tf);
+  // one Newton step of g t^2 + d t - g = 0 (its derivative is at least 2 |g|),
+  // the residual in FP64, the step in FP32
+  const double f = fma(t, fma(g, t, d), -g);
+  // u = t / (1 + q), q = sqrt(1 + t^2), to FP32 accuracy and corrected to first
+  // order for its rounding, found from (u^2 - 1) t + 2 u = 0 (derivative
+  // 2 (1 + t u)), and for the Newton step, du = dt / (q (1 + q))
+  const float q = jp_sqrt1p2(tf);
+  const float uf = __fdividef(tf, 1.f + q);
+  const double ud = jp_to_double(uf);
+  const double w = fma(ud, fma(t, ud, 2.0), -t);
+  const float dt = -__fdividef(jp_to_float(f, e), fmaf(2.f * fg, tf, fd));
+  u = ud + jp_to_double(__fdividef(dt, q * (1.f + q)) -
+                        __fdividef(jp_to_float(w, 1023), 2.f * fmaf(tf, uf, 1.f)));
+  // s = 2 u / (1 + u^2): the reciprocal from FP32, its error removed to second order
+  const double x = fma(u, u, 1.0);
+  const double r = jp_to_double(__fdividef(1.f, fmaf(uf, uf, 1.f)));
+  const double s0 = (u + u) * r;
+  const double er = fma(-x, r, 1.0);
+  s = fma(s0, fma(er, er, er), s0);
+  if (!rot) t = u = s = 0.0;
+  return rot;
+}
+// A squared norm that shrank to less than about a quarter (or cancelled to a
+// negative number) is computed afresh.
+__device__ __forceinline__ bool jp_shrunk(float now, float before) { return now < 0.25f * before; }
+__device__ __forceinline__ bool jp_shrunk(double now, double before) {
+  return (__double2hiint(now) >> 20) + 2 <= (__double2hiint(before) >> 20);
+}
+
+constexpr int64_t JR_MAX_M = 2048;  // rows held in registers: 8 for each of 256 threads
+
+// `prev`: nullptr, or the rotated flag of the sweep before (the step does
+// nothing when that sweep had converged; lets several sweeps be queued).
+template <class T, int WB, int RPT, bool VEC, bool FIRST, int MAXT>
+__global__ void __launch_bounds__(MAXT)
+k_jacobi_reg_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, float tol, float tol_conv, T amin,
+                  T amin_conv, int step, const int* prev, int* rotated) {
+  constexpr int C2 = 2 * WB;                 // columns of the pair
+  constexpr int NR = FIRST ? C2 - 1 : WB;    // rounds
+  constexpr int MAXW = MAXT / 32;
+  struct __align__(2 * sizeof(T)) Rot {
+    T u, s;
+  };
+  __shared__ T red[2][MAXW][WB];
+  __shared__ T nred[MAXW][C2];
+  __shared__ Rot rots[NR][WB];           // all rounds, for V
+  __shared__ Rot rotw[MAXW][WB];         // the current round, one copy a warp
+  __shared__ unsigned rmask[NR];
+  // the previous step's kernel must be done before its columns are read
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (prev && *(const volatile int*)prev == 0) return;
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
   const int bi = jp_player(blockIdx.x, step, nbp), bj = jp_player(nbp - 1 - blockIdx.x, step, nbp);
-  const int t = threadIdx.x;
-  const int m4 = (int)(m >> 2), n4 = n >> 2;
-  float4* cols4 = reinterpret_cast<float4*>(cols);
-  float4* W4 = reinterpret_cast<float4*>(W);
-  float4* V4 = reinterpret_cast<float4*>(V);
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  int gcs[C2];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nw = blockDim.x >> 5;
+  const int64_t c0 = (int64_t)bi * WB, c1 = (int64_t)bj * WB;
+  const int nI = bi < nb ? (n - c0 < WB ? (int)(n - c0) : WB) : 0;  // columns of each block
+  const int nJ = bj < nb ? (n - c1 < WB ? (int)(n - c1) : WB) : 0;
+  const int bd = (int)blockDim.x;
+
+  T x[C2][RPT];
+  // row of this thread's element k, counted from r0
+  auto row = [&](int k) { return VEC ? 4 * (int64_t)(t + (k >> 2) * bd) + (k & 3) : t + (int64_t)k * bd; };
+  // rows r0 + ... of the pair's columns of X (leading dimension and row count ld)
+  auto load = [&](const T* X, int64_t ld, int64_t r0) {
 #pragma unroll
-  for (int c = 0; c < C2; ++c) {
-    const int blk = c < WB ? bi : bj;
-    const int gc = blk * WB + (c < WB ? c : c - WB);
-    gcs[c] = (blk < nb && gc < n) ? gc : -1;
-  }
-  if (t == 0) any = major = 0;
-  for (int i = t; i < m4; i += THREADS) {
-    float4 v[C2];
+    for (int c = 0; c < C2; ++c) {
+      const bool in = c < WB ? c < nI : c - WB < nJ;
+      const T* col = X + (c < WB ? c0 + c : c1 + c - WB) * ld + r0;
+      const int64_t left = in ? ld - r0 : 0;
+      if constexpr (VEC) {
 #pragma unroll
-    for (int c = 0; c < C2; ++c) v[c] = gcs[c] >= 0 ? W4[(int64_t)gcs[c] * m4 + i] : zero4;
+        for (int k = 0; k < RPT; k += 4) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (row(k) < left) v = *reinterpret_cast<const float4*>(col + row(k));
+          x[c][k] = v.x;
+          x[c][k + 1] = v.y;
+          x[c][k + 2] = v.z;
+          x[c][k + 3] = v.w;
+        }
+      } else {
 #pragma unroll
-    for (int c = 0; c < C2; ++c) cols4[(int64_t)c * m4 + i] = v[c];
-  }
-  for (int i = t; i < C2 * C2; i += THREADS) Q[i] = (i % (C2 + 1) == 0) ? 1.f : 0.f;
-  __syncthreads();
-  const int g = t / TP, lt = t % TP, wg = lt / 32, lane = t & 31;
-  const int rounds = first ? C2 - 1 : WB;
-  for (int r = 0; r < rounds; ++r) {
-    int p, q;
-    if (first) {
-      p = jp_player(g, r, C2);
-      q = jp_player(C2 - 1 - g, r, C2);
-    } else {
-      p = g;
-      q = WB + (g + r) % WB;
-    }
-    if (p > q) {
-      const int tmp = p;
-      p = q;
-      q = tmp;
-    }
-    float4* xp = cols4 + (int64_t)p * m4;
-    float4* xq = cols4 + (int64_t)q * m4;
-    float a = 0.f, b = 0.f, gg = 0.f, a1 = 0.f, b1 = 0.f, g1 = 0.f;
-    int i = lt;
-    for (; i + TP < m4; i += 2 * TP) {
-      const float4 x0 = xp[i], y0 = xq[i], x1 = xp[i + TP], y1 = xq[i + TP];
-      a = fmaf(x0.x, x0.x, a);
-      b = fmaf(y0.x, y0.x, b);
-      gg = fmaf(x0.x, y0.x, gg);
-      a1 = fmaf(x0.y, x0.y, a1);
-      b1 = fmaf(y0.y, y0.y, b1);
-      g1 = fmaf(x0.y, y0.y, g1);
-      a = fmaf(x0.z, x0.z, a);
-      b = fmaf(y0.z, y0.z, b);
-      gg = fmaf(x0.z, y0.z, gg);
-      a1 = fmaf(x0.w, x0.w, a1);
-      b1 = fmaf(y0.w, y0.w, b1);
-      g1 = fmaf(x0.w, y0.w, g1);
-      a = fmaf(x1.x, x1.x, a);
-      b = fmaf(y1.x, y1.x, b);
-      gg = fmaf(x1.x, y1.x, gg);
-      a1 = fmaf(x1.y, x1.y, a1);
-      b1 = fmaf(y1.y, y1.y, b1);
-      g1 = fmaf(x1.y, y1.y, g1);
-      a = fmaf(x1.z, x1.z, a);
-      b = fmaf(y1.z, y1.z, b);
-      gg = fmaf(x1.z, y1.z, gg);
-      a1 = fmaf(x1.w, x1.w, a1);
-      b1 = fmaf(y1.w, y1.w, b1);
-      g1 = fmaf(x1.w, y1.w, g1);
-    }
-    if (i < m4) {
-      const float4 x0 = xp[i], y0 = xq[i];
-      a = fmaf(x0.x, x0.x, a);
-      b = fmaf(y0.x, y0.x, b);
-      gg = fmaf(x0.x, y0.x, gg);
-      a1 = fmaf(x0.y, x0.y, a1);
-      b1 = fmaf(y0.y, y0.y, b1);
-      g1 = fmaf(x0.y, y0.y, g1);
-      a = fmaf(x0.z, x0.z, a);
-      b = fmaf(y0.z, y0.z, b);
-      gg = fmaf(x0.z, y0.z, gg);
-      a1 = fmaf(x0.w, x0.w, a1);
-      b1 = fmaf(y0.w, y0.w, b1);
-      g1 = fmaf(x0.w, y0.w, g1);
-    }
-    a += a1;
-    b += b1;
-    gg += g1;
-    a = jp_warp_sum(a);
-    b = jp_warp_sum(b);
-    gg = jp_warp_sum(gg);
-    if constexpr (WPG > 1) {
-      if (lane == 0) {
-        red[(g * WPG + wg) * 3 + 0] = a;
-        red[(g * WPG + wg) * 3 + 1] = b;
-        red[(g * WPG + wg) * 3 + 2] = gg;
+        for (int k = 0; k < RPT; ++k) x[c][k] = row(k) < left ? col[row(k)] : T(0);
       }
+    }
+  };
+  auto store = [&](T* X, int64_t ld, int64_t r0) {
+#pragma unroll
+    for (int c = 0; c < C2; ++c) {
+      const bool in = c < WB ? c < nI : c - WB < nJ;
+      T* col = X + (c < WB ? c0 + c : c1 + c - WB) * ld + r0;
+      const int64_t left = in ? ld - r0 : 0;
+      if constexpr (VEC) {
+#pragma unroll
+        for (int k = 0; k < RPT; k += 4)
+          if (row(k) < left)
+            *reinterpret_cast<float4*>(col + row(k)) = make_float4(x[c][k], x[c][k + 1], x[c][k + 2], x[c][k + 3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < RPT; ++k)
+          if (row(k) < left) col[row(k)] = x[c][k];
+      }
+    }
+  };
+  auto rotate = [&](int p, int q, const Rot& o) {
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const T y = x[p][k], z = x[q][k];
+      x[p][k] = fma(-o.s, fma(o.u, y, z), y);
+      x[q][k] = fma(o.s, fma(-o.u, z, y), z);
+    }
+  };
+  // A round always rotates the same register columns (position g with partner(g));
+  // the columns move one position on between rounds and are back in place after
+  // the last, so the rounds are one loop: unrolled, they ran once each from a
+  // cold instruction cache (FP64, n = 120: 4 us of a 5 us round).
+  auto partner = [](int g) { return FIRST ? C2 - 1 - g : WB + g; };
+  auto advance = [&]() {
+    constexpr int lo = FIRST ? 1 : WB;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      const T y = x[lo][k];
+#pragma unroll
+      for (int c = lo; c + 1 < C2; ++c) x[c][k] = x[c + 1][k];
+      x[C2 - 1][k] = y;
+    }
+  };
+  const int next_lane = FIRST ? (lane == 0 ? 0 : (lane == C2 - 1 ? 1 : lane + 1))
+                              : (lane < WB ? lane : (lane == C2 - 1 ? WB : lane + 1));
+
+  load(W, m, 0);
+  // every warp computes the angles of a round (one barrier a round; shuffles
+  // inside a branch for one warp cost about 500 clocks each)
+  T norm = T(0);  // lane c < C2: squared norm of the column at position c
+  bool dirty = true;
+  unsigned any = 0, any_major = 0;
+#pragma unroll 1
+  for (int r = 0; r < NR; ++r) {
+    if (dirty) {  // block-uniform
+      T v[C2];
+#pragma unroll
+      for (int c = 0; c < C2; ++c) {
+        v[c] = x[c][0] * x[c][0];
+#pragma unroll
+        for (int k = 1; k < RPT; ++k) v[c] = fma(x[c][k], x[c][k], v[c]);
+      }
+      constexpr int SH = C2 == 16 ? 1 : 2;  // 5 - log2 C2
+      const T sum = jp_transpose_sum<T, C2>(v, lane);
+      if ((lane & ((1 << SH) - 1)) == 0) nred[warp][lane >> SH] = sum;
       __syncthreads();
-      a = 0.f;
-      b = 0.f;
-      gg = 0.f;
-#pragma unroll
-      for (int w = 0; w < WPG; ++w) {
-        a += red[(g * WPG + w) * 3 + 0];
-        b += red[(g * WPG + w) * 3 + 1];
-        gg += red[(g * WPG + w) * 3 + 2];
-      }
+      T a = nred[0][lane & (C2 - 1)];
+      for (int w = 1; w < nw; ++w) a += nred[w][lane & (C2 - 1)];
+      norm = a;
+      // nred is rewritten only after later barriers of this loop
     }
-    const bool rot = !(a <= amin || b <= amin || fabsf(gg) <= tol * sqrtf(a) * sqrtf(b));
-    if (rot) {
-      const float zeta = (b - a) / (2.f * gg);
-      const float tt = copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
-      const float c = 1.f / sqrtf(1.f + tt * tt), sn = c * tt;
-      for (int j = lt; j < m4; j += TP) {
-        const float4 x = xp[j], y = xq[j];
-        xp[j] = make_float4(c * x.x - sn * y.x, c * x.y - sn * y.y, c * x.z - sn * y.z, c * x.w - sn * y.w);
-        xq[j] = make_float4(sn * x.x + c * y.x, sn * x.y + c * y.y, sn * x.z + c * y.z, sn * x.w + c * y.w);
+    {
+      T v[WB];
+#pragma unroll
+      for (int g = 0; g < WB; ++g) {
+        v[g] = x[g][0] * x[partner(g)][0];
+#pragma unroll
+        for (int k = 1; k < RPT; ++k) v[g] = fma(x[g][k], x[partner(g)][k], v[g]);
       }
-      if (lt < C2) {
-        const float x = Q[lt + p * C2], y = Q[lt + q * C2];
-        Q[lt + p * C2] = c * x - sn * y;
-        Q[lt + q * C2] = sn * x + c * y;
-      }
-      if (lt == 0) {
-        any = 1;
-        if (a > amin_conv && b > amin_conv && fabsf(gg) > tol_conv * sqrtf(a) * sqrtf(b)) major = 1;
-      }
+      constexpr int SH = WB == 8 ? 2 : 3;  // 5 - log2 WB
+      const T sum = jp_transpose_sum<T, WB>(v, lane);
+      if ((lane & ((1 << SH) - 1)) == 0) red[r & 1][warp][lane >> SH] = sum;
     }
-    __syncthreads();  // columns, Q and red are reused by the next round
-  }
-  if (!any) return;  // block-uniform (read after the last barrier)
+    __syncthreads();
+    const int pr = lane & (WB - 1);
+    T g = T(0);
 #pragma unroll
-  for (int c = 0; c < C2; ++c) {
-    if (gcs[c] < 0) continue;
-    const float4* src = cols4 + (int64_t)c * m4;
-    float4* dst = W4 + (int64_t)gcs[c] * m4;
-    for (int i = t; i < m4; i += THREADS) dst[i] = src[i];
-  }
-  __syncthreads();  // the column buffer now takes V's columns
-  for (int i = t; i < n4; i += THREADS) {
-    float4 v[C2];
-#pragma unroll
-    for (int c = 0; c < C2; ++c) v[c] = gcs[c] >= 0 ? V4[(int64_t)gcs[c] * n4 + i] : zero4;
-#pragma unroll
-    for (int c = 0; c < C2; ++c) cols4[(int64_t)c * n4 + i] = v[c];
-  }
-  __syncthreads();
-  // V[:, cols] <- V[:, cols] Q: output columns 4 og .. 4 og + 3, rows 4 r4 .. 4 r4 + 3
-  const int og = t % NG;
-  int ogc[4];  // global columns of this thread's outputs (-1: none)
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int c = 4 * og + j;
-    const int blk = c < WB ? bi : bj;
-    const int gc = blk * WB + (c < WB ? c : c - WB);
-    ogc[j] = (blk < nb && gc < n) ? gc : -1;
-  }
-  float qr[C2][4];
-#pragma unroll
-  for (int d = 0; d < C2; ++d)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) qr[d][j] = Q[d + (4 * og + j) * C2];
-  for (int r4 = t / NG; r4 < n4; r4 += THREADS / NG) {
-    float4 acc[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = zero4;
-#pragma unroll
-    for (int d = 0; d < C2; ++d) {
-      const float4 x = cols4[(int64_t)d * n4 + r4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[j].x = fmaf(x.x, qr[d][j], acc[j].x);
-        acc[j].y = fmaf(x.y, qr[d][j], acc[j].y);
-        acc[j].z = fmaf(x.z, qr[d][j], acc[j].z);
-        acc[j].w = fmaf(x.w, qr[d][j], acc[j].w);
-      }
+    for (int w0 = 0; w0 < MAXW; w0 += 32 / WB) {
+      const int w = w0 + lane / WB;
+      const T part = red[r & 1][w < MAXW ? w : 0][pr];  // rows of absent warps are never written
+      g += w < nw ? part : T(0);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (ogc[j] >= 0) V4[(int64_t)ogc[j] * n4 + r4] = acc[j];
+    for (int o = WB; o < 32; o <<= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    const T a = __shfl_sync(0xffffffffu, norm, pr), b = __shfl_sync(0xffffffffu, norm, partner(pr));
+    T tt, u, s;
+    bool major;
+    const bool rot = jp_angle(a, b, g, tol, tol_conv, amin, amin_conv, tt, u, s, major);
+    const T an = a - tt * g, bn = b + tt * g;
+    const unsigned mask = __ballot_sync(0xffffffffu, rot) & ((1u << WB) - 1u);
+    any_major |= __ballot_sync(0xffffffffu, rot && major);
+    dirty = __any_sync(0xffffffffu, rot && (jp_shrunk(an, a) || jp_shrunk(bn, b)));
+    // lane c takes the new norm of position c from its pair's lane, then the
+    // norms move on with the columns
+    const int src = lane < WB ? lane : (FIRST ? C2 - 1 - lane : lane - WB) & (WB - 1);
+    const T na = __shfl_sync(0xffffffffu, an, src), nb2 = __shfl_sync(0xffffffffu, bn, src);
+    norm = __shfl_sync(0xffffffffu, lane < WB ? na : nb2, next_lane & 31);
+    if (lane < WB) {
+      const Rot o{u, s};
+      rotw[warp][lane] = o;
+      if (warp == 0) {
+        rots[r][lane] = o;
+        if (lane == 0) rmask[r] = mask;
+      }
+    }
+    __syncwarp();
+    any |= mask;
+    if (mask) {
+#pragma unroll
+      for (int g = 0; g < WB; ++g) rotate(g, partner(g), rotw[warp][g]);
+    }
+    advance();
+    __syncwarp();  // rotw is rewritten by the next round
   }
-  if (t == 0 && major) *rotated = 1;
+  if (!any) return;  // block-uniform
+  store(W, m, 0);
+  __syncthreads();  // rots and rmask of the last round (written by warp 0)
+  for (int64_t r0 = 0; r0 < n; r0 += (int64_t)RPT * bd) {
+    load(V, n, r0);
+#pragma unroll 1
+    for (int r = 0; r < NR; ++r) {
+      if (rmask[r]) {
+#pragma unroll
+        for (int g = 0; g < WB; ++g) rotate(g, partner(g), rots[r][g]);
+      }
+      advance();
+    }
+    store(V, n, r0);
+  }
+  if (t == 0 && any_major) *rotated = 1;
 }
 
 // Self-test of the grid barrier's timeout path: every block arrives at a
@@ -706,46 +822,27 @@ size_t jb_smem_bytes(int64_t m) {
   return sizeof(T) * ((size_t)2 * WB * m + (size_t)4 * WB * WB + (size_t)WB * (JB_THREADS / WB / 32) * 3);
 }
 
-template <class T, int WB, int THREADS>
-int jb_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_conv, int max_sweeps, int* flag,
-             int* sweeps) {
-  const size_t smem = jb_smem_bytes<T, WB>(m);
-  // FP32 with 16-byte aligned columns of W and V (and V's columns fitting in
-  // the column buffer): the vectorised step
-  const bool vec = std::is_same<T, float>::value && m % 4 == 0 && n % 4 == 0 && n <= m &&
-                   ((uintptr_t)W % 16) == 0 && ((uintptr_t)V % 16) == 0;
-  static bool attr = false;
-  if (!attr) {
-    ITG_CUDA(h, cudaFuncSetAttribute(k_jacobi_block_step<T, WB, THREADS>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    if constexpr (std::is_same<T, float>::value)
-      ITG_CUDA(h, cudaFuncSetAttribute(k_jacobi_block_step_f4<WB, THREADS>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
-  const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
+// Sweeps of a block-cyclic kernel: launch(sweep, step) enqueues one step whose
+// rotations raise flag[sweep].  Up to `chunk` sweeps are queued between two
+// reads of the flags (the steps of a sweep after a converged one return at
+// once), so that small problems do not wait for the host after every sweep.
+template <class F>
+int jb_sweeps(itg_handle* h, int steps, int max_sweeps, int chunk, int* flag, int* sweeps, F&& launch) {
   int* hp = (int*)h->pinned;
-  for (int sw = 0; sw < max_sweeps; ++sw) {
-    ITG_CUDA(h, cudaMemsetAsync(flag, 0, sizeof(int), h->stream));
-    for (int step = 0; step < nbp - 1; ++step) {
-      if constexpr (std::is_same<T, float>::value) {
-        if (vec) {
-          k_jacobi_block_step_f4<WB, THREADS><<<nbp / 2, THREADS, smem, h->stream>>>(
-              W, m, n, V, tol, conv_tol(tol), amin, amin_conv, step, step == 0, flag);
-          continue;
-        }
-      }
-      k_jacobi_block_step<T, WB, THREADS><<<nbp / 2, THREADS, smem, h->stream>>>(W, m, n, V, tol, conv_tol(tol),
-                                                                                 amin, amin_conv, step, step == 0,
-                                                                                 flag);
-    }
+  ITG_CUDA(h, cudaMemsetAsync(flag, 0, sizeof(int) * max_sweeps, h->stream));
+  for (int sw = 0; sw < max_sweeps;) {
+    const int end = sw + chunk < max_sweeps ? sw + chunk : max_sweeps;
+    for (int q = sw; q < end; ++q)
+      for (int step = 0; step < steps; ++step) launch(q, step, q > sw ? flag + q - 1 : nullptr, flag + q);
     ITG_CHECK_LAUNCH(h);
-    ITG_CUDA(h, cudaMemcpyAsync(hp, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    ITG_CUDA(h, cudaMemcpyAsync(hp, flag + sw, sizeof(int) * (end - sw), cudaMemcpyDeviceToHost, h->stream));
     ITG_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (hp[0] == 0) {
-      *sweeps = sw + 1;
-      return ITG_OK;
-    }
+    for (int q = sw; q < end; ++q)
+      if (hp[q - sw] == 0) {
+        *sweeps = q + 1;
+        return ITG_OK;
+      }
+    sw = end;
   }
   *sweeps = max_sweeps;
   return ITG_ERR_NOTCONVERGED;
@@ -754,9 +851,71 @@ int jb_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_
 template <class T, int WB>
 int jb_run(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_conv, int max_sweeps, int* flag,
            int* sweeps) {
-  if (sizeof(T) == 8 && m <= JB_SMALL_M)
-    return jb_run_t<T, WB, 32 * WB>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
-  return jb_run_t<T, WB, JB_THREADS>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+  const size_t smem = jb_smem_bytes<T, WB>(m);
+  static bool attr = false;
+  if (!attr) {
+    ITG_CUDA(h, cudaFuncSetAttribute(k_jacobi_block_step<T, WB, JB_THREADS>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    attr = true;
+  }
+  const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
+  return jb_sweeps(h, nbp - 1, max_sweeps, 1, flag, sweeps, [&](int, int step, const int*, int* rot) {
+    k_jacobi_block_step<T, WB, JB_THREADS><<<nbp / 2, JB_THREADS, smem, h->stream>>>(
+        W, m, n, V, tol, conv_tol(tol), amin, amin_conv, step, step == 0, rot);
+  });
+}
+
+// Register-resident steps (m <= JR_MAX_M), each launched so that it may start
+// while its predecessor drains (it waits for its results itself).
+template <class T, int WB, int RPT, bool VEC, int MAXT>
+int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_conv, int max_sweeps, int* flag,
+             int* sweeps) {
+  const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
+  const int threads = (int)((m + RPT - 1) / RPT + 31) / 32 * 32;
+  // a queued step costs about 2 us when it has nothing to do, a look at the
+  // flags about 20 us
+  const int chunk = n <= 48 ? 5 : (n <= 160 ? 2 : 1);
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nbp / 2));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = h->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const float tolf = (float)tol, tolc = (float)conv_tol(tol);
+  return jb_sweeps(h, nbp - 1, max_sweeps, chunk, flag, sweeps, [&](int, int step, const int* prev, int* rot) {
+    if (step == 0)
+      cudaLaunchKernelEx(&cfg, k_jacobi_reg_step<T, WB, RPT, VEC, true, MAXT>, W, m, n, V, tolf, tolc, amin, amin_conv,
+                         step, prev, rot);
+    else
+      cudaLaunchKernelEx(&cfg, k_jacobi_reg_step<T, WB, RPT, VEC, false, MAXT>, W, m, n, V, tolf, tolc, amin,
+                         amin_conv, step, prev, rot);
+  });
+}
+
+// FP32: 8-column blocks, at most eight warps (each computes the angles again).
+// FP64: 4-column blocks and, up to
+// 1024 rows, four warps (one for each quarter of the SM, whose FP64 pipes are
+// separate).
+template <class T>
+int jr_run(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_conv, int max_sweeps, int* flag,
+           int* sweeps) {
+  if constexpr (sizeof(T) == 4) {
+    const bool vec = m % 4 == 0 && n % 4 == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)V % 16) == 0;
+    if (m <= 1024) {
+      if (vec) return jr_run_t<T, 8, 4, true, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+      return jr_run_t<T, 8, 4, false, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    }
+    if (vec) return jr_run_t<T, 8, 8, true, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    return jr_run_t<T, 8, 8, false, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+  } else {
+    if (m <= 128) return jr_run_t<T, 4, 1, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    if (m <= 256) return jr_run_t<T, 4, 2, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    if (m <= 512) return jr_run_t<T, 4, 4, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    return jr_run_t<T, 4, 8, false, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+  }
 }
 
 // Blocked Jacobi with the widest block whose column pair fits in 200 KB of
@@ -769,6 +928,8 @@ int jacobi_blocked(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, i
     *sweeps = 0;
     return ITG_OK;
   }
+  if (h->jacobi_mode == 0 && m <= JR_MAX_M)
+    return jr_run<T>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
   // jacobi_mode 3 keeps the blocks at 4 columns (half the shared memory per CTA, more CTAs per SM)
   if (h->jacobi_mode != 3 && jb_smem_bytes<T, 8>(m) <= LIM && n >= 64)
     return jb_run<T, 8>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
