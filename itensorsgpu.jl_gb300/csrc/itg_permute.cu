@@ -4,10 +4,17 @@
 // side first fuses modes that stay adjacent in both layouts, then picks one of
 // two HBM-bound kernels:
 //   * row copy  — A's fastest mode is also B's fastest: both sides stream
-//                 contiguous rows; one div/mod chain per row.
-//   * transpose — different fastest modes: 32x32 tiles staged through shared
-//                 memory so that reads of A and writes of B are both coalesced.
+//                 contiguous rows, several short ones or a segment of a long
+//                 one per CTA.
+//   * transpose — different fastest modes: tiles staged through shared memory
+//                 so that reads of A and writes of B are both coalesced.
+// Both walk items of about 4096 elements by a linear index whose quotient is a
+// multiply, so that no lane idles on a ragged edge, with eight loads of every
+// thread in flight.
 #include "itg_internal.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace {
 
@@ -32,7 +39,9 @@ __device__ __forceinline__ void rest_offsets(const RestDesc& r, int64_t lin, int
   ob = 0;
   for (int i = 0; i < r.n; ++i) {
     int64_t d = r.dims[i];
-    int64_t q = lin / d;
+    int64_t q;
+    if (((lin | d) >> 32) == 0) q = (int64_t)((uint32_t)lin / (uint32_t)d);
+    else q = lin / d;
     int64_t c = lin - q * d;
     lin = q;
     oa += c * r.strA[i];
@@ -40,69 +49,213 @@ __device__ __forceinline__ void rest_offsets(const RestDesc& r, int64_t lin, int
   }
 }
 
-// One CTA handles `rows_per_block` rows of length d0 (stride 1 in A and B).
-__global__ void k_perm_rows(const double* __restrict__ A, double* __restrict__ B,
-                            const double* __restrict__ Bin, double alpha, double beta,
-                            int64_t d0, int64_t nrows, RestDesc rest) {
-  for (int64_t row = blockIdx.x; row < nrows; row += gridDim.x) {
-    int64_t oa, ob;
-    rest_offsets(rest, row, oa, ob);
-    const double* a = A + oa;
-    double* b = B + ob;
-    const double* bi = Bin ? Bin + ob : nullptr;
-    for (int64_t i = threadIdx.x; i < d0; i += blockDim.x) {
-      double v = alpha * a[i];
-      if (bi) v = fma(beta, bi[i], v);
-      b[i] = v;
+// x / d for x, d <= 2^16: the upper half of x * ceil(2^32 / d)
+struct FastDiv {
+  uint32_t d, m;
+  __device__ __forceinline__ uint32_t div(uint32_t x) const { return d == 1 ? x : __umulhi(x, m); }
+};
+inline FastDiv fast_div(uint32_t d) {
+  return {d, d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d)};
+}
+
+constexpr int PERM_THREADS = 256;
+constexpr int PERM_ITEM = 4096;  // elements per item
+constexpr int PERM_FLIGHT = 8;   // loads of a thread in flight
+constexpr int PERM_ROWS = 256;   // rows per item at most
+
+// B = alpha A + beta Bin element by element.  The FP64 pipe (two operations a
+// clock and SM, 0.6 of HBM's rate in 16-byte element copies) is spared where
+// the scalars allow: a copy with alpha = +-1 takes no FP64 operation, a sum
+// with beta = 1 and alpha = +-1 one, each with the bits of the general form.
+enum PermOp { PERM_COPY, PERM_SCALE, PERM_ADD, PERM_AXPBY };
+struct PermScalars {
+  double alpha, beta;
+  long long flip;  // sign bit of alpha (PERM_COPY, PERM_ADD)
+};
+template <int OP>
+__device__ __forceinline__ double perm_op(const PermScalars& s, double a, double b) {
+  if (OP == PERM_COPY || OP == PERM_ADD) {
+    const double x = __longlong_as_double(__double_as_longlong(a) ^ s.flip);
+    return OP == PERM_COPY ? x : x + b;
+  }
+  return OP == PERM_SCALE ? s.alpha * a : fma(s.beta, b, s.alpha * a);
+}
+constexpr bool perm_reads_b(int op) { return op == PERM_ADD || op == PERM_AXPBY; }
+
+// Item: `rows` rows of length d0 (stride 1 in A and B), or (nseg > 1) one
+// segment of seg elements of a row.  The rows' offsets are decomposed once per
+// item, one row a thread.  Bin may be B: every element is read before it is
+// written, by the same thread.  Measured: (d0, d2, d1, d3) of 129 x 250 x 64 x 63
+// 767 -> 322 us (95% of measured HBM); a sum of 2^26 elements in one order, which
+// is a single row, 110 ms (one CTA) -> 0.27 ms.
+template <int OP>
+__global__ void __launch_bounds__(PERM_THREADS, 4)
+k_perm_rows(const double* __restrict__ A, double* B, const double* Bin, PermScalars sc, int64_t d0, int64_t nrows,
+            int rows, int64_t seg, int64_t nseg, FastDiv by_d0, int64_t items, RestDesc rest) {
+  __shared__ int64_t oa[PERM_ROWS], ob[PERM_ROWS];
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const int64_t row0 = nseg > 1 ? it / nseg : it * rows;
+    const int64_t i0 = nseg > 1 ? (it - row0 * nseg) * seg : 0;
+    const int nr = (int)(nrows - row0 < rows ? nrows - row0 : rows);
+    __syncthreads();  // the offsets of the item before
+    if ((int)threadIdx.x < nr) {
+      int64_t x, y;
+      rest_offsets(rest, row0 + threadIdx.x, x, y);
+      oa[threadIdx.x] = x + i0;
+      ob[threadIdx.x] = y + i0;
+    }
+    __syncthreads();
+    const int len = (int)(nseg > 1 ? (d0 - i0 < seg ? d0 - i0 : seg) : d0);
+    const int total = nr * len;
+    for (int e0 = threadIdx.x; e0 < total; e0 += PERM_THREADS * PERM_FLIGHT) {
+      double v[PERM_FLIGHT], w[PERM_FLIGHT];
+      int64_t o[PERM_FLIGHT];
+#pragma unroll
+      for (int u = 0; u < PERM_FLIGHT; ++u) {
+        const int e = e0 + u * PERM_THREADS;
+        o[u] = -1;
+        if (e < total) {
+          const int r = nseg > 1 ? 0 : (int)by_d0.div(e);
+          const int i = e - r * len;
+          v[u] = A[oa[r] + i];
+          o[u] = ob[r] + i;
+          if (perm_reads_b(OP)) w[u] = Bin[o[u]];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < PERM_FLIGHT; ++u)
+        if (o[u] >= 0) B[o[u]] = perm_op<OP>(sc, v[u], perm_reads_b(OP) ? w[u] : 0.0);
     }
   }
 }
 
 // Tiled transpose between A's mode 0 (size n0, stride 1 in A, stride s0B in B)
-// and A's mode q (size nq, stride sqA in A, stride 1 in B).  blockIdx.y walks
-// the batches (the other modes), so their offsets are decomposed once per
-// batch, and blockIdx.x the 32 x 32 tiles of one batch; the index arithmetic
-// inside a batch is 32-bit.
-#define TP 32
-__global__ void __launch_bounds__(256)
-k_perm_transpose(const double* __restrict__ A, double* __restrict__ B, const double* __restrict__ Bin,
-                 double alpha, double beta, int64_t n0, int64_t nq, int64_t sqA, int64_t s0B, int64_t nbatch,
+// and A's mode q (size nq, stride sqA in A, stride 1 in B): e0 x eq tiles,
+// equal within a mode, so a length just above a multiple leaves no sliver (129
+// = 3 x 43); up to 64 wide, so that a tile row is 512 contiguous bytes on both
+// sides.  Lanes run along the contiguous mode in two halves, 2^l0 (2^lq) of
+// them to a row where the mode is short.  Four CTAs to an SM (at 78 registers,
+// three, sums ran at 86 instead of 94% of HBM).  Measured against 32 x 32
+// tiles with the general scalars: 129 x 250 x 64 x 63 reversed 495 -> 410 us,
+// 128 x 256 x 64 x 64 reversed 392 -> 340 us (94% of measured HBM), its sum 625
+// -> 530 us.
+template <int OP>
+__global__ void __launch_bounds__(PERM_THREADS, 4)
+k_perm_transpose(const double* __restrict__ A, double* B, const double* Bin, PermScalars sc, int64_t n0, int64_t nq,
+                 int64_t sqA, int64_t s0B, int e0, int eq, int l0, int lq, int64_t t0, int64_t tq, int64_t items,
                  RestDesc rest) {
-  __shared__ double tile[TP][TP + 1];
-  const int t0 = (int)((n0 + TP - 1) / TP), tq = (int)((nq + TP - 1) / TP);
-  const int tiles = t0 * tq;
-  for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
+  extern __shared__ double tile[];  // [eq][pitch], the pitch odd: no bank conflicts along either side
+  const int pitch = e0 | 1;
+  const int rx = threadIdx.x & ((1 << l0) - 1), ry = threadIdx.x >> l0, rstep = PERM_THREADS >> l0;
+  const int wx = threadIdx.x & ((1 << lq) - 1), wy = threadIdx.x >> lq, wstep = PERM_THREADS >> lq;
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const int64_t tiles = t0 * tq;
+    int64_t b, r, iq;
+    if ((items >> 32) == 0) {
+      b = (uint32_t)it / (uint32_t)tiles;
+      r = it - b * tiles;
+      iq = (uint32_t)r / (uint32_t)t0;
+    } else {
+      b = it / tiles;
+      r = it - b * tiles;
+      iq = r / t0;
+    }
+    const int64_t i0 = (r - iq * t0) * e0, k0 = iq * eq;
     int64_t oa, ob;
     rest_offsets(rest, b, oa, ob);
-    for (int r = blockIdx.x; r < tiles; r += gridDim.x) {
-      const int iq = r / t0, i0 = r - iq * t0;
-      const int64_t base0 = (int64_t)i0 * TP, baseq = (int64_t)iq * TP;
-      // read: threadIdx.x runs along mode 0 (contiguous in A); all loads first
-      double v[TP / 8];
+    const int w0 = (int)(n0 - i0 < e0 ? n0 - i0 : e0), wq = (int)(nq - k0 < eq ? nq - k0 : eq);
+    // read along mode 0 (contiguous in A): rows ry, ry + rstep, ..., lanes rx and rx + 2^l0, ...
+    {
+      const double* a = A + oa + i0 + k0 * sqA;
+      for (int x = rx; x < w0; x += 2 << l0) {
+        const bool two = x + (1 << l0) < w0;
+        for (int k = ry; k < wq; k += 4 * rstep) {
+          double v[4][2];
+          const double* p = a + x + k * sqA;
 #pragma unroll
-      for (int j = 0; j < TP / 8; ++j) {
-        const int y = threadIdx.y + 8 * j;
-        const int64_t i = base0 + threadIdx.x, k = baseq + y;
-        v[j] = (i < n0 && k < nq) ? A[oa + i + k * sqA] : 0.0;
-      }
+          for (int j = 0; j < 4; ++j)
+            if (k + j * rstep < wq) {
+              v[j][0] = p[j * rstep * sqA];
+              if (two) v[j][1] = p[j * rstep * sqA + (1 << l0)];
+            }
+          double* q = tile + k * pitch + x;
 #pragma unroll
-      for (int j = 0; j < TP / 8; ++j) tile[threadIdx.y + 8 * j][threadIdx.x] = v[j];
-      __syncthreads();
-      // write: threadIdx.x runs along mode q (contiguous in B)
-#pragma unroll
-      for (int j = 0; j < TP / 8; ++j) {
-        const int y = threadIdx.y + 8 * j;
-        const int64_t k = baseq + threadIdx.x, i = base0 + y;
-        if (i < n0 && k < nq) {
-          const int64_t o = ob + k + i * s0B;
-          double w = alpha * tile[threadIdx.x][y];
-          if (Bin) w = fma(beta, Bin[o], w);
-          B[o] = w;
+          for (int j = 0; j < 4; ++j)
+            if (k + j * rstep < wq) {
+              q[j * rstep * pitch] = v[j][0];
+              if (two) q[j * rstep * pitch + (1 << l0)] = v[j][1];
+            }
         }
       }
-      __syncthreads();
     }
+    __syncthreads();
+    // write along mode q (contiguous in B)
+    {
+      const int64_t o0 = ob + k0 + i0 * s0B;
+      for (int x = wx; x < wq; x += 2 << lq) {
+        const bool two = x + (1 << lq) < wq;
+        for (int i = wy; i < w0; i += 4 * wstep) {
+          double v[4][2], w[4][2];
+          const double* q = tile + x * pitch + i;
+          double* p = B + o0 + x + i * s0B;
+          const double* pb = Bin + o0 + x + i * s0B;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i + j * wstep < w0) {
+              if (perm_reads_b(OP)) {
+                w[j][0] = pb[j * wstep * s0B];
+                if (two) w[j][1] = pb[j * wstep * s0B + (1 << lq)];
+              }
+              v[j][0] = q[j * wstep];
+              if (two) v[j][1] = q[j * wstep + (pitch << lq)];
+            }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i + j * wstep < w0) {
+              p[j * wstep * s0B] = perm_op<OP>(sc, v[j][0], perm_reads_b(OP) ? w[j][0] : 0.0);
+              if (two)
+                p[j * wstep * s0B + (1 << lq)] = perm_op<OP>(sc, v[j][1], perm_reads_b(OP) ? w[j][1] : 0.0);
+            }
+        }
+      }
+    }
+    __syncthreads();
   }
+}
+
+// Tile of the transpose: about 64 x 64, the other side longer where one mode
+// is short, and equal tiles within each mode; padded rows fit in 35 KB, so six
+// CTAs share an SM.  l0, lq: log2 of the lanes along each mode.
+void perm_tile(int64_t n0, int64_t nq, int& e0, int& eq, int& l0, int& lq) {
+  auto even = [](int64_t n, int64_t cap) { return (int)((n + (n + cap - 1) / cap - 1) / ((n + cap - 1) / cap)); };
+  int64_t c0 = 64, cq = 64;
+  if (n0 < 64) cq = 4352 / (n0 | 1);
+  else if (nq < 64) c0 = 4352 / nq - 1;
+  e0 = even(n0, c0);
+  eq = even(nq, cq);
+  auto lanes = [](int e) {
+    int l = 0;
+    while (l < 5 && (1 << l) < e) ++l;
+    return l;
+  };
+  l0 = lanes(e0);
+  lq = lanes(eq);
+}
+
+template <int OP>
+void perm_launch_rows(int blocks, cudaStream_t st, const double* A, double* B, const double* Bin, PermScalars sc,
+                      int64_t d0, int64_t nrows, int rows, int64_t seg, int64_t nseg, int64_t items,
+                      const RestDesc& rest) {
+  k_perm_rows<OP><<<blocks, PERM_THREADS, 0, st>>>(A, B, Bin, sc, d0, nrows, rows, seg, nseg,
+                                                   fast_div(nseg > 1 ? 1 : (uint32_t)d0), items, rest);
+}
+
+template <int OP>
+void perm_launch_transpose(int blocks, size_t smem, cudaStream_t st, const double* A, double* B, const double* Bin,
+                           PermScalars sc, int64_t n0, int64_t nq, int64_t sqA, int64_t s0B, int e0, int eq, int l0,
+                           int lq, int64_t t0, int64_t tq, int64_t items, const RestDesc& rest) {
+  k_perm_transpose<OP><<<blocks, PERM_THREADS, smem, st>>>(A, B, Bin, sc, n0, nq, sqA, s0B, e0, eq, l0, lq, t0, tq,
+                                                           items, rest);
 }
 
 // Resolve modesB as a permutation of modesA.  perm[j] = A-position of B's mode j.
@@ -164,6 +317,9 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
     d.rank++;
   }
   const double* bin = (beta == 0.0) ? nullptr : Bin;
+  const bool unit = alpha == 1.0 || alpha == -1.0;
+  const int op = !bin ? (unit ? PERM_COPY : PERM_SCALE) : (unit && beta == 1.0 ? PERM_ADD : PERM_AXPBY);
+  const PermScalars sc{alpha, beta, alpha < 0.0 ? (long long)(1ull << 63) : 0ll};
   if (d.rank == 0) {  // single element
     d.rank = 1;
     d.dims[0] = 1;
@@ -183,10 +339,20 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
       rest.strB[rest.n] = d.strB[i];
       rest.n++;
     }
-    int64_t nrows = total / d.dims[0];
-    int threads = d.dims[0] >= 256 ? 256 : (d.dims[0] >= 64 ? 64 : 32);
-    int blocks = (int)std::min<int64_t>(nrows, (int64_t)h->num_sms * 64);
-    k_perm_rows<<<blocks, threads, 0, h->stream>>>(A, B, bin, alpha, beta, d.dims[0], nrows, rest);
+    const int64_t d0 = d.dims[0], nrows = total / d0;
+    // short rows share an item, long ones are cut into segments
+    const int64_t seg = PERM_ITEM, nseg = d0 > 2 * PERM_ITEM ? (d0 + seg - 1) / seg : 1;
+    int64_t rows = nseg > 1 ? 1 : std::min<int64_t>(std::max<int64_t>(1, PERM_ITEM / d0), PERM_ROWS);
+    const int64_t items = nseg > 1 ? nrows * nseg : (nrows + rows - 1) / rows;
+    const int blocks = (int)std::min<int64_t>(items, (int64_t)h->num_sms * 64);
+    auto run = [&](auto tag) {
+      perm_launch_rows<decltype(tag)::value>(blocks, h->stream, A, B, bin, sc, d0, nrows, (int)rows, seg, nseg, items,
+                                             rest);
+    };
+    if (op == PERM_COPY) run(std::integral_constant<int, PERM_COPY>());
+    else if (op == PERM_SCALE) run(std::integral_constant<int, PERM_SCALE>());
+    else if (op == PERM_ADD) run(std::integral_constant<int, PERM_ADD>());
+    else run(std::integral_constant<int, PERM_AXPBY>());
   } else {
     rest.n = 0;
     for (int i = 1; i < d.rank; ++i) {
@@ -198,14 +364,22 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
     }
     int64_t n0 = d.dims[0], nq = d.dims[q];
     int64_t nbatch = total / (n0 * nq);
-    const int64_t tiles = ((n0 + TP - 1) / TP) * ((nq + TP - 1) / TP);
-    if (tiles > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "permute: transpose too large");
-    const int64_t want = (int64_t)h->num_sms * 32;  // resident CTAs
-    const int64_t gx = std::min<int64_t>(tiles, want);
-    const int64_t gy = std::min<int64_t>(std::min<int64_t>(nbatch, std::max<int64_t>(1, want / gx)), 65535);
-    dim3 thr(TP, 8);
-    k_perm_transpose<<<dim3((unsigned)gx, (unsigned)gy), thr, 0, h->stream>>>(A, B, bin, alpha, beta, n0, nq,
-                                                                            d.strA[q], d.strB[0], nbatch, rest);
+    int e0, eq, l0, lq;
+    perm_tile(n0, nq, e0, eq, l0, lq);
+    const int64_t t0 = (n0 + e0 - 1) / e0, tq = (nq + eq - 1) / eq;
+    if (t0 * tq > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "permute: transpose too large");
+    const int64_t items = t0 * tq * nbatch;
+    const int blocks = (int)std::min<int64_t>(items, (int64_t)h->num_sms * 48);
+    const size_t smem = sizeof(double) * (size_t)eq * (e0 | 1);
+    const int64_t sqA = d.strA[q], s0B = d.strB[0];
+    auto run = [&](auto tag) {
+      perm_launch_transpose<decltype(tag)::value>(blocks, smem, h->stream, A, B, bin, sc, n0, nq, sqA, s0B, e0, eq, l0,
+                                                  lq, t0, tq, items, rest);
+    };
+    if (op == PERM_COPY) run(std::integral_constant<int, PERM_COPY>());
+    else if (op == PERM_SCALE) run(std::integral_constant<int, PERM_SCALE>());
+    else if (op == PERM_ADD) run(std::integral_constant<int, PERM_ADD>());
+    else run(std::integral_constant<int, PERM_AXPBY>());
   }
   ITG_CHECK_LAUNCH(h);
   return ITG_OK;
