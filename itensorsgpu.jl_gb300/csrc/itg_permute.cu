@@ -136,7 +136,7 @@ k_perm_rows(const double* __restrict__ A, double* B, const double* Bin, PermScal
 // sides.  Lanes run along the contiguous mode in two halves, 2^l0 (2^lq) of
 // them to a row where the mode is short.  Four CTAs to an SM (at 78 registers,
 // three, sums ran at 86 instead of 94% of HBM).  Measured against 32 x 32
-// tiles with the general scalars: 129 x 250 x 64 x 63 reversed 495 -> 410 us,
+// tiles with the general scalars: 129 x 250 x 64 x 63 reversed 495 -> 365 us,
 // 128 x 256 x 64 x 64 reversed 392 -> 340 us (94% of measured HBM), its sum 625
 // -> 530 us.
 template <int OP>
@@ -362,6 +362,15 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
       rest.strB[rest.n] = d.strB[i];
       rest.n++;
     }
+    // batches next to each other in B first: a tile row of A is 512 bytes of its
+    // own whatever the order, while B's rows then continue one another
+    // (129 x 250 x 64 x 63 reversed 412 -> 365 us, no order slower)
+    for (int i = 1; i < rest.n; ++i)
+      for (int j = i; j > 0 && rest.strB[j] < rest.strB[j - 1]; --j) {
+        std::swap(rest.dims[j], rest.dims[j - 1]);
+        std::swap(rest.strA[j], rest.strA[j - 1]);
+        std::swap(rest.strB[j], rest.strB[j - 1]);
+      }
     int64_t n0 = d.dims[0], nq = d.dims[q];
     int64_t nbatch = total / (n0 * nq);
     int e0, eq, l0, lq;
