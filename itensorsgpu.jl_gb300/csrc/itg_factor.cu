@@ -421,56 +421,145 @@ namespace {
 // (never written during the step) and forms the same reflector
 //   beta = -sign(alpha) |x|, tau = (beta - alpha) / beta, v = x / (alpha - beta), v_j = 1;
 // CTA 0 stores v, tau and beta; CTA c > 0 applies I - tau v v^T to column j + c.
-template <int T>
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int w = 0; w < T / 32; ++w) s += sh[w];
-  __syncthreads();
-  return s;
+//
+// Bound by a chain of FP64 instructions, 64 clocks each on a quarter of the
+// SM: one pass forms |x|^2 and x . a_c together (v . a_c is the latter times
+// 1 / (alpha - beta)), one reduction sums both, the square root and the
+// reciprocals take 20 instructions from FP32 seeds (hypot, sqrt and two
+// divisions took over 100), and the block has one warp for each quarter of the
+// SM.  A step starts while its predecessor drains.  Together with the panel's
+// shorter tail (itg_qr_blocked.cu) the 2048 x 2048 mixed split went from 134 to
+// 118 ms, the 378 x 366 one from 16.2 to 10.7 ms.
+constexpr int HOUSE_THREADS = 128;
+
+// beta, tau and 1 / (alpha - beta) of the reflector from alpha and s2 > 0, the
+// squared norm below alpha.  Scaled by powers of two so that alpha^2 + s2 is
+// in [1, 8); square root and reciprocals by Newton's iteration from FP32.
+__device__ __forceinline__ void house_scalars(double alpha, double s2, double& beta, double& tau, double& scale) {
+  const int ea = ((__double2hiint(alpha) >> 20) & 0x7FF) - 1023, es = (((__double2hiint(s2) >> 20) & 0x7FF) - 1023) >> 1;
+  int e = ea > es ? ea : es;
+  e = e < -1000 ? -1000 : (e > 1000 ? 1000 : e);
+  const double p = __hiloint2double((1023 - e) << 20, 0), ip = __hiloint2double((1023 + e) << 20, 0);
+  const double as = fabs(alpha) * p;
+  const double t = fma(as, as, s2 * p * p);
+  double y = (double)rsqrtf((float)t);
+  const double ht = -0.5 * t;
+  y *= fma(ht, y * y, 1.5);
+  y *= fma(ht, y * y, 1.5);
+  double n = t * y;
+  n = fma(fma(-n, n, t), 0.5 * y, n);
+  tau = fma(as, y, 1.0);
+  const double d = as + n;
+  double r = (double)__fdividef(1.f, (float)d);
+  r = fma(r, fma(-d, r, 1.0), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  beta = -copysign(n * ip, alpha);
+  scale = copysign(r * p, alpha);
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(HOUSE_THREADS)
 k_house_step(double* __restrict__ A, int64_t m, int j, double* __restrict__ Vh, double* __restrict__ tau,
              double* __restrict__ rdiag) {
-  __shared__ double sh[8];
+  __shared__ double red[HOUSE_THREADS / 32][2];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const double* x = A + (int64_t)j * m;
-  const double alpha = x[j];
-  double s2 = 0.0;
-  for (int64_t i = j + 1 + threadIdx.x; i < m; i += 256) s2 = fma(x[i], x[i], s2);
-  s2 = block_sum<256>(s2, sh);
-  double tj = 0.0, beta = alpha, scale = 0.0;
-  if (s2 > 0.0) {
-    beta = -copysign(hypot(alpha, sqrt(s2)), alpha);
-    tj = (beta - alpha) / beta;
-    scale = 1.0 / (alpha - beta);
+  double* col = A + (int64_t)(j + blockIdx.x) * m;
+  const int t = threadIdx.x, lane = t & 31;
+  const double cj = col[j];
+  double alpha = x[j], ps = 1.0, s2, w;
+  // s2 = |x below alpha|^2 and w = x . col, x scaled by ps
+  auto sums = [&](bool scaled) {
+    double a = 0.0, c = 0.0;
+    if (!scaled) {
+#pragma unroll 8
+      for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) {
+        const double xi = x[i];
+        a = fma(xi, xi, a);
+        if (blockIdx.x) c = fma(xi, col[i], c);
+      }
+    } else {
+      for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) {
+        const double xi = x[i] * ps;
+        a = fma(xi, xi, a);
+        c = fma(xi, col[i], c);
+      }
+    }
+    // lanes below 16 sum the one, the others the other
+    const bool up = lane & 16;
+    double v = (up ? c : a) + __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((lane & 15) == 0) red[t >> 5][lane >> 4] = v;
+    __syncthreads();
+    s2 = (red[0][0] + red[1][0]) + (red[2][0] + red[3][0]);
+    w = (red[0][1] + red[1][1]) + (red[2][1] + red[3][1]);
+  };
+  sums(false);
+  // squares near the ends of the range (or lost below it): once more with x
+  // scaled by a power of two to at most 1
+  const bool scaled = !(s2 >= 0x1p-960 && s2 <= 0x1p960);
+  if (scaled) {
+    int mx = 0;  // largest exponent field
+    for (int64_t i = j + t; i < m; i += HOUSE_THREADS) {
+      const int e = (__double2hiint(x[i]) >> 20) & 0x7FF;
+      mx = e > mx ? e : mx;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const int y = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = y > mx ? y : mx;
+    }
+    __syncthreads();
+    if (lane == 0) red[t >> 5][0] = (double)mx;
+    __syncthreads();
+    mx = (int)fmax(fmax(red[0][0], red[1][0]), fmax(red[2][0], red[3][0]));
+    __syncthreads();
+    const int k = mx - 1022 < -1000 ? -1000 : (mx - 1022 > 1000 ? 1000 : mx - 1022);
+    ps = __hiloint2double((1023 - k) << 20, 0);
+    alpha *= ps;
+    sums(true);
   }
+  double tj = 0.0, beta = alpha, scale = 0.0;
+  if (s2 > 0.0) house_scalars(alpha, s2, beta, tj, scale);
   if (blockIdx.x == 0) {
     double* v = Vh + (int64_t)j * m;
-    for (int64_t i = threadIdx.x; i < m; i += 256) v[i] = i < j ? 0.0 : (i == j ? 1.0 : x[i] * scale);
-    if (threadIdx.x == 0) {
+    for (int64_t i = t; i < m; i += HOUSE_THREADS)
+      v[i] = i < j ? 0.0 : (i == j ? 1.0 : (scaled ? x[i] * ps : x[i]) * scale);
+    if (t == 0) {
       tau[j] = tj;
-      rdiag[j] = beta;
+      rdiag[j] = scaled ? beta / ps : beta;
     }
     return;
   }
   if (tj == 0.0) return;
-  double* col = A + (int64_t)(j + blockIdx.x) * m;
-  double w = 0.0;
-  for (int64_t i = j + 1 + threadIdx.x; i < m; i += 256) w = fma(x[i] * scale, col[i], w);
-  w = block_sum<256>(w, sh) + col[j];
-  const double f = tj * w;
-  for (int64_t i = j + threadIdx.x; i < m; i += 256) col[i] -= f * (i == j ? 1.0 : x[i] * scale);
+  const double f = tj * fma(w, scale, cj), g = -f * scale;
+  if (!scaled) {
+#pragma unroll 8
+    for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) col[i] = fma(g, x[i], col[i]);
+  } else {
+    for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) col[i] = fma(g, x[i] * ps, col[i]);
+  }
+  if (t == 0) col[j] = cj - f;
 }
 
 }  // namespace
 
 namespace itg {
-void house_step_launch(itg_handle* h, double* A, int64_t m, int j, int ncta, double* Vh, double* tau,
-                       double* rdiag) {
-  k_house_step<<<(unsigned)ncta, 256, 0, h->stream>>>(A, m, j, Vh, tau, rdiag);
+// Steps j0 .. j0 + count - 1 on columns up to jend, on the handle's stream.
+int house_panel(itg_handle* h, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh, double* tau,
+                double* rdiag) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  for (int64_t j = j0; j < j0 + count; ++j) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(jend - j));
+    cfg.blockDim = dim3(HOUSE_THREADS);
+    cfg.stream = h->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = j > j0 ? 1 : 0;  // the first step waits for everything before it
+    ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step, A, m, (int)j, Vh, tau, rdiag));
+  }
+  return ITG_OK;
 }
 }  // namespace itg
 
@@ -704,9 +793,6 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
   double* J = W;
   double *Vh = nullptr, *tau = nullptr, *Vh2 = nullptr, *tau2 = nullptr;
   double *Tq = nullptr, *Tq2 = nullptr, *Qws = nullptr;
-  // products of the QR's trailing updates: FP64 (their depth is one 32-column
-  // panel, too shallow for the split path's operand preparation to pay off)
-  const int qr_prec = ITG_PREC_FP64;
   if (pre) {
     Vh = (double*)(base + oVh);
     tau = (double*)(base + oTau);
@@ -715,7 +801,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     Tq = (double*)(base + oTq);
     Qws = (double*)(base + oQws);
     ProfScope prof(h, ITG_KERNEL_SVD_QR);
-    ITG_TRY(itg::qr_blocked(h, W, mm, nn, nn, Vh, tau, rd, Tq, Qws, qr_prec));
+    ITG_TRY(itg::qr_blocked(h, W, mm, nn, nn, Vh, tau, rd, Tq, Qws));
     k_build_rt<<<itg_blocks_for(nn * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, mm, (int)nn, rd, J);
     ITG_CHECK_LAUNCH(h);
     if (two) {
@@ -724,7 +810,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
       double* rd2 = (double*)(base + oRd2);
       double* J2 = (double*)(base + oB2);
       Tq2 = (double*)(base + oTq2);
-      ITG_TRY(itg::qr_blocked(h, J, nn, nn, nn, Vh2, tau2, rd2, Tq2, Qws, qr_prec));
+      ITG_TRY(itg::qr_blocked(h, J, nn, nn, nn, Vh2, tau2, rd2, Tq2, Qws));
       k_build_rt<<<itg_blocks_for(nn * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(J, nn, (int)nn, rd2, J2);
       ITG_CHECK_LAUNCH(h);
       J = J2;
@@ -975,7 +1061,7 @@ extern "C" int itg_qr(itg_handle* h, int64_t m, int64_t n, const double* A, int6
   double* ws = (double*)(base + oWs);
   k_copy_matrix<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, m, n, W, 0.0);
   ITG_CHECK_LAUNCH(h);
-  ITG_TRY(itg::qr_blocked(h, W, m, n, r, Vh, tau, rd, Tq, ws, ITG_PREC_FP64));
+  ITG_TRY(itg::qr_blocked(h, W, m, n, r, Vh, tau, rd, Tq, ws));
   k_extract_r<<<itg_blocks_for(r * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m, r, n, rd, R);
   k_eye_cols<<<itg_blocks_for(m * r, 256, h->num_sms * 16), 256, 0, h->stream>>>(Q, m, r);
   ITG_CHECK_LAUNCH(h);

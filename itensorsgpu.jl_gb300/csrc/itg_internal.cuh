@@ -18,7 +18,6 @@
 #define ITG_PINNED_DOUBLES 4096  // host staging for small results (Davidson subspace <= 32x32)
 #define ITG_GEMV_MAX_PART 65536  // partial sums of itg_gemv_t
 #define QR_NB 32                 // panel width of the blocked Householder QR
-#define QR_NB_MAX 64
 
 // A lowered contraction C[m,n] = sum_k A[m,k] B[k,n] with every operand
 // addressed through offset tables (see itg_contract.cu).
@@ -112,15 +111,11 @@ struct itg_handle {
   int64_t tune_runs = 0;
   void* cplx_buf = nullptr;   // realified operands / temporaries of complex contractions
   size_t cplx_buf_bytes = 0;
-  int64_t* tab_buf = nullptr; // offset tables of the blocked QR's submatrix products
-  int64_t tab_buf_elems = 0;
   // Look-ahead of the blocked QR: the trailing updates run on qr_stream while
-  // the next panel is factored on `stream` (own offset tables, two events).
+  // the next panel is factored on `stream` (two events).
   cudaStream_t qr_stream = nullptr;
   cudaEvent_t qr_ev_ready = nullptr;  // panel's reflectors and T are final (on `stream`)
   cudaEvent_t qr_ev_done = nullptr;   // trailing update finished (on qr_stream)
-  int64_t* tab_buf2 = nullptr;
-  int64_t tab_buf2_elems = 0;
   // Split operand slice reuse: [0] the A operand, [1] the B operand of the
   // next split contraction when slice_keep[i] is set (see SliceCache).
   SliceCache slice_cache[2];
@@ -150,10 +145,10 @@ template <class T>
 int jacobi_persistent(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, int max_sweeps, int* aux,
                       int* sweeps, T amin_conv = T(0));
 // Blocked Householder QR (itg_qr_blocked.cu): panels of QR_NB columns, WY
-// trailing updates through the contraction engine at `precision`; nref
-// reflectors (nref <= min(m, n)) applied to all n columns.
+// trailing updates in FP64; nref reflectors (nref <= min(m, n)) applied to all
+// n columns.
 int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, double* Vh, double* tau, double* rd,
-               double* Tbuf, double* ws, int precision);
+               double* Tbuf, double* ws);
 int q_apply_blocked(itg_handle* h, double* Y, int64_t m, int64_t n, int64_t ncols, const double* Vh,
                     const double* Tbuf, double* ws);
 size_t qr_blocked_ws_doubles(int64_t n);
