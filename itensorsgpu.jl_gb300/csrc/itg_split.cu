@@ -378,34 +378,23 @@ struct Part {
   }
 };
 
-// v * 2^exp2 rounded to nearest even, built with integer instructions.
+// v * 2^exp2 rounded to nearest even (|v| < 2^63), built with about 25 integer
+// instructions: |v| normalised to 64 bits, the rounding bit added to the upper
+// 53, and the exponent field added below them so that a carry moves into it.
 __device__ __forceinline__ double i64_to_double_scaled(long long v, int exp2) {
-  if (v == 0) return 0.0;
-  const unsigned long long sgn = v < 0 ? (1ull << 63) : 0ull;
-  unsigned long long u = v < 0 ? (unsigned long long)(-v) : (unsigned long long)v;
-  const int top = 63 - __clzll((long long)u);
-  unsigned long long mant;
-  int e2 = top + exp2;
-  if (top <= 52) {
-    mant = u << (52 - top);
-  } else {
-    const int sh = top - 52;
-    const unsigned long long rem = u & ((1ull << sh) - 1);
-    const unsigned long long half = 1ull << (sh - 1);
-    mant = u >> sh;
-    if (rem > half || (rem == half && (mant & 1ull))) {
-      mant++;
-      if (mant >> 53) {
-        mant >>= 1;
-        e2++;
-      }
-    }
-  }
-  const int be = e2 + 1023;
-  if (be <= 0) return __longlong_as_double((long long)sgn);
-  if (be >= 2047) return __longlong_as_double((long long)(sgn | 0x7FF0000000000000ull));
-  return __longlong_as_double(
-      (long long)(sgn | ((unsigned long long)be << 52) | (mant & ((1ull << 52) - 1))));
+  const long long sg = v >> 63;
+  unsigned long long u = (unsigned long long)((v ^ sg) - sg);
+  if (u == 0) return 0.0;
+  const int lz = __clzll((long long)u);
+  u <<= lz;
+  const unsigned long long m = u >> 11;
+  const uint32_t low = (uint32_t)u & 0x7FFu;
+  const unsigned long long mant = m + (uint32_t)(low > 0x400u || (low == 0x400u && ((uint32_t)m & 1u)));
+  const int be = 63 - lz + exp2 + 1023, bc = be + (int)(mant >> 53);
+  unsigned long long bits = ((unsigned long long)(long long)(be - 1) << 52) + mant;
+  if (bc <= 0) bits = 0;
+  if (bc >= 2047) bits = 0x7FF0000000000000ull;
+  return __longlong_as_double((long long)(bits | ((unsigned long long)sg & 0x8000000000000000ull)));
 }
 
 // Tile variants: BN = 256 keeps the int64 accumulators in global memory
@@ -874,41 +863,49 @@ __global__ void k_row_expfield_mmajor(const double* __restrict__ X, const int64_
   if (e) atomicMax(&efield[r], e);
 }
 
-// Balanced base-2^8 digits of |X[r,k]| * 2^-e_r rounded to 48 fractional bits
-// (S = 6 digits), and the sign of X[r,k]; the digits of X are the digits of
-// |X| negated.  Y = |X| 2^(48 - e_r) (at most 2^48) splits into 24 + 24 bits
-// whose bytes are the unbalanced digits u_p; one carry pass from the least
-// significant digit makes them balanced (v = u_p + carry; v >= 128 -> digit
-// v - 256, carry 1), so |d_0| <= 256 and |d_p| <= 128 for p >= 1, all exact
-// in bf16.
-__device__ __forceinline__ void make_digits_abs(double x, int efield_r, int (&d)[S_SLICES], bool& neg) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-  neg = (bits >> 63) != 0;
-  const int E = (int)((bits >> 52) & 0x7FF);
-  unsigned long long M = bits & ((1ull << 52) - 1);
-  if (E) M |= 1ull << 52;
-  const int Ee = E ? E : 1;
-  const int sh = Ee - 1075 - (efield_r - 1022) + 48;
-  unsigned long long Y;
-  if (M == 0 || E == 2047) {
-    Y = 0;
-  } else if (sh >= 0) {
-    Y = M << sh;
-  } else if (sh <= -60) {
-    Y = 0;
-  } else {
-    Y = (M >> (-sh)) + ((M >> (-sh - 1)) & 1ull);
-  }
-  const uint32_t lo = (uint32_t)Y & 0x00FFFFFFu, hi = (uint32_t)(Y >> 24);
-  const uint32_t u[6] = {hi >> 16, (hi >> 8) & 255u, hi & 255u, lo >> 16, (lo >> 8) & 255u, lo & 255u};
-  int c = 0;
-#pragma unroll
-  for (int p = 5; p >= 1; --p) {
-    const int v = (int)u[p] + c;
-    c = v >= 128;
-    d[p] = c ? v - 256 : v;
-  }
-  d[0] = (int)u[0] + c;
+// The balanced base-2^8 digits of |X[r,k]| * 2^-e_r rounded to 48 fractional
+// bits (S = 6 digits), as one word, and the sign of X[r,k]; the digits of X are
+// those of |X| negated.  Y = |X| 2^(48 - e_r) (an integer of at most 2^48,
+// rounded half up) plus 128 in each of its five lower bytes: byte q < 5 of the
+// word is then digit d_(5-q) + 128 with d in [-128, 127], and what is above them
+// d_0 in [0, 256], all exact in bf16.
+constexpr unsigned long long DIGIT_BIAS = 0x0000008080808080ull;
+__device__ __forceinline__ unsigned long long digit_word(double x, int efield_r) {
+  const int hi = __double2hiint(x);
+  const int E = (hi >> 20) & 0x7FF;
+  unsigned long long M = ((unsigned long long)((hi & 0xFFFFF) | (E ? 0x100000 : 0)) << 32) |
+                         (unsigned)__double2loint(x);
+  const int n = efield_r - (E ? E : 1) + 5;  // Y = M 2^-n, n >= 4
+  M = ((M >> (n < 56 ? n - 1 : 55)) + 1) >> 1;
+  if (n >= 56 || E == 2047) M = 0;
+  return M + DIGIT_BIAS;
+}
+// Sign bits of two elements as they go into a packed pair of bf16 (a zero digit
+// may so become -0, which changes no product or sum).
+__device__ __forceinline__ uint32_t digit_signs(double lo, double hi) {
+  return ((uint32_t)__double2hiint(lo) >> 31 << 15) | ((uint32_t)__double2hiint(hi) & 0x80000000u);
+}
+
+// bf16 bits of digit p of two such words, packed low | high.  A byte b below
+// 0x4B000000 is the float 2^23 + b, d + 0x4B400000 the float 1.5 2^23 + d; the
+// bf16 of a float with at most 8 significant bits is its upper half.
+template <int P>
+__device__ __forceinline__ float digit_float(unsigned long long w) {
+  if (P == 0) return __int_as_float(0x4B400000 + (int)((uint32_t)(w >> 32) >> 8)) - 12582912.0f;
+  const uint32_t half = P == 1 ? (uint32_t)(w >> 32) : (uint32_t)w;
+  constexpr uint32_t sel = 0x7440u + (P == 1 ? 0u : (uint32_t)(5 - P));
+  return __int_as_float((int)__byte_perm(half, 0x4B000000u, sel)) - 8388736.0f;
+}
+template <int P>
+__device__ __forceinline__ uint32_t pack_digits(unsigned long long lo, unsigned long long hi) {
+  return __byte_perm((uint32_t)__float_as_int(digit_float<P>(lo)), (uint32_t)__float_as_int(digit_float<P>(hi)),
+                     0x7632);
+}
+// Digit p of eight elements; sg: their signs in pairs.
+template <int P>
+__device__ __forceinline__ uint4 pack_digits8(const unsigned long long (&w)[8], const uint32_t (&sg)[4]) {
+  return make_uint4(pack_digits<P>(w[0], w[1]) ^ sg[0], pack_digits<P>(w[2], w[3]) ^ sg[1],
+                    pack_digits<P>(w[4], w[5]) ^ sg[2], pack_digits<P>(w[6], w[7]) ^ sg[3]);
 }
 
 // ------------------------------------------------- H_eff middle step
@@ -921,25 +918,34 @@ __device__ __forceinline__ void make_digits_abs(double x, int efield_r, int (&d)
 // 128-byte swizzle into shared memory, two slices per 128-byte row (slice p
 // at k offset 32 (p % 2) of tile p / 2); Weff's column digits are written the
 // same way once per CTA.  One thread issues the 21 digit products (one or two
-// K = 16 steps each) into six TMEM level accumulators of NJP columns; one
+// K = 16 steps each) into six TMEM level accumulators of 16 columns, in two
+// passes for nj > 16 (the second beside the conversion of the first); one
 // group per level suffices because sum_{p+q=L} nc |a_p| |b_q| <= 32 (2 * 2^15
 // + 4 * 2^14) = 2^22 keeps every FP32 partial sum an exact integer.  Each thread then reads
 // its row's level sums, forms the int64 fixed-point value and converts it to
 // FP64 with integer instructions: the same bits as k_split_gemm computes for
 // this product (same digits, same fixed point, same rounding).
+//
+// Bound by the chain load - digits - MMA - drain - store of a block; three CTAs
+// of an SM overlap theirs.  At chi = 1024 (2^20 rows, nc = nj = 20; its reads and
+// writes take 50 us at the measured HBM rate) 379 -> 255 us: digits as one biased
+// word (33 instead of 65 instructions an element), level sums combined in
+// pairs in 32 bits, 128 instead of 256 TMEM columns (two CTAs an SM before).
 constexpr int MID_ROWS = 128;
 constexpr int MID_THREADS = 128;
 constexpr int MID_KSLICE = 32;  // padded K per slice (nc <= 32)
 constexpr int MID_A_TILE = MID_ROWS * 128;     // bytes: 128 rows x 128 B (two slices)
 constexpr int MID_NTILE = (S_SLICES + 1) / 2;  // 3 tiles hold the 6 slices
 
-template <int NJP>
+constexpr uint32_t MID_TMEM_COLS = 128;        // six level accumulators of 16 columns
+
+// NPASS: passes over 16 output columns.
+template <int NPASS>
 struct MidSmem {
-  static constexpr int B_TILE = NJP * 128;
+  static constexpr int B_TILE = NPASS * 16 * 128;
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = MID_NTILE * MID_A_TILE;
   static constexpr int TOTAL = 1024 /*align slack*/ + B_OFF + MID_NTILE * B_TILE + 256;
-  static constexpr uint32_t TMEM_COLS = (S_SLICES * NJP <= 128) ? 128u : 256u;
 };
 
 // byte offset of element (row i, k) of a K-major 128-byte-swizzled tile
@@ -947,59 +953,35 @@ __device__ __forceinline__ uint32_t sw128_off(int i, int k) {
   return (uint32_t)(i * 128 + ((((k >> 3) ^ (i & 7))) << 4) + ((k & 7) << 1));
 }
 
-// bf16 bits of two small integers (|d| <= 2^8, exact in bf16) packed low | high:
-// float(d) = (0x4B400000 + d as float bits) - 1.5 * 2^23 exactly, and the bf16
-// of a float with at most 8 significant bits is its upper half.
-__device__ __forceinline__ uint32_t pack_bf16x2(int lo, int hi) {
-  const float fl = __int_as_float(0x4B400000 + lo) - 12582912.0f;
-  const float fh = __int_as_float(0x4B400000 + hi) - 12582912.0f;
-  return __byte_perm((uint32_t)__float_as_int(fl), (uint32_t)__float_as_int(fh), 0x7632);
-}
-
-// Writes the digits of 8 consecutive k (c0 .. c0 + 7 of slice p) of row i;
-// sgn[q] holds the sign bits (0x8000 per half) of elements 2q, 2q + 1.
-__device__ __forceinline__ void store_digit_chunk(uint8_t* tile, int i, int p, int c0, const int (&dg)[8],
-                                                  const uint32_t (&sgn)[4]) {
-  const int k = (p & 1) * MID_KSLICE + c0;
-  uint4 v;
-  v.x = pack_bf16x2(dg[0], dg[1]) ^ sgn[0];
-  v.y = pack_bf16x2(dg[2], dg[3]) ^ sgn[1];
-  v.z = pack_bf16x2(dg[4], dg[5]) ^ sgn[2];
-  v.w = pack_bf16x2(dg[6], dg[7]) ^ sgn[3];
-  *(uint4*)(tile + sw128_off(i, k)) = v;
-}
-
-// The 6 digits of 8 elements (x[c0 .. c0 + 7], row exponent field ef) into the
-// 7 slices' chunks of row i.  A negative element's digits are the negated
-// digits of its magnitude (bf16 sign bit; a zero digit may so become -0,
-// which changes no product or sum).
+// The 6 digits of 8 elements (x[0 .. 7] = columns c0 .. c0 + 7, row exponent
+// field ef) of row i into the slices' chunks: slice p at k offset 32 (p % 2) of
+// tile p / 2.
 __device__ __forceinline__ void digits8(uint8_t* tiles, int tile_bytes, int i, int c0, const double* x, int ef) {
-  constexpr int S = S_SLICES;
-  int dg[S][8];
-  uint32_t sgn[4] = {0u, 0u, 0u, 0u};
+  unsigned long long w[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    int d[S];
-    bool neg;
-    make_digits_abs(x[e], ef, d, neg);
-    if (neg) sgn[e >> 1] |= (e & 1) ? 0x80000000u : 0x00008000u;
-#pragma unroll
-    for (int p = 0; p < S; ++p) dg[p][e] = d[p];
-  }
-#pragma unroll
-  for (int p = 0; p < S; ++p) store_digit_chunk(tiles + (p >> 1) * tile_bytes, i, p, c0, dg[p], sgn);
+  for (int e = 0; e < 8; ++e) w[e] = digit_word(x[e], ef);
+  const uint32_t sg[4] = {digit_signs(x[0], x[1]), digit_signs(x[2], x[3]), digit_signs(x[4], x[5]),
+                          digit_signs(x[6], x[7])};
+  const uint32_t even = sw128_off(i, c0), odd = sw128_off(i, MID_KSLICE + c0);
+  *(uint4*)(tiles + even) = pack_digits8<0>(w, sg);
+  *(uint4*)(tiles + odd) = pack_digits8<1>(w, sg);
+  *(uint4*)(tiles + tile_bytes + even) = pack_digits8<2>(w, sg);
+  *(uint4*)(tiles + tile_bytes + odd) = pack_digits8<3>(w, sg);
+  *(uint4*)(tiles + 2 * tile_bytes + even) = pack_digits8<4>(w, sg);
+  *(uint4*)(tiles + 2 * tile_bytes + odd) = pack_digits8<5>(w, sg);
 }
 
-template <int NJP>
-__global__ void __launch_bounds__(MID_THREADS)
+template <int NPASS>
+__global__ void __launch_bounds__(MID_THREADS, 3)
 k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff, double* __restrict__ T3,
                  int64_t R, int nc, int nj, uint64_t wait_ns, int* err) {
   constexpr int S = S_SLICES;
+  constexpr int NJP = 16 * NPASS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = base + MidSmem<NJP>::A_OFF;
-  uint8_t* sB = base + MidSmem<NJP>::B_OFF;
-  uint8_t* tail = sB + MID_NTILE * MidSmem<NJP>::B_TILE;
+  uint8_t* sA = base + MidSmem<NPASS>::A_OFF;
+  uint8_t* sB = base + MidSmem<NPASS>::B_OFF;
+  uint8_t* tail = sB + MID_NTILE * MidSmem<NPASS>::B_TILE;
   uint64_t* done = (uint64_t*)tail;
   uint32_t* tmem_slot = (uint32_t*)(tail + 8);
   int* fB = (int*)(tail + 16);  // [NJP] column exponent fields of Weff
@@ -1014,17 +996,14 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(MidSmem<NJP>::TMEM_COLS));
+                 "r"(MID_TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   // A chunks no block writes (k groups past nc): zero once
-  {
-    const int zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const uint32_t nosign[4] = {0u, 0u, 0u, 0u};
-    for (int cg = ngrp; cg < MID_KSLICE / 8; ++cg)
+  for (int cg = ngrp; cg < MID_KSLICE / 8; ++cg)
 #pragma unroll
-      for (int p = 0; p < S; ++p) store_digit_chunk(sA + (p >> 1) * MID_A_TILE, t, p, cg * 8, zero, nosign);
-  }
+    for (int p = 0; p < S; ++p)
+      *(uint4*)(sA + (p >> 1) * MID_A_TILE + sw128_off(t, (p & 1) * MID_KSLICE + cg * 8)) = make_uint4(0u, 0u, 0u, 0u);
   // B: digits of Weff's columns (row j of the B tiles, k = c), once per CTA
   {
     const int j = t >> 2, cg = t & 3;  // NJP * 4 <= 128 threads
@@ -1046,7 +1025,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
         const int c = cg * 8 + e;
         w[e] = (j < nj && c < nc) ? Weff[c + (int64_t)nc * j] : 0.0;
       }
-      digits8(sB, MidSmem<NJP>::B_TILE, j, cg * 8, w, ef);
+      digits8(sB, MidSmem<NPASS>::B_TILE, j, cg * 8, w, ef);
     }
   }
   tc_fence_before();
@@ -1055,87 +1034,89 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
   const int ksteps = nc > 16 ? 2 : 1;
-  int lk = 0;
-  while ((1 << lk) < nc) ++lk;
-  const int F = 62 - 17 - lk;
   const int64_t nblk = (R + MID_ROWS - 1) / MID_ROWS;
+  // the 21 digit products of output columns 16 h .. 16 h + 15 (one thread)
+  auto issue = [&](int h) {
+    constexpr uint32_t idesc = idesc_bf16(MID_ROWS, 16);
+    for (int L = 0; L < S; ++L) {
+      for (int p = 0; p <= L; ++p) {
+        const int q = L - p;
+        const uint64_t ad = sdesc_sw128(smem_u32(sA + (p >> 1) * MID_A_TILE));
+        const uint64_t bd = sdesc_sw128(smem_u32(sB + (q >> 1) * MidSmem<NPASS>::B_TILE + h * 16 * 128));
+        for (int s = 0; s < ksteps; ++s) {
+          const uint64_t ka = (uint64_t)(2 * (2 * (p & 1) + s)), kb = (uint64_t)(2 * (2 * (q & 1) + s));
+          tc_mma_bf16(tmem_base + (uint32_t)(L * 16), ad + ka, bd + kb, idesc, (p > 0 || s > 0) ? 1u : 0u);
+        }
+      }
+    }
+    tc_commit(done);
+  };
   bool ok = true;
   uint32_t phase = 0;
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x, phase ^= 1u) {
+  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     const int64_t r = blk * MID_ROWS + t;
     // ---- A: this thread's row of T1 (all loads first)
-    double x[MID_KSLICE];
+    int eA;
+    {
+      double x[MID_KSLICE];
 #pragma unroll
-    for (int c = 0; c < MID_KSLICE; ++c) x[c] = (c < nc && r < R) ? __ldcs(T1 + r + R * c) : 0.0;
-    unsigned long long mx = 0;
+      for (int c = 0; c < MID_KSLICE; ++c) x[c] = (c < nc && r < R) ? __ldcs(T1 + r + R * c) : 0.0;
+      unsigned mx = 0;  // the exponent is in the upper word
 #pragma unroll
-    for (int c = 0; c < MID_KSLICE; ++c) {
-      const unsigned long long b = (unsigned long long)__double_as_longlong(x[c]) & 0x7FFFFFFFFFFFFFFFull;
-      mx = b > mx ? b : mx;
+      for (int c = 0; c < MID_KSLICE; ++c) {
+        const unsigned b = (unsigned)__double2hiint(x[c]) & 0x7FFFFFFFu;
+        mx = b > mx ? b : mx;
+      }
+      eA = (int)(mx >> 20);
+#pragma unroll
+      for (int cg = 0; cg < MID_KSLICE / 8; ++cg)
+        if (cg < ngrp) digits8(sA, MID_A_TILE, t, cg * 8, x + cg * 8, eA);
     }
-    const int eA = (int)((mx >> 52) & 0x7FF);
-#pragma unroll
-    for (int cg = 0; cg < MID_KSLICE / 8; ++cg)
-      if (cg < ngrp) digits8(sA, MID_A_TILE, t, cg * 8, x + cg * 8, eA);
     // generic-proxy smem writes -> visible to the tensor core (async proxy)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (t == 0) {
-      constexpr uint32_t idesc = idesc_bf16(MID_ROWS, NJP);
-      for (int L = 0; L < S; ++L) {
-        for (int p = 0; p <= L; ++p) {
-          const int q = L - p;
-          const uint64_t ad = sdesc_sw128(smem_u32(sA + (p >> 1) * MID_A_TILE));
-          const uint64_t bd = sdesc_sw128(smem_u32(sB + (q >> 1) * MidSmem<NJP>::B_TILE));
-          for (int s = 0; s < ksteps; ++s) {
-            const uint64_t ka = (uint64_t)(2 * (2 * (p & 1) + s)), kb = (uint64_t)(2 * (2 * (q & 1) + s));
-            tc_mma_bf16(tmem_base + (uint32_t)(L * NJP), ad + ka, bd + kb, idesc, (p > 0 || s > 0) ? 1u : 0u);
-          }
-        }
+    if (t == 0) issue(0);
+    const int em = eA - 1022;
+#pragma unroll
+    for (int h = 0; h < NPASS; ++h) {
+      // every thread waits (bounded) for the products, then takes its row's level sums
+      ok = mbar_wait(done, phase, err, abort_flag, wait_ns);
+      tc_fence_after();
+      // CTA-uniform decision: every thread reaches this barrier whatever its wait returned
+      if (__syncthreads_or(!ok)) {
+        ok = false;
+        break;
       }
-      tc_commit(done);
-    }
-    // every thread waits (bounded) for the products, then drains its row
-    ok = mbar_wait(done, phase, err, abort_flag, wait_ns);
-    tc_fence_after();
-    // CTA-uniform decision: every thread reaches this barrier whatever its wait returned
-    if (__syncthreads_or(!ok)) {
-      ok = false;
-      break;
-    }
-    // int64 fixed point: acc = sum_L s_L 2^(F - 8L) (F >= 40 here, so every
-    // shift is a left shift), by Horner over the levels and one final shift
-    long long acc[NJP];
+      phase ^= 1u;
+      uint32_t v[S][16];
 #pragma unroll
-    for (int L = 0; L < S; ++L) {
+      for (int L = 0; L < S; ++L) tc_ld_32x32b_x16_nowait(lane_base + (uint32_t)(L * 16), v[L]);
+      tc_wait_ld();
+      // the accumulators (after the last pass also the A tiles) may be reused:
+      // the next pass's products run beside this one's conversion
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      if (h + 1 < NPASS && t == 0) issue(h + 1);
+      // fixed point sum_L s_L 2^(8 (5 - L)), the level sums in pairs first: each
+      // is an integer of at most 2^22 in magnitude (float -> int by the
+      // 1.5 * 2^23 shift), so s_L 2^8 + s_(L+1) fits in 32 bits
 #pragma unroll
-      for (int h = 0; h < NJP / 16; ++h) {
-        if (16 * h < nj) {
-          uint32_t v[16];
-          tc_ld_32x32b_x16(lane_base + (uint32_t)(L * NJP + 16 * h), v);
+      for (int j = 0; j < 16; ++j) {
+        if (16 * h + j < nj) {
+          int q[S];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            // exact integer of magnitude <= 2^22: float -> int by the 1.5 * 2^23 shift
-            const long long tv = (long long)(__float_as_int(__uint_as_float(v[j]) + 12582912.0f) - 0x4B400000);
-            acc[16 * h + j] = L == 0 ? tv : (long long)((unsigned long long)acc[16 * h + j] << 8) + tv;
-          }
+          for (int L = 0; L < S; ++L) q[L] = __float_as_int(__uint_as_float(v[L][j]) + 12582912.0f) - 0x4B400000;
+          const long long acc = (long long)((unsigned long long)(long long)((q[0] << 8) + q[1]) << 32) +
+                                ((long long)((q[2] << 8) + q[3]) * 65536ll) + (long long)((q[4] << 8) + q[5]);
+          if (r < R)
+            __stcs(T3 + r + R * (16 * h + j), i64_to_double_scaled(acc, em + fB[16 * h + j] - 1022 - 16 - 40));
         }
       }
     }
-    if (r < R) {
-      const int em = eA - 1022;
-#pragma unroll
-      for (int j = 0; j < NJP; ++j)
-        if (j < nj)
-          __stcs(T3 + r + R * j, i64_to_double_scaled((long long)((unsigned long long)acc[j] << (F - 40)),
-                                                      em + fB[j] - 1022 - 16 - F));
-    }
-    // the TMEM accumulators and the A tiles are reused by the next block
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    if (!ok) break;
   }
   tc_fence_before();
   __syncthreads();
@@ -1145,7 +1126,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
     if (!ok) mbar_drain(done, phase, wait_ns);
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(MidSmem<NJP>::TMEM_COLS));
+                 "r"(MID_TMEM_COLS));
   }
 }
 
@@ -1181,32 +1162,24 @@ k_make_slices(const double* __restrict__ X, const int64_t* __restrict__ offR,
   }
   __syncthreads();
   // each thread: 8 consecutive k of one row -> one 16-byte store per slice
-  static_assert(S == S_SLICES, "digit routine is written for 6 slices");
+  static_assert(S == 6, "the digit word holds 6 slices");
   const int rr = t >> 3, kc = t & 7;
   const int64_t r = r0 + rr;
   const int ef = (r < R) ? efield[r] : 0;
-  int dg[S][8];
-  uint32_t sgn[4] = {0u, 0u, 0u, 0u};
+  unsigned long long w[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    int d[S];
-    bool neg;
-    make_digits_abs(tile[rr][kc * 8 + e], ef, d, neg);
-    if (neg) sgn[e >> 1] |= (e & 1) ? 0x80000000u : 0x00008000u;
+  for (int e = 0; e < 8; ++e) w[e] = digit_word(tile[rr][kc * 8 + e], ef);
+  uint32_t sg[4];
 #pragma unroll
-    for (int p = 0; p < S; ++p) dg[p][e] = d[p];
-  }
+  for (int e = 0; e < 4; ++e) sg[e] = digit_signs(tile[rr][kc * 8 + 2 * e], tile[rr][kc * 8 + 2 * e + 1]);
   const size_t plane = (size_t)Rpad * Kpad;
-  const size_t o = (size_t)r * Kpad + k0 + kc * 8;
-#pragma unroll
-  for (int p = 0; p < S; ++p) {
-    uint4 v;
-    v.x = pack_bf16x2(dg[p][0], dg[p][1]) ^ sgn[0];
-    v.y = pack_bf16x2(dg[p][2], dg[p][3]) ^ sgn[1];
-    v.z = pack_bf16x2(dg[p][4], dg[p][5]) ^ sgn[2];
-    v.w = pack_bf16x2(dg[p][6], dg[p][7]) ^ sgn[3];
-    *(uint4*)(out + (size_t)p * plane + o) = v;
-  }
+  uint4* o = (uint4*)(out + (size_t)r * Kpad + k0 + kc * 8);
+  o[0] = pack_digits8<0>(w, sg);
+  o[plane / 8] = pack_digits8<1>(w, sg);
+  o[2 * (plane / 8)] = pack_digits8<2>(w, sg);
+  o[3 * (plane / 8)] = pack_digits8<3>(w, sg);
+  o[4 * (plane / 8)] = pack_digits8<4>(w, sg);
+  o[5 * (plane / 8)] = pack_digits8<5>(w, sg);
 }
 
 // --------------------------------------------------------------- host
@@ -1341,7 +1314,6 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   const size_t oAcc = take(Smem<BN>::TACC ? 0 : tile_bytes * (size_t)grid);
   const size_t oTacc = take(shares ? tile_bytes * (size_t)grid : 0);
   const size_t oCnt = take(shares ? sizeof(int) * (size_t)grid : 0);
-  const size_t oErr = take(sizeof(int));
   ITG_TRY(ws_reserve(h, off));
   char* ws = (char*)h->split_ws;
   int* eA = (int*)(ws + oEA);
@@ -1359,8 +1331,7 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   long long* acc = (long long*)(ws + oAcc);
   long long* tacc = (long long*)(ws + oTacc);
   int* cnt = (int*)(ws + oCnt);
-  int* err = (int*)(ws + oErr);
-  ITG_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), h->stream));
+  int* err = h->dev_status;  // written only by a wait that runs out
   if (shares) {
     ITG_CUDA(h, cudaMemsetAsync(tacc, 0, tile_bytes * (size_t)grid, h->stream));
     ITG_CUDA(h, cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)grid, h->stream));
@@ -1448,8 +1419,6 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
     k_split_gemm<BN><<<(unsigned)grid, NUM_THREADS, Smem<BN>::TOTAL, h->stream>>>(mA, mB, a);
   }
   ITG_CHECK_LAUNCH(h);
-  // surface a device-side timeout on the next synchronising call
-  ITG_CUDA(h, cudaMemcpyAsync(h->dev_status, err, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
   return ITG_OK;
 }
 
@@ -1460,39 +1429,30 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
   if (nc < 1 || nj < 1 || nc > MID_KSLICE || nj > 32) return ITG_ERR_UNSUPPORTED;
   const int64_t grid = (R + MID_ROWS - 1) / MID_ROWS;
   if (grid > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "heff mid: too many rows");
-  ITG_TRY(ws_reserve(h, 256));
-  int* err = (int*)h->split_ws;
-  ITG_CUDA(h, cudaMemsetAsync(err, 0, sizeof(int), h->stream));
-  auto launch = [&](auto njp_tag) -> int {
-    constexpr int NJP = decltype(njp_tag)::value;
+  int* err = h->dev_status;
+  auto launch = [&](auto tag) -> int {
+    constexpr int NPASS = decltype(tag)::value;
     static bool attr = false;
     if (!attr) {
-      ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NJP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       MidSmem<NJP>::TOTAL));
-      ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NJP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       MidSmem<NPASS>::TOTAL));
+      ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NPASS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
       attr = true;
     }
-    // CTAs per SM: by shared memory (the carveout is set to its maximum) and by
-    // TMEM (512 columns per SM)
-    int smem_sm = 0;
-    ITG_CUDA(h, cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device));
-    int per_sm = smem_sm / (MidSmem<NJP>::TOTAL + 1024);
-    const int tmem_cap = (int)(512u / MidSmem<NJP>::TMEM_COLS);
-    if (per_sm > tmem_cap) per_sm = tmem_cap;
-    if (per_sm < 1) per_sm = 1;
-    const int64_t g = std::min<int64_t>(grid, (int64_t)per_sm * h->num_sms);
-    k_heff_mid_split<NJP><<<(unsigned)g, MID_THREADS, MidSmem<NJP>::TOTAL, h->stream>>>(T1, Weff, T3, R, nc, nj,
-                                                                                         h->wait_ns, err);
+    // three CTAs per SM: by shared memory (the carveout is set to its maximum)
+    // and registers; TMEM (512 columns per SM) would allow four
+    const int64_t g = std::min<int64_t>(grid, (int64_t)3 * h->num_sms);
+    k_heff_mid_split<NPASS><<<(unsigned)g, MID_THREADS, MidSmem<NPASS>::TOTAL, h->stream>>>(T1, Weff, T3, R, nc, nj,
+                                                                                            h->wait_ns, err);
     ITG_CHECK_LAUNCH(h);
     return ITG_OK;
   };
   {
     ProfScope prof(h, ITG_KERNEL_HEFF_MID);
-    if (nj <= 16) ITG_TRY(launch(std::integral_constant<int, 16>()));
-    else ITG_TRY(launch(std::integral_constant<int, 32>()));
+    if (nj <= 16) ITG_TRY(launch(std::integral_constant<int, 1>()));
+    else ITG_TRY(launch(std::integral_constant<int, 2>()));
   }
-  ITG_CUDA(h, cudaMemcpyAsync(h->dev_status, err, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
   return ITG_OK;
 }
 
