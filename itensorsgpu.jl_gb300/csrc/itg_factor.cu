@@ -457,107 +457,181 @@ __device__ __forceinline__ void house_scalars(double alpha, double s2, double& b
   scale = copysign(r * p, alpha);
 }
 
-__global__ void __launch_bounds__(HOUSE_THREADS)
-k_house_step(double* __restrict__ A, int64_t m, int j, double* __restrict__ Vh, double* __restrict__ tau,
-             double* __restrict__ rdiag) {
-  __shared__ double red[HOUSE_THREADS / 32][2];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// Sums of two values over a block of THREADS threads; red: 2 THREADS / 32 doubles.
+template <int THREADS>
+__device__ __forceinline__ void house_sum2(double& a, double& b, double* red) {
+  // lanes below 16 sum the one, the others the other
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16;
+  double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((lane & 15) == 0) red[2 * (threadIdx.x >> 5) + (lane >> 4)] = v;
+  __syncthreads();
+  a = b = 0.0;
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) {
+    a += red[2 * w];
+    b += red[2 * w + 1];
+  }
+}
+
+__device__ __forceinline__ bool house_in_range(double s2) { return s2 >= 0x1p-960 && s2 <= 0x1p960; }
+
+// The step with x scaled by a power of two to at most 1: for columns whose
+// squares are near the ends of the range, or are lost below it.
+template <int THREADS>
+__device__ __noinline__ void house_step_scaled(double* A, int64_t m, int j, double* Vh, double* tau, double* rdiag,
+                                               double* red) {
   const double* x = A + (int64_t)j * m;
   double* col = A + (int64_t)(j + blockIdx.x) * m;
-  const int t = threadIdx.x, lane = t & 31;
-  const double cj = col[j];
-  double alpha = x[j], ps = 1.0, s2, w;
-  // s2 = |x below alpha|^2 and w = x . col, x scaled by ps
-  auto sums = [&](bool scaled) {
-    double a = 0.0, c = 0.0;
-    if (!scaled) {
-#pragma unroll 8
-      for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) {
-        const double xi = x[i];
-        a = fma(xi, xi, a);
-        if (blockIdx.x) c = fma(xi, col[i], c);
-      }
-    } else {
-      for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) {
-        const double xi = x[i] * ps;
-        a = fma(xi, xi, a);
-        c = fma(xi, col[i], c);
-      }
-    }
-    // lanes below 16 sum the one, the others the other
-    const bool up = lane & 16;
-    double v = (up ? c : a) + __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((lane & 15) == 0) red[t >> 5][lane >> 4] = v;
-    __syncthreads();
-    s2 = (red[0][0] + red[1][0]) + (red[2][0] + red[3][0]);
-    w = (red[0][1] + red[1][1]) + (red[2][1] + red[3][1]);
-  };
-  sums(false);
-  // squares near the ends of the range (or lost below it): once more with x
-  // scaled by a power of two to at most 1
-  const bool scaled = !(s2 >= 0x1p-960 && s2 <= 0x1p960);
-  if (scaled) {
-    int mx = 0;  // largest exponent field
-    for (int64_t i = j + t; i < m; i += HOUSE_THREADS) {
-      const int e = (__double2hiint(x[i]) >> 20) & 0x7FF;
-      mx = e > mx ? e : mx;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const int y = __shfl_xor_sync(0xffffffffu, mx, o);
-      mx = y > mx ? y : mx;
-    }
-    __syncthreads();
-    if (lane == 0) red[t >> 5][0] = (double)mx;
-    __syncthreads();
-    mx = (int)fmax(fmax(red[0][0], red[1][0]), fmax(red[2][0], red[3][0]));
-    __syncthreads();
-    const int k = mx - 1022 < -1000 ? -1000 : (mx - 1022 > 1000 ? 1000 : mx - 1022);
-    ps = __hiloint2double((1023 - k) << 20, 0);
-    alpha *= ps;
-    sums(true);
+  const int t = threadIdx.x;
+  int mx = 0;  // largest exponent field
+  for (int64_t i = j + t; i < m; i += THREADS) {
+    const int e = (__double2hiint(x[i]) >> 20) & 0x7FF;
+    mx = e > mx ? e : mx;
   }
+  double pair[2] = {(double)__reduce_max_sync(0xffffffffu, (unsigned)mx), 0.0};
+  __syncthreads();
+  if ((t & 31) == 0) red[t >> 5] = pair[0];
+  __syncthreads();
+  for (int w = 0; w < THREADS / 32; ++w) pair[0] = fmax(pair[0], red[w]);
+  __syncthreads();
+  const int k = (int)pair[0] - 1022 < -1000 ? -1000 : ((int)pair[0] - 1022 > 1000 ? 1000 : (int)pair[0] - 1022);
+  const double ps = __hiloint2double((1023 - k) << 20, 0), alpha = x[j] * ps, cj = col[j];
+  double s2 = 0.0, w = 0.0;
+  for (int64_t i = j + 1 + t; i < m; i += THREADS) {
+    const double xi = x[i] * ps;
+    s2 = fma(xi, xi, s2);
+    w = fma(xi, col[i], w);
+  }
+  house_sum2<THREADS>(s2, w, red);
   double tj = 0.0, beta = alpha, scale = 0.0;
   if (s2 > 0.0) house_scalars(alpha, s2, beta, tj, scale);
   if (blockIdx.x == 0) {
     double* v = Vh + (int64_t)j * m;
-    for (int64_t i = t; i < m; i += HOUSE_THREADS)
-      v[i] = i < j ? 0.0 : (i == j ? 1.0 : (scaled ? x[i] * ps : x[i]) * scale);
+    for (int64_t i = t; i < m; i += THREADS) v[i] = i < j ? 0.0 : (i == j ? 1.0 : x[i] * ps * scale);
     if (t == 0) {
       tau[j] = tj;
-      rdiag[j] = scaled ? beta / ps : beta;
+      rdiag[j] = beta / ps;
     }
     return;
   }
   if (tj == 0.0) return;
   const double f = tj * fma(w, scale, cj), g = -f * scale;
-  if (!scaled) {
-#pragma unroll 8
-    for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) col[i] = fma(g, x[i], col[i]);
-  } else {
-    for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) col[i] = fma(g, x[i] * ps, col[i]);
-  }
+  for (int64_t i = j + 1 + t; i < m; i += THREADS) col[i] = fma(g, x[i] * ps, col[i]);
   if (t == 0) col[j] = cj - f;
+}
+
+__global__ void __launch_bounds__(HOUSE_THREADS)
+k_house_step(double* __restrict__ A, int64_t m, int j, double* __restrict__ Vh, double* __restrict__ tau,
+             double* __restrict__ rdiag) {
+  __shared__ double red[HOUSE_THREADS / 16];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const double* x = A + (int64_t)j * m;
+  double* col = A + (int64_t)(j + blockIdx.x) * m;
+  const int t = threadIdx.x;
+  const double alpha = x[j], cj = col[j];
+  double s2 = 0.0, w = 0.0;
+#pragma unroll 8
+  for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) {
+    const double xi = x[i];
+    s2 = fma(xi, xi, s2);
+    if (blockIdx.x) w = fma(xi, col[i], w);
+  }
+  house_sum2<HOUSE_THREADS>(s2, w, red);
+  if (!house_in_range(s2)) {
+    house_step_scaled<HOUSE_THREADS>(A, m, j, Vh, tau, rdiag, red);
+    return;
+  }
+  double tj, beta, scale;
+  house_scalars(alpha, s2, beta, tj, scale);
+  if (blockIdx.x == 0) {
+    double* v = Vh + (int64_t)j * m;
+    for (int64_t i = t; i < m; i += HOUSE_THREADS) v[i] = i < j ? 0.0 : (i == j ? 1.0 : x[i] * scale);
+    if (t == 0) {
+      tau[j] = tj;
+      rdiag[j] = beta;
+    }
+    return;
+  }
+  const double f = tj * fma(w, scale, cj), g = -f * scale;
+#pragma unroll 8
+  for (int64_t i = j + 1 + t; i < m; i += HOUSE_THREADS) col[i] = fma(g, x[i], col[i]);
+  if (t == 0) col[j] = cj - f;
+}
+
+// The step in LAPACK's operations throughout (norm by hypot, the scaled
+// reflector in every product): what itg_qr runs on.  Its factors are results in
+// their own right and start iterations (the gauge of an MPS before its first
+// sweep) that carry a difference in the last bit far, so they stay as they are;
+// the factorisations, which refine what their QR gives them, take the step above.
+__global__ void __launch_bounds__(256)
+k_house_step_plain(double* __restrict__ A, int64_t m, int j, double* __restrict__ Vh, double* __restrict__ tau,
+                   double* __restrict__ rdiag) {
+  __shared__ double sh[16];
+  auto sum = [&](double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s += sh[w];
+    __syncthreads();
+    return s;
+  };
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const double* x = A + (int64_t)j * m;
+  const double alpha = x[j];
+  double s2 = 0.0;
+  for (int64_t i = j + 1 + threadIdx.x; i < m; i += 256) s2 = fma(x[i], x[i], s2);
+  s2 = sum(s2);
+  if (!house_in_range(s2)) {
+    house_step_scaled<256>(A, m, j, Vh, tau, rdiag, sh);
+    return;
+  }
+  double tj = 0.0, beta = alpha, scale = 0.0;
+  if (s2 > 0.0) {
+    beta = -copysign(hypot(alpha, sqrt(s2)), alpha);
+    tj = (beta - alpha) / beta;
+    scale = 1.0 / (alpha - beta);
+  }
+  if (blockIdx.x == 0) {
+    double* v = Vh + (int64_t)j * m;
+    for (int64_t i = threadIdx.x; i < m; i += 256) v[i] = i < j ? 0.0 : (i == j ? 1.0 : x[i] * scale);
+    if (threadIdx.x == 0) {
+      tau[j] = tj;
+      rdiag[j] = beta;
+    }
+    return;
+  }
+  if (tj == 0.0) return;
+  double* col = A + (int64_t)(j + blockIdx.x) * m;
+  double w = 0.0;
+  for (int64_t i = j + 1 + threadIdx.x; i < m; i += 256) w = fma(x[i] * scale, col[i], w);
+  w = sum(w) + col[j];
+  const double f = tj * w;
+  for (int64_t i = j + threadIdx.x; i < m; i += 256) col[i] -= f * (i == j ? 1.0 : x[i] * scale);
 }
 
 }  // namespace
 
 namespace itg {
 // Steps j0 .. j0 + count - 1 on columns up to jend, on the handle's stream.
-int house_panel(itg_handle* h, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh, double* tau,
-                double* rdiag) {
+int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
+                double* tau, double* rdiag) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   for (int64_t j = j0; j < j0 + count; ++j) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(jend - j));
-    cfg.blockDim = dim3(HOUSE_THREADS);
+    cfg.blockDim = dim3(fast ? HOUSE_THREADS : 256);
     cfg.stream = h->stream;
     cfg.attrs = &at;
     cfg.numAttrs = j > j0 ? 1 : 0;  // the first step waits for everything before it
-    ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step, A, m, (int)j, Vh, tau, rdiag));
+    if (fast) ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step, A, m, (int)j, Vh, tau, rdiag));
+    else ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step_plain, A, m, (int)j, Vh, tau, rdiag));
   }
   return ITG_OK;
 }
@@ -801,7 +875,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     Tq = (double*)(base + oTq);
     Qws = (double*)(base + oQws);
     ProfScope prof(h, ITG_KERNEL_SVD_QR);
-    ITG_TRY(itg::qr_blocked(h, W, mm, nn, nn, Vh, tau, rd, Tq, Qws));
+    ITG_TRY(itg::qr_blocked(h, W, mm, nn, nn, Vh, tau, rd, Tq, Qws, true));
     k_build_rt<<<itg_blocks_for(nn * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, mm, (int)nn, rd, J);
     ITG_CHECK_LAUNCH(h);
     if (two) {
@@ -810,7 +884,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
       double* rd2 = (double*)(base + oRd2);
       double* J2 = (double*)(base + oB2);
       Tq2 = (double*)(base + oTq2);
-      ITG_TRY(itg::qr_blocked(h, J, nn, nn, nn, Vh2, tau2, rd2, Tq2, Qws));
+      ITG_TRY(itg::qr_blocked(h, J, nn, nn, nn, Vh2, tau2, rd2, Tq2, Qws, true));
       k_build_rt<<<itg_blocks_for(nn * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(J, nn, (int)nn, rd2, J2);
       ITG_CHECK_LAUNCH(h);
       J = J2;
@@ -1061,7 +1135,7 @@ extern "C" int itg_qr(itg_handle* h, int64_t m, int64_t n, const double* A, int6
   double* ws = (double*)(base + oWs);
   k_copy_matrix<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, m, n, W, 0.0);
   ITG_CHECK_LAUNCH(h);
-  ITG_TRY(itg::qr_blocked(h, W, m, n, r, Vh, tau, rd, Tq, ws));
+  ITG_TRY(itg::qr_blocked(h, W, m, n, r, Vh, tau, rd, Tq, ws, false));
   k_extract_r<<<itg_blocks_for(r * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m, r, n, rd, R);
   k_eye_cols<<<itg_blocks_for(m * r, 256, h->num_sms * 16), 256, 0, h->stream>>>(Q, m, r);
   ITG_CHECK_LAUNCH(h);

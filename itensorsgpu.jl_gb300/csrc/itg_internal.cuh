@@ -148,7 +148,7 @@ int jacobi_persistent(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin
 // trailing updates in FP64; nref reflectors (nref <= min(m, n)) applied to all
 // n columns.
 int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, double* Vh, double* tau, double* rd,
-               double* Tbuf, double* ws);
+               double* Tbuf, double* ws, bool fast);
 int q_apply_blocked(itg_handle* h, double* Y, int64_t m, int64_t n, int64_t ncols, const double* Vh,
                     const double* Tbuf, double* ws);
 size_t qr_blocked_ws_doubles(int64_t n);

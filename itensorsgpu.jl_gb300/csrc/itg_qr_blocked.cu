@@ -13,49 +13,39 @@
 #include "itg_internal.cuh"
 
 namespace itg {
-int house_panel(itg_handle* h, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh, double* tau,
-                double* rdiag);
+int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
+                double* tau, double* rdiag);
 }  // namespace itg
 
 namespace {
 
 // T (32 x 32, upper triangular) from the partial sums of Y = V^T V (column c
-// of chunk q at part[32 (q bw + c)]):  T = [T1, -T1 Y12 T2; 0, T2] for blocks of
-// 1, 2, 4, 8, 16 (each element two short dot products; the column recurrence
-// of larft is a chain of 500 FP64 instructions, 44 us, this one 8 us).
-__global__ void __launch_bounds__(256)
+// of chunk q at part[32 (q bw + c)]): LAPACK's larft,
+//   T(j,j) = tau_j, T(0:j, j) = -tau_j T(0:j, 0:j) Y(0:j, j),
+// with its sums formed one term a step for all elements at once (thread (i, j)
+// adds T(i,l) Y(l,j) as soon as column l is final: the order of the recurrence,
+// 32 steps instead of a chain of 500 FP64 instructions; 44 -> 12 us).
+__global__ void __launch_bounds__(1024)
 k_larft(const double* __restrict__ part, int nchunk, const double* __restrict__ tau, int bw, double* __restrict__ T) {
   constexpr int NB = QR_NB;
-  __shared__ double Y[NB][NB + 1], S[NB][NB + 1], M[NB][NB + 1];  // [column][row]
-  const int t = threadIdx.x;
-  for (int i = t; i < NB * NB; i += 256) {
-    const int c = i / NB, r = i % NB;
-    double y = 0.0;
-    if (r < c && c < bw)
-      for (int q = 0; q < nchunk; ++q) y += part[(int64_t)q * NB * bw + i];
-    Y[c][r] = y;
-    S[c][r] = r == c && c < bw ? tau[c] : 0.0;
-  }
+  __shared__ double Y[NB][NB + 1], col[2][NB];  // Y[column][row]; column l of T
+  const int i = threadIdx.x % NB, j = threadIdx.x / NB;
+  double y = 0.0;
+  if (i < j && j < bw)
+    for (int q = 0; q < nchunk; ++q) y += part[((int64_t)q * bw + j) * NB + i];
+  Y[j][i] = y;
+  const double tj = j < bw ? tau[j] : 0.0;
+  double s = 0.0, t = 0.0;
   __syncthreads();
-  for (int s = 1; s < NB; s *= 2) {
-    // element (r, c) of the off-diagonal block of pair b: rows 2 s b + r, columns 2 s b + s + c
-    const int b = t / (s * s), r = t % s, c = t / s % s;
-    const int o = 2 * s * b;
-    const bool in = o < NB;
-    if (in) {
-      double m = 0.0;
-      for (int l = 0; l <= c; ++l) m = fma(Y[o + s + l][o + r], S[o + s + c][o + s + l], m);
-      M[o + s + c][o + r] = m;
+  for (int l = 0; l < NB; ++l) {
+    if (j == l) {
+      t = i < l ? -tj * s : (i == l ? tj : 0.0);
+      col[l & 1][i] = t;
     }
     __syncthreads();
-    if (in) {
-      double m = 0.0;
-      for (int l = r; l < s; ++l) m = fma(S[o + l][o + r], M[o + s + c][o + l], m);
-      S[o + s + c][o + r] = -m;
-    }
-    __syncthreads();
+    if (j > l && i <= l) s = fma(col[l & 1][i], Y[j][l], s);
   }
-  for (int i = t; i < NB * NB; i += 256) T[i] = S[i / NB][i % NB];
+  T[j * NB + i] = t;
 }
 
 // Partial sums of V_p^T B for the panel's reflectors V_p (columns jb..jb+bw of
@@ -149,18 +139,18 @@ k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const 
     zs[c][k] = n0 + c < N ? Z2[(n0 + c) * NB + k] : 0.0;
   }
   const int tr = t % 16, tc = t / 16;
-  double acc[2][2];
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, old[2][2];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       const int64_t r = r0 + tr + 16 * a, c = n0 + tc + 8 * b;
-      acc[a][b] = (r < m && c < N) ? C[(c0 + c) * m + r] : 0.0;
+      old[a][b] = (r < m && c < N) ? C[(c0 + c) * m + r] : 0.0;
     }
   __syncthreads();
 #pragma unroll 8
   for (int k = 0; k < NB; ++k) {
-    const double v0 = vs[k][tr], v1 = vs[k][tr + 16], z0 = -zs[tc][k], z1 = -zs[tc + 8][k];
+    const double v0 = vs[k][tr], v1 = vs[k][tr + 16], z0 = zs[tc][k], z1 = zs[tc + 8][k];
     acc[0][0] = fma(v0, z0, acc[0][0]);
     acc[0][1] = fma(v0, z1, acc[0][1]);
     acc[1][0] = fma(v1, z0, acc[1][0]);
@@ -171,7 +161,7 @@ k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const 
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       const int64_t r = r0 + tr + 16 * a, c = n0 + tc + 8 * b;
-      if (r < m && c < N) C[(c0 + c) * m + r] = acc[a][b];
+      if (r < m && c < N) C[(c0 + c) * m + r] = old[a][b] - acc[a][b];
     }
 }
 
@@ -217,7 +207,8 @@ int wy_apply(itg_handle* h, double* C, int64_t m, int64_t jb, int bw, const doub
 
 namespace itg {
 
-// Blocked Householder QR of W (m x n, ld m) in place with nref <= min(m, n)
+// Blocked Householder QR (fast: with the column steps of house_panel's fast
+// form) of W (m x n, ld m) in place with nref <= min(m, n)
 // reflectors (nref = n for the tall case, m for a wide matrix): reflectors in
 // Vh (m x nref, explicit unit diagonal, zeros above), tau, R's diagonal in rd,
 // the rest of R's rows above the diagonal in W; Tbuf holds QR_NB^2 doubles
@@ -255,7 +246,7 @@ int qr_lookahead_init(itg_handle* h) {
 }  // namespace
 
 int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, double* Vh, double* tau, double* rd,
-               double* Tbuf, double* ws) {
+               double* Tbuf, double* ws, bool fast) {
   const int NB = QR_NB;
   const int64_t part_doubles = QR_PART_CHUNKS * 32 * n;
   double *Zp = ws, *partp = Zp + (int64_t)NB * n;                          // panel stream
@@ -269,7 +260,7 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
     ITG_CUDA(h, cudaStreamWaitEvent(h->stream, h->qr_ev_done, 0));
     if (nref > 0) {
       const int64_t w = nref < NB ? nref : NB;
-      ITG_TRY(house_panel(h, W, m, 0, w, w, Vh, tau, rd));
+      ITG_TRY(house_panel(h, fast, W, m, 0, w, w, Vh, tau, rd));
     }
   }
   for (int64_t jb = 0, panel = 0; jb < nref; jb += NB, ++panel) {
@@ -283,7 +274,7 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
       OnStream on(h, h->qr_stream);
       int nchunk = 0;
       ITG_TRY(skinny_vt_b(h, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
-      k_larft<<<1, 256, 0, h->stream>>>(partp, nchunk, tau + jb, (int)bw, Tp);
+      k_larft<<<1, QR_NB * QR_NB, 0, h->stream>>>(partp, nchunk, tau + jb, (int)bw, Tp);
       ITG_CHECK_LAUNCH(h);
       if (nt <= 0) continue;
       // V_p and T_p are final: the handle's stream may update the rest
@@ -299,7 +290,7 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
     ITG_CUDA(h, cudaEventRecord(h->qr_ev_done, main_stream));
     if (nnext > 0) {
       OnStream on(h, h->qr_stream);
-      ITG_TRY(house_panel(h, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
+      ITG_TRY(house_panel(h, fast, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
     }
   }
   // the handle's stream continues after the last panel's work
