@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <fstream>
 #include <sstream>
 
@@ -483,6 +484,31 @@ std::string plan_key(int rankA, const int64_t* dimsA, const int32_t* modesA, int
   return os.str();
 }
 
+// The same identity in binary, for the plan lookup of every call: per tensor
+// its rank, then per mode the canonical label and the dimension.  (Formatting
+// the text key cost 3 us a call.)
+std::string plan_key_bin(int rankA, const int64_t* dimsA, const int32_t* modesA, int rankB, const int64_t* dimsB,
+                         const int32_t* modesB, int rankC, const int64_t* dimsC, const int32_t* modesC) {
+  char buf[3 + 9 * 3 * ITG_MAX_RANK];
+  int32_t seen[3 * ITG_MAX_RANK];
+  int nseen = 0, n = 0;
+  auto put = [&](int r, const int64_t* d, const int32_t* m) {
+    buf[n++] = (char)r;
+    for (int i = 0; i < r; ++i) {
+      int l = 0;
+      while (l < nseen && seen[l] != m[i]) ++l;
+      if (l == nseen) seen[nseen++] = m[i];
+      buf[n++] = (char)l;
+      std::memcpy(buf + n, d + i, 8);
+      n += 8;
+    }
+  };
+  put(rankC, dimsC, modesC);
+  put(rankA, dimsA, modesA);
+  put(rankB, dimsB, modesB);
+  return std::string(buf, n);
+}
+
 }  // namespace
 
 int itg_split_gemm(itg_handle* h, const ContractPlan& p, const double* A, const double* B, double* C,
@@ -724,15 +750,15 @@ namespace itg {
 int get_plan(itg_handle* h, int rankA, const int64_t* dimsA, const int32_t* modesA, int rankB,
              const int64_t* dimsB, const int32_t* modesB, int rankC, const int64_t* dimsC,
              const int32_t* modesC, std::shared_ptr<ContractPlan>& plan) {
-  std::string key = plan_key(rankA, dimsA, modesA, rankB, dimsB, modesB, rankC, dimsC, modesC);
+  std::string key = plan_key_bin(rankA, dimsA, modesA, rankB, dimsB, modesB, rankC, dimsC, modesC);
   auto it = h->plans.find(key);
   if (it != h->plans.end()) {
     plan = it->second;
     return ITG_OK;
   }
   ITG_TRY(build_plan(h, rankA, dimsA, modesA, rankB, dimsB, modesB, rankC, dimsC, modesC, plan));
-  plan->key = key;
-  h->plans[key] = plan;
+  plan->key = plan_key(rankA, dimsA, modesA, rankB, dimsB, modesB, rankC, dimsC, modesC);
+  h->plans[std::move(key)] = plan;
   return ITG_OK;
 }
 

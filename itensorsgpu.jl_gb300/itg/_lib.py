@@ -12,6 +12,7 @@ first call raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import threading
 from pathlib import Path
 
@@ -189,14 +190,19 @@ def load_library(path: Path | None = None) -> C.CDLL:
         return lib
 
 
+@functools.lru_cache(maxsize=8192)
+def _const_array(ctype, vals):
+    return (ctype * max(1, len(vals)))(*vals)
+
+
 def i64arr(vals):
-    a = (C.c_int64 * max(1, len(vals)))(*[int(v) for v in vals])
-    return a
+    """int64 input array (dims); shared between calls of the same values, so read-only."""
+    return _const_array(C.c_int64, tuple(map(int, vals)))
 
 
 def i32arr(vals):
-    a = (C.c_int32 * max(1, len(vals)))(*[int(v) for v in vals])
-    return a
+    """int32 input array (mode labels); shared between calls of the same values, so read-only."""
+    return _const_array(C.c_int32, tuple(map(int, vals)))
 
 
 class Handle:
@@ -226,7 +232,8 @@ class Handle:
 
     def call(self, name: str, *args):
         st = getattr(self.lib, name)(self.ptr, *args)
-        self.check(st, name)
+        if st:
+            self.check(st, name)
 
     def close(self):
         if getattr(self, "ptr", None):

@@ -12,6 +12,7 @@ itg.dmrg over the instances (same algorithm; the SVD is always FP64 Jacobi here)
 from __future__ import annotations
 
 import ctypes as C
+import math
 import time
 
 import numpy as np
@@ -23,15 +24,15 @@ from .mps import MPO, MPS
 
 
 def _ptrs(ts):
-    return (C.c_void_p * len(ts))(*[C.c_void_p(t.data_ptr()) for t in ts])
+    return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
 def _grouped(h, A, dA, mA, B, dB, mB, dC, mC):
     """C_i = A_i * B_i for all i (same modes, per-instance dims); returns the C_i."""
-    outs = [T.empty_dev(int(np.prod(d))) for d in dC]
-    flat = lambda ds: [int(x) for d in ds for x in d]
-    h.call("itg_contract_grouped", len(A), C.c_double(1.0), _ptrs(A), len(mA), i64arr(flat(dA)), i32arr(mA),
-           _ptrs(B), len(mB), i64arr(flat(dB)), i32arr(mB), C.c_double(0.0), _ptrs(outs), len(mC),
+    outs = [T.empty_dev(math.prod(d)) for d in dC]
+    flat = lambda ds: [x for d in ds for x in d]
+    h.call("itg_contract_grouped", len(A), 1.0, _ptrs(A), len(mA), i64arr(flat(dA)), i32arr(mA),
+           _ptrs(B), len(mB), i64arr(flat(dB)), i32arr(mB), 0.0, _ptrs(outs), len(mC),
            i64arr(flat(dC)), i32arr(mC))
     return outs
 
@@ -106,11 +107,11 @@ def dmrg_batched(Hs, psis, nsweep: int, maxdims, cutoff: float, *, mindim: int =
             W1d, W2d = chains[0].Wd[b], chains[0].Wd[b + 1]
             e = (C.c_double * cnt)()
             nmv = (C.c_int * cnt)()
-            h.call("itg_davidson_heff2_batched", cnt, i64arr(chiL), i64arr(chiR), C.c_int64(d),
-                   C.c_int64(W1d[0]), C.c_int64(W1d[3]), C.c_int64(W2d[3]),
+            h.call("itg_davidson_heff2_batched", cnt, i64arr(chiL), i64arr(chiR), d,
+                   W1d[0], W1d[3], W2d[3],
                    _ptrs([Lenv[i][b][0] for i in range(cnt)]), _ptrs([c.W[b] for c in chains]),
                    _ptrs([c.W[b + 1] for c in chains]), _ptrs([Renv[i][b + 2][0] for i in range(cnt)]),
-                   _ptrs(phis), int(krylovdim), int(maxiter), C.c_double(eigsolve_tol), e, nmv)
+                   _ptrs(phis), int(krylovdim), int(maxiter), eigsolve_tol, e, nmv)
             energies[:] = np.frombuffer(e, dtype=np.float64)
             ms = [chiL[i] * d for i in range(cnt)]
             ns = [d * chiR[i] for i in range(cnt)]
@@ -121,7 +122,7 @@ def dmrg_batched(Hs, psis, nsweep: int, maxdims, cutoff: float, *, mindim: int =
             ks = (C.c_int64 * cnt)()
             tes = (C.c_double * cnt)()
             h.call("itg_svd_trunc_batched", cnt, i64arr(ms), i64arr(ns), _ptrs(phis),
-                   i64arr([at(md[i], sw) for i in range(cnt)]), C.c_int64(mindim), C.c_double(cutoff), 0, 1, 0,
+                   i64arr([at(md[i], sw) for i in range(cnt)]), mindim, cutoff, 0, 1, 0,
                    _ptrs(Us), _ptrs(Ss), _ptrs(Vs), ks, tes)
             for i, c in enumerate(chains):
                 kk = int(ks[i])

@@ -14,6 +14,7 @@ precision.  The host only orchestrates.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import time
 from dataclasses import dataclass, field
 
@@ -102,31 +103,29 @@ class DMRGResult:
 
 # ---------------------------------------------------------- raw helpers
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _contract_raw(h, A, dA, mA, B, dB, mB, dC, mC, precision=PREC_FP64, out=None):
-    n = int(np.prod(dC)) if len(dC) else 1
     if out is None:
-        out = T.empty_dev(n)
-    h.call("itg_contract", ITG_F64, C.c_double(1.0), _ptr(A), len(dA), i64arr(dA), i32arr(mA),
-           _ptr(B), len(dB), i64arr(dB), i32arr(mB), C.c_double(0.0), _ptr(out), len(dC),
+        out = T.empty_dev(math.prod(dC))
+    h.call("itg_contract", ITG_F64, 1.0, _ptr(A), len(dA), i64arr(dA), i32arr(mA),
+           _ptr(B), len(dB), i64arr(dB), i32arr(mB), 0.0, _ptr(out), len(dC),
            i64arr(dC), i32arr(mC), int(precision))
     return out
 
 
 def _diag_raw(h, d, dD, mD, Tt, dT, mT, dC, mC):
-    n = int(np.prod(dC))
-    out = T.empty_dev(n)
-    h.call("itg_diag_contract", ITG_F64, C.c_double(1.0), _ptr(d), 0, len(dD), i64arr(dD), i32arr(mD),
-           _ptr(Tt), len(dT), i64arr(dT), i32arr(mT), C.c_double(0.0), _ptr(out), len(dC),
+    out = T.empty_dev(math.prod(dC))
+    h.call("itg_diag_contract", ITG_F64, 1.0, _ptr(d), 0, len(dD), i64arr(dD), i32arr(mD),
+           _ptr(Tt), len(dT), i64arr(dT), i32arr(mT), 0.0, _ptr(out), len(dC),
            i64arr(dC), i32arr(mC))
     return out
 
 
 def _permute_raw(h, A, dA, mA, mB):
-    out = T.empty_dev(int(np.prod(dA)))
-    h.call("itg_permute", ITG_F64, C.c_double(1.0), _ptr(A), len(dA), i64arr(dA), i32arr(mA),
+    out = T.empty_dev(math.prod(dA))
+    h.call("itg_permute", ITG_F64, 1.0, _ptr(A), len(dA), i64arr(dA), i32arr(mA),
            _ptr(out), i32arr(mB))
     return out
 
@@ -174,8 +173,8 @@ def _env_right(h, Rt, Rd, A, Ad, W, Wd, prec):
 
 def _contract_acc(h, alpha, A, dA, mA, B, dB, mB, out, dC, mC, precision):
     """out = alpha * (A x B) + out."""
-    h.call("itg_contract", ITG_F64, C.c_double(alpha), _ptr(A), len(dA), i64arr(dA), i32arr(mA),
-           _ptr(B), len(dB), i64arr(dB), i32arr(mB), C.c_double(1.0), _ptr(out), len(dC),
+    h.call("itg_contract", ITG_F64, alpha, _ptr(A), len(dA), i64arr(dA), i32arr(mA),
+           _ptr(B), len(dB), i64arr(dB), i32arr(mB), 1.0, _ptr(out), len(dC),
            i64arr(dC), i32arr(mC), int(precision))
 
 
@@ -227,8 +226,8 @@ def _noise_split(h, phi, shape, Lt, Ld, W1, W1d, W2, W2d, Rt, Rd, ha, noise, max
     k = C.c_int64()
     te = C.c_double()
     dc = C.c_double()
-    h.call("itg_eigh_trunc", C.c_int64(m), _ptr(rho), C.c_int64(m), C.c_int64(maxdim), C.c_int64(mindim),
-           C.c_double(cutoff), 0, 1, int(legacy), _ptr(D), _ptr(U), C.byref(k), C.byref(te), C.byref(dc))
+    h.call("itg_eigh_trunc", m, _ptr(rho), m, maxdim, mindim,
+           cutoff, 0, 1, int(legacy), _ptr(D), _ptr(U), C.byref(k), C.byref(te), C.byref(dc))
     kk = int(k.value)
     Uk = U[: m * kk]
     if ha == 1:
@@ -252,7 +251,7 @@ def _orthogonalize_left_end(h, ch: _Chain):
         r = min(m, n)
         Q = T.empty_dev(m * r)
         R = T.empty_dev(r * n)
-        h.call("itg_qr", C.c_int64(m), C.c_int64(n), _ptr(Mt), C.c_int64(m), _ptr(Q), _ptr(R))
+        h.call("itg_qr", m, n, _ptr(Mt), m, _ptr(Q), _ptr(R))
         # A_j = Q^T as (r, d, b)
         ch.A[j] = _permute_raw(h, Q, (d, b, r), [2, 3, 1], [1, 2, 3])
         ch.Ad[j] = (r, d, b)
@@ -262,8 +261,8 @@ def _orthogonalize_left_end(h, ch: _Chain):
                                     (pa, pd, r), [1, 2, 4])
         ch.Ad[j - 1] = (pa, pd, r)
     nrm = C.c_double()
-    h.call("itg_nrm2", C.c_int64(ch.A[0].numel()), _ptr(ch.A[0]), C.byref(nrm))
-    h.call("itg_scal", C.c_int64(ch.A[0].numel()), C.c_double(1.0 / nrm.value), _ptr(ch.A[0]))
+    h.call("itg_nrm2", ch.A[0].numel(), _ptr(ch.A[0]), C.byref(nrm))
+    h.call("itg_scal", ch.A[0].numel(), C.c_double(1.0 / nrm.value), _ptr(ch.A[0]))
 
 
 def _dmrg_complex(H: MPO, psi0: MPS, sweeps: Sweeps, krylovdim: int, maxiter: int, eigsolve_tol: float,
@@ -436,15 +435,15 @@ def dmrg(H: MPO, psi0: MPS, sweeps: Sweeps, *, krylovdim: int = 3, maxiter: int 
             e = C.c_double()
             nmv = C.c_int()
             if preconditioner is None:
-                h.call("itg_davidson_heff2", C.c_int64(a), C.c_int64(c), C.c_int64(d1), C.c_int64(W1d[0]),
-                       C.c_int64(W1d[3]), C.c_int64(W2d[3]), _ptr(Lt), _ptr(W1), _ptr(W2), _ptr(Rt),
-                       _ptr(phi), int(krylovdim), int(maxiter), C.c_double(eigsolve_tol), int(precision),
+                h.call("itg_davidson_heff2", a, c, d1, W1d[0],
+                       W1d[3], W2d[3], _ptr(Lt), _ptr(W1), _ptr(W2), _ptr(Rt),
+                       _ptr(phi), int(krylovdim), int(maxiter), eigsolve_tol, int(precision),
                        C.byref(e), C.byref(nmv))
             else:
                 fb = C.c_int()
-                h.call("itg_davidson_heff2_learned", C.c_int64(a), C.c_int64(c), C.c_int64(d1),
-                       C.c_int64(W1d[0]), C.c_int64(W1d[3]), C.c_int64(W2d[3]), _ptr(Lt), _ptr(W1), _ptr(W2),
-                       _ptr(Rt), _ptr(phi), int(krylovdim), int(maxiter), C.c_double(eigsolve_tol),
+                h.call("itg_davidson_heff2_learned", a, c, d1,
+                       W1d[0], W1d[3], W2d[3], _ptr(Lt), _ptr(W1), _ptr(W2),
+                       _ptr(Rt), _ptr(phi), int(krylovdim), int(maxiter), eigsolve_tol,
                        int(precision), preconditioner.ptr,
                        _ptr(lamL) if lamL is not None else None, _ptr(lamR) if lamR is not None else None,
                        C.byref(e), C.byref(nmv), C.byref(fb))
@@ -479,8 +478,8 @@ def dmrg(H: MPO, psi0: MPS, sweeps: Sweeps, *, krylovdim: int = 3, maxiter: int 
             te = C.c_double()
             dc = C.c_double()
             try:
-                h.call("itg_factorize_trunc", C.c_int64(m), C.c_int64(n), _ptr(phi), C.c_int64(m),
-                       C.c_int64(maxdim), C.c_int64(mindim), C.c_double(cutoff), 0, 1,
+                h.call("itg_factorize_trunc", m, n, _ptr(phi), m,
+                       maxdim, mindim, cutoff, 0, 1,
                        int(legacy_gpu_truncate), 0 if ha == 1 else 1, int(svd_method), int(precision),
                        _ptr(Lb), _ptr(S), _ptr(Cb), C.byref(k), C.byref(te), C.byref(dc))
             except NotConverged:

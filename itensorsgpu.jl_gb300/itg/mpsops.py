@@ -32,6 +32,7 @@ itg_factorize_trunc, itg_nrm2); torch only allocates.
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 
@@ -63,7 +64,7 @@ def _pc(A: ITensor, la, B: ITensor, lb, lc):
     code = {lab: k + 1 for k, lab in enumerate(dims)}
     dC = tuple(dims[lab] for lab in lc)
     if A.is_complex or B.is_complex:
-        out = T.empty_dev(int(np.prod(dC)) if dC else 1, True)
+        out = T.empty_dev(math.prod(dC), True)
         one, zero = (C.c_double * 2)(1.0, 0.0), (C.c_double * 2)(0.0, 0.0)
         T._h().call("itg_contract_z", T._dt(A), T._dt(B), one, T._ptr(A.store.data), len(la), i64arr(A.dims),
                     i32arr([code[x] for x in la]), T._ptr(B.store.data), len(lb), i64arr(B.dims),

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import itertools
+import math
 from dataclasses import dataclass
 
 import numpy as np
@@ -58,12 +59,19 @@ def _h():
     return _lib.handle(_state["device"])
 
 
+_devices = {}
+
+
 def _dev():
-    return torch.device("cuda", _state["device"])
+    d = _state["device"]
+    dev = _devices.get(d)
+    if dev is None:
+        dev = _devices[d] = torch.device("cuda", d)
+    return dev
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def empty_dev(n: int, cplx: bool = False):
@@ -85,7 +93,7 @@ def _to_complex_data(d):
     """Complex copy of real device data through itg_real_to_complex."""
     out = empty_dev(len(d), True)
     if len(d):
-        _h().call("itg_real_to_complex", C.c_int64(len(d)), _ptr(d), _ptr(out))
+        _h().call("itg_real_to_complex", len(d), _ptr(d), _ptr(out))
     return out
 
 
@@ -315,12 +323,12 @@ def randomCuITensor(*inds, seed: int | None = None) -> ITensor:
     s = next(_seed_counter) if seed is None else int(seed)
     if not cplx:
         t = torch.empty(max(n, 1), dtype=torch.float64, device=_dev())
-        _h().call("itg_random_normal", C.c_int64(n), C.c_uint64(s), C.c_uint64(0), _ptr(t))
+        _h().call("itg_random_normal", n, s, 0, _ptr(t))
         return ITensor(Dense(t[:n]), inds)
     t = torch.empty(max(n, 1), dtype=torch.complex128, device=_dev())
-    _h().call("itg_random_normal", C.c_int64(2 * n), C.c_uint64(s), C.c_uint64(0), _ptr(t))
+    _h().call("itg_random_normal", 2 * n, s, 0, _ptr(t))
     if n:
-        _h().call("itg_scal", C.c_int64(2 * n), C.c_double(0.5 ** 0.5), _ptr(t))
+        _h().call("itg_scal", 2 * n, C.c_double(0.5 ** 0.5), _ptr(t))
     return ITensor(Dense(t[:n]), inds)
 
 
@@ -385,11 +393,11 @@ def _scale(t: ITensor, x) -> ITensor:
         out = t.store.data.clone() if t.is_complex else _to_complex_data(t.store.data)
         if len(out):
             a = (C.c_double * 2)(complex(x).real, complex(x).imag)
-            _h().call("itg_zscal", C.c_int64(len(out)), a, _ptr(out))
+            _h().call("itg_zscal", len(out), a, _ptr(out))
         return ITensor(Dense(out), t.inds)
     out = t.store.data.clone()
     if len(out):
-        _h().call("itg_scal", C.c_int64(len(out)), C.c_double(float(x)), _ptr(out))
+        _h().call("itg_scal", len(out), C.c_double(float(x)), _ptr(out))
     st = Dense(out) if isinstance(t.store, Dense) else Diag(out, t.store.uniform)
     return ITensor(st, t.inds)
 
@@ -408,7 +416,7 @@ def dag(x):
     _require_cuda(x)
     out = torch.empty_like(x.store.data)
     if len(out):
-        _h().call("itg_conj", C.c_int64(len(out)), _ptr(x.store.data), _ptr(out))
+        _h().call("itg_conj", len(out), _ptr(x.store.data), _ptr(out))
     return ITensor(Dense(out), x.inds)
 
 
@@ -434,7 +442,7 @@ def permute(t: ITensor, *inds) -> ITensor:
     lab = _labels(t.inds)
     out = empty_dev(dim(inds), t.is_complex)
     if dim(inds) > 0:
-        _h().call("itg_permute", _dt(t), C.c_double(1.0), _ptr(t.store.data), len(t.inds),
+        _h().call("itg_permute", _dt(t), 1.0, _ptr(t.store.data), len(t.inds),
                   i64arr(t.dims), i32arr([lab[i] for i in t.inds]), _ptr(out),
                   i32arr([lab[i] for i in inds]))
     return ITensor(Dense(out), inds)
@@ -452,8 +460,8 @@ def _axpby(alpha: float, a: ITensor, beta: float, b: ITensor) -> ITensor:
     lab = _labels(b.inds)
     out = empty_dev(dim(b.inds), b.is_complex)
     if dim(b.inds) > 0:
-        _h().call("itg_axpby_permuted", _dt(b), C.c_double(alpha), _ptr(a.store.data), len(a.inds),
-                  i64arr(a.dims), i32arr([lab[i] for i in a.inds]), C.c_double(beta),
+        _h().call("itg_axpby_permuted", _dt(b), alpha, _ptr(a.store.data), len(a.inds),
+                  i64arr(a.dims), i32arr([lab[i] for i in a.inds]), beta,
                   _ptr(b.store.data), i32arr([lab[i] for i in b.inds]), _ptr(out))
     return ITensor(Dense(out), b.inds)
 
@@ -471,7 +479,7 @@ def norm(t: ITensor) -> float:
         t = ITensor(Dense(d), (Index(len(d)),))
     r = C.c_double()
     n = len(t.store.data) * (2 if t.is_complex else 1)
-    _h().call("itg_nrm2", C.c_int64(n), _ptr(t.store.data), C.byref(r))
+    _h().call("itg_nrm2", n, _ptr(t.store.data), C.byref(r))
     return r.value
 
 
@@ -500,34 +508,33 @@ def contract(A: ITensor, B: ITensor, precision: int | None = None, **kw) -> ITen
         from .mpsops import contract as _contract_chain
         return _contract_chain(A, B, **kw)
     _require_cuda(A, B)
-    common = [i for i in A.inds if i in B.inds]
-    out_inds = tuple([i for i in A.inds if i not in common] + [i for i in B.inds if i not in common])
+    # an index is its (id, prime level); mode labels in order of first appearance
+    ka = [(i.id, i.plev) for i in A.inds]
+    kb = [(i.id, i.plev) for i in B.inds]
+    sa, sb = set(ka), set(kb)
+    out_inds = tuple([i for i, k in zip(A.inds, ka) if k not in sb] + [i for i, k in zip(B.inds, kb) if k not in sa])
     prec = _state["precision"] if precision is None else precision
-    if A.isdiag() and B.isdiag():
-        return _diag_diag(A, B, common, out_inds)
     if A.isdiag() or B.isdiag():
+        if A.isdiag() and B.isdiag():
+            return _diag_diag(A, B, [i for i, k in zip(A.inds, ka) if k in sb], out_inds)
         D, T = (A, B) if A.isdiag() else (B, A)
         return _diag_dense(D, T, out_inds)
-    lab = _labels(A.inds, B.inds)
-    if A.is_complex or B.is_complex:
-        out = empty_dev(dim(out_inds), True)
-        if dim(out_inds) > 0:
+    lab = {k: n for n, k in enumerate(dict.fromkeys(ka + kb), 1)}
+    dA, dB, dC = A.dims, B.dims, tuple([i.dim for i in out_inds])
+    mA, mB = i32arr([lab[k] for k in ka]), i32arr([lab[k] for k in kb])
+    mC = i32arr([lab[k] for k in ka if k not in sb] + [lab[k] for k in kb if k not in sa])
+    n = math.prod(dC)
+    cplx = A.is_complex or B.is_complex
+    out = empty_dev(n, cplx)
+    if n > 0:
+        if cplx:
             one = (C.c_double * 2)(1.0, 0.0)
             zero = (C.c_double * 2)(0.0, 0.0)
-            _h().call("itg_contract_z", _dt(A), _dt(B), one,
-                      _ptr(A.store.data), len(A.inds), i64arr(A.dims), i32arr([lab[i] for i in A.inds]),
-                      _ptr(B.store.data), len(B.inds), i64arr(B.dims), i32arr([lab[i] for i in B.inds]),
-                      zero, _ptr(out), len(out_inds), i64arr([i.dim for i in out_inds]),
-                      i32arr([lab[i] for i in out_inds]), int(prec))
-        return ITensor(Dense(out), out_inds)
-    out = empty_dev(dim(out_inds))
-    if dim(out_inds) > 0:
-        _h().call("itg_contract", ITG_F64, C.c_double(1.0),
-                  _ptr(A.store.data), len(A.inds), i64arr(A.dims), i32arr([lab[i] for i in A.inds]),
-                  _ptr(B.store.data), len(B.inds), i64arr(B.dims), i32arr([lab[i] for i in B.inds]),
-                  C.c_double(0.0),
-                  _ptr(out), len(out_inds), i64arr([i.dim for i in out_inds]),
-                  i32arr([lab[i] for i in out_inds]), int(prec))
+            _h().call("itg_contract_z", _dt(A), _dt(B), one, _ptr(A.store.data), len(dA), i64arr(dA), mA,
+                      _ptr(B.store.data), len(dB), i64arr(dB), mB, zero, _ptr(out), len(dC), i64arr(dC), mC, int(prec))
+        else:
+            _h().call("itg_contract", ITG_F64, 1.0, _ptr(A.store.data), len(dA), i64arr(dA), mA, _ptr(B.store.data),
+                      len(dB), i64arr(dB), mB, 0.0, _ptr(out), len(dC), i64arr(dC), mC, int(prec))
     return ITensor(Dense(out), out_inds)
 
 
@@ -537,7 +544,7 @@ def _split_cplx(d):
     n = len(d)
     out = empty_dev(2 * n)
     if n:
-        _h().call("itg_permute", ITG_F64, C.c_double(1.0), _ptr(d), 2, i64arr([2, n]), i32arr([1, 2]), _ptr(out),
+        _h().call("itg_permute", ITG_F64, 1.0, _ptr(d), 2, i64arr([2, n]), i32arr([1, 2]), _ptr(out),
                   i32arr([2, 1]))
     return out[:n], out[n:]
 
@@ -548,7 +555,7 @@ def _join_cplx(re, im):
     buf = torch.cat([re, im]) if n else re
     out = empty_dev(n, True)
     if n:
-        _h().call("itg_permute", ITG_F64, C.c_double(1.0), _ptr(buf), 2, i64arr([n, 2]), i32arr([1, 2]), _ptr(out),
+        _h().call("itg_permute", ITG_F64, 1.0, _ptr(buf), 2, i64arr([n, 2]), i32arr([1, 2]), _ptr(out),
                   i32arr([2, 1]))
     return out
 
@@ -569,10 +576,10 @@ def _diag_dense(D: ITensor, T: ITensor, out_inds) -> ITensor:
     lab = _labels(D.inds, T.inds)
     out = empty_dev(dim(out_inds), T.is_complex)
     if dim(out_inds) > 0:
-        _h().call("itg_diag_contract", _dt(T), C.c_double(1.0), _ptr(D.store.data),
+        _h().call("itg_diag_contract", _dt(T), 1.0, _ptr(D.store.data),
                   int(D.store.uniform), len(D.inds), i64arr(D.dims), i32arr([lab[i] for i in D.inds]),
                   _ptr(T.store.data), len(T.inds), i64arr(T.dims), i32arr([lab[i] for i in T.inds]),
-                  C.c_double(0.0), _ptr(out), len(out_inds), i64arr([i.dim for i in out_inds]),
+                  0.0, _ptr(out), len(out_inds), i64arr([i.dim for i in out_inds]),
                   i32arr([lab[i] for i in out_inds]))
     return ITensor(Dense(out), out_inds)
 
@@ -610,13 +617,13 @@ def _diag_diag(A: ITensor, B: ITensor, common, out_inds) -> ITensor:
     dims_all = [i.dim for i in A.inds] + [i.dim for i in B.inds]
     n = min(lens) if lens else min(dims_all)
     out = empty_dev(max(n, 1))
-    _h().call("itg_diag_diag", C.c_int64(n), C.c_double(1.0), _ptr(A.store.data),
+    _h().call("itg_diag_diag", n, 1.0, _ptr(A.store.data),
               int(A.store.uniform), _ptr(B.store.data), int(B.store.uniform), _ptr(out))
     if len(out_inds) == 0:
         # full contraction of two diagonals: the sum of the products
         ones = torch.ones(max(n, 1), dtype=torch.float64, device=_dev())
         r = C.c_double()
-        _h().call("itg_dot", C.c_int64(n), _ptr(out), _ptr(ones), C.byref(r))
+        _h().call("itg_dot", n, _ptr(out), _ptr(ones), C.byref(r))
         return ITensor(Dense(torch.full((1,), r.value, dtype=torch.float64, device=_dev())), ())
     uni = A.store.uniform and B.store.uniform
     return ITensor(Diag(out[: (1 if uni else n)], uni), out_inds)
@@ -668,9 +675,9 @@ def svd(A: ITensor, *left_inds, **kw):
     dc = C.c_double()
     maxdim, mindim, cutoff, ab, rel, legacy = _trunc_args(m, n, kw)
     # complex: A ~ U S V^H (so U * S * dag(V) rebuilds A, test/test_cuitensor.jl:100-106)
-    _h().call("itg_svd_trunc_z" if cplx else "itg_svd_trunc", C.c_int64(m), C.c_int64(n), _ptr(Am.store.data),
-              C.c_int64(m),
-              C.c_int64(maxdim), C.c_int64(mindim), C.c_double(cutoff), ab, rel, legacy,
+    _h().call("itg_svd_trunc_z" if cplx else "itg_svd_trunc", m, n, _ptr(Am.store.data),
+              m,
+              maxdim, mindim, cutoff, ab, rel, legacy,
               _ptr(U), _ptr(S), _ptr(V), C.byref(k), C.byref(te), C.byref(dc))
     kk = int(k.value)
     u = Index(kk, kw.get("lefttags", "Link,u"))
@@ -728,8 +735,8 @@ def factorize(A: ITensor, *left_inds, ortho: str = "left", **kw):
     dc = C.c_double()
     maxdim, mindim, cutoff, ab, rel, legacy = _trunc_args(m, n, kw)
     prec = _precision_code(kw.get("precision", get_precision()))
-    _h().call("itg_factorize_trunc", C.c_int64(m), C.c_int64(n), _ptr(Am.store.data), C.c_int64(m),
-              C.c_int64(maxdim), C.c_int64(mindim), C.c_double(cutoff), ab, rel, legacy,
+    _h().call("itg_factorize_trunc", m, n, _ptr(Am.store.data), m,
+              maxdim, mindim, cutoff, ab, rel, legacy,
               0 if ortho == "left" else 1, int(kw.get("method", 0)), prec,
               _ptr(Lb), _ptr(S), _ptr(Cb), C.byref(k), C.byref(te), C.byref(dc))
     kk = int(k.value)
@@ -767,8 +774,8 @@ def eigen(A: ITensor, left_inds, right_inds, **kw):
     te = C.c_double()
     dc = C.c_double()
     maxdim, mindim, cutoff, ab, rel, legacy = _trunc_args(n, n, kw)
-    _h().call("itg_eigh_trunc_z" if cplx else "itg_eigh_trunc", C.c_int64(n), _ptr(Am.store.data), C.c_int64(n),
-              C.c_int64(maxdim), C.c_int64(mindim), C.c_double(cutoff), ab, rel, legacy,
+    _h().call("itg_eigh_trunc_z" if cplx else "itg_eigh_trunc", n, _ptr(Am.store.data), n,
+              maxdim, mindim, cutoff, ab, rel, legacy,
               _ptr(D), _ptr(U), C.byref(k), C.byref(te), C.byref(dc))
     kk = int(k.value)
     l = Index(kk, "Link,eigen,l")
@@ -791,7 +798,7 @@ def qr(A: ITensor, *left_inds):
     cplx = Am.is_complex
     Q = empty_dev(m * r, cplx)
     R = empty_dev(r * n, cplx)
-    _h().call("itg_qr_z" if cplx else "itg_qr", C.c_int64(m), C.c_int64(n), _ptr(Am.store.data), C.c_int64(m),
+    _h().call("itg_qr_z" if cplx else "itg_qr", m, n, _ptr(Am.store.data), m,
               _ptr(Q), _ptr(R))
     q = Index(r, "Link,qr")
     return ITensor(Dense(Q), (*left, q)), ITensor(Dense(R), (q, *right))
