@@ -655,6 +655,7 @@ __global__ void k_build_rt(const double* __restrict__ A, int64_t m, int n, const
 namespace itg {
 int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, double fro, double* ws, float* ws32,
                    int* flag);
+int64_t start32_ws_doubles(int64_t m, int64_t n);
 }
 
 namespace {
@@ -662,17 +663,20 @@ constexpr int JACOBI_MAX_SWEEPS = 60;
 constexpr int JACOBI_AUX_INTS = 8 + JACOBI_MAX_SWEEPS;
 constexpr int64_t ONECTA_MAX_N = 192;
 constexpr int64_t PRECOND_MIN_N = 24;
-constexpr int64_t START32_MIN_N = 192;  // FP64 Jacobi starts from the FP32 rotations above this (jacobi_run)
+// From this many columns the FP64 Jacobi starts from the FP32 rotations
+// (jacobi_start32): below, its products cost what the sweeps do (n = 16 random
+// 0.59 -> 0.55 ms, sigma = exp(-32 k / n) 0.90 -> 0.91 ms).
+constexpr int64_t START32_MIN_N = 16;
 // Below this many columns one CTA runs all sweeps in one launch (n = 10: 0.64
 // against 0.75 ms for the queued steps, n = 12: 0.87 against 0.82 ms).
 constexpr int64_t REG_MIN_N = 12;
 
 // Workspace of jacobi_run's FP32 start, 0 where it is not taken.
 bool start32(const itg_handle* h, int64_t m, int64_t n) {
-  return n > START32_MIN_N && h->jacobi_mode == 0 && m <= 2048;
+  return n >= START32_MIN_N && h->jacobi_mode == 0 && m <= 2048;
 }
 size_t start32_bytes(const itg_handle* h, int64_t m, int64_t n) {
-  return start32(h, m, n) ? itg_align256(sizeof(double) * (n * n + m * n)) + sizeof(float) * (m * n + n * n) : 0;
+  return start32(h, m, n) ? itg_align256(sizeof(double) * itg::start32_ws_doubles(m, n)) + sizeof(float) * (m * n + n * n) : 0;
 }
 
 // Runs Jacobi on W (m x n, m >= n) with V = I.  Returns ITG_ERR_NOTCONVERGED
@@ -709,7 +713,7 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   }
   if (start32(h, m, n) && std::isfinite(fro) && fro > 0.0)
     ITG_TRY(itg::jacobi_start32(h, W, m, n, V, fro, (double*)ws,
-                                (float*)(ws + itg_align256(sizeof(double) * (n * n + m * n))), flag_dev));
+                                (float*)(ws + itg_align256(sizeof(double) * itg::start32_ws_doubles(m, n))), flag_dev));
   if (h->jacobi_mode == 0 || h->jacobi_mode == 3) {
     const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, JACOBI_MAX_SWEEPS, flag_dev,
                                                sweeps_done, amin_conv);

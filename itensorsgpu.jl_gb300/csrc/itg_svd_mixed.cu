@@ -485,17 +485,89 @@ int ns_polish(itg_handle* h, double* L, int64_t rows, int64_t cols, double* ws, 
   return gemm(h, false, rows, cols, cols, 1.0, tmp, Q, 1.0, L, precision);
 }
 
-// Start of the FP64 Jacobi on W (m x n, m >= n, Frobenius norm fro): the FP32
-// Jacobi of the mixed method finds V to about 1e-6, two Newton-Schulz steps in
-// FP64 make it orthonormal to rounding and W <- W V, so that fewer FP64 sweeps
-// are left: on a symmetric matrix of n = 700 the eigendecomposition takes 46
-// instead of 99 ms, on a graded R^T of n = 2048 (whose small columns FP32 does
-// not resolve) the FP64 split 0.87 instead of 1.22 s.  Nothing of the result
-// rests on FP32: the FP64 sweeps go on to their own tolerance.
-// ws: n^2 + m n doubles, ws32: m n + n^2 floats.
+namespace {
+
+// Rotations that diagonalise G = W^T W to first order: K antisymmetric,
+// k_ij = g_ij / (g_jj - g_ii), for the pairs that are nearly orthogonal and
+// well separated (a pair inside a cluster, or of two columns of rounding noise,
+// is left to the Jacobi sweeps).
+__device__ __forceinline__ double rotation_generator(double gii, double gjj, double gij) {
+  const double d = gjj - gii;
+  const bool ok = fabs(d) > 1e-4 * fmax(gii, gjj) && gij * gij <= 1e-6 * gii * gjj && fabs(gij) <= 0.05 * fabs(d);
+  return ok ? gij / d : 0.0;
+}
+
+// Row j's sum of |k_ij|, and the diagonal of G.
+__global__ void __launch_bounds__(128)
+k_generator_rows(const double* __restrict__ G, int n, double* __restrict__ diag, double* __restrict__ rows) {
+  __shared__ double sh[4];
+  const int j = blockIdx.x;
+  const double gjj = G[(int64_t)j * (n + 1)];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 128)
+    if (i != j) s += fabs(rotation_generator(G[(int64_t)i * (n + 1)], gjj, G[i + (int64_t)j * n]));
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    diag[j] = gjj;
+    rows[j] = sh[0] + sh[1] + sh[2] + sh[3];
+  }
+}
+
+// K and I + K.  Rows with a large sum are left out (with their columns), so
+// that |K| <= 0.015 and I + K + K^2/2 is orthogonal to |K|^4/4 <= 1.3e-8: one
+// Newton-Schulz step then makes it so to rounding.
+__global__ void k_generator(const double* __restrict__ G, int n, const double* __restrict__ diag,
+                            const double* __restrict__ rows, double* __restrict__ K, double* __restrict__ M) {
+  const int64_t nn = (int64_t)n * n;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x) {
+    const int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
+    const int p = i < j ? i : j, q = i < j ? j : i;  // both triangles from the upper one
+    double k = 0.0;
+    if (i != j && rows[p] <= 0.015 && rows[q] <= 0.015) k = rotation_generator(diag[p], diag[q], G[p + (int64_t)q * n]);
+    if (i > j) k = -k;
+    K[t] = k;
+    M[t] = i == j ? 1.0 : k;
+  }
+}
+
+__global__ void k_copy_scaled(const double* __restrict__ x, int64_t n, double a, double* __restrict__ y) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    y[i] = a * x[i];
+}
+
+// P <- (3 I - P) / 2: X P is the Newton-Schulz step for P = X^T X
+__global__ void k_newton_schulz(double* P, int n) {
+  const int64_t nn = (int64_t)n * n;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x)
+    P[t] = (t % (n + 1) == 0 ? 1.5 : 0.0) - 0.5 * P[t];
+}
+
+}  // namespace
+
+// Start of the FP64 Jacobi on W (m x n, m >= n, Frobenius norm fro).  The FP32
+// Jacobi finds V to about 1e-6 (columns of every size: one-sided rotations keep
+// the accuracy of graded columns relative to their own norms); a Newton-Schulz
+// step makes it orthonormal.  Then twice: W <- A V (scaled), the remaining rotations to
+// first order from W^T W (k_generator), V <- V (I + K + K^2/2) and another
+// Newton-Schulz step.  The error falls quadratically, so that of the FP64 sweeps,
+// each bound by the FP64 pipes of a few SMs, only one is left where the spectrum
+// has no clusters (8 to 12 without this start, 3 without the two refinements);
+// the products are spread over the GPU.  Nothing of the result rests on FP32:
+// the FP64 sweeps go on to their own tolerance, and K is bounded so that V
+// stays orthonormal to rounding.
+// SVD of n x n, random / sigma = exp(-32 k / n): n = 32 1.16 / 1.17 -> 0.90 / 0.99
+// ms, n = 120 4.6 / 5.2 -> 2.7 / 2.9, n = 192 9.7 / 10.3 -> 4.3 / 4.6; n = 378
+// (FP32 start without the refinements before) 16.5 / 15.1 -> 14.4 / 10.9.
+// ws: start32_ws_doubles(m, n) doubles, ws32: m n + n^2 floats.
+int64_t start32_ws_doubles(int64_t m, int64_t n) { return 3 * n * n + m * n + 2 * n; }
+
 int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, double fro, double* ws, float* ws32,
                    int* flag) {
-  const double scale = std::ldexp(1.0, -std::ilogb(fro));
+  // a power of two: A's squares then stay in range, and scaling it is exact
+  const int ex = std::ilogb(fro);
+  const double scale = std::ldexp(1.0, ex < -1000 ? 1000 : -ex);
   float* W32 = ws32;
   float* V32 = ws32 + m * n;
   k_to_float<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m * n, scale, W32);
@@ -503,34 +575,46 @@ int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, do
   ITG_CHECK_LAUNCH(h);
   const double f = fro * scale;  // in [1, 2)
   int sweeps = 0;
-  const int st = itg::jacobi_blocked<float>(h, W32, m, (int)n, V32, 1e-5f, (float)(1e-14 * f * f), 30, flag, &sweeps);
+  // columns below 1e-15 of the norm are left alone (their squares leave FP32's
+  // range), those below 1e-7 do not keep the sweeps running
+  const int st = itg::jacobi_blocked<float>(h, W32, m, (int)n, V32, 1e-5f, (float)(1e-30 * f * f), 30, flag, &sweeps,
+                                            (float)(1e-14 * f * f));
   if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
-  k_to_double<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(V32, n * n, V);
-  ITG_CHECK_LAUNCH(h);
   double* P = ws;
-  double* T = ws + n * n;
-  const int gb = itg_blocks_for(n * n, 256, h->num_sms * 16);
-  // heuristic tiles: timing the variants of each new shape would cost more than the products
-  const bool tune = h->autotune;
-  h->autotune = false;
-  int gs = ITG_OK;
-  for (int it = 0; it < 2 && gs == ITG_OK; ++it) {
-    gs = gemm(h, true, n, n, n, 1.0, V, V, 0.0, P, ITG_PREC_FP64);
-    if (gs != ITG_OK) break;
-    k_half_identity_minus<<<gb, 256, 0, h->stream>>>(P, (int)n, P);
-    if (cudaMemcpyAsync(T, V, sizeof(double) * n * n, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess) {
-      gs = itg_fail(h, ITG_ERR_CUDA, "copy of the rotations failed");
-      break;
-    }
-    gs = gemm(h, false, n, n, n, 1.0, T, P, 1.0, V, ITG_PREC_FP64);
-  }
-  if (gs == ITG_OK && cudaMemcpyAsync(T, W, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess)
-    gs = itg_fail(h, ITG_ERR_CUDA, "copy of the columns failed");
-  if (gs == ITG_OK) gs = gemm(h, false, m, n, n, 1.0, T, V, 0.0, W, ITG_PREC_FP64);
-  h->autotune = tune;
-  ITG_TRY(gs);
+  double* M = P + n * n;
+  double* Y = M + n * n;
+  double* A = Y + n * n;
+  double* diag = A + m * n;
+  double* rows = diag + n;
+  k_to_double<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(V32, n * n, Y);
+  k_copy_scaled<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m * n, scale, A);
   ITG_CHECK_LAUNCH(h);
-  return ITG_OK;
+  // heuristic tiles: timing the variants of each new shape would cost more than the products
+  struct NoTune {
+    itg_handle* h;
+    bool was;
+    explicit NoTune(itg_handle* hh) : h(hh), was(hh->autotune) { h->autotune = false; }
+    ~NoTune() { h->autotune = was; }
+  } no_tune(h);
+  const int gb = itg_blocks_for(n * n, 256, h->num_sms * 16);
+  auto newton_schulz = [&](const double* X, double* Q, double* out) -> int {  // out = X (3 I - X^T X) / 2
+    ITG_TRY(gemm(h, true, n, n, n, 1.0, X, X, 0.0, Q, ITG_PREC_FP64));
+    k_newton_schulz<<<gb, 256, 0, h->stream>>>(Q, (int)n);
+    ITG_CHECK_LAUNCH(h);
+    return gemm(h, false, n, n, n, 1.0, X, Q, 0.0, out, ITG_PREC_FP64);
+  };
+  ITG_TRY(newton_schulz(Y, P, V));
+  for (int it = 0; it < 2; ++it) {
+    ITG_TRY(gemm(h, false, m, n, n, 1.0, A, V, 0.0, W, ITG_PREC_FP64));
+    ITG_TRY(gemm(h, true, n, n, m, 1.0, W, W, 0.0, P, ITG_PREC_FP64));
+    k_generator_rows<<<(int)n, 128, 0, h->stream>>>(P, (int)n, diag, rows);
+    k_generator<<<gb, 256, 0, h->stream>>>(P, (int)n, diag, rows, Y, M);
+    ITG_CHECK_LAUNCH(h);
+    ITG_TRY(gemm(h, false, n, n, n, 0.5, Y, Y, 1.0, M, ITG_PREC_FP64));
+    ITG_TRY(gemm(h, false, n, n, n, 1.0, V, M, 0.0, P, ITG_PREC_FP64));
+    ITG_TRY(newton_schulz(P, Y, V));
+  }
+  return gemm(h, false, m, n, n, 1.0 / scale, A, V, 0.0, W, ITG_PREC_FP64);
 }
 
 size_t svd_mixed_ws_doubles(int64_t mm, int64_t nn) {
