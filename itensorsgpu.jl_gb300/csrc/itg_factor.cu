@@ -618,8 +618,9 @@ k_house_step_plain(double* __restrict__ A, int64_t m, int j, double* __restrict_
 
 namespace itg {
 // Steps j0 .. j0 + count - 1 on columns up to jend, on the handle's stream.
-int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
-                double* tau, double* rdiag) {
+// after_kernel: the last thing put on the stream is a kernel.
+int house_panel(itg_handle* h, bool fast, bool after_kernel, double* A, int64_t m, int64_t j0, int64_t count,
+                int64_t jend, double* Vh, double* tau, double* rdiag) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -629,7 +630,7 @@ int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int6
     cfg.blockDim = dim3(fast ? HOUSE_THREADS : 256);
     cfg.stream = h->stream;
     cfg.attrs = &at;
-    cfg.numAttrs = j > j0 ? 1 : 0;  // the first step waits for everything before it
+    cfg.numAttrs = j > j0 || after_kernel ? 1 : 0;
     if (fast) ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step, A, m, (int)j, Vh, tau, rdiag));
     else ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step_plain, A, m, (int)j, Vh, tau, rdiag));
   }

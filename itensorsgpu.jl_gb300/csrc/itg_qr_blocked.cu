@@ -13,84 +13,122 @@
 #include "itg_internal.cuh"
 
 namespace itg {
-int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
-                double* tau, double* rdiag);
+int house_panel(itg_handle* h, bool fast, bool after_kernel, double* A, int64_t m, int64_t j0, int64_t count,
+                int64_t jend, double* Vh, double* tau, double* rdiag);
 }  // namespace itg
 
 namespace {
 
+// Every kernel here starts while its predecessor on the stream drains and waits
+// for its results itself.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// after_kernel: the last thing put on the stream is a kernel (not an event or a copy)
+template <class... P, class... A>
+int launch_after(itg_handle* h, bool after_kernel, dim3 grid, int threads, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = h->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = after_kernel ? 1 : 0;
+  ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
+  return ITG_OK;
+}
+
 // T (32 x 32, upper triangular) from the partial sums of Y = V^T V (column c
 // of chunk q at part[32 (q bw + c)]): LAPACK's larft,
 //   T(j,j) = tau_j, T(0:j, j) = -tau_j T(0:j, 0:j) Y(0:j, j),
-// with its sums formed one term a step for all elements at once (thread (i, j)
-// adds T(i,l) Y(l,j) as soon as column l is final: the order of the recurrence,
-// 32 steps instead of a chain of 500 FP64 instructions; 44 -> 12 us).
-__global__ void __launch_bounds__(1024)
+// with its sums formed one term a step for all elements at once (lane i of warp
+// j % 8 adds T(i,l) Y(l,j) as soon as column l is final: the order of the
+// recurrence, bw steps instead of a chain of 500 FP64 instructions).  Bound by
+// a step's latency (a product, a barrier, a sum of up to four columns a warp);
+// eight warps instead of 32 shorten its barrier (21 -> 14 us at bw = 32).
+__global__ void __launch_bounds__(256)
 k_larft(const double* __restrict__ part, int nchunk, const double* __restrict__ tau, int bw, double* __restrict__ T) {
-  constexpr int NB = QR_NB;
+  constexpr int NB = QR_NB, NW = 8, CW = NB / NW;
   __shared__ double Y[NB][NB + 1], col[2][NB];  // Y[column][row]; column l of T
-  const int i = threadIdx.x % NB, j = threadIdx.x / NB;
-  double y = 0.0;
-  if (i < j && j < bw)
-    for (int q = 0; q < nchunk; ++q) y += part[((int64_t)q * bw + j) * NB + i];
-  Y[j][i] = y;
-  const double tj = j < bw ? tau[j] : 0.0;
-  double s = 0.0, t = 0.0;
-  __syncthreads();
-  for (int l = 0; l < NB; ++l) {
-    if (j == l) {
-      t = i < l ? -tj * s : (i == l ? tj : 0.0);
-      col[l & 1][i] = t;
-    }
-    __syncthreads();
-    if (j > l && i <= l) s = fma(col[l & 1][i], Y[j][l], s);
+  grid_wait();
+  const int i = threadIdx.x % NB, w = threadIdx.x / NB;
+  double tj[CW], s[CW], t[CW];
+#pragma unroll
+  for (int c = 0; c < CW; ++c) {
+    const int j = w + NW * c;
+    tj[c] = j < bw ? tau[j] : 0.0;
+    s[c] = t[c] = 0.0;
+    double y = 0.0;
+    if (i < j && j < bw)
+      for (int q = 0; q < nchunk; ++q) y += part[((int64_t)q * bw + j) * NB + i];
+    Y[j][i] = y;
   }
-  T[j * NB + i] = t;
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < CW; ++c) {
+    const int end = bw < NW * (c + 1) ? bw : NW * (c + 1);
+    for (int l = NW * c; l < end; ++l) {
+      if (w == l % NW) {
+        t[c] = i < l ? -tj[c] * s[c] : (i == l ? tj[c] : 0.0);
+        col[l & 1][i] = t[c];
+      }
+      __syncthreads();
+      if (i <= l) {
+        const double x = col[l & 1][i];
+#pragma unroll
+        for (int d = c; d < CW; ++d)
+          if (w + NW * d > l) s[d] = fma(x, Y[w + NW * d][l], s[d]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CW; ++c) T[(w + NW * c) * NB + i] = t[c];
 }
 
 // Partial sums of V_p^T B for the panel's reflectors V_p (columns jb..jb+bw of
 // Vh, rows jb..m) and N columns of B (ld ldb, rows jb..m): bw <= 32 rows of
 // dot products of length K = m - jb.  The product is too thin for the tiled
 // GEMM (it would run N / 64 CTAs), so the K range is split over gridDim.y
-// chunks whose partial results are summed in chunk order by the consumer.
-constexpr int SK_TILE_K = 64;
+// chunks whose partial results are summed in chunk order by the consumer, and
+// the 32 rows over gridDim.z: FP64 runs at 2 FMAs a clock and SM whatever the
+// tile, so a tile is one element a thread (8 rows by 32 columns, a warp a row).
+// With 32 rows a block (four elements a thread) a panel's 32 columns at K = 378
+// took 18.7 us on 6 SMs; now 7 on 24, the same sums.
+constexpr int SK_TILE_K = 64, SK_ROWS = 8;
 constexpr int QR_PART_CHUNKS = 16;  // K chunks of the thin products (partials: 16 x 32 x N)
 __global__ void __launch_bounds__(256)
 k_skinny_partial(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const double* __restrict__ B,
                  int64_t ldb, int64_t b0, int64_t N, int64_t kchunk, double* __restrict__ part) {
-  __shared__ double vs[32][SK_TILE_K + 1];
+  __shared__ double vs[SK_ROWS][SK_TILE_K];
   __shared__ double bs[32][SK_TILE_K + 1];
-  const int t = threadIdx.x;
+  grid_wait();
+  const int t = threadIdx.x, r = t / 32, c = t % 32, r0 = blockIdx.z * SK_ROWS;
   const int64_t c0 = (int64_t)blockIdx.x * 32;
   const int64_t K = m - jb;
   const int64_t k_lo = (int64_t)blockIdx.y * kchunk;
   const int64_t k_hi = k_lo + kchunk < K ? k_lo + kchunk : K;
-  const int r = t / 8, cq = (t % 8) * 4;  // each thread: row r, columns cq..cq+3
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  double acc = 0.0;
   for (int64_t k0 = k_lo; k0 < k_hi; k0 += SK_TILE_K) {
+#pragma unroll
+    for (int i = t; i < SK_ROWS * SK_TILE_K; i += 256) {
+      const int col = i / SK_TILE_K, kk = i % SK_TILE_K;
+      vs[col][kk] = (k0 + kk < k_hi && r0 + col < bw) ? Vh[(jb + r0 + col) * m + jb + k0 + kk] : 0.0;
+    }
+#pragma unroll
     for (int i = t; i < 32 * SK_TILE_K; i += 256) {
       const int col = i / SK_TILE_K, kk = i % SK_TILE_K;
-      const int64_t k = k0 + kk;
-      const bool kin = k < k_hi;
-      vs[col][kk] = (kin && col < bw) ? Vh[(jb + col) * m + jb + k] : 0.0;
-      const int64_t c = c0 + col;
-      bs[col][kk] = (kin && c < N) ? B[(b0 + c) * ldb + jb + k] : 0.0;
+      bs[col][kk] = (k0 + kk < k_hi && c0 + col < N) ? B[(b0 + c0 + col) * ldb + jb + k0 + kk] : 0.0;
     }
     __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < SK_TILE_K; ++kk) {
-      const double v = vs[r][kk];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = fma(v, bs[cq + q][kk], acc[q]);
-    }
+#pragma unroll 16
+    for (int kk = 0; kk < SK_TILE_K; ++kk) acc = fma(vs[r][kk], bs[c][kk], acc);
     __syncthreads();
   }
-  double* P = part + (int64_t)blockIdx.y * 32 * N;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int64_t c = c0 + cq + q;
-    if (c < N) P[r + 32 * c] = acc[q];
-  }
+  if (c0 + c < N) part[((int64_t)blockIdx.y * N + c0 + c) * 32 + r0 + r] = acc;
 }
 
 // Z2 (32 x N) = op(T) Z with Z the sum of the partial results in chunk order,
@@ -104,6 +142,7 @@ k_skinny_t(const double* __restrict__ part, int nchunk, int bw, int64_t N, const
   __shared__ double z[8][NB], Ts[NB][NB + 1];
   const int t = threadIdx.x, r = t % NB, cl = t / NB;
   const int64_t c = (int64_t)blockIdx.x * 8 + cl;
+  grid_wait();
   for (int i = t; i < NB * NB; i += 256) Ts[i / NB][i % NB] = T[i];  // [column][row]
   double s = 0.0;
   if (c < N && r < bw)
@@ -120,53 +159,57 @@ k_skinny_t(const double* __restrict__ part, int nchunk, int bw, int64_t N, const
   Z2[c * NB + r] = r < bw ? a : 0.0;
 }
 
-// C(jb:m, c0 : c0 + N) -= V_p Z2 (C of leading dimension m).  32 x 16 tiles of
-// four elements a thread: like every FP64 product here bound by the FP64 pipe
-// whatever its tile, so the tile is small to fill the SMs when N is one panel.
+// C(jb:m, c0 : c0 + N) -= V_p Z2 (C of leading dimension m).  Like every FP64
+// product here bound by the FP64 pipe whatever its tile: 32 x 16 tiles of four
+// elements a thread, or 16 x 8 of one (HALF) when those would leave SMs idle.
+// One panel's columns at m = 378: 9.7 -> 7 us.
+template <bool HALF>
 __global__ void __launch_bounds__(128)
 k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const double* __restrict__ Z2, int64_t N,
             double* __restrict__ C, int64_t c0) {
-  constexpr int NB = QR_NB;
-  __shared__ double vs[NB][33], zs[16][NB + 1];
+  constexpr int NB = QR_NB, TM = HALF ? 16 : 32, TN = HALF ? 8 : 16, U = HALF ? 1 : 2;
+  __shared__ double vs[NB][TM + 1], zs[TN][NB + 1];
+  grid_wait();
   const int t = threadIdx.x;
-  const int64_t r0 = jb + (int64_t)blockIdx.x * 32, n0 = (int64_t)blockIdx.y * 16;
-  for (int i = t; i < 32 * NB; i += 128) {
-    const int k = i / 32, r = i % 32;
+  const int64_t r0 = jb + (int64_t)blockIdx.x * TM, n0 = (int64_t)blockIdx.y * TN;
+#pragma unroll
+  for (int i = t; i < TM * NB; i += 128) {
+    const int k = i / TM, r = i % TM;
     vs[k][r] = (k < bw && r0 + r < m) ? Vh[(jb + k) * m + r0 + r] : 0.0;
   }
-  for (int i = t; i < 16 * NB; i += 128) {
+#pragma unroll
+  for (int i = t; i < TN * NB; i += 128) {
     const int c = i / NB, k = i % NB;
     zs[c][k] = n0 + c < N ? Z2[(n0 + c) * NB + k] : 0.0;
   }
   const int tr = t % 16, tc = t / 16;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, old[2][2];
+  double acc[U][U], old[U][U];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < U; ++a)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < U; ++b) {
       const int64_t r = r0 + tr + 16 * a, c = n0 + tc + 8 * b;
       old[a][b] = (r < m && c < N) ? C[(c0 + c) * m + r] : 0.0;
+      acc[a][b] = 0.0;
     }
   __syncthreads();
 #pragma unroll 8
-  for (int k = 0; k < NB; ++k) {
-    const double v0 = vs[k][tr], v1 = vs[k][tr + 16], z0 = zs[tc][k], z1 = zs[tc + 8][k];
-    acc[0][0] = fma(v0, z0, acc[0][0]);
-    acc[0][1] = fma(v0, z1, acc[0][1]);
-    acc[1][0] = fma(v1, z0, acc[1][0]);
-    acc[1][1] = fma(v1, z1, acc[1][1]);
-  }
+  for (int k = 0; k < NB; ++k)
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < U; ++a)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
+      for (int b = 0; b < U; ++b) acc[a][b] = fma(vs[k][tr + 16 * a], zs[tc + 8 * b][k], acc[a][b]);
+#pragma unroll
+  for (int a = 0; a < U; ++a)
+#pragma unroll
+    for (int b = 0; b < U; ++b) {
       const int64_t r = r0 + tr + 16 * a, c = n0 + tc + 8 * b;
       if (r < m && c < N) C[(c0 + c) * m + r] = old[a][b] - acc[a][b];
     }
 }
 
 // Partial sums of V_p^T B into part; nchunk: how many.
-int skinny_vt_b(itg_handle* h, const double* Vh, int64_t m, int64_t jb, int bw, const double* B, int64_t ldb,
+int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, int64_t jb, int bw, const double* B, int64_t ldb,
                 int64_t b0, int64_t N, double* part, int64_t part_doubles, int* nchunk_out) {
   const int64_t K = m - jb;
   const int64_t ntile = (N + 31) / 32;
@@ -177,9 +220,8 @@ int skinny_vt_b(itg_handle* h, const double* Vh, int64_t m, int64_t jb, int bw, 
   if (nchunk < 1) return itg_fail(h, ITG_ERR_INVALID, "skinny product: partial buffer too small");
   const int64_t kchunk = ((K + nchunk - 1) / nchunk + SK_TILE_K - 1) / SK_TILE_K * SK_TILE_K;
   nchunk = (K + kchunk - 1) / kchunk;
-  k_skinny_partial<<<dim3((unsigned)ntile, (unsigned)nchunk), 256, 0, h->stream>>>(Vh, m, jb, bw, B, ldb, b0, N,
-                                                                                   kchunk, part);
-  ITG_CHECK_LAUNCH(h);
+  const dim3 grid((unsigned)ntile, (unsigned)nchunk, 32 / SK_ROWS);
+  ITG_TRY(launch_after(h, after_kernel, grid, 256, k_skinny_partial, Vh, m, jb, bw, B, ldb, b0, N, kchunk, part));
   *nchunk_out = (int)nchunk;
   return ITG_OK;
 }
@@ -187,19 +229,20 @@ int skinny_vt_b(itg_handle* h, const double* Vh, int64_t m, int64_t jb, int bw, 
 // C(jb:m, c0 : c0 + N) -= V_p (op(T_p) (V_p^T C(jb:m, c0 : c0 + N))) on the
 // handle's current stream; Z2 holds 32 N doubles.
 template <bool TRANS>
-int wy_apply(itg_handle* h, double* C, int64_t m, int64_t jb, int bw, const double* Vh, const double* Tp, int64_t c0,
+int wy_apply(itg_handle* h, bool after_kernel, double* C, int64_t m, int64_t jb, int bw, const double* Vh, const double* Tp, int64_t c0,
              int64_t N, double* Z2, double* part, int64_t part_doubles) {
   if (N <= 0) return ITG_OK;
   int nchunk = 0;
-  ITG_TRY(skinny_vt_b(h, Vh, m, jb, bw, C, m, c0, N, part, part_doubles, &nchunk));
-  k_skinny_t<TRANS><<<(unsigned)((N + 7) / 8), 256, 0, h->stream>>>(part, nchunk, bw, N, Tp, Z2);
-  const int64_t gx = (m - jb + 31) / 32, gy = (N + 15) / 16;
+  ITG_TRY(skinny_vt_b(h, after_kernel, Vh, m, jb, bw, C, m, c0, N, part, part_doubles, &nchunk));
+  ITG_TRY(launch_after(h, true, dim3((unsigned)((N + 7) / 8)), 256, k_skinny_t<TRANS>, part, nchunk, bw, N, Tp, Z2));
+  const bool half = ((m - jb + 31) / 32) * ((N + 15) / 16) < h->num_sms;
+  const int tm = half ? 16 : 32, tn = half ? 8 : 16;
+  const int64_t gx = (m - jb + tm - 1) / tm, gy = (N + tn - 1) / tn;
   for (int64_t y = 0; y < gy; y += 65535) {  // the grid's y limit
-    const int64_t ny = gy - y < 65535 ? gy - y : 65535;
-    k_wy_update<<<dim3((unsigned)gx, (unsigned)ny), 128, 0, h->stream>>>(
-        Vh, m, jb, bw, Z2 + y * 16 * QR_NB, N - y * 16, C, c0 + y * 16);
+    const dim3 grid((unsigned)gx, (unsigned)(gy - y < 65535 ? gy - y : 65535));
+    ITG_TRY(launch_after(h, true, grid, 128, half ? k_wy_update<true> : k_wy_update<false>, Vh, m, jb, bw,
+                         Z2 + y * tn * QR_NB, N - y * tn, C, c0 + y * tn));
   }
-  ITG_CHECK_LAUNCH(h);
   return ITG_OK;
 }
 
@@ -260,7 +303,7 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
     ITG_CUDA(h, cudaStreamWaitEvent(h->stream, h->qr_ev_done, 0));
     if (nref > 0) {
       const int64_t w = nref < NB ? nref : NB;
-      ITG_TRY(house_panel(h, fast, W, m, 0, w, w, Vh, tau, rd));
+      ITG_TRY(house_panel(h, fast, false, W, m, 0, w, w, Vh, tau, rd));
     }
   }
   for (int64_t jb = 0, panel = 0; jb < nref; jb += NB, ++panel) {
@@ -273,24 +316,23 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
     {
       OnStream on(h, h->qr_stream);
       int nchunk = 0;
-      ITG_TRY(skinny_vt_b(h, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
-      k_larft<<<1, QR_NB * QR_NB, 0, h->stream>>>(partp, nchunk, tau + jb, (int)bw, Tp);
-      ITG_CHECK_LAUNCH(h);
+      ITG_TRY(skinny_vt_b(h, true, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
+      ITG_TRY(launch_after(h, true, dim3(1), 256, k_larft, partp, nchunk, tau + jb, (int)bw, Tp));
       if (nt <= 0) continue;
       // V_p and T_p are final: the handle's stream may update the rest
       ITG_CUDA(h, cudaEventRecord(h->qr_ev_ready, h->stream));
       // panel p + 1's columns got panel p - 1's update on the handle's stream
       if (panel > 0) ITG_CUDA(h, cudaStreamWaitEvent(h->stream, h->qr_ev_done, 0));
-      ITG_TRY(wy_apply<true>(h, W, m, jb, (int)bw, Vh, Tp, jn, nnext, Zp, partp, part_doubles));
+      ITG_TRY(wy_apply<true>(h, false, W, m, jb, (int)bw, Vh, Tp, jn, nnext, Zp, partp, part_doubles));
     }
     if (nrest > 0) {
       ITG_CUDA(h, cudaStreamWaitEvent(main_stream, h->qr_ev_ready, 0));
-      ITG_TRY(wy_apply<true>(h, W, m, jb, (int)bw, Vh, Tp, jn + nnext, nrest, Zu, partu, part_doubles));
+      ITG_TRY(wy_apply<true>(h, false, W, m, jb, (int)bw, Vh, Tp, jn + nnext, nrest, Zu, partu, part_doubles));
     }
     ITG_CUDA(h, cudaEventRecord(h->qr_ev_done, main_stream));
     if (nnext > 0) {
       OnStream on(h, h->qr_stream);
-      ITG_TRY(house_panel(h, fast, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
+      ITG_TRY(house_panel(h, fast, true, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
     }
   }
   // the handle's stream continues after the last panel's work
@@ -310,7 +352,7 @@ int q_apply_blocked(itg_handle* h, double* Y, int64_t m, int64_t n, int64_t ncol
   for (int64_t panel = npanel - 1; panel >= 0; --panel) {
     const int64_t jb = panel * NB;
     const int64_t bw = (n - jb < NB) ? n - jb : NB;
-    ITG_TRY(wy_apply<false>(h, Y, m, jb, (int)bw, Vh, Tbuf + panel * NB * NB, 0, ncols, Z2, part,
+    ITG_TRY(wy_apply<false>(h, panel != npanel - 1, Y, m, jb, (int)bw, Vh, Tbuf + panel * NB * NB, 0, ncols, Z2, part,
                             QR_PART_CHUNKS * 32 * ncols));
   }
   return ITG_OK;
