@@ -696,14 +696,38 @@ int choose_f64(itg_handle* h, const ContractPlan& p, const double* A, const doub
   return ITG_OK;
 }
 
+// Split-precision variant where nothing was timed, by the time of a work item
+// (64 of K of one digit product): 0.235 us in a 128-wide tile (0.28 when all SMs
+// stay busy), 0.40 in a 256-wide one, whose int64 sums move through L2 at the
+// end of each level (40 us a tile); stream-K shares whole levels, so it cannot
+// beat the largest one, and costs about 35 us for its shared accumulators.
+// n = 384: 64 to 129 us by variant; 1536 x 384 x 1920 145 to 308; 4096 x 1024 x
+// 5120 853 to 983; the choice is within 10 % of the best on 16 shapes, N <= 128
+// or not.
+int heuristic_split(itg_handle* h, int64_t M, int64_t N, int64_t K) {
+  const double nkb = (double)((K + 63) / 64), items = 21.0 * nkb, top = 6.0 * nkb, sms = (double)h->num_sms;
+  const double t1 = (double)((M + 127) / 128) * ((N + 127) / 128), t2 = (double)((M + 127) / 128) * ((N + 255) / 256);
+  auto shared = [&](double tiles, double item, double flush) {
+    const double share = tiles / sms * items;
+    return (share > top ? share : top) * item + flush * (tiles / sms) + 35.0;
+  };
+  const double c[4] = {std::ceil(t1 / sms) * items * 0.235, shared(t1, t1 > sms ? 0.28 : 0.235, 0.0),
+                       std::ceil(t2 / sms) * (items * 0.40 + 40.0), shared(t2, 0.40, 40.0)};
+  const int v[4] = {ITG_SPLIT_BN_128, ITG_SPLIT_BN_128 | ITG_SPLIT_STREAMK, ITG_SPLIT_BN_256,
+                    ITG_SPLIT_BN_256 | ITG_SPLIT_STREAMK};
+  int best = 0;
+  for (int i = 1; i < (N <= 128 ? 2 : 4); ++i)
+    if (c[i] < c[best]) best = i;
+  return v[best];
+}
+
 int choose_split(itg_handle* h, const ContractPlan& p, const double* A, const double* B, double alpha, int& bn) {
   if (p.split_bn) {
     bn = p.split_bn;
     return ITG_OK;
   }
-  // heuristic: 128-wide tiles for narrow outputs, else 256-wide
   const bool narrow = p.N <= 128;
-  bn = narrow ? ITG_SPLIT_BN_128 : ITG_SPLIT_BN_256;
+  bn = heuristic_split(h, p.M, p.N, p.K);
   if (p.key.empty() || narrow) {
     if (!p.key.empty()) p.split_bn = bn;
     return ITG_OK;
@@ -1031,7 +1055,7 @@ extern "C" int itg_autotune_query(itg_handle* h, int rankA, const int64_t* dimsA
   else *tile = tune::heuristic_tile(h, p.M, p.N, p.K);
   if (p.split_bn) *split_bn = p.split_bn;
   else if (tune::lookup("split|" + p.key, v)) *split_bn = v;
-  else *split_bn = p.N <= 128 ? ITG_SPLIT_BN_128 : ITG_SPLIT_BN_256;
+  else *split_bn = tune::heuristic_split(h, p.M, p.N, p.K);
   return ITG_OK;
 }
 

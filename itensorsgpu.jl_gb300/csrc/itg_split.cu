@@ -29,9 +29,9 @@
 //
 // Kernel roles (10 warps per CTA; a CTA computes one 128 x BN output tile,
 // or, persistent, a sequence of tiles and parts of tiles, see Part):
-//   warp 0    TMA producer: A/B slice tiles (64 bf16 of K per stage, 128B
-//             swizzle) into a 4-stage shared-memory ring, mbarrier complete_tx
-//   warp 1    TMEM allocator and single-thread tcgen05.mma issuer
+//   warp 0    TMA producer: A/B slice tiles (items of 64 bf16 of K, 128B
+//             swizzle) into a shared-memory ring, mbarrier complete_tx
+//   warp 1    TMEM allocator and tcgen05.mma issuer (one elected lane issues)
 //   warps 2-9 TMEM drain / epilogue: warp w reads TMEM lanes 32*(w%4)..+31 and
 //             owns half of the tile's columns
 // Every mbarrier wait is bounded (%globaltimer; the handle's wait limit,
@@ -93,19 +93,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // role of the CTA raised the flag first.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err,
                                           volatile int* abort_flag, uint64_t wait_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer();
+  uint64_t t0 = 0;
   for (uint32_t it = 0;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63) == 63) {
       if (*abort_flag) return false;
-      if (globaltimer() - t0 > wait_ns) {
+      const uint64_t now = globaltimer();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > wait_ns) {
         atomicExch(err, ITG_ERR_TIMEOUT);
         *abort_flag = 1;
         return false;
       }
     }
   }
+}
+// The same by a whole warp, with one outcome for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, volatile int* abort_flag,
+                                               uint64_t wait_ns) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, abort_flag, wait_ns));
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
 }
 // Bounded wait that ignores the abort flag: on the way out, for this CTA's own
 // TMA copies and MMAs still in flight (they complete by themselves; the bound
@@ -226,69 +238,44 @@ __host__ __device__ __forceinline__ int digit_log2(int p) { return p == 0 ? 8 : 
 
 // Exact-accumulation schedule shared by every role.  Items are
 // (level L, pair p, k-block kb) in level-major order; a group is a run of
-// items of one level whose summed |product| bound stays <= 2^24.
+// items of one level whose summed |product| bound stays <= 2^24.  It is walked
+// in runs of k-blocks of one pair inside one group: the two roles that issue an
+// item are one thread each, and stepping the schedule item by item cost them
+// 640 clocks of an item's 900 (its four products take 512).
+constexpr int GROUP_LOG2 = 24, BK_LOG2 = 6;
+static_assert(BK == 1 << BK_LOG2, "");
 struct Sched {
   int S, nkb;
-  // iteration state
-  int L, p, kb;
-  int group;     // group index of the current item
-  int64_t used;  // bound used in the current group (log-domain sums as integers)
-  bool first_in_group;
-  __host__ __device__ void begin(int S_, int nkb_) {
+  int L, p, kb;  // next item
+  int used;      // bound used in the current group
+  bool first;    // the next item opens a group
+  __host__ __device__ void begin(int S_, int nkb_, int L0) {
     S = S_;
     nkb = nkb_;
-    L = 0;
-    p = 0;
-    kb = 0;
-    group = 0;
-    used = 0;
-    first_in_group = true;
-    used = cost();
-  }
-  // Jump to the first item of level L0 (a group always starts there).
-  __host__ __device__ void seek(int L0) {
     L = L0;
-    p = 0;
-    kb = 0;
-    first_in_group = true;
-    used = L < S ? cost() : 0;
+    p = kb = used = 0;
+    first = true;
   }
-  __host__ __device__ int q() const { return L - p; }
-  __host__ __device__ int64_t cost() const {
-    return (int64_t)BK << (digit_log2(p) + digit_log2(L - p));
-  }
-  __host__ __device__ bool valid() const { return L < S; }
-  // Advance; reports whether the item just finished closed its group.
-  __host__ __device__ bool advance() {
-    int nL = L, np = p, nkb2 = kb + 1;
-    if (nkb2 == nkb) {
-      nkb2 = 0;
-      np = p + 1;
-      if (np > L) {
-        np = 0;
-        nL = L + 1;
+  __host__ __device__ int cost_log2() const { return BK_LOG2 + digit_log2(p) + digit_log2(L - p); }
+  // Takes the next run: n items of pair (p, L - p) from k-block kb on.
+  // Reports whether it ends its group.
+  __host__ __device__ bool take(int& n) {
+    const int c = cost_log2(), room = ((1 << GROUP_LOG2) - used) >> c;
+    n = nkb - kb < room ? nkb - kb : room;
+    used += n << c;
+    kb += n;
+    bool closes = false;
+    if (kb == nkb) {
+      kb = 0;
+      if (++p > L) {
+        p = 0;
+        ++L;
+        closes = true;
       }
     }
-    bool closes;
-    if (nL >= S) {
-      closes = true;
-    } else if (nL != L) {
-      closes = true;
-    } else {
-      int64_t c = (int64_t)BK << (digit_log2(np) + digit_log2(nL - np));
-      closes = used + c > ((int64_t)1 << 24);
-    }
-    L = nL;
-    p = np;
-    kb = nkb2;
-    if (closes) {
-      group++;
-      used = 0;
-      first_in_group = true;
-    } else {
-      first_in_group = false;
-    }
-    if (L < S) used += cost();
+    closes = closes || ((1 << GROUP_LOG2) - used) >> cost_log2() == 0;
+    first = closes;
+    if (closes) used = 0;
     return closes;
   }
 };
@@ -400,14 +387,16 @@ __device__ __forceinline__ double i64_to_double_scaled(long long v, int exp2) {
 // Tile variants: BN = 256 keeps the int64 accumulators in global memory
 // (two 256-column FP32 TMEM buffers fill the TMEM); BN = 128 keeps them in
 // TMEM columns 256..511 (low / high words), so a drain never leaves the SM,
-// and runs a 6-stage operand ring.
+// and runs a ring of three stages of two items.
 template <int BN>
 struct Smem {
   static constexpr bool TACC = BN == 128;
-  static constexpr int NSTAGE = TACC ? 6 : STAGES;
+  static constexpr int SUB = TACC ? 2 : 1;  // items a stage holds
+  static constexpr int NSTAGE = TACC ? 3 : STAGES;
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int ITEM_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGE_BYTES = SUB * ITEM_BYTES;
   static constexpr int TOTAL = 1024 /*align slack*/ + NSTAGE * STAGE_BYTES + 256;
 };
 
@@ -438,6 +427,16 @@ __device__ __forceinline__ void load_acc16(uint32_t lane_base, const long long* 
 // accumulator into the tile's shared one with 64-bit integer atomics (exact,
 // so the result does not depend on their order), then counts itself in; the
 // last one to arrive converts.  Nobody waits for anybody else.
+//
+// What bounds it: per item of four products, first the issuing warp, not the
+// copies (without any loads the time was the same): stepping the schedule, its
+// operands moved to uniform registers inside a one-lane branch and a fence took
+// 900 clocks where the products take 512 (BN = 256) or 256.  Runs of k-blocks
+// (Sched), warp-wide loops with one elected lane and two items a stage
+// (BN = 128) brought an item from 0.49 to 0.39 us (256) and 0.23 (128), the two
+// products of a chi = 1024 matvec from 0.92 + 0.83 to 0.77 + 0.65 ms.  Now the
+// operands' reads from shared memory bound BN = 128 (8 KB a product of 64
+// clocks), the products and the flushes of the int64 sums BN = 256.
 template <int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
@@ -446,6 +445,7 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int NST = Smem<BN>::NSTAGE;
   constexpr bool TACC = Smem<BN>::TACC;
+  constexpr int SUB = Smem<BN>::SUB;
   uint8_t* stage_mem = base;
   uint64_t* bars = (uint64_t*)(base + NST * Smem<BN>::STAGE_BYTES);
   uint64_t* full = bars;                 // [NST]
@@ -496,85 +496,108 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      int it = 0;
-      bool ok = true;
-      int ct, L0, Le;
-      for (int si = 0; ok && part.seg(gcl, si, tb, lb, te, le, ct, L0, Le); ++si) {
-        const int m_grp = ct / args.tiles_n;
-        const int n_tile = ct - m_grp * args.tiles_n;
-        const int m0 = m_grp * BM, n0 = n_tile * BN;
-        Sched sc;
-        sc.begin(args.S, args.nkb);
-        sc.seek(L0);
-        while (sc.valid() && sc.L < Le) {
-          if (*abort_flag) {
+    // The whole warp walks the schedule and one lane issues (as below): inside
+    // a branch for one lane every operand of a copy or product would have to be
+    // moved to the uniform registers again.
+    const bool leader = elect_one();
+    int it = 0, s = 0;
+    uint32_t ph = 1;  // parity of the stage's last release (none before the first round)
+    bool ok = true;
+    int ct, L0, Le;
+    for (int si = 0; ok && part.seg(gcl, si, tb, lb, te, le, ct, L0, Le); ++si) {
+      const int m_grp = ct / args.tiles_n;
+      const int n_tile = ct - m_grp * args.tiles_n;
+      const int m0 = m_grp * BM, n0 = n_tile * BN;
+      Sched sc;
+      sc.begin(args.S, args.nkb, L0);
+      while (ok && sc.L < Le) {
+        int x = sc.kb * BK;
+        const int ya = sc.p * args.Mpad + m0, yb = (sc.L - sc.p) * args.Npad + n0;
+        int n;
+        sc.take(n);
+        for (; n > 0; n -= SUB) {
+          if (it >= NST && !mbar_wait_warp(&empty[s], ph, args.err, abort_flag, args.wait_ns)) {
             ok = false;
             break;
           }
-          const int s = it % NST;
-          if (it >= NST) {
-            if (!mbar_wait(&empty[s], ((it / NST) - 1) & 1, args.err, abort_flag, args.wait_ns)) {
-              ok = false;
-              break;
+          uint8_t* sa = stage_mem + s * Smem<BN>::STAGE_BYTES;
+          if (leader) {
+            const int c = n < SUB ? n : SUB;
+            mbar_arrive_expect_tx(&full[s], c * Smem<BN>::ITEM_BYTES);
+#pragma unroll
+            for (int j = 0; j < SUB; ++j) {
+              if (j == c) break;
+              tma_load_2d(sa, &mapA, x + j * BK, ya, &full[s]);
+              tma_load_2d(sa + Smem<BN>::A_BYTES, &mapB, x + j * BK, yb, &full[s]);
+              sa += Smem<BN>::ITEM_BYTES;
             }
           }
-          uint8_t* sa = stage_mem + s * Smem<BN>::STAGE_BYTES;
-          uint8_t* sb = sa + Smem<BN>::A_BYTES;
-          mbar_arrive_expect_tx(&full[s], Smem<BN>::STAGE_BYTES);
-          tma_load_2d(sa, &mapA, sc.kb * BK, sc.p * args.Mpad + m0, &full[s]);
-          tma_load_2d(sb, &mapB, sc.kb * BK, sc.q() * args.Npad + n0, &full[s]);
-          sc.advance();
+          x += SUB * BK;
           ++it;
+          if (++s == NST) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
-      // make sure no copy is still landing in shared memory when we leave
-      for (int j = std::max(0, it - NST); j < it; ++j) mbar_drain(&full[j % NST], (j / NST) & 1, args.wait_ns);
     }
+    // make sure no copy is still landing in shared memory when we leave
+    for (int j = std::max(0, it - NST); j < it; ++j) mbar_drain(&full[j % NST], (j / NST) & 1, args.wait_ns);
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(BM, BN);
-      int it = 0, lg = 0;  // items and groups issued by this CTA
-      bool ok = true;
-      int ct, L0, Le;
-      for (int si = 0; ok && part.seg(gcl, si, tb, lb, te, le, ct, L0, Le); ++si) {
-        Sched sc;
-        sc.begin(args.S, args.nkb);
-        sc.seek(L0);
-        while (sc.valid() && sc.L < Le) {
-          const int b = lg & 1;
-          const bool first = sc.first_in_group;
-          if (first && lg >= 2) {
-            ok = mbar_wait(&acc_empty[b], ((lg >> 1) - 1) & 1, args.err, abort_flag, args.wait_ns);
-            tc_fence_after();
-            if (!ok) break;
-          }
-          const int s = it % NST;
-          ok = mbar_wait(&full[s], (it / NST) & 1, args.err, abort_flag, args.wait_ns);
-          if (!ok) break;
+    const bool leader = elect_one();
+    constexpr uint32_t idesc = idesc_bf16(BM, BN);
+    const uint64_t desc0 = sdesc_sw128(smem_u32(stage_mem));
+    int s = 0, lg = 0;  // stage; groups issued by this CTA
+    uint32_t ph = 0;
+    bool ok = true;
+    int ct, L0, Le;
+    for (int si = 0; ok && part.seg(gcl, si, tb, lb, te, le, ct, L0, Le); ++si) {
+      Sched sc;
+      sc.begin(args.S, args.nkb, L0);
+      while (ok && sc.L < Le) {
+        const int b = lg & 1;
+        uint32_t accum = sc.first ? 0u : 1u;
+        if (sc.first && lg >= 2) {
+          ok = mbar_wait_warp(&acc_empty[b], ((lg >> 1) - 1) & 1, args.err, abort_flag, args.wait_ns);
           tc_fence_after();
-          const uint32_t sa = smem_u32(stage_mem + s * Smem<BN>::STAGE_BYTES);
-          const uint32_t sb = sa + Smem<BN>::A_BYTES;
-          const uint64_t ad = sdesc_sw128(sa), bd = sdesc_sw128(sb);
-          const uint32_t tmem_d = tmem_base + (uint32_t)(b * BN);
+          if (!ok) break;
+        }
+        const uint32_t tmem_d = tmem_base + (uint32_t)(b * BN);
+        int n;
+        const bool closes = sc.take(n);
+        for (; n > 0; n -= SUB) {
+          ok = mbar_wait_warp(&full[s], ph, args.err, abort_flag, args.wait_ns);
+          if (!ok) break;
+          const uint64_t stage = desc0 + (uint64_t)(s * (Smem<BN>::STAGE_BYTES >> 4));
+          if (leader) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint32_t accum = (first && kk == 0) ? 0u : 1u;
-            tc_mma_bf16(tmem_d, ad + (uint64_t)(2 * kk), bd + (uint64_t)(2 * kk), idesc, accum);
+            for (int j = 0; j < SUB; ++j) {
+              if (j == n) break;
+              const uint64_t ad = stage + (uint64_t)(j * (Smem<BN>::ITEM_BYTES >> 4));
+              const uint64_t bd = ad + (uint64_t)(Smem<BN>::A_BYTES >> 4);
+              tc_mma_bf16(tmem_d, ad, bd, idesc, j == 0 ? accum : 1u);
+#pragma unroll
+              for (int kk = 1; kk < BK / 16; ++kk)
+                tc_mma_bf16(tmem_d, ad + (uint64_t)(2 * kk), bd + (uint64_t)(2 * kk), idesc, 1u);
+            }
+            tc_commit(&empty[s]);
           }
-          tc_commit(&empty[s]);
-          if (sc.advance()) {
-            tc_commit(&acc_full[b]);
-            ++lg;
+          accum = 1u;
+          if (++s == NST) {
+            s = 0;
+            ph ^= 1u;
           }
-          ++it;
+        }
+        if (closes && ok) {
+          if (leader) tc_commit(&acc_full[b]);
+          ++lg;
         }
       }
-      // all MMAs issued by this thread complete before TMEM is released
-      tc_commit(done_bar);
-      mbar_drain(done_bar, 0, args.wait_ns);
     }
+    // all MMAs issued by this thread complete before TMEM is released
+    if (leader) tc_commit(done_bar);
+    mbar_drain(done_bar, 0, args.wait_ns);
   } else {
     // ------------------------------------------------------ drain/epilogue
     // Each thread owns one row and NCOL columns.  A group's FP32 values are
@@ -603,13 +626,12 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
       int nsum = 0;
       bool have_acc = false, complete = false;
       Sched sc;
-      sc.begin(args.S, args.nkb);
-      sc.seek(L0);
-      while (sc.valid() && sc.L < Le) {
+      sc.begin(args.S, args.nkb, L0);
+      while (sc.L < Le) {
         const int L = sc.L;
-        while (!sc.advance()) {
+        for (int n; !sc.take(n);) {
         }
-        const bool seg_last = !sc.valid() || sc.L >= Le;
+        const bool seg_last = sc.L >= Le;
         const bool flush = seg_last || sc.L != L || nsum + 1 == 127;
         const int b = lg & 1;
         // every lane polls; the outcome is made warp-uniform because the TMEM
@@ -1483,10 +1505,9 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
 }  // namespace itg
 
 // bn: tcgen05 tile variant: 128 or 256 columns, optionally | ITG_SPLIT_STREAMK
-// (persistent CTAs sharing the work evenly); 0: 128 when N <= 128, else 256.
+// (persistent CTAs sharing the work evenly).
 int itg_split_gemm(itg_handle* h, const ContractPlan& p, const double* A, const double* B, double* C,
                    double alpha, double beta, int bn) {
-  if (bn == 0) bn = p.N <= 128 ? 128 : 256;
   const bool sk = (bn & ITG_SPLIT_STREAMK) != 0;
   bn &= ~ITG_SPLIT_STREAMK;
   if (bn == 128) return split::run<128>(h, p, A, B, C, alpha, beta, sk);
