@@ -54,29 +54,41 @@ __global__ void k_weff(const double* __restrict__ W1, const double* __restrict__
 }
 
 // T3[r + R*j] = sum_c T1[r + R*c] * Weff[c + nc*j]   (R = chiL*chiR rows)
-__global__ void __launch_bounds__(256)
+// FP64-bound: 64 rows by 4 columns a block, so that a small R still reaches many
+// SMs (256 rows by all columns: 9.5 us on 3 SMs at chi = 24, now 4.5; T1's
+// re-reads are cheap next to the FMAs, nj / 4 of them to 2 nj nc flops).
+constexpr int MID_R = 64, MID_J = 4;
+__global__ void __launch_bounds__(MID_R)
 k_heff_mid(const double* __restrict__ T1, const double* __restrict__ Weff, double* __restrict__ T3,
            int64_t R, int nc, int nj) {
-  extern __shared__ double wsh[];
-  for (int i = threadIdx.x; i < nc * nj; i += blockDim.x) wsh[i] = Weff[i];
+  extern __shared__ double wsh[];  // MID_J columns of Weff
+  const int j0 = blockIdx.x * MID_J;
+  const int jn = nj - j0 < MID_J ? nj - j0 : MID_J;
+  for (int i = threadIdx.x; i < nc * jn; i += MID_R) wsh[i] = Weff[(int64_t)j0 * nc + i];
   __syncthreads();
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < R;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    for (int j0 = 0; j0 < nj; j0 += 8) {
-      double acc[8];
+  for (int64_t r = (int64_t)blockIdx.y * MID_R + threadIdx.x; r < R; r += (int64_t)gridDim.y * MID_R) {
+    double acc[MID_J];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = 0.0;
-      for (int c = 0; c < nc; ++c) {
-        double x = T1[r + R * c];
+    for (int q = 0; q < MID_J; ++q) acc[q] = 0.0;
+#pragma unroll 5
+    for (int c = 0; c < nc; ++c) {
+      const double x = T1[r + R * c];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (j0 + q < nj) acc[q] = fma(x, wsh[c + nc * (j0 + q)], acc[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (j0 + q < nj) T3[r + R * (j0 + q)] = acc[q];
+      for (int q = 0; q < MID_J; ++q)
+        if (q < jn) acc[q] = fma(x, wsh[c + nc * q], acc[q]);
     }
+#pragma unroll
+    for (int q = 0; q < MID_J; ++q)
+      if (q < jn) T3[r + R * (j0 + q)] = acc[q];
   }
+}
+
+int launch_heff_mid(itg_handle* h, const double* T1, const double* Weff, double* T3, int64_t R, int nc, int nj) {
+  const int64_t gy = (R + MID_R - 1) / MID_R;
+  k_heff_mid<<<dim3((unsigned)((nj + MID_J - 1) / MID_J), (unsigned)(gy < 65535 ? gy : 65535)), MID_R,
+               sizeof(double) * nc * (nj < MID_J ? nj : MID_J), h->stream>>>(T1, Weff, T3, R, nc, nj);
+  ITG_CHECK_LAUNCH(h);
+  return ITG_OK;
 }
 
 // diag(H_eff)[a', s1', s2', b'] = sum_{w,y} L[a',w,a'] Wd[w,s1',s2',y] R[b',y,b']
@@ -190,9 +202,7 @@ int heff_apply(itg_handle* h, const HeffDims& D, const double* L, const double* 
   if (precision == ITG_PREC_SPLIT) mid = itg::heff_mid_split(h, Rrows, nc, nj, w.T1, w.Weff, w.T3);
   if (mid == ITG_ERR_UNSUPPORTED) {
     ProfScope prof(h, ITG_KERNEL_HEFF_MID);
-    k_heff_mid<<<itg_blocks_for(Rrows, 256, h->num_sms * 8), 256, sizeof(double) * nc * nj, h->stream>>>(
-        w.T1, w.Weff, w.T3, Rrows, nc, nj);
-    ITG_CHECK_LAUNCH(h);
+    ITG_TRY(launch_heff_mid(h, w.T1, w.Weff, w.T3, Rrows, nc, nj));
   } else {
     ITG_TRY(mid);
   }
@@ -359,6 +369,56 @@ __device__ __forceinline__ double dv_block_sum(double v, double* sh) {
   return v;
 }
 
+// NV sums over the block at once; thread 8 c of the block gets the c-th (the
+// others 0 or part of it).  Each is the same tree as dv_block_sum's (lanes 16,
+// 8, ... 1 apart, then warps 4, 2, 1 apart), so the same bits, but a warp halves
+// the number of values it carries along with the distance: nine sums take 16
+// FP64 additions a warp instead of 45 (each holds a quarter of the SM for 64
+// clocks) and one barrier instead of 18.  Nine sums over n = 579072 (k_dv_gram<3>)
+// 36 -> 23 us, over n = 2300 17 -> 7 us.
+template <int NV>
+__device__ __forceinline__ double dv_block_sums(const double (&in)[NV], double (*sh)[DV_THREADS / 32 + 1]) {
+  constexpr int N2 = NV <= 1 ? 1 : (NV <= 2 ? 2 : (NV <= 4 ? 4 : (NV <= 8 ? 8 : 16)));
+  static_assert(NV <= 16 && DV_THREADS == 256, "");
+  double v[N2];
+#pragma unroll
+  for (int c = 0; c < N2; ++c) v[c] = c < NV ? in[c] : 0.0;
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int m = N2; m > 1; m >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int c = 0; c < m / 2; ++c) {
+      const double send = up ? v[c] : v[c + m / 2], keep = up ? v[c + m / 2] : v[c];
+      v[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    o >>= 1;
+  }
+  constexpr int LANES = 32 / N2;  // lanes that hold one value's sum
+#pragma unroll
+  for (int d = LANES / 2; d > 0; d >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+  if (lane % LANES == 0) sh[lane / LANES][threadIdx.x >> 5] = v[0];
+  __syncthreads();
+  double s = threadIdx.x < 8 * N2 ? sh[threadIdx.x / 8][threadIdx.x % 8] : 0.0;
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  __syncthreads();  // sh may be used again
+  return s;
+}
+
+// The same for partial sums part[c np + ...] of np blocks.
+template <int NV>
+__device__ __forceinline__ double dv_reduce_all(const double* part, int np, double (*sh)[DV_THREADS / 32 + 1]) {
+  double s[NV];
+#pragma unroll
+  for (int c = 0; c < NV; ++c) s[c] = 0.0;
+  for (int i = threadIdx.x; i < np; i += DV_THREADS)
+#pragma unroll
+    for (int c = 0; c < NV; ++c) s[c] += __ldcg(part + (int64_t)c * np + i);
+  return dv_block_sums(s, sh);
+}
+
 // True in every thread of the block that arrives last of `total` (the counter
 // wraps to zero for the next use); its reads of the others' partials are
 // ordered after their writes.
@@ -406,15 +466,13 @@ template <int K>
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_gram(int64_t n, const double* __restrict__ V, const double* __restrict__ AV, double* part, unsigned* counter,
           double* G_host) {
-  __shared__ double sh[32];
+  __shared__ double sh[16][DV_THREADS / 32 + 1];
   const int nb = gridDim.x, b = blockIdx.x;
   const int64_t chunk = (n + nb - 1) / nb;
   const int64_t lo = (int64_t)b * chunk, hi = lo + chunk < n ? lo + chunk : n;
-  double s[K][K];
+  double s[K * K];
 #pragma unroll
-  for (int i = 0; i < K; ++i)
-#pragma unroll
-    for (int j = 0; j < K; ++j) s[i][j] = 0.0;
+  for (int c = 0; c < K * K; ++c) s[c] = 0.0;
 #pragma unroll 2
   for (int64_t e = lo + threadIdx.x; e < hi; e += blockDim.x) {
     double v[K], a[K];
@@ -424,22 +482,17 @@ k_dv_gram(int64_t n, const double* __restrict__ V, const double* __restrict__ AV
       a[i] = AV[e + i * n];
     }
 #pragma unroll
-    for (int i = 0; i < K; ++i)
+    for (int j = 0; j < K; ++j)
 #pragma unroll
-      for (int j = 0; j < K; ++j) s[i][j] = fma(v[i], a[j], s[i][j]);
+      for (int i = 0; i < K; ++i) s[j * K + i] = fma(v[i], a[j], s[j * K + i]);
   }
-#pragma unroll
-  for (int j = 0; j < K; ++j)
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const double t = dv_block_sum(s[i][j], sh);
-      if (threadIdx.x == 0) part[(int64_t)(j * K + i) * nb + b] = t;
-    }
+  const int c = threadIdx.x / 8;
+  const bool mine = threadIdx.x % 8 == 0 && c < K * K;
+  double t = dv_block_sums(s, sh);
+  if (mine) part[(int64_t)c * nb + b] = t;
   if (!dv_last(counter, nb)) return;
-  for (int c = 0; c < K * K; ++c) {
-    const double t = dv_reduce(part + (int64_t)c * nb, nb, sh);
-    if (threadIdx.x == 0) G_host[c] = t;
-  }
+  t = dv_reduce_all<K * K>(part, nb, sh);
+  if (mine) G_host[c] = t;
 }
 
 struct DvCoef {
@@ -454,7 +507,7 @@ __global__ void __launch_bounds__(DV_THREADS)
 k_dv_ritz(int64_t n, int k, const double* V, const double* __restrict__ AV, DvCoef c, double theta, double guard,
           const double* __restrict__ dg, double* __restrict__ X, double* __restrict__ HX,
           double* __restrict__ Rv, double* t, double* part, unsigned* counter, double* sc, double* sc_host) {
-  __shared__ double sh[32];
+  __shared__ double sh[4][DV_THREADS / 32 + 1];
   const int kk = K ? K : k;
   double sr = 0.0, sx = 0.0, st = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -477,20 +530,14 @@ k_dv_ritz(int64_t n, int k, const double* V, const double* __restrict__ AV, DvCo
       st = fma(v, v, st);
     }
   }
-  sr = dv_block_sum(sr, sh);
-  sx = dv_block_sum(sx, sh);
-  st = dv_block_sum(st, sh);
-  const int nb = gridDim.x;
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = sr;
-    part[nb + blockIdx.x] = sx;
-    part[2 * nb + blockIdx.x] = st;
-  }
+  const int nb = gridDim.x, q = threadIdx.x / 8;
+  const bool mine = threadIdx.x % 8 == 0 && q < 3;
+  const double sums[3] = {sr, sx, st};
+  double s = dv_block_sums(sums, sh);
+  if (mine) part[q * nb + blockIdx.x] = s;
   if (!dv_last(counter, nb)) return;
-  for (int q = 0; q < 3; ++q) {
-    const double s = dv_reduce(part + q * nb, nb, sh);
-    if (threadIdx.x == 0) sc[q] = sc_host[q] = sqrt(s);
-  }
+  s = dv_reduce_all<3>(part, nb, sh);
+  if (mine) sc[q] = sc_host[q] = sqrt(s);
 }
 
 // c[j] = -V[:, j] . t, chunks as itg_gemv_t cuts them
@@ -498,7 +545,7 @@ template <int K>
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_proj(int64_t n, const double* __restrict__ V, const double* __restrict__ t, double* part, unsigned* counter,
           double* c) {
-  __shared__ double sh[32];
+  __shared__ double sh[4][DV_THREADS / 32 + 1];
   const int nb = gridDim.x, b = blockIdx.x;
   const int64_t chunk = (n + nb - 1) / nb;
   const int64_t lo = (int64_t)b * chunk, hi = lo + chunk < n ? lo + chunk : n;
@@ -511,16 +558,13 @@ k_dv_proj(int64_t n, const double* __restrict__ V, const double* __restrict__ t,
 #pragma unroll
     for (int j = 0; j < K; ++j) s[j] = fma(V[e + j * n], y, s[j]);
   }
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    const double v = dv_block_sum(s[j], sh);
-    if (threadIdx.x == 0) part[(int64_t)j * nb + b] = v;
-  }
+  const int j = threadIdx.x / 8;
+  const bool mine = threadIdx.x % 8 == 0 && j < K;
+  double v = dv_block_sums(s, sh);
+  if (mine) part[(int64_t)j * nb + b] = v;
   if (!dv_last(counter, nb)) return;
-  for (int j = 0; j < K; ++j) {
-    const double v = dv_reduce(part + (int64_t)j * nb, nb, sh);
-    if (threadIdx.x == 0) c[j] = -1.0 * v;
-  }
+  v = dv_reduce_all<K>(part, nb, sh);
+  if (mine) c[j] = -1.0 * v;
 }
 
 // t += V c; with out: |t| (device and host copies)
@@ -568,10 +612,7 @@ int heff_form_weff(itg_handle* h, int64_t d, int64_t wL, int64_t wM, int64_t wR,
 }
 int heff_mid(itg_handle* h, int64_t rows, int nc, int nj, const double* T1, const double* Weff,
              double* T3) {
-  k_heff_mid<<<itg_blocks_for(rows, 256, h->num_sms * 8), 256, sizeof(double) * nc * nj, h->stream>>>(
-      T1, Weff, T3, rows, nc, nj);
-  ITG_CHECK_LAUNCH(h);
-  return ITG_OK;
+  return launch_heff_mid(h, T1, Weff, T3, rows, nc, nj);
 }
 }  // namespace itg
 
