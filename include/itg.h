@@ -540,6 +540,13 @@ ITG_API int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m, co
                                   double* const* U, double* const* S, double* const* V,
                                   int64_t* k, double* truncerr);
 
+/* The kept factors of itg_svd_trunc_batched as chain tensors, sigma absorbed
+ * into the left (to_left) or the right one: A_i (m_i x k_i) = U_i [S_i] and
+ * B_i (k_i x n_i) = [S_i] V_i^T, U_i m_i and V_i n_i rows. */
+ITG_API int itg_svd_absorb_batched(itg_handle* h, int count, const int64_t* m, const int64_t* n, const int64_t* k,
+                                   const double* const* U, const double* const* S, const double* const* V,
+                                   int to_left, double* const* A, double* const* B);
+
 /* itg_davidson_heff2 for `count` instances sharing d and the MPO bond
  * dimensions (the same bond of equally long chains), each with its own chiL,
  * chiR and tensors.  The H_eff chain runs as grouped launches over all

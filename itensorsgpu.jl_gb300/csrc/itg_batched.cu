@@ -4,6 +4,7 @@
 // per chain step for all instances) and whose vector operations are segmented
 // kernels over all instances' vectors at once.
 #include "itg_internal.cuh"
+#include "itg_truncate.cuh"
 
 #include <cmath>
 #include <algorithm>
@@ -29,7 +30,6 @@ struct SvdJob {
   double* sig;       // nn
   double* P;         // nn
   int* order;        // nn
-  double* out3;      // keep, truncerr, docut
   int m, n, mm, nn, tr;
   int64_t maxdim;
 };
@@ -44,9 +44,22 @@ __device__ __forceinline__ double wsum(double v) {
   return v;
 }
 
-// One CTA per instance: copy, all Jacobi sweeps, norms, ranking.
+struct TruncRule {
+  int64_t mindim;
+  double cutoff;
+  int absoluteCutoff, doRelCutoff, legacy;
+};
+
+// One CTA per instance: copy, all Jacobi sweeps, norms, ranking, truncation
+// (out: keep, truncerr, docut of each, in host memory) and the sorted factors.
+// Bound by FP64 instructions (64 clocks of a quarter of the SM each): a step
+// forms its pairs' sums a warp a pair, the rotations one thread a pair (square
+// roots and divisions, about 70 instructions, once for 32 pairs instead of once
+// a pair), then applies them a warp a pair.  16 instances of 10 sites, maxdim 16:
+// 427 -> 310 us a bond, gather and truncation included.
+constexpr int SVDB_MAX_N = 512;
 __global__ void __launch_bounds__(1024)
-k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __restrict__ sweeps_out) {
+k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, TruncRule rule, double* out) {
   SvdJob J = jobs[blockIdx.x];
   const int mm = J.mm, nn = J.nn;
   // copy (transpose for wide inputs) and identity
@@ -57,20 +70,28 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __
   for (int t = threadIdx.x; t < nn * nn; t += blockDim.x) J.Vw[t] = (t % (nn + 1) == 0) ? 1.0 : 0.0;
   __syncthreads();
   __shared__ int rotated;
+  __shared__ double sums[3][SVDB_MAX_N / 2], rot[2][SVDB_MAX_N / 2];  // |p|^2, |q|^2, p.q; c and s of each pair
   const int np = nn + (nn & 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const double tol = tol_eps * sqrt((double)mm);
+  // columns of pair pi, p < q; false for the absent column of an odd nn
+  auto columns = [&](int pi, int step, int& p, int& q) {
+    p = rr_p(pi, step, np);
+    q = rr_p(np - 1 - pi, step, np);
+    if (p >= nn || q >= nn) return false;
+    if (p > q) { const int t = p; p = q; q = t; }
+    return true;
+  };
   int sweep = 0;
   for (; sweep < max_sweeps && nn > 1; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
     for (int step = 0; step < np - 1; ++step) {
+      int p, q;
       for (int pi = warp; pi < np / 2; pi += nw) {
-        int p = rr_p(pi, step, np), q = rr_p(np - 1 - pi, step, np);
-        if (p >= nn || q >= nn) continue;
-        if (p > q) { const int t = p; p = q; q = t; }
-        double* wp = J.W + (int64_t)p * mm;
-        double* wq = J.W + (int64_t)q * mm;
+        if (!columns(pi, step, p, q)) continue;
+        const double* wp = J.W + (int64_t)p * mm;
+        const double* wq = J.W + (int64_t)q * mm;
         double a = 0, b = 0, g = 0;
         for (int i = lane; i < mm; i += 32) {
           const double x = wp[i], y = wq[i];
@@ -78,11 +99,40 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __
           b = fma(y, y, b);
           g = fma(x, y, g);
         }
-        a = wsum(a); b = wsum(b); g = wsum(g);
-        if (a == 0.0 || b == 0.0 || fabs(g) <= tol * sqrt(a) * sqrt(b)) continue;
-        const double zeta = (b - a) / (2.0 * g);
-        const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
+        // the three sums in one tree: lanes 0-7 end with a, 8-15 with b, 16-23 with g
+        const bool hi = lane & 16, mid = lane & 8;
+        const double u = (hi ? g : a) + __shfl_xor_sync(0xffffffffu, hi ? a : g, 16);
+        const double v = (hi ? 0.0 : b) + __shfl_xor_sync(0xffffffffu, hi ? b : 0.0, 16);
+        double w = (mid ? v : u) + __shfl_xor_sync(0xffffffffu, mid ? u : v, 8);
+        for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if ((lane & 7) == 0 && lane < 24) sums[lane >> 3][pi] = w;
+      }
+      __syncthreads();
+      for (int pi = threadIdx.x; pi < np / 2; pi += blockDim.x) {
+        if (!columns(pi, step, p, q)) continue;
+        const double a = sums[0][pi], b = sums[1][pi], g = sums[2][pi];
+        double c = 1.0, s = 0.0;
+        if (!(a == 0.0 || b == 0.0 || fabs(g) <= tol * sqrt(a) * sqrt(b))) {
+          const double zeta = (b - a) / (2.0 * g);
+          const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+          c = 1.0 / sqrt(1.0 + t * t);
+          s = c * t;
+          // converged once no pair above the rounding floor of the dot product
+          // (4 tol, as in the single-matrix kernels) needed a rotation
+          if (fabs(g) > 4.0 * tol * sqrt(a) * sqrt(b)) rotated = 1;
+        } else {
+          c = 2.0;  // no rotation
+        }
+        rot[0][pi] = c;
+        rot[1][pi] = s;
+      }
+      __syncthreads();
+      for (int pi = warp; pi < np / 2; pi += nw) {
+        if (!columns(pi, step, p, q)) continue;
+        const double c = rot[0][pi], s = rot[1][pi];
+        if (c == 2.0) continue;
+        double* wp = J.W + (int64_t)p * mm;
+        double* wq = J.W + (int64_t)q * mm;
         for (int i = lane; i < mm; i += 32) {
           const double x = wp[i], y = wq[i];
           wp[i] = c * x - s * y;
@@ -95,9 +145,6 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __
           vp[i] = c * x - s * y;
           vq[i] = s * x + c * y;
         }
-        // converged once no pair above the rounding floor of the dot product
-        // (4 tol, as in the single-matrix kernels) needed a rotation
-        if (lane == 0 && fabs(g) > 4.0 * tol * sqrt(a) * sqrt(b)) rotated = 1;
       }
       __syncthreads();
     }
@@ -105,7 +152,6 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __
     __syncthreads();
     if (!r) break;
   }
-  if (threadIdx.x == 0) sweeps_out[blockIdx.x] = sweep;
   // column norms of W, unit-norm V columns
   for (int j = warp; j < nn; j += nw) {
     double s = 0.0, v2 = 0.0;
@@ -129,32 +175,49 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, int* __
     J.S[r] = v;
     J.P[r] = v * v;
   }
-}
-
-// Gather the sorted factors: U[:, r] = W[:, order[r]] / sigma (rows mm), V[:, r] = Vw[:, order[r]].
-__global__ void k_svd_batched_gather(SvdJob* __restrict__ jobs) {
-  const SvdJob J = jobs[blockIdx.x];
-  const int mm = J.mm, nn = J.nn;
+  __syncthreads();
+  // the last warp's first lane truncates while the others gather the sorted
+  // factors: U[:, r] = W[:, order[r]] / sigma (rows mm), V[:, r] = Vw[:, order[r]]
+  if (warp == nw - 1) {
+    if (lane == 0)
+      truncate_spectrum(J.P, nn, J.maxdim, rule.mindim, rule.cutoff, rule.absoluteCutoff, rule.doRelCutoff,
+                        rule.legacy, out + 3 * blockIdx.x);
+    return;
+  }
+  const int nt = blockDim.x - 32;
   double* Ud = J.tr ? J.V : J.U;  // rows mm
   double* Vd = J.tr ? J.U : J.V;  // rows nn
-  for (int t = threadIdx.x; t < mm * nn; t += blockDim.x) {
+  for (int t = threadIdx.x; t < mm * nn; t += nt) {
     const int r = t / mm, i = t - r * mm;
     const int j = J.order[r];
     const double sv = J.sig[j];
     Ud[t] = sv > 0.0 ? J.W[i + (int64_t)j * mm] / sv : 0.0;
   }
-  for (int t = threadIdx.x; t < nn * nn; t += blockDim.x) {
+  for (int t = threadIdx.x; t < nn * nn; t += nt) {
     const int r = t / nn, i = t - r * nn;
     Vd[t] = J.Vw[i + (int64_t)J.order[r] * nn];
   }
 }
 
-}  // namespace
-
-namespace itg {
-int truncate_dev(itg_handle* h, const double* P, int64_t n, int64_t maxdim, int64_t mindim,
-                 double cutoff, int absoluteCutoff, int doRelCutoff, int legacy_gpu, double* out3);
+// The factors kept of each instance in the layout of the chain, sigma absorbed
+// to the left or to the right: A (m x k) = U [S], B (k x n) = [S] V^T.
+struct AbsorbJob {
+  const double *U, *S, *V;
+  double *A, *B;
+  int64_t m, n, k;
+};
+__global__ void __launch_bounds__(256)
+k_svd_absorb(const AbsorbJob* __restrict__ jobs, int to_left) {
+  const AbsorbJob J = jobs[blockIdx.y];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t t = t0; t < J.m * J.k; t += stride) J.A[t] = to_left ? J.S[t / J.m] * J.U[t] : J.U[t];
+  for (int64_t t = t0; t < J.n * J.k; t += stride) {
+    const int64_t j = t / J.k, r = t - j * J.k;
+    J.B[t] = to_left ? J.V[j + r * J.n] : J.S[r] * J.V[j + r * J.n];
+  }
 }
+
+}  // namespace
 
 extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m, const int64_t* n,
                                      const double* const* A, const int64_t* maxdim, int64_t mindim,
@@ -167,11 +230,11 @@ extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m,
   std::vector<SvdJob> jobs(count);
   size_t off = 0;
   auto take = [&](size_t b) { size_t o = off; off += itg_align256(b); return o; };
-  std::vector<size_t> oW(count), oV(count), oSig(count), oP(count), oOrd(count), oOut(count);
+  std::vector<size_t> oW(count), oV(count), oSig(count), oP(count), oOrd(count);
   for (int i = 0; i < count; ++i) {
     if (m[i] <= 0 || n[i] <= 0) return itg_fail(h, ITG_ERR_SHAPE, "batched svd: empty matrix %d", i);
     const int64_t mm = m[i] >= n[i] ? m[i] : n[i], nn = m[i] >= n[i] ? n[i] : m[i];
-    if (nn > 512 || mm > 8192)
+    if (nn > SVDB_MAX_N || mm > 8192)
       return itg_fail(h, ITG_ERR_UNSUPPORTED, "batched svd: instance %d (%lld x %lld) above 512 columns",
                       i, (long long)m[i], (long long)n[i]);
     oW[i] = take(sizeof(double) * mm * nn);
@@ -179,9 +242,9 @@ extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m,
     oSig[i] = take(sizeof(double) * nn);
     oP[i] = take(sizeof(double) * nn);
     oOrd[i] = take(sizeof(int) * nn);
-    oOut[i] = take(4 * sizeof(double));
   }
-  const size_t oJobs = take(sizeof(SvdJob) * count), oSw = take(sizeof(int) * count);
+  if (count * 3 > ITG_PINNED_DOUBLES) return itg_fail(h, ITG_ERR_UNSUPPORTED, "batched svd: too many instances");
+  const size_t oJobs = take(sizeof(SvdJob) * count);
   ITG_TRY(itg_scratch_reserve(h, off));
   char* base = (char*)h->scratch;
   for (int i = 0; i < count; ++i) {
@@ -195,7 +258,6 @@ extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m,
     J.sig = (double*)(base + oSig[i]);
     J.P = (double*)(base + oP[i]);
     J.order = (int*)(base + oOrd[i]);
-    J.out3 = (double*)(base + oOut[i]);
     J.m = (int)m[i];
     J.n = (int)n[i];
     J.tr = m[i] < n[i];
@@ -205,24 +267,36 @@ extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m,
   }
   SvdJob* djobs = (SvdJob*)(base + oJobs);
   ITG_CUDA(h, cudaMemcpyAsync(djobs, jobs.data(), sizeof(SvdJob) * count, cudaMemcpyHostToDevice, h->stream));
-  k_svd_batched<<<count, 1024, 0, h->stream>>>(djobs, 2.220446049250313e-16, 60, (int*)(base + oSw));
+  const TruncRule rule = {mindim, cutoff, absoluteCutoff, doRelCutoff, legacy_gpu};
+  k_svd_batched<<<count, 1024, 0, h->stream>>>(djobs, 2.220446049250313e-16, 60, rule, h->pinned);
   ITG_CHECK_LAUNCH(h);
-  for (int i = 0; i < count; ++i)
-    ITG_TRY(itg::truncate_dev(h, jobs[i].P, jobs[i].nn, maxdim[i], mindim, cutoff, absoluteCutoff,
-                              doRelCutoff, legacy_gpu, jobs[i].out3));
-  k_svd_batched_gather<<<count, 512, 0, h->stream>>>(djobs);
-  ITG_CHECK_LAUNCH(h);
-  // read all truncation results (contiguous copies would need one buffer; the
-  // out3 slots are 256 bytes apart, so copy them one by one into pinned memory)
-  if (count * 3 > ITG_PINNED_DOUBLES) return itg_fail(h, ITG_ERR_UNSUPPORTED, "batched svd: too many instances");
-  for (int i = 0; i < count; ++i)
-    ITG_CUDA(h, cudaMemcpyAsync(h->pinned + 3 * i, jobs[i].out3, 3 * sizeof(double), cudaMemcpyDeviceToHost,
-                                h->stream));
   ITG_CUDA(h, cudaStreamSynchronize(h->stream));
   for (int i = 0; i < count; ++i) {
     k[i] = (int64_t)h->pinned[3 * i];
     truncerr[i] = h->pinned[3 * i + 1];
   }
+  return ITG_OK;
+}
+
+extern "C" int itg_svd_absorb_batched(itg_handle* h, int count, const int64_t* m, const int64_t* n, const int64_t* k,
+                                      const double* const* U, const double* const* S, const double* const* V,
+                                      int to_left, double* const* A, double* const* B) {
+  if (!h || count < 0 || (count > 0 && (!m || !n || !k || !U || !S || !V || !A || !B))) return ITG_ERR_INVALID;
+  if (count == 0) return ITG_OK;
+  if (count > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "batched absorb: too many instances");
+  std::vector<AbsorbJob> jobs(count);
+  int64_t most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (m[i] <= 0 || n[i] <= 0 || k[i] <= 0) return itg_fail(h, ITG_ERR_SHAPE, "batched absorb: empty factor %d", i);
+    if (!U[i] || !S[i] || !V[i] || !A[i] || !B[i]) return itg_fail(h, ITG_ERR_INVALID, "batched absorb: null pointer");
+    jobs[i] = {U[i], S[i], V[i], A[i], B[i], m[i], n[i], k[i]};
+    most = std::max(most, std::max(m[i], n[i]) * k[i]);
+  }
+  ITG_TRY(itg_scratch_reserve(h, sizeof(AbsorbJob) * count));
+  ITG_CUDA(h, cudaMemcpyAsync(h->scratch, jobs.data(), sizeof(AbsorbJob) * count, cudaMemcpyHostToDevice, h->stream));
+  const int64_t gx = (most + 255) / 256;
+  k_svd_absorb<<<dim3((unsigned)(gx < 64 ? gx : 64), count), 256, 0, h->stream>>>((const AbsorbJob*)h->scratch, to_left);
+  ITG_CHECK_LAUNCH(h);
   return ITG_OK;
 }
 

@@ -152,6 +152,7 @@ SIGNATURES = {
                                        _P, C.c_int, _I64P, _I32P, C.c_double, _P, C.c_int, _I64P, _I32P]),
     "itg_svd_trunc_batched": (C.c_int, [_P, C.c_int, _I64P, _I64P, _P, _I64P, C.c_int64, C.c_double,
                                         C.c_int, C.c_int, C.c_int, _P, _P, _P, _I64P, _DP]),
+    "itg_svd_absorb_batched": (C.c_int, [_P, C.c_int, _I64P, _I64P, _I64P, _P, _P, _P, C.c_int, _P, _P]),
     "itg_davidson_heff2_batched": (C.c_int, [_P, C.c_int, _I64P, _I64P, C.c_int64, C.c_int64, C.c_int64,
                                              C.c_int64, _P, _P, _P, _P, _P, C.c_int, C.c_int, C.c_double,
                                              _DP, C.POINTER(C.c_int)]),

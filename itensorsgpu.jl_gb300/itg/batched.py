@@ -19,12 +19,20 @@ import numpy as np
 
 from . import tensor as T
 from ._lib import i32arr, i64arr
-from .dmrg import _Chain, _diag_raw, _orthogonalize_left_end, _permute_raw, sweepnext
+from .dmrg import _Chain, _orthogonalize_left_end, sweepnext
 from .mps import MPO, MPS
 
 
 def _ptrs(ts):
     return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+
+
+def _pool(sizes):
+    """Tensors of these lengths in one allocation, each on a 256-byte boundary, and their addresses."""
+    parts = [x for n in sizes for x in (n, -n % 32)]
+    buf = T.empty_dev(sum(parts))
+    out = buf.split(parts)[::2]
+    return out, _ptrs(out)
 
 
 def _grouped(h, A, dA, mA, B, dB, mB, dC, mC):
@@ -116,30 +124,20 @@ def dmrg_batched(Hs, psis, nsweep: int, maxdims, cutoff: float, *, mindim: int =
             ms = [chiL[i] * d for i in range(cnt)]
             ns = [d * chiR[i] for i in range(cnt)]
             rs = [min(a, bb) for a, bb in zip(ms, ns)]
-            Us = [T.empty_dev(m * r) for m, r in zip(ms, rs)]
-            Ss = [T.empty_dev(r) for r in rs]
-            Vs = [T.empty_dev(n * r) for n, r in zip(ns, rs)]
+            # one buffer each for the factors and the new tensors of all instances
+            U, Up = _pool([m * r for m, r in zip(ms, rs)])
+            S, Sp = _pool(rs)
+            V, Vp = _pool([n * r for n, r in zip(ns, rs)])
             ks = (C.c_int64 * cnt)()
             tes = (C.c_double * cnt)()
             h.call("itg_svd_trunc_batched", cnt, i64arr(ms), i64arr(ns), _ptrs(phis),
-                   i64arr([at(md[i], sw) for i in range(cnt)]), mindim, cutoff, 0, 1, 0,
-                   _ptrs(Us), _ptrs(Ss), _ptrs(Vs), ks, tes)
+                   i64arr([at(md[i], sw) for i in range(cnt)]), mindim, cutoff, 0, 1, 0, Up, Sp, Vp, ks, tes)
+            new, newp = _pool([m * k for m, k in zip(ms, ks)])
+            new1, new1p = _pool([n * k for n, k in zip(ns, ks)])
+            h.call("itg_svd_absorb_batched", cnt, i64arr(ms), i64arr(ns), ks, Up, Sp, Vp, int(ha != 1), newp, new1p)
             for i, c in enumerate(chains):
-                kk = int(ks[i])
-                a, d1, d2, cc = chiL[i], d, d, chiR[i]
-                Uk, Vk, Sk = Us[i][: ms[i] * kk], Vs[i][: ns[i] * kk], Ss[i][:kk]
-                if ha == 1:
-                    c.A[b] = Uk.clone()
-                    c.Ad[b] = (a, d1, kk)
-                    c.A[b + 1] = _diag_raw(h, Sk, (kk, kk), [1, 2], Vk, (d2, cc, kk), [3, 4, 1], (kk, d2, cc),
-                                           [2, 3, 4])
-                    c.Ad[b + 1] = (kk, d2, cc)
-                else:
-                    c.A[b] = _diag_raw(h, Sk, (kk, kk), [1, 2], Uk, (a, d1, kk), [3, 4, 1], (a, d1, kk),
-                                       [3, 4, 2])
-                    c.Ad[b] = (a, d1, kk)
-                    c.A[b + 1] = _permute_raw(h, Vk, (d2, cc, kk), [1, 2, 3], [3, 1, 2])
-                    c.Ad[b + 1] = (kk, d2, cc)
+                c.A[b], c.Ad[b] = new[i], (chiL[i], d, ks[i])
+                c.A[b + 1], c.Ad[b + 1] = new1[i], (ks[i], d, chiR[i])
             if ha == 1:
                 Ln, Ld = _env_left_g(h, [Lenv[i][b][0] for i in range(cnt)], [Lenv[i][b][1] for i in range(cnt)],
                                      [c.A[b] for c in chains], [c.Ad[b] for c in chains],
@@ -159,6 +157,6 @@ def dmrg_batched(Hs, psis, nsweep: int, maxdims, cutoff: float, *, mindim: int =
     for c, psi in zip(chains, psis):
         links = [T.Index(1, "Link,l=0")] + [T.Index(c.Ad[j][2], f"Link,l={j + 1}") for j in range(N - 1)] + \
                 [T.Index(1, f"Link,l={N}")]
-        ts = [T.ITensor(T.Dense(c.A[j]), (links[j], psi.sites[j], links[j + 1])) for j in range(N)]
+        ts = [T.ITensor(T.Dense(c.A[j].clone()), (links[j], psi.sites[j], links[j + 1])) for j in range(N)]
         out.append(MPS(ts, psi.sites, 0, 1))
     return energies.copy(), out, secs
