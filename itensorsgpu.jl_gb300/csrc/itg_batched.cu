@@ -8,6 +8,7 @@
 
 #include <cmath>
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace itg {
@@ -304,6 +305,9 @@ extern "C" int itg_svd_absorb_batched(itg_handle* h, int count, const int64_t* m
 // Same algorithm as itg_davidson_heff2, run for many instances at once.  Each
 // instance keeps its own state (basis size, restart count, convergence); every
 // phase runs one launch over the instances that are in that phase.
+// Bound by launches and waits: the correction vectors are queued behind the Ritz
+// step before its norms are known, so a basis vector takes two waits for the host
+// instead of four (16 instances of 10 sites, maxdim 16: 905 -> 675 us a bond).
 namespace {
 
 struct Seg {
@@ -364,9 +368,9 @@ __global__ void k_seg_ritz(const int* __restrict__ ids, const Seg* __restrict__ 
   }
 }
 
-// out[i] = |buf_i| where buf_i starts at base + (col >= 0 ? V + col*n : v1)
+// out[i] (and host[i] where given) = |buf_i| where buf_i starts at base + (col >= 0 ? V + col*n : v1)
 __global__ void k_seg_nrm(const int* __restrict__ ids, const Seg* __restrict__ seg, const double* __restrict__ buf,
-                          int col, const int* __restrict__ colv, double* __restrict__ out) {
+                          int col, const int* __restrict__ colv, double* out, double* host) {
   __shared__ double sh[32];
   const int i = ids[blockIdx.x];
   const Seg s = seg[i];
@@ -375,7 +379,11 @@ __global__ void k_seg_nrm(const int* __restrict__ ids, const Seg* __restrict__ s
   double acc = 0.0;
   for (int64_t e = threadIdx.x; e < s.n; e += blockDim.x) acc = fma(x[e], x[e], acc);
   acc = bsum(acc, sh);
-  if (threadIdx.x == 0) out[i] = sqrt(acc);
+  if (threadIdx.x == 0) {
+    acc = sqrt(acc);
+    if (out) out[i] = acc;
+    if (host) host[i] = acc;
+  }
 }
 
 // t_i (basis column kk[i] of V) = Rv / (dg - theta), guarded; or = Rv (plain)
@@ -429,16 +437,17 @@ __global__ void k_seg_sub(const int* __restrict__ ids, const Seg* __restrict__ s
   }
 }
 
-// dst_i = src_i * f[i]; src/dst given as (buffer, column or -1 for v1 slots).
+// dst_i = src_i * f[i], or / f[i] rounded as a product with 1 / f[i] (inv);
+// src/dst given as (buffer, column or -1 for v1 slots).
 __global__ void k_seg_scale(const int* __restrict__ ids, const Seg* __restrict__ seg, const double* __restrict__ src,
                             int scol, const int* __restrict__ scolv, double* __restrict__ dst, int dcol,
-                            const double* __restrict__ f, double* const* __restrict__ extdst) {
+                            const double* __restrict__ f, bool inv, double* const* __restrict__ extdst) {
   const int i = ids[blockIdx.y];
   const Seg s = seg[i];
   const int sc = scolv ? scolv[i] : scol;
   const double* x = src + (sc >= 0 ? s.V + sc * s.n : s.v1);
   double* y = extdst ? extdst[i] : dst + (dcol >= 0 ? s.V + dcol * s.n : s.v1);
-  const double a = f[i];
+  const double a = inv ? 1.0 / f[i] : f[i];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < s.n; e += (int64_t)gridDim.x * blockDim.x)
     y[e] = x[e] * a;
 }
@@ -626,12 +635,9 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   auto take = [&](size_t b) { size_t o = off; off += itg_align256(b); return o; };
   const size_t oV = take(8 * vtot), oAV = take(8 * vtot), oX = take(8 * v1tot), oHX = take(8 * v1tot),
                oR = take(8 * v1tot), oDg = take(8 * v1tot), oT1 = take(8 * t1tot), oT3 = take(8 * t3tot),
-               oW = take(8 * (size_t)count * nc * nj), oSeg = take(sizeof(Seg) * count),
-               oHp = take(sizeof(HeffPtrs) * count), oIds = take(sizeof(int) * count),
-               oKk = take(sizeof(int) * count), oG = take(8 * (size_t)count * kmax * kmax),
-               oY = take(8 * (size_t)count * kmax), oTh = take(8 * (size_t)count), oHc = take(8 * (size_t)count * kmax),
-               oNr = take(8 * (size_t)count), oF = take(8 * (size_t)count), oCol = take(sizeof(int) * count),
-               oPsi = take(sizeof(double*) * count);
+               oW = take(8 * (size_t)count * nc * nj), oHc = take(8 * (size_t)count * kmax),
+               oNr = take(8 * (size_t)count), oSeg = take(sizeof(Seg) * count), oHp = take(sizeof(HeffPtrs) * count),
+               oPsi = take(sizeof(double*) * count), oDesc = oSeg;
   ITG_TRY(itg_scratch_reserve(h, off));
   char* base = (char*)h->scratch;
   double* V = (double*)(base + oV);
@@ -645,21 +651,45 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   double* Weff = (double*)(base + oW);
   Seg* dseg = (Seg*)(base + oSeg);
   HeffPtrs* dhp = (HeffPtrs*)(base + oHp);
-  int* dids = (int*)(base + oIds);
-  int* dkk = (int*)(base + oKk);
-  double* dG = (double*)(base + oG);
-  double* dY = (double*)(base + oY);
-  double* dTh = (double*)(base + oTh);
   double* dHc = (double*)(base + oHc);
   double* dNr = (double*)(base + oNr);
-  double* dF = (double*)(base + oF);
-  int* dCol = (int*)(base + oCol);
   double** dPsi = (double**)(base + oPsi);
-  std::vector<HeffPtrs> hps(count);
-  for (int i = 0; i < count; ++i) hps[i] = {L[i], W1[i], W2[i], R[i]};
-  ITG_CUDA(h, cudaMemcpyAsync(dseg, seg.data(), sizeof(Seg) * count, cudaMemcpyHostToDevice, h->stream));
-  ITG_CUDA(h, cudaMemcpyAsync(dhp, hps.data(), sizeof(HeffPtrs) * count, cudaMemcpyHostToDevice, h->stream));
-  ITG_CUDA(h, cudaMemcpyAsync(dPsi, psi, sizeof(double*) * count, cudaMemcpyHostToDevice, h->stream));
+  // What the kernels need from the host (which instances, basis sizes,
+  // coefficients) is read from pinned memory in place: a few bytes a block, where
+  // a copy each took 5 us of the host.  The ring starts anew after every wait and
+  // holds all that is staged between two of them (fewer than 60 arrays of at
+  // most count x kmax doubles; its tail: the start vectors' norms).
+  const size_t desc_bytes = off - oDesc;
+  const size_t ring = itg_align256(desc_bytes) + 64 * 1024 + (size_t)count * (256 + 16 * kmax);
+  if (ring + 8 * (size_t)count > h->stage_bytes) {
+    if (h->stage) cudaFreeHost(h->stage);
+    h->stage = nullptr;
+    h->stage_bytes = 0;
+    if (cudaMallocHost(&h->stage, ring + 8 * (size_t)count) != cudaSuccess)
+      return itg_fail(h, ITG_ERR_ALLOC, "batched davidson: pinned staging allocation failed");
+    h->stage_bytes = ring + 8 * (size_t)count;
+  }
+  char* stage = (char*)h->stage;
+  double* norm0 = (double*)(stage + (ring & ~(size_t)255));
+  size_t staged = 0;
+  auto put = [&](const void* src, size_t bytes) -> const void* {
+    void* at = stage + staged;
+    std::memcpy(at, src, bytes);
+    staged += itg_align256(bytes);
+    return at;
+  };
+  {
+    Seg* sp = (Seg*)(stage + (oSeg - oDesc));
+    HeffPtrs* hp = (HeffPtrs*)(stage + (oHp - oDesc));
+    double** pp = (double**)(stage + (oPsi - oDesc));
+    for (int i = 0; i < count; ++i) {
+      sp[i] = seg[i];
+      hp[i] = {L[i], W1[i], W2[i], R[i]};
+      pp[i] = psi[i];
+    }
+    ITG_CUDA(h, cudaMemcpyAsync(base + oDesc, stage, desc_bytes, cudaMemcpyHostToDevice, h->stream));
+    staged = itg_align256(desc_bytes);
+  }
   const int gx = (int)((nmax + 255) / 256 < 64 ? (nmax + 255) / 256 : 64);
   k_seg_weff<<<count, 256, 0, h->stream>>>(dhp, (int)wL, (int)wM, (int)wR, (int)d, Weff);
   k_seg_diag<<<dim3(gx, count), 256, sizeof(double) * wL * d * d * wR, h->stream>>>(dhp, dseg, (int)d, (int)wL,
@@ -671,17 +701,11 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   std::vector<double> theta(count, 0.0), rn(count, 0.0);
   std::vector<int> ids;
   double* hpin = h->pinned;
-  auto upload_ids = [&](const std::vector<int>& v) -> int {
-    ITG_CUDA(h, cudaMemcpyAsync(dids, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, h->stream));
-    return ITG_OK;
-  };
-  auto upload_kk = [&]() -> int {
-    ITG_CUDA(h, cudaMemcpyAsync(dkk, kk.data(), sizeof(int) * count, cudaMemcpyHostToDevice, h->stream));
-    return ITG_OK;
-  };
-  auto read = [&](const double* src, size_t nd) -> int {
-    ITG_CUDA(h, cudaMemcpyAsync(hpin, src, 8 * nd, cudaMemcpyDeviceToHost, h->stream));
+  auto ints = [&](const std::vector<int>& v) { return (const int*)put(v.data(), sizeof(int) * v.size()); };
+  auto doubles = [&](const std::vector<double>& v) { return (const double*)put(v.data(), 8 * v.size()); };
+  auto wait = [&]() -> int {
     ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    staged = 0;
     return ITG_OK;
   };
   // grouped H_eff matvec for the instances in `v`, from column kcol[i] of V into AV
@@ -713,12 +737,11 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
     const int32_t mT3[5] = {3, 6, 7, 9, 10}, mR[3] = {6, 10, 11}, mO[4] = {3, 7, 9, 11};
     ITG_TRY(itg::contract_grouped_f64(h, c, 1.0, a1.data(), 3, dA1.data(), mL, b1.data(), 4, dB1.data(), mP,
                                       0.0, c1.data(), 5, dC1.data(), mT1));
-    ITG_TRY(upload_ids(v));
     int64_t rmax = 0;
     for (int i : v) rmax = seg[i].rows > rmax ? seg[i].rows : rmax;
     const int64_t gr = (rmax + SEG_MID_R - 1) / SEG_MID_R;
     const dim3 grid((nj + SEG_MID_J - 1) / SEG_MID_J, (unsigned)(gr < 65535 ? gr : 65535), c);
-    k_seg_mid<<<grid, SEG_MID_R, sizeof(double) * nc * (nj < SEG_MID_J ? nj : SEG_MID_J), h->stream>>>(dids, dseg, T1, Weff, T3, nc, nj);
+    k_seg_mid<<<grid, SEG_MID_R, sizeof(double) * nc * (nj < SEG_MID_J ? nj : SEG_MID_J), h->stream>>>(ints(v), dseg, T1, Weff, T3, nc, nj);
     ITG_CHECK_LAUNCH(h);
     ITG_TRY(itg::contract_grouped_f64(h, c, 1.0, a3.data(), 5, dA3.data(), mT3, b3.data(), 3, dB3.data(), mR,
                                       0.0, c3.data(), 4, dC3.data(), mO));
@@ -731,25 +754,18 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   for (int i = 0; i < count; ++i) all[i] = i;
   {
     // X_i = psi_i (external pointers), then V0 = X / |X|
-    ITG_TRY(upload_ids(all));
     for (int i = 0; i < count; ++i)
       ITG_CUDA(h, cudaMemcpyAsync(X + seg[i].v1, psi[i], 8 * seg[i].n, cudaMemcpyDeviceToDevice, h->stream));
-    k_seg_nrm<<<count, 256, 0, h->stream>>>(dids, dseg, X, -1, nullptr, dNr);
-    ITG_CHECK_LAUNCH(h);
-    ITG_TRY(read(dNr, count));
-    std::vector<double> inv(count);
-    for (int i = 0; i < count; ++i) {
-      if (!(hpin[i] > 0.0)) return itg_fail(h, ITG_ERR_INVALID, "batched davidson: zero start vector %d", i);
-      inv[i] = 1.0 / hpin[i];
-    }
-    ITG_CUDA(h, cudaMemcpyAsync(dF, inv.data(), 8 * count, cudaMemcpyHostToDevice, h->stream));
-    k_seg_scale<<<dim3(gx, count), 256, 0, h->stream>>>(dids, dseg, X, -1, nullptr, V, 0, dF, nullptr);
+    const int* ids = ints(all);
+    k_seg_nrm<<<count, 256, 0, h->stream>>>(ids, dseg, X, -1, nullptr, dNr, norm0);
+    k_seg_scale<<<dim3(gx, count), 256, 0, h->stream>>>(ids, dseg, X, -1, nullptr, V, 0, dNr, true, nullptr);
     ITG_CHECK_LAUNCH(h);
     std::vector<int> col0(count, 0);
     ITG_TRY(matvec(all, col0));
   }
   std::vector<double> Gh, yv;
   std::vector<double> ycoef((size_t)count * kmax, 0.0);
+  bool first = true;  // the start vectors' norms have not been looked at
   for (;;) {
     // Rayleigh-Ritz for every instance still running
     ids.clear();
@@ -757,73 +773,82 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
       if (!done[i]) ids.push_back(i);
     if (ids.empty()) break;
     const int c = (int)ids.size();
-    ITG_TRY(upload_ids(ids));
-    ITG_TRY(upload_kk());
-    k_seg_gram<<<dim3(kmax * kmax, c), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, AV, dG);
+    const int* dids = ints(ids);
+    const int* dkk = ints(kk);
+    k_seg_gram<<<dim3(kmax * kmax, c), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, AV, hpin);
     ITG_CHECK_LAUNCH(h);
-    ITG_TRY(read(dG, (size_t)count * kmax * kmax));
+    ITG_TRY(wait());
+    if (first) {
+      for (int i = 0; i < count; ++i)
+        if (!(norm0[i] > 0.0))
+          return itg_fail(h, ITG_ERR_INVALID, "batched davidson: zero start vector %d", i);
+      first = false;
+    }
     for (int i : ids) {
       small_lowest(kk[i], hpin + (size_t)i * kmax * kmax, kmax, theta[i], yv);
       for (int j = 0; j < kmax; ++j) ycoef[(size_t)i * kmax + j] = j < kk[i] ? yv[j] : 0.0;
     }
-    ITG_CUDA(h, cudaMemcpyAsync(dY, ycoef.data(), 8 * (size_t)count * kmax, cudaMemcpyHostToDevice, h->stream));
-    ITG_CUDA(h, cudaMemcpyAsync(dTh, theta.data(), 8 * (size_t)count, cudaMemcpyHostToDevice, h->stream));
-    k_seg_ritz<<<dim3(gx, c), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, AV, dY, dTh, X, HX, Rv);
-    k_seg_nrm<<<c, 256, 0, h->stream>>>(dids, dseg, Rv, -1, nullptr, dNr);
+    // Ritz vectors and residuals, and for the instances whose basis can grow the
+    // correction vectors too, before the host has seen any of the norms (an
+    // instance whose residual turns out converged drops its correction)
+    dids = ints(ids);
+    dkk = ints(kk);
+    const double* dTh = doubles(theta);
+    double *rnh = hpin, *t0h = hpin + count, *tnh = hpin + 2 * (size_t)count;
+    k_seg_ritz<<<dim3(gx, c), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, AV, doubles(ycoef), dTh, X, HX, Rv);
+    k_seg_nrm<<<c, 256, 0, h->stream>>>(dids, dseg, Rv, -1, nullptr, nullptr, rnh);
     ITG_CHECK_LAUNCH(h);
-    ITG_TRY(read(dNr, count));
+    auto corrections = [&](const std::vector<int>& cur, int attempt) -> int {
+      const int cc = (int)cur.size();
+      const int *di = ints(cur), *dk = ints(kk);
+      k_seg_correction<<<dim3(gx, cc), 256, 0, h->stream>>>(di, dseg, dk, Rv, dg, doubles(theta), attempt, V);
+      k_seg_nrm<<<cc, 256, 0, h->stream>>>(di, dseg, V, 0, dk, nullptr, t0h);
+      for (int pass = 0; pass < 2; ++pass) {
+        k_seg_proj<<<dim3(kmax, cc), 256, 0, h->stream>>>(di, dseg, dk, kmax, V, dHc);
+        k_seg_sub<<<dim3(gx, cc), 256, 0, h->stream>>>(di, dseg, dk, kmax, V, dHc);
+      }
+      k_seg_nrm<<<cc, 256, 0, h->stream>>>(di, dseg, V, 0, dk, nullptr, tnh);
+      ITG_CHECK_LAUNCH(h);
+      return ITG_OK;
+    };
     std::vector<int> grow, stop;
+    for (int i : ids)
+      if (kk[i] < kmax) grow.push_back(i);
+    if (!grow.empty()) ITG_TRY(corrections(grow, 0));
+    ITG_TRY(wait());
+    grow.clear();
     for (int i : ids) {
-      rn[i] = hpin[i];
+      rn[i] = rnh[i];
       if (rn[i] < tol || kk[i] == kmax) stop.push_back(i);
       else grow.push_back(i);
     }
-    // correction vectors for the instances that grow their basis
     std::vector<int> accepted;
     std::vector<double> tscale(count, 0.0);
-    if (!grow.empty()) {
-      std::vector<int> cur = grow;
-      for (int attempt = 0; attempt < 2 && !cur.empty(); ++attempt) {
-        const int cc = (int)cur.size();
-        ITG_TRY(upload_ids(cur));
-        k_seg_correction<<<dim3(gx, cc), 256, 0, h->stream>>>(dids, dseg, dkk, Rv, dg, dTh, attempt, V);
-        ITG_CHECK_LAUNCH(h);
-        std::vector<int> colk(count, 0);
-        for (int i = 0; i < count; ++i) colk[i] = kk[i];
-        ITG_CUDA(h, cudaMemcpyAsync(dCol, colk.data(), sizeof(int) * count, cudaMemcpyHostToDevice, h->stream));
-        k_seg_nrm<<<cc, 256, 0, h->stream>>>(dids, dseg, V, 0, dCol, dNr);
-        ITG_CHECK_LAUNCH(h);
-        ITG_TRY(read(dNr, count));
-        std::vector<double> t0(count, 0.0);
-        for (int i : cur) t0[i] = hpin[i];
-        for (int pass = 0; pass < 2; ++pass) {
-          k_seg_proj<<<dim3(kmax, cc), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, dHc);
-          k_seg_sub<<<dim3(gx, cc), 256, 0, h->stream>>>(dids, dseg, dkk, kmax, V, dHc);
-        }
-        k_seg_nrm<<<cc, 256, 0, h->stream>>>(dids, dseg, V, 0, dCol, dNr);
-        ITG_CHECK_LAUNCH(h);
-        ITG_TRY(read(dNr, count));
-        std::vector<int> retry;
-        for (int i : cur) {
-          const double tn = hpin[i];
-          if (tn > 1e-6 * t0[i]) {
-            if (tn > 1e-14) {
-              accepted.push_back(i);
-              tscale[i] = 1.0 / tn;
-            } else {
-              stop.push_back(i);
-            }
-          } else if (attempt == 0) {
-            retry.push_back(i);
+    for (int attempt = 0; attempt < 2 && !grow.empty(); ++attempt) {
+      if (attempt > 0) {
+        ITG_TRY(corrections(grow, attempt));
+        ITG_TRY(wait());
+      }
+      std::vector<int> retry;
+      for (int i : grow) {
+        const double tn = tnh[i];
+        if (tn > 1e-6 * t0h[i]) {
+          if (tn > 1e-14) {
+            accepted.push_back(i);
+            tscale[i] = 1.0 / tn;
           } else {
             stop.push_back(i);
           }
+        } else if (attempt == 0) {
+          retry.push_back(i);
+        } else {
+          stop.push_back(i);
         }
-        cur = retry;
       }
+      grow = retry;
     }
     if (!accepted.empty()) {
-      ITG_CUDA(h, cudaMemcpyAsync(dF, tscale.data(), 8 * count, cudaMemcpyHostToDevice, h->stream));
+      const double* dF = doubles(tscale);
       // normalise column kk[i] in place; one launch per distinct kk value
       std::vector<int> kvals;
       for (int i : accepted)
@@ -832,8 +857,8 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
         std::vector<int> sub;
         for (int i : accepted)
           if (kk[i] == kv) sub.push_back(i);
-        ITG_TRY(upload_ids(sub));
-        k_seg_scale<<<dim3(gx, (int)sub.size()), 256, 0, h->stream>>>(dids, dseg, V, kv, nullptr, V, kv, dF, nullptr);
+        k_seg_scale<<<dim3(gx, (int)sub.size()), 256, 0, h->stream>>>(ints(sub), dseg, V, kv, nullptr, V, kv, dF, false,
+                                                                      nullptr);
         ITG_CHECK_LAUNCH(h);
       }
       ITG_TRY(matvec(accepted, kk));
@@ -847,18 +872,14 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
     }
     auto normalise_into = [&](const std::vector<int>& v, bool to_psi) -> int {
       if (v.empty()) return ITG_OK;
-      ITG_TRY(upload_ids(v));
-      k_seg_nrm<<<(int)v.size(), 256, 0, h->stream>>>(dids, dseg, X, -1, nullptr, dNr);
-      ITG_CHECK_LAUNCH(h);
-      ITG_TRY(read(dNr, count));
-      std::vector<double> f(count, 0.0);
-      for (int i : v) f[i] = 1.0 / hpin[i];
-      ITG_CUDA(h, cudaMemcpyAsync(dF, f.data(), 8 * count, cudaMemcpyHostToDevice, h->stream));
+      const int* di = ints(v);
+      const dim3 grid(gx, (int)v.size());
+      k_seg_nrm<<<(int)v.size(), 256, 0, h->stream>>>(di, dseg, X, -1, nullptr, dNr, nullptr);
       if (to_psi) {
-        k_seg_scale<<<dim3(gx, (int)v.size()), 256, 0, h->stream>>>(dids, dseg, X, -1, nullptr, nullptr, 0, dF, dPsi);
+        k_seg_scale<<<grid, 256, 0, h->stream>>>(di, dseg, X, -1, nullptr, nullptr, 0, dNr, true, dPsi);
       } else {
-        k_seg_scale<<<dim3(gx, (int)v.size()), 256, 0, h->stream>>>(dids, dseg, X, -1, nullptr, V, 0, dF, nullptr);
-        k_seg_scale<<<dim3(gx, (int)v.size()), 256, 0, h->stream>>>(dids, dseg, HX, -1, nullptr, AV, 0, dF, nullptr);
+        k_seg_scale<<<grid, 256, 0, h->stream>>>(di, dseg, X, -1, nullptr, V, 0, dNr, true, nullptr);
+        k_seg_scale<<<grid, 256, 0, h->stream>>>(di, dseg, HX, -1, nullptr, AV, 0, dNr, true, nullptr);
       }
       ITG_CHECK_LAUNCH(h);
       return ITG_OK;

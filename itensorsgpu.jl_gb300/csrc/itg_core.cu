@@ -143,6 +143,7 @@ extern "C" int itg_destroy(itg_handle* h) {
   if (h->group_desc) cudaFree(h->group_desc);
   if (h->tune_buf) cudaFree(h->tune_buf);
   if (h->pinned) cudaFreeHost(h->pinned);
+  if (h->stage) cudaFreeHost(h->stage);
   if (h->dev_status) cudaFree(h->dev_status);
   if (h->gemv_part) cudaFree(h->gemv_part);
   if (h->qr_ev_ready) cudaEventDestroy(h->qr_ev_ready);

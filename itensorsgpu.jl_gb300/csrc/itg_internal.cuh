@@ -84,6 +84,9 @@ struct itg_handle {
   size_t split_ws_bytes = 0;
   // Small pinned host buffer for scalar results (dot, truncation outputs).
   double* pinned = nullptr;
+  // Pinned staging ring of the batched Davidson (read by its kernels in place).
+  void* stage = nullptr;
+  size_t stage_bytes = 0;
   // Partial sums of itg_gemv_t (its own buffer: callers hold scratch regions).
   double* gemv_part = nullptr;
   // Persistent device buffers of the contraction plans, keyed by shape.
