@@ -137,6 +137,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// A kernel started while its predecessor on the stream drains: everything before
+// this call may overlap it, everything after sees its results.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -493,6 +499,7 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -843,46 +850,72 @@ __global__ void k_mbar_selftest(int* err, uint64_t wait_ns) {
 }
 
 // ----------------------------------------------------------- slicing
-// Exponent field (11 bits) of max_k |X[r,k]| for every row r < R.
-__global__ void k_row_expfield(const double* __restrict__ X, const int64_t* __restrict__ offR,
-                               const int64_t* __restrict__ offK, int64_t R, int64_t K,
-                               int* __restrict__ efield) {
-  {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); r < R; r += warps) {
-      const double* x = X + offR[r];
-      unsigned long long mx = 0;
-      for (int64_t k = lane; k < K; k += 32) {
-        unsigned long long b = (unsigned long long)__double_as_longlong(x[offK[k]]) & 0x7FFFFFFFFFFFFFFFull;
-        mx = b > mx ? b : mx;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, o);
-        mx = y > mx ? y : mx;
-      }
-      if (lane == 0) efield[r] = (int)((mx >> 52) & 0x7FF);
-    }
-  }
-}
+// One operand of a product on its way into digit slices.
+struct PrepOp {
+  const double* X;
+  const int64_t *offR, *offK;
+  int64_t R, K, Rpad, Kpad;
+  int kmaj;              // k is the contiguous direction (else the rows are)
+  int nchunk;            // chunks of K whose maxima are found apart
+  int64_t chunk;         // their length
+  int* part;             // [nchunk][Rpad] exponent fields of the chunks (ef itself when there is one)
+  int* ef;               // exponent field (11 bits) of max_k |X[r,k]|
+  __nv_bfloat16* out;    // slices [digit][Rpad][Kpad]
+  int64_t eblocks, sblocks;  // blocks of k_split_exponents and k_make_slices
+};
 
-// Rows contiguous in memory: a 2-D grid, threads along rows, blockIdx.y over
-// K chunks of 64; partial maxima meet through atomicMax on the exponent field
-// (integer max, order independent).  efield must start at 0.
-__global__ void k_row_expfield_mmajor(const double* __restrict__ X, const int64_t* __restrict__ offR,
-                                      const int64_t* __restrict__ offK, int64_t R, int64_t K,
-                                      int* __restrict__ efield) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const int64_t k0 = (int64_t)blockIdx.y * 64, k1 = k0 + 64 < K ? k0 + 64 : K;
-  const double* x = X + offR[r];
-  unsigned long long mx = 0;
-  for (int64_t k = k0; k < k1; ++k) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(x[offK[k]]) & 0x7FFFFFFFFFFFFFFFull;
-    mx = b > mx ? b : mx;
+// Exponent fields of both operands, and zeros for the sums that the product's
+// CTAs share.  One launch for all of it, the slices the second and the product
+// the third: the preparation of a small product is bound by its launches (eight,
+// with the memsets, each a few us; H_eff at chi = 189 159 -> 135 us).
+constexpr int ZERO_BLOCK = 16 * 256;  // 16-byte words a block
+__global__ void __launch_bounds__(256)
+k_split_exponents(PrepOp a, PrepOp b, uint4* zero, int64_t nzero) {
+  grid_wait();
+  int64_t blk = blockIdx.x;
+  if (blk >= a.eblocks + b.eblocks) {
+    const int64_t z0 = (blk - a.eblocks - b.eblocks) * ZERO_BLOCK;
+#pragma unroll
+    for (int i = 0; i < ZERO_BLOCK / 256; ++i) {
+      const int64_t z = z0 + threadIdx.x + 256 * i;
+      if (z < nzero) zero[z] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    return;
   }
-  const int e = (int)((mx >> 52) & 0x7FF);
-  if (e) atomicMax(&efield[r], e);
+  if (blk >= a.eblocks) {
+    blk -= a.eblocks;
+    a = b;
+  }
+  auto magnitude = [](double x) { return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull; };
+  unsigned long long mx = 0;
+  if (a.kmaj) {  // a warp a row
+    const int lane = threadIdx.x & 31;
+    const int64_t r = blk * 8 + (threadIdx.x >> 5);
+    if (r >= a.R) return;
+    const double* x = a.X + a.offR[r];
+#pragma unroll 4
+    for (int64_t k = lane; k < a.K; k += 32) {
+      const unsigned long long m = magnitude(x[a.offK[k]]);
+      mx = m > mx ? m : mx;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = y > mx ? y : mx;
+    }
+    if (lane == 0) a.ef[r] = (int)((mx >> 52) & 0x7FF);
+  } else {  // threads along the rows, a chunk of K a block
+    const int c = (int)(blk % a.nchunk);
+    const int64_t r = blk / a.nchunk * 256 + threadIdx.x;
+    if (r >= a.R) return;
+    const int64_t k0 = c * a.chunk, k1 = k0 + a.chunk < a.K ? k0 + a.chunk : a.K;
+    const double* x = a.X + a.offR[r];
+#pragma unroll 8
+    for (int64_t k = k0; k < k1; ++k) {
+      const unsigned long long m = magnitude(x[a.offK[k]]);
+      mx = m > mx ? m : mx;
+    }
+    a.part[c * a.Rpad + r] = (int)((mx >> 52) & 0x7FF);
+  }
 }
 
 // The balanced base-2^8 digits of |X[r,k]| * 2^-e_r rounded to 48 fractional
@@ -1026,6 +1059,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
 #pragma unroll
     for (int p = 0; p < S; ++p)
       *(uint4*)(sA + (p >> 1) * MID_A_TILE + sw128_off(t, (p & 1) * MID_KSLICE + cg * 8)) = make_uint4(0u, 0u, 0u, 0u);
+  grid_wait();
   // B: digits of Weff's columns (row j of the B tiles, k = c), once per CTA
   {
     const int j = t >> 2, cg = t & 3;  // NJP * 4 <= 128 threads
@@ -1152,42 +1186,58 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
   }
 }
 
-// out[p][r][k] (bf16, k contiguous, padded to Rpad x Kpad) for the gathered X.
-template <bool KMAJ, int S>
+// out[p][r][k] (bf16, k contiguous, padded to Rpad x Kpad) for the gathered X
+// of both operands.
 __global__ void __launch_bounds__(256)
-k_make_slices(const double* __restrict__ X, const int64_t* __restrict__ offR,
-              const int64_t* __restrict__ offK, int64_t R, int64_t K, int64_t Rpad, int64_t Kpad,
-              const int* __restrict__ efield, __nv_bfloat16* __restrict__ out) {
+k_make_slices(PrepOp a, PrepOp b) {
   __shared__ double tile[32][65];
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;
+  grid_wait();
+  int64_t blk = blockIdx.x;
+  if (blk >= a.sblocks) {
+    blk -= a.sblocks;
+    a = b;
+  }
+  const int64_t kblocks = a.Kpad / 64, r0 = blk / kblocks * 32, k0 = blk % kblocks * 64, R = a.R, K = a.K;
   const int t = threadIdx.x;
-  if (KMAJ) {
+  if (a.kmaj) {
     const int kk = t & 63;
     const int64_t k = k0 + kk;
-    const int64_t ok = (k < K) ? offK[k] : 0;
+    const int64_t ok = (k < K) ? a.offK[k] : 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int rr = (t >> 6) + 4 * i;
       const int64_t r = r0 + rr;
-      tile[rr][kk] = (r < R && k < K) ? X[offR[r] + ok] : 0.0;
+      tile[rr][kk] = (r < R && k < K) ? a.X[a.offR[r] + ok] : 0.0;
     }
   } else {
     const int rr = t & 31;
     const int64_t r = r0 + rr;
-    const int64_t orr = (r < R) ? offR[r] : 0;
+    const int64_t orr = (r < R) ? a.offR[r] : 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int kk = (t >> 5) + 8 * i;
       const int64_t k = k0 + kk;
-      tile[rr][kk] = (r < R && k < K) ? X[orr + offK[k]] : 0.0;
+      tile[rr][kk] = (r < R && k < K) ? a.X[orr + a.offK[k]] : 0.0;
     }
   }
-  __syncthreads();
-  // each thread: 8 consecutive k of one row -> one 16-byte store per slice
-  static_assert(S == 6, "the digit word holds 6 slices");
+  // each thread: 8 consecutive k of one row -> one 16-byte store per slice; the
+  // eight threads of a row share its chunks' exponents
   const int rr = t >> 3, kc = t & 7;
   const int64_t r = r0 + rr;
-  const int ef = (r < R) ? efield[r] : 0;
+  int ef = 0;
+  if (r < R)
+    for (int c = kc; c < a.nchunk; c += 8) {
+      const int x = a.part[c * a.Rpad + r];
+      ef = x > ef ? x : ef;
+    }
+  for (int o = 1; o < 8; o <<= 1) {
+    const int x = __shfl_xor_sync(0xffffffffu, ef, o);
+    ef = x > ef ? x : ef;
+  }
+  if (a.nchunk > 1 && k0 == 0 && kc == 0 && r < R) a.ef[r] = ef;
+  __syncthreads();
+  const int64_t Rpad = a.Rpad, Kpad = a.Kpad;
+  __nv_bfloat16* out = a.out;
   unsigned long long w[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) w[e] = digit_word(tile[rr][kc * 8 + e], ef);
@@ -1234,6 +1284,25 @@ int make_map(itg_handle* h, CUtensorMap* map, void* base, int64_t inner, int64_t
 }
 
 int ws_reserve(itg_handle* h, size_t bytes);
+
+// Launches a kernel that waits for its predecessor itself (grid_wait), so that
+// it may start while that one drains; not inside a capture.
+template <class... P, class... A>
+int launch_waiting(itg_handle* h, bool capturing, unsigned grid, int threads, size_t smem, void (*kernel)(P...),
+                   A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = capturing ? 0 : 1;
+  ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
+  return ITG_OK;
+}
 
 // CTAs of one variant that fit on the GPU at once (one per SM at this shared
 // memory size), queried once per variant.
@@ -1334,8 +1403,25 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   const size_t oSA = take(cache[0] ? 0 : (size_t)2 * S * Mpad * Kpad);
   const size_t oSB = take(cache[1] ? 0 : (size_t)2 * S * Npad * Kpad);
   const size_t oAcc = take(Smem<BN>::TACC ? 0 : tile_bytes * (size_t)grid);
-  const size_t oTacc = take(shares ? tile_bytes * (size_t)grid : 0);
+  const size_t oTacc = take(shares ? tile_bytes * (size_t)grid : 0);  // (the counters follow: zeroed together)
   const size_t oCnt = take(shares ? sizeof(int) * (size_t)grid : 0);
+  const size_t zero_bytes = off - oTacc;
+  // exponents of an operand with contiguous rows: enough chunks of K to fill the SMs
+  const bool kmaj[2] = {p.a_kmaj, p.b_kmaj};
+  const int64_t rows[2] = {p.M, p.N};
+  int nchunk[2] = {1, 1};
+  int64_t chunk[2] = {p.K, p.K};
+  size_t oPart[2] = {0, 0};
+  for (int i = 0; i < 2; ++i) {
+    if (kmaj[i] || hit[i]) continue;
+    const int64_t ky = (p.K + 63) / 64;
+    if (ky > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: contraction depth too large");
+    int64_t want = (8 * 256 * (int64_t)h->num_sms + rows[i] - 1) / rows[i];
+    want = std::min<int64_t>(std::min<int64_t>(want, 32), ky);
+    chunk[i] = (ky + want - 1) / want * 64;
+    nchunk[i] = (int)((p.K + chunk[i] - 1) / chunk[i]);
+    if (nchunk[i] > 1) oPart[i] = take(sizeof(int) * (size_t)nchunk[i] * rpads[i]);
+  }
   ITG_TRY(ws_reserve(h, off));
   char* ws = (char*)h->split_ws;
   int* eA = (int*)(ws + oEA);
@@ -1354,50 +1440,38 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   long long* tacc = (long long*)(ws + oTacc);
   int* cnt = (int*)(ws + oCnt);
   int* err = h->dev_status;  // written only by a wait that runs out
-  if (shares) {
-    ITG_CUDA(h, cudaMemsetAsync(tacc, 0, tile_bytes * (size_t)grid, h->stream));
-    ITG_CUDA(h, cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)grid, h->stream));
-  }
-  // exponents
+  if (Mpad / 32 > 65535 || Npad / 32 > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: too many rows");
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
   {
     ProfScope prof(h, ITG_KERNEL_SPLIT_PREP);
-    const int thr = 256;
-    auto expo = [&](bool kmaj, const double* X, const int64_t* offR, const int64_t* offK, int64_t R,
-                    int* ef) -> int {
-      if (kmaj) {
-        k_row_expfield<<<itg_blocks_for(R, thr / 32, h->num_sms * 16), thr, 0, h->stream>>>(
-            X, offR, offK, R, p.K, ef);
-      } else {
-        ITG_CUDA(h, cudaMemsetAsync(ef, 0, sizeof(int) * R, h->stream));
-        const int64_t ky = (p.K + 63) / 64;
-        if (ky > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: contraction depth too large");
-        dim3 g((unsigned)((R + thr - 1) / thr), (unsigned)ky);
-        k_row_expfield_mmajor<<<g, thr, 0, h->stream>>>(X, offR, offK, R, p.K, ef);
-      }
-      return ITG_OK;
-    };
-    if (!hit[0]) ITG_TRY(expo(p.a_kmaj, A, p.offAm(), p.offAk(), p.M, eA));
-    if (!hit[1]) ITG_TRY(expo(p.b_kmaj, B, p.offBn(), p.offBk(), p.N, eB));
-    ITG_CHECK_LAUNCH(h);
-  }
-  // slices
-  {
-    ProfScope prof(h, ITG_KERNEL_SPLIT_PREP);
-    dim3 gA((unsigned)(Kpad / 64), (unsigned)(Mpad / 32)), gB((unsigned)(Kpad / 64), (unsigned)(Npad / 32));
-    if (gA.y > 65535 || gB.y > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: too many rows");
-    if (!hit[0]) {
-      if (p.a_kmaj)
-        k_make_slices<true, S><<<gA, 256, 0, h->stream>>>(A, p.offAm(), p.offAk(), p.M, p.K, Mpad, Kpad, eA, sA);
-      else
-        k_make_slices<false, S><<<gA, 256, 0, h->stream>>>(A, p.offAm(), p.offAk(), p.M, p.K, Mpad, Kpad, eA, sA);
+    PrepOp op[2] = {};
+    int* efs[2] = {eA, eB};
+    for (int i = 0; i < 2; ++i) {
+      if (hit[i]) continue;  // no blocks
+      PrepOp& o = op[i];
+      o.X = srcs[i];
+      o.offR = i ? p.offBn() : p.offAm();
+      o.offK = i ? p.offBk() : p.offAk();
+      o.R = rows[i];
+      o.K = p.K;
+      o.Rpad = rpads[i];
+      o.Kpad = Kpad;
+      o.kmaj = kmaj[i];
+      o.nchunk = nchunk[i];
+      o.chunk = chunk[i];
+      o.ef = efs[i];
+      o.part = nchunk[i] > 1 ? (int*)(ws + oPart[i]) : efs[i];
+      o.out = i ? sB : sA;
+      o.eblocks = kmaj[i] ? (rows[i] + 7) / 8 : (rows[i] + 255) / 256 * nchunk[i];
+      o.sblocks = (Kpad / 64) * (rpads[i] / 32);
     }
-    if (!hit[1]) {
-      if (p.b_kmaj)
-        k_make_slices<true, S><<<gB, 256, 0, h->stream>>>(B, p.offBn(), p.offBk(), p.N, p.K, Npad, Kpad, eB, sB);
-      else
-        k_make_slices<false, S><<<gB, 256, 0, h->stream>>>(B, p.offBn(), p.offBk(), p.N, p.K, Npad, Kpad, eB, sB);
-    }
-    ITG_CHECK_LAUNCH(h);
+    const int64_t nzero = shares ? (int64_t)(zero_bytes / 16) : 0;
+    const int64_t eb = op[0].eblocks + op[1].eblocks + (nzero + ZERO_BLOCK - 1) / ZERO_BLOCK;
+    const int64_t sb = op[0].sblocks + op[1].sblocks;
+    if (eb > INT32_MAX || sb > INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: problem too large");
+    if (eb > 0)
+      ITG_TRY(launch_waiting(h, capturing, (unsigned)eb, 256, 0, k_split_exponents, op[0], op[1], (uint4*)tacc, nzero));
+    if (sb > 0) ITG_TRY(launch_waiting(h, capturing, (unsigned)sb, 256, 0, k_make_slices, op[0], op[1]));
   }
   for (int i = 0; i < 2; ++i) {
     if (!cache[i] || hit[i]) continue;
@@ -1438,7 +1512,7 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   a.err = err;
   {
     ProfScope prof(h, ITG_KERNEL_GEMM_SPLIT);
-    k_split_gemm<BN><<<(unsigned)grid, NUM_THREADS, Smem<BN>::TOTAL, h->stream>>>(mA, mB, a);
+    ITG_TRY(launch_waiting(h, capturing, (unsigned)grid, NUM_THREADS, Smem<BN>::TOTAL, k_split_gemm<BN>, mA, mB, a));
   }
   ITG_CHECK_LAUNCH(h);
   return ITG_OK;
@@ -1465,9 +1539,10 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
     // three CTAs per SM: by shared memory (the carveout is set to its maximum)
     // and registers; TMEM (512 columns per SM) would allow four
     const int64_t g = std::min<int64_t>(grid, (int64_t)3 * h->num_sms);
-    k_heff_mid_split<NPASS><<<(unsigned)g, MID_THREADS, MidSmem<NPASS>::TOTAL, h->stream>>>(T1, Weff, T3, R, nc, nj,
-                                                                                            h->wait_ns, err);
-    ITG_CHECK_LAUNCH(h);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    ITG_CUDA(h, cudaStreamIsCapturing(h->stream, &cap));
+    ITG_TRY(launch_waiting(h, cap != cudaStreamCaptureStatusNone, (unsigned)g, MID_THREADS, MidSmem<NPASS>::TOTAL,
+                           k_heff_mid_split<NPASS>, T1, Weff, T3, R, nc, nj, h->wait_ns, err));
     return ITG_OK;
   };
   {

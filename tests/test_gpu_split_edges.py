@@ -36,3 +36,27 @@ def test_variants_agree(gpu, m, n, k):
     ref = (An.astype(np.longdouble) @ Bn.astype(np.longdouble)) if m * n * k < 2e7 else An @ Bn
     bound = _lib.load_library().itg_split_error_bound(k) + k * 2.0 ** -53
     assert np.linalg.norm((outs[0].reshape(n, m).T - ref).astype(float)) <= bound * np.linalg.norm(An) * np.linalg.norm(Bn)
+
+
+@pytest.mark.parametrize("m,n,k", [(3, 700, 300), (257, 33, 2100), (900, 260, 64), (40, 5, 9000)])
+def test_operand_orders_agree(gpu, m, n, k):
+    """Row exponents of operands with contiguous k and with contiguous rows (found in chunks of k): the same bits."""
+    from itg import _lib
+    import torch
+    h = _lib.handle(0)
+    g = torch.Generator().manual_seed(m + n + k)
+    A = torch.randn(k, m, dtype=torch.float64, generator=g) * torch.exp2(torch.randint(-40, 40, (k, m), generator=g))
+    B = torch.randn(n, k, dtype=torch.float64, generator=g)
+    c = (2, _lib.i64arr([m, n]), _lib.i32arr([1, 2]))
+    outs = []
+    for ta in (0, 1):
+        for tb in (0, 1):  # column-major, so the first mode is contiguous
+            a = (2, _lib.i64arr([k, m] if ta else [m, k]), _lib.i32arr([3, 1] if ta else [1, 3]))
+            b = (2, _lib.i64arr([n, k] if tb else [k, n]), _lib.i32arr([2, 3] if tb else [3, 2]))
+            x, y = (A.T if ta else A).contiguous().cuda(), (B.T if tb else B).contiguous().cuda()
+            out = torch.empty(m * n, dtype=torch.float64, device="cuda")
+            h.call("itg_contract", 0, 1.0, x.data_ptr(), *a, y.data_ptr(), *b, 0.0, out.data_ptr(), *c, 1)
+            h.call("itg_synchronize")
+            outs.append(out.cpu().numpy())
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])
