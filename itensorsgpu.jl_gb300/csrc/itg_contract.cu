@@ -196,6 +196,7 @@ k_gemm_gather_f64(const double* __restrict__ A, const double* __restrict__ B,
                   const int64_t* __restrict__ offCn, int64_t M, int64_t N, int64_t K,
                   double alpha, double beta) {
   extern __shared__ double smem[];
+  itg_grid_wait();
   gemm_tile_f64<BM, BN, AK, BK>(A, B, C, offAm, offAk, offBk, offBn, offCm, offCn, M, N, K, alpha, beta,
                                 (int64_t)blockIdx.x * BM, (int64_t)blockIdx.y * BN, smem);
 }
@@ -264,11 +265,9 @@ int launch_gemm_t(itg_handle* h, const ContractPlan& p, const double* A, const d
   if (gy > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "N=%lld too large", (long long)p.N);
   dim3 grid((unsigned)gx, (unsigned)gy);
   ProfScope prof(h, ITG_KERNEL_GEMM_F64);
-  k_gemm_gather_f64<BM, BN, AK, BK><<<grid, GTHREADS, smem, h->stream>>>(
-      A, B, C, p.offAm(), p.offAk(), p.offBk(), p.offBn(), p.offCm(), p.offCn(), p.M, p.N, p.K,
-      alpha, beta);
-  ITG_CHECK_LAUNCH(h);
-  return ITG_OK;
+  const bool overlap = itg_small_grid(h, gx * gy) && !itg_capturing(h);
+  return itg_launch_after(h, overlap, grid, GTHREADS, smem, k_gemm_gather_f64<BM, BN, AK, BK>, A, B, C, p.offAm(),
+                          p.offAk(), p.offBk(), p.offBn(), p.offCm(), p.offCn(), p.M, p.N, p.K, alpha, beta);
 }
 
 template <bool AK, bool BK>

@@ -61,6 +61,7 @@ constexpr int MID_R = 64, MID_J = 4;
 __global__ void __launch_bounds__(MID_R)
 k_heff_mid(const double* __restrict__ T1, const double* __restrict__ Weff, double* __restrict__ T3,
            int64_t R, int nc, int nj) {
+  itg_grid_wait();
   extern __shared__ double wsh[];  // MID_J columns of Weff
   const int j0 = blockIdx.x * MID_J;
   const int jn = nj - j0 < MID_J ? nj - j0 : MID_J;
@@ -84,11 +85,10 @@ k_heff_mid(const double* __restrict__ T1, const double* __restrict__ Weff, doubl
 }
 
 int launch_heff_mid(itg_handle* h, const double* T1, const double* Weff, double* T3, int64_t R, int nc, int nj) {
-  const int64_t gy = (R + MID_R - 1) / MID_R;
-  k_heff_mid<<<dim3((unsigned)((nj + MID_J - 1) / MID_J), (unsigned)(gy < 65535 ? gy : 65535)), MID_R,
-               sizeof(double) * nc * (nj < MID_J ? nj : MID_J), h->stream>>>(T1, Weff, T3, R, nc, nj);
-  ITG_CHECK_LAUNCH(h);
-  return ITG_OK;
+  const int64_t gx = (nj + MID_J - 1) / MID_J, gy = (R + MID_R - 1) / MID_R;
+  const bool overlap = itg_small_grid(h, gx * gy) && !itg_capturing(h);
+  return itg_launch_after(h, overlap, dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535)), MID_R,
+                          sizeof(double) * nc * (nj < MID_J ? nj : MID_J), k_heff_mid, T1, Weff, T3, R, nc, nj);
 }
 
 // diag(H_eff)[a', s1', s2', b'] = sum_{w,y} L[a',w,a'] Wd[w,s1',s2',y] R[b',y,b']
@@ -441,6 +441,7 @@ __device__ __forceinline__ double dv_reduce(const double* part, int np, double* 
 // out = |x| (device and host copies)
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_norm(int64_t n, const double* __restrict__ x, double* part, unsigned* counter, double* out, double* out_host) {
+  itg_grid_wait();
   __shared__ double sh[32];
   double s = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -454,6 +455,7 @@ k_dv_norm(int64_t n, const double* __restrict__ x, double* part, unsigned* count
 
 // y = x / *nrm, and y2 = x2 / *nrm where given (may be in place)
 __global__ void k_dv_scale(int64_t n, const double* nrm, const double* x, double* y, const double* x2, double* y2) {
+  itg_grid_wait();
   const double a = 1.0 / *nrm;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     y[i] = a * x[i];
@@ -466,6 +468,7 @@ template <int K>
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_gram(int64_t n, const double* __restrict__ V, const double* __restrict__ AV, double* part, unsigned* counter,
           double* G_host) {
+  itg_grid_wait();
   __shared__ double sh[16][DV_THREADS / 32 + 1];
   const int nb = gridDim.x, b = blockIdx.x;
   const int64_t chunk = (n + nb - 1) / nb;
@@ -507,6 +510,7 @@ __global__ void __launch_bounds__(DV_THREADS)
 k_dv_ritz(int64_t n, int k, const double* V, const double* __restrict__ AV, DvCoef c, double theta, double guard,
           const double* __restrict__ dg, double* __restrict__ X, double* __restrict__ HX,
           double* __restrict__ Rv, double* t, double* part, unsigned* counter, double* sc, double* sc_host) {
+  itg_grid_wait();
   __shared__ double sh[4][DV_THREADS / 32 + 1];
   const int kk = K ? K : k;
   double sr = 0.0, sx = 0.0, st = 0.0;
@@ -545,6 +549,7 @@ template <int K>
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_proj(int64_t n, const double* __restrict__ V, const double* __restrict__ t, double* part, unsigned* counter,
           double* c) {
+  itg_grid_wait();
   __shared__ double sh[4][DV_THREADS / 32 + 1];
   const int nb = gridDim.x, b = blockIdx.x;
   const int64_t chunk = (n + nb - 1) / nb;
@@ -572,6 +577,7 @@ template <int K>
 __global__ void __launch_bounds__(DV_THREADS)
 k_dv_sub(int64_t n, int k, const double* V, const double* __restrict__ c, double* t, double* part, unsigned* counter,
          double* out, double* out_host) {
+  itg_grid_wait();
   __shared__ double sh[32];
   const int kk = K ? K : k;
   double a = 0.0;
@@ -727,6 +733,9 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
     if (nb > ITG_GEMV_MAX_PART / k) nb = ITG_GEMV_MAX_PART / k;
     return (int)(nb < 1 ? 1 : nb);
   };
+  auto launch = [&](auto kernel, int grid, auto... args) -> int {
+    return itg_launch_after(h, itg_small_grid(h, grid), dim3((unsigned)grid), DV_THREADS, 0, kernel, args...);
+  };
   auto gram = [&](int k) -> int {
     if (k > DV_KMAX || (int64_t)k * k * chunks(k) > ITG_GEMV_MAX_PART) {
       double* G = coef + 32;
@@ -734,12 +743,12 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
       ITG_CUDA(h, cudaMemcpyAsync(hG, G, sizeof(double) * k * k, cudaMemcpyDeviceToHost, h->stream));
       return ITG_OK;
     }
+    int st = ITG_OK;
     dv_dispatch(k, [&](auto K) {
       if constexpr (decltype(K)::value > 0)
-        k_dv_gram<decltype(K)::value><<<chunks(k), DV_THREADS, 0, h->stream>>>(n, V, AV, h->gemv_part, cnt, hG);
+        st = launch(k_dv_gram<decltype(K)::value>, chunks(k), n, V, AV, h->gemv_part, cnt, hG);
     });
-    ITG_CHECK_LAUNCH(h);
-    return ITG_OK;
+    return st;
   };
   // two passes of t -= V (V^T t), then |t| into dsc[3]
   auto orthogonalise = [&](int k, double* t) -> int {
@@ -748,26 +757,26 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
         ITG_TRY(itg_gemv_t(h, n, k, V, n, t, coef));
         ITG_TRY(itg_scal(h, k, -1.0, coef));
       } else {
+        int st = ITG_OK;
         dv_dispatch(k, [&](auto K) {
           if constexpr (decltype(K)::value > 0)
-            k_dv_proj<decltype(K)::value><<<chunks(k), DV_THREADS, 0, h->stream>>>(n, V, t, h->gemv_part, cnt + 1,
-                                                                                  coef);
+            st = launch(k_dv_proj<decltype(K)::value>, chunks(k), n, V, t, h->gemv_part, cnt + 1, coef);
         });
+        ITG_TRY(st);
       }
       double* out = pass ? dsc + 3 : nullptr;
+      int st = ITG_OK;
       dv_dispatch(k, [&](auto K) {
-        k_dv_sub<decltype(K)::value><<<nbn, DV_THREADS, 0, h->stream>>>(n, k, V, coef, t, part, cnt + 2, out, hp + 3);
+        st = launch(k_dv_sub<decltype(K)::value>, nbn, n, k, V, coef, t, part, cnt + 2, out, hp + 3);
       });
-      ITG_CHECK_LAUNCH(h);
+      ITG_TRY(st);
     }
     return ITG_OK;
   };
   auto scale = [&](const double* nrm, const double* x, double* y, const double* x2, double* y2) -> int {
-    k_dv_scale<<<gb, 256, 0, h->stream>>>(n, nrm, x, y, x2, y2);
-    ITG_CHECK_LAUNCH(h);
-    return ITG_OK;
+    return launch(k_dv_scale, gb, n, nrm, x, y, x2, y2);
   };
-  k_dv_norm<<<nbn, DV_THREADS, 0, h->stream>>>(n, psi, part, cnt + 3, dsc + 4, hp + 4);
+  ITG_TRY(launch(k_dv_norm, nbn, n, psi, part, cnt + 3, dsc + 4, hp + 4));
   ITG_TRY(scale(dsc + 4, psi, V, nullptr, nullptr));
   ITG_TRY(matvec_direct(V, AV));
   if (h->use_graphs) ITG_TRY(capture());
@@ -796,7 +805,7 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
         // preconditioned residual lies almost in span(V)): the plain residual instead
         double* t = V + (int64_t)(k - 1) * n;
         ITG_CUDA(h, cudaMemcpyAsync(t, Rv, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
-        k_dv_norm<<<nbn, DV_THREADS, 0, h->stream>>>(n, t, part, cnt + 3, dsc + 2, hp + 2);
+        ITG_TRY(launch(k_dv_norm, nbn, n, t, part, cnt + 3, dsc + 2, hp + 2));
         ITG_TRY(orthogonalise(k - 1, t));
         ITG_CUDA(h, cudaStreamSynchronize(h->stream));
         accept = hp[3] > 1e-6 * hp[2] && hp[3] > 1e-14;
@@ -828,11 +837,12 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
     for (int i = 0; i < k; ++i) c.y[i] = y[i];
     const double guard = 1e-8 * (fabs(theta) > 1.0 ? fabs(theta) : 1.0);
     double* t = k < kmax ? V + (int64_t)k * n : nullptr;
+    int st = ITG_OK;
     dv_dispatch(k, [&](auto K) {
-      k_dv_ritz<decltype(K)::value><<<nbn, DV_THREADS, 0, h->stream>>>(n, k, V, AV, c, theta, guard, dg, X, HX, Rv,
-                                                                      t, part, cnt + 3, dsc, hp);
+      st = launch(k_dv_ritz<decltype(K)::value>, nbn, n, k, V, AV, c, theta, guard, dg, X, HX, Rv, t, part, cnt + 3, dsc,
+                  hp);
     });
-    ITG_CHECK_LAUNCH(h);
+    ITG_TRY(st);
     if (k == kmax) {
       if (restart == maxiter - 1) break;
       // restart from the Ritz pair, unless its residual turns out converged

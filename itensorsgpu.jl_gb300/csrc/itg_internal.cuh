@@ -176,6 +176,45 @@ int itg_fail(itg_handle* h, int code, const char* fmt, ...);
 
 #define ITG_CHECK_LAUNCH(h) ITG_CUDA((h), cudaGetLastError())
 
+// A kernel that was started while its predecessor on the stream drains: what
+// comes before this call may overlap it, what comes after sees its results (and
+// those of everything before it, as every kernel so launched waits in turn).
+__device__ __forceinline__ void itg_grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a kernel that calls itg_grid_wait.  overlap: it may start early (not
+// when the last thing put on the stream is an event or a wait for one, nor
+// inside a capture).
+// Blocks that start early are placed on the SMs that drain first.  A grid of up
+// to one block an SM gains its launch (N = 20 DMRG, some 100 small kernels a
+// bond, 79 -> 68 ms); a larger one that is bound by the FP64 pipes ends up uneven (H_eff at
+// chi = 181 457 -> 504 us), so those launch plainly (itg_small_grid).
+template <class... P, class... A>
+int itg_launch_after(itg_handle* h, bool overlap, dim3 grid, int threads, size_t smem, void (*kernel)(P...),
+                     A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
+  return ITG_OK;
+}
+
+inline bool itg_small_grid(const itg_handle* h, int64_t blocks) { return blocks <= h->num_sms; }
+
+inline bool itg_capturing(itg_handle* h) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
 #define ITG_TRY(expr)            \
   do {                           \
     int _s = (expr);             \

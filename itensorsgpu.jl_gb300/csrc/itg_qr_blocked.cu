@@ -19,29 +19,6 @@ int house_panel(itg_handle* h, bool fast, bool after_kernel, double* A, int64_t 
 
 namespace {
 
-// Every kernel here starts while its predecessor on the stream drains and waits
-// for its results itself.
-__device__ __forceinline__ void grid_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// after_kernel: the last thing put on the stream is a kernel (not an event or a copy)
-template <class... P, class... A>
-int launch_after(itg_handle* h, bool after_kernel, dim3 grid, int threads, void (*kernel)(P...), A... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.stream = h->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = after_kernel ? 1 : 0;
-  ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
-  return ITG_OK;
-}
-
 // T (32 x 32, upper triangular) from the partial sums of Y = V^T V (column c
 // of chunk q at part[32 (q bw + c)]): LAPACK's larft,
 //   T(j,j) = tau_j, T(0:j, j) = -tau_j T(0:j, 0:j) Y(0:j, j),
@@ -54,7 +31,7 @@ __global__ void __launch_bounds__(256)
 k_larft(const double* __restrict__ part, int nchunk, const double* __restrict__ tau, int bw, double* __restrict__ T) {
   constexpr int NB = QR_NB, NW = 8, CW = NB / NW;
   __shared__ double Y[NB][NB + 1], col[2][NB];  // Y[column][row]; column l of T
-  grid_wait();
+  itg_grid_wait();
   const int i = threadIdx.x % NB, w = threadIdx.x / NB;
   double tj[CW], s[CW], t[CW];
 #pragma unroll
@@ -105,7 +82,7 @@ k_skinny_partial(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, c
                  int64_t ldb, int64_t b0, int64_t N, int64_t kchunk, double* __restrict__ part) {
   __shared__ double vs[SK_ROWS][SK_TILE_K];
   __shared__ double bs[32][SK_TILE_K + 1];
-  grid_wait();
+  itg_grid_wait();
   const int t = threadIdx.x, r = t / 32, c = t % 32, r0 = blockIdx.z * SK_ROWS;
   const int64_t c0 = (int64_t)blockIdx.x * 32;
   const int64_t K = m - jb;
@@ -142,7 +119,7 @@ k_skinny_t(const double* __restrict__ part, int nchunk, int bw, int64_t N, const
   __shared__ double z[8][NB], Ts[NB][NB + 1];
   const int t = threadIdx.x, r = t % NB, cl = t / NB;
   const int64_t c = (int64_t)blockIdx.x * 8 + cl;
-  grid_wait();
+  itg_grid_wait();
   for (int i = t; i < NB * NB; i += 256) Ts[i / NB][i % NB] = T[i];  // [column][row]
   double s = 0.0;
   if (c < N && r < bw)
@@ -169,7 +146,7 @@ k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const 
             double* __restrict__ C, int64_t c0) {
   constexpr int NB = QR_NB, TM = HALF ? 16 : 32, TN = HALF ? 8 : 16, U = HALF ? 1 : 2;
   __shared__ double vs[NB][TM + 1], zs[TN][NB + 1];
-  grid_wait();
+  itg_grid_wait();
   const int t = threadIdx.x;
   const int64_t r0 = jb + (int64_t)blockIdx.x * TM, n0 = (int64_t)blockIdx.y * TN;
 #pragma unroll
@@ -209,8 +186,8 @@ k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const 
 }
 
 // Partial sums of V_p^T B into part; nchunk: how many.
-int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, int64_t jb, int bw, const double* B, int64_t ldb,
-                int64_t b0, int64_t N, double* part, int64_t part_doubles, int* nchunk_out) {
+int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, int64_t jb, int bw, const double* B,
+                int64_t ldb, int64_t b0, int64_t N, double* part, int64_t part_doubles, int* nchunk_out) {
   const int64_t K = m - jb;
   const int64_t ntile = (N + 31) / 32;
   int64_t nchunk = (4 * (int64_t)h->num_sms + ntile - 1) / ntile;
@@ -221,7 +198,8 @@ int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, i
   const int64_t kchunk = ((K + nchunk - 1) / nchunk + SK_TILE_K - 1) / SK_TILE_K * SK_TILE_K;
   nchunk = (K + kchunk - 1) / kchunk;
   const dim3 grid((unsigned)ntile, (unsigned)nchunk, 32 / SK_ROWS);
-  ITG_TRY(launch_after(h, after_kernel, grid, 256, k_skinny_partial, Vh, m, jb, bw, B, ldb, b0, N, kchunk, part));
+  ITG_TRY(itg_launch_after(h, after_kernel, grid, 256, 0, k_skinny_partial, Vh, m, jb, bw, B, ldb, b0, N, kchunk,
+                           part));
   *nchunk_out = (int)nchunk;
   return ITG_OK;
 }
@@ -229,19 +207,20 @@ int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, i
 // C(jb:m, c0 : c0 + N) -= V_p (op(T_p) (V_p^T C(jb:m, c0 : c0 + N))) on the
 // handle's current stream; Z2 holds 32 N doubles.
 template <bool TRANS>
-int wy_apply(itg_handle* h, bool after_kernel, double* C, int64_t m, int64_t jb, int bw, const double* Vh, const double* Tp, int64_t c0,
-             int64_t N, double* Z2, double* part, int64_t part_doubles) {
+int wy_apply(itg_handle* h, bool after_kernel, double* C, int64_t m, int64_t jb, int bw, const double* Vh,
+             const double* Tp, int64_t c0, int64_t N, double* Z2, double* part, int64_t part_doubles) {
   if (N <= 0) return ITG_OK;
   int nchunk = 0;
   ITG_TRY(skinny_vt_b(h, after_kernel, Vh, m, jb, bw, C, m, c0, N, part, part_doubles, &nchunk));
-  ITG_TRY(launch_after(h, true, dim3((unsigned)((N + 7) / 8)), 256, k_skinny_t<TRANS>, part, nchunk, bw, N, Tp, Z2));
+  ITG_TRY(itg_launch_after(h, true, dim3((unsigned)((N + 7) / 8)), 256, 0, k_skinny_t<TRANS>, part, nchunk, bw, N, Tp,
+                           Z2));
   const bool half = ((m - jb + 31) / 32) * ((N + 15) / 16) < h->num_sms;
   const int tm = half ? 16 : 32, tn = half ? 8 : 16;
   const int64_t gx = (m - jb + tm - 1) / tm, gy = (N + tn - 1) / tn;
   for (int64_t y = 0; y < gy; y += 65535) {  // the grid's y limit
     const dim3 grid((unsigned)gx, (unsigned)(gy - y < 65535 ? gy - y : 65535));
-    ITG_TRY(launch_after(h, true, grid, 128, half ? k_wy_update<true> : k_wy_update<false>, Vh, m, jb, bw,
-                         Z2 + y * tn * QR_NB, N - y * tn, C, c0 + y * tn));
+    ITG_TRY(itg_launch_after(h, true, grid, 128, 0, half ? k_wy_update<true> : k_wy_update<false>, Vh, m, jb, bw,
+                             Z2 + y * tn * QR_NB, N - y * tn, C, c0 + y * tn));
   }
   return ITG_OK;
 }
@@ -317,7 +296,7 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
       OnStream on(h, h->qr_stream);
       int nchunk = 0;
       ITG_TRY(skinny_vt_b(h, true, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
-      ITG_TRY(launch_after(h, true, dim3(1), 256, k_larft, partp, nchunk, tau + jb, (int)bw, Tp));
+      ITG_TRY(itg_launch_after(h, true, dim3(1), 256, 0, k_larft, partp, nchunk, tau + jb, (int)bw, Tp));
       if (nt <= 0) continue;
       // V_p and T_p are final: the handle's stream may update the rest
       ITG_CUDA(h, cudaEventRecord(h->qr_ev_ready, h->stream));

@@ -137,12 +137,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
-// A kernel started while its predecessor on the stream drains: everything before
-// this call may overlap it, everything after sees its results.
-__device__ __forceinline__ void grid_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -499,7 +493,7 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  grid_wait();
+  itg_grid_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -871,7 +865,7 @@ struct PrepOp {
 constexpr int ZERO_BLOCK = 16 * 256;  // 16-byte words a block
 __global__ void __launch_bounds__(256)
 k_split_exponents(PrepOp a, PrepOp b, uint4* zero, int64_t nzero) {
-  grid_wait();
+  itg_grid_wait();
   int64_t blk = blockIdx.x;
   if (blk >= a.eblocks + b.eblocks) {
     const int64_t z0 = (blk - a.eblocks - b.eblocks) * ZERO_BLOCK;
@@ -1059,7 +1053,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
 #pragma unroll
     for (int p = 0; p < S; ++p)
       *(uint4*)(sA + (p >> 1) * MID_A_TILE + sw128_off(t, (p & 1) * MID_KSLICE + cg * 8)) = make_uint4(0u, 0u, 0u, 0u);
-  grid_wait();
+  itg_grid_wait();
   // B: digits of Weff's columns (row j of the B tiles, k = c), once per CTA
   {
     const int j = t >> 2, cg = t & 3;  // NJP * 4 <= 128 threads
@@ -1191,7 +1185,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
 __global__ void __launch_bounds__(256)
 k_make_slices(PrepOp a, PrepOp b) {
   __shared__ double tile[32][65];
-  grid_wait();
+  itg_grid_wait();
   int64_t blk = blockIdx.x;
   if (blk >= a.sblocks) {
     blk -= a.sblocks;
@@ -1284,25 +1278,6 @@ int make_map(itg_handle* h, CUtensorMap* map, void* base, int64_t inner, int64_t
 }
 
 int ws_reserve(itg_handle* h, size_t bytes);
-
-// Launches a kernel that waits for its predecessor itself (grid_wait), so that
-// it may start while that one drains; not inside a capture.
-template <class... P, class... A>
-int launch_waiting(itg_handle* h, bool capturing, unsigned grid, int threads, size_t smem, void (*kernel)(P...),
-                   A... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = h->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = capturing ? 0 : 1;
-  ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
-  return ITG_OK;
-}
 
 // CTAs of one variant that fit on the GPU at once (one per SM at this shared
 // memory size), queried once per variant.
@@ -1470,8 +1445,9 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
     const int64_t sb = op[0].sblocks + op[1].sblocks;
     if (eb > INT32_MAX || sb > INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: problem too large");
     if (eb > 0)
-      ITG_TRY(launch_waiting(h, capturing, (unsigned)eb, 256, 0, k_split_exponents, op[0], op[1], (uint4*)tacc, nzero));
-    if (sb > 0) ITG_TRY(launch_waiting(h, capturing, (unsigned)sb, 256, 0, k_make_slices, op[0], op[1]));
+      ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)eb), 256, 0, k_split_exponents, op[0], op[1], (uint4*)tacc,
+                               nzero));
+    if (sb > 0) ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)sb), 256, 0, k_make_slices, op[0], op[1]));
   }
   for (int i = 0; i < 2; ++i) {
     if (!cache[i] || hit[i]) continue;
@@ -1512,7 +1488,8 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   a.err = err;
   {
     ProfScope prof(h, ITG_KERNEL_GEMM_SPLIT);
-    ITG_TRY(launch_waiting(h, capturing, (unsigned)grid, NUM_THREADS, Smem<BN>::TOTAL, k_split_gemm<BN>, mA, mB, a));
+    ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)grid), NUM_THREADS, Smem<BN>::TOTAL, k_split_gemm<BN>, mA, mB,
+                             a));
   }
   ITG_CHECK_LAUNCH(h);
   return ITG_OK;
@@ -1539,10 +1516,8 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
     // three CTAs per SM: by shared memory (the carveout is set to its maximum)
     // and registers; TMEM (512 columns per SM) would allow four
     const int64_t g = std::min<int64_t>(grid, (int64_t)3 * h->num_sms);
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    ITG_CUDA(h, cudaStreamIsCapturing(h->stream, &cap));
-    ITG_TRY(launch_waiting(h, cap != cudaStreamCaptureStatusNone, (unsigned)g, MID_THREADS, MidSmem<NPASS>::TOTAL,
-                           k_heff_mid_split<NPASS>, T1, Weff, T3, R, nc, nj, h->wait_ns, err));
+    ITG_TRY(itg_launch_after(h, !itg_capturing(h), dim3((unsigned)g), MID_THREADS, MidSmem<NPASS>::TOTAL,
+                             k_heff_mid_split<NPASS>, T1, Weff, T3, R, nc, nj, h->wait_ns, err));
     return ITG_OK;
   };
   {
