@@ -741,6 +741,81 @@ k_jacobi_reg_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, float 
   if (t == 0 && any_major) *rotated = 1;
 }
 
+// All FP32 sweeps of a small start in one launch: n <= 48 columns of W (m <= 32 RPT
+// rows, FP64, times a power of two `scale`) and of V in shared memory, a warp a
+// pair of the element-wise round robin, one barrier a round.  V goes out in FP64.
+// Bound by a round's latency (sums over a warp, angle, barrier: 0.45 us); the
+// blocked steps above take 8 us for eight rounds and a launch each, and the host
+// has to wait for their flags: n = 48 (all of the start but its products) 390 -> 177
+// us, n = 20 250 -> 52; n = 64 no longer gains.
+constexpr int JS_MAX_N = 48, JS_V = 64;  // columns; rows kept of V
+template <int RPT>
+__global__ void __launch_bounds__(JS_MAX_N / 2 * 32)
+k_jacobi32_small(const double* __restrict__ W, int m, int n, double scale, float tol, float amin,
+                 float amin_conv, int max_sweeps, double* __restrict__ V) {
+  constexpr int ROWS = 32 * RPT;
+  extern __shared__ float js_smem[];
+  float* w = js_smem;                  // [n][ROWS]
+  float* v = js_smem + n * ROWS;       // [n][JS_V]
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, bd = (int)blockDim.x, np = n + (n & 1);
+  for (int i = t; i < n * ROWS; i += bd) {
+    const int c = i / ROWS, r = i % ROWS;
+    w[i] = r < m ? (float)(W[(int64_t)c * m + r] * scale) : 0.f;
+  }
+  for (int i = t; i < n * JS_V; i += bd) v[i] = i / JS_V == i % JS_V ? 1.f : 0.f;
+  __syncthreads();
+  int p = warp, q = np - 1 - warp;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    int major_any = 0;
+    for (int step = 0; step < np - 1; ++step) {
+      if (p < n && q < n) {  // warp-uniform
+        float *wp = w + p * ROWS + lane, *wq = w + q * ROWS + lane;
+        float *vp = v + p * JS_V + lane, *vq = v + q * JS_V + lane;
+        float x[RPT], y[RPT], a = 0.f, b = 0.f, g = 0.f;
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+          x[k] = wp[32 * k];
+          y[k] = wq[32 * k];
+          a = fmaf(x[k], x[k], a);
+          b = fmaf(y[k], y[k], b);
+          g = fmaf(x[k], y[k], g);
+        }
+        const float v0 = vp[0], v1 = vp[32], u0 = vq[0], u1 = vq[32];
+        // the three sums in one tree: lanes 0-7 end with a, 8-15 with b, 16-23 with g
+        const bool hi = lane & 16, mid = lane & 8;
+        const float e = (hi ? g : a) + __shfl_xor_sync(0xffffffffu, hi ? a : g, 16);
+        const float f = (hi ? 0.f : b) + __shfl_xor_sync(0xffffffffu, hi ? b : 0.f, 16);
+        float d = (mid ? f : e) + __shfl_xor_sync(0xffffffffu, mid ? e : f, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        a = __shfl_sync(0xffffffffu, d, 0);
+        b = __shfl_sync(0xffffffffu, d, 8);
+        g = __shfl_sync(0xffffffffu, d, 16);
+        float tt, u, s;
+        bool major;
+        if (jp_angle(a, b, g, tol, tol, amin, amin_conv, tt, u, s, major)) {
+#pragma unroll
+          for (int k = 0; k < RPT; ++k) {
+            wp[32 * k] = fmaf(-s, fmaf(u, x[k], y[k]), x[k]);
+            wq[32 * k] = fmaf(s, fmaf(-u, y[k], x[k]), y[k]);
+          }
+          vp[0] = fmaf(-s, fmaf(u, v0, u0), v0);
+          vq[0] = fmaf(s, fmaf(-u, u0, v0), u0);
+          vp[32] = fmaf(-s, fmaf(u, v1, u1), v1);
+          vq[32] = fmaf(s, fmaf(-u, u1, v1), u1);
+          major_any |= major;
+        }
+      }
+      // the players of the next step (0 keeps its place)
+      if (p > 0 && ++p == np) p = 1;
+      if (++q == np) q = 1;
+      __syncthreads();
+    }
+    if (!__syncthreads_or(major_any)) break;
+  }
+  for (int i = t; i < n * n; i += bd) V[i] = (double)v[i / n * JS_V + i % n];
+}
+
 // Self-test of the grid barrier's timeout path: every block arrives at a
 // barrier that counts one participant more than the grid has, so the count
 // is never met; each block waits until the limit, the first to give up raises
@@ -769,6 +844,30 @@ int grid_barrier_selftest(itg_handle* h, int* status, int* blocks_out) {
 }
 
 int jacobi_aux_ints(int max_sweeps) { return 8 + max_sweeps; }
+
+// The rotations V (n x n) of the FP32 start of W (m x n); false when it is too
+// large for the one-launch kernel.
+bool jacobi32_small_fits(const itg_handle* h, int64_t m, int64_t n) {
+  return h->jacobi_mode == 0 && n >= 2 && n <= JS_MAX_N && m <= 128;
+}
+int jacobi32_small(itg_handle* h, const double* W, int64_t m, int64_t n, double scale, float tol, float amin,
+                   float amin_conv, int max_sweeps, double* V) {
+  const bool tall = m > 64;
+  const size_t smem = sizeof(float) * (size_t)n * ((tall ? 128 : 64) + JS_V);
+  const int threads = 32 * (int)((n + 1) / 2);
+  static bool attr = false;
+  if (!attr) {
+    ITG_CUDA(h, cudaFuncSetAttribute(k_jacobi32_small<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    ITG_CUDA(h, cudaFuncSetAttribute(k_jacobi32_small<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    attr = true;
+  }
+  if (tall)
+    k_jacobi32_small<4><<<1, threads, smem, h->stream>>>(W, (int)m, (int)n, scale, tol, amin, amin_conv, max_sweeps, V);
+  else
+    k_jacobi32_small<2><<<1, threads, smem, h->stream>>>(W, (int)m, (int)n, scale, tol, amin, amin_conv, max_sweeps, V);
+  ITG_CHECK_LAUNCH(h);
+  return ITG_OK;
+}
 
 // Runs up to max_sweeps sweeps on W (m x n) accumulating into V (n x n, set
 // by the caller).  *sweeps = sweeps run; ITG_ERR_NOTCONVERGED when the limit
@@ -872,9 +971,10 @@ int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_
              int* sweeps) {
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
   const int threads = (int)((m + RPT - 1) / RPT + 31) / 32 * 32;
-  // a queued step costs about 2 us when it has nothing to do, a look at the
-  // flags about 20 us
-  const int chunk = n <= 48 ? 5 : (n <= 160 ? 2 : 1);
+  // a queued step costs about 1 us when it has nothing to do, a look at the flags
+  // about 25: FP32 takes six sweeps and more, FP64 (after the FP32 start, which
+  // smaller problems do not take) mostly one
+  const int chunk = sizeof(T) == 4 ? (n <= 160 ? 7 : (n <= 512 ? 4 : 1)) : (n < 16 ? 5 : 1);
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;

@@ -500,6 +500,7 @@ __device__ __forceinline__ double rotation_generator(double gii, double gjj, dou
 // Row j's sum of |k_ij|, and the diagonal of G.
 __global__ void __launch_bounds__(128)
 k_generator_rows(const double* __restrict__ G, int n, double* __restrict__ diag, double* __restrict__ rows) {
+  itg_grid_wait();
   __shared__ double sh[4];
   const int j = blockIdx.x;
   const double gjj = G[(int64_t)j * (n + 1)];
@@ -520,6 +521,7 @@ k_generator_rows(const double* __restrict__ G, int n, double* __restrict__ diag,
 // Newton-Schulz step then makes it so to rounding.
 __global__ void k_generator(const double* __restrict__ G, int n, const double* __restrict__ diag,
                             const double* __restrict__ rows, double* __restrict__ K, double* __restrict__ M) {
+  itg_grid_wait();
   const int64_t nn = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x) {
     const int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
@@ -539,6 +541,7 @@ __global__ void k_copy_scaled(const double* __restrict__ x, int64_t n, double a,
 
 // P <- (3 I - P) / 2: X P is the Newton-Schulz step for P = X^T X
 __global__ void k_newton_schulz(double* P, int n) {
+  itg_grid_wait();
   const int64_t nn = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x)
     P[t] = (t % (n + 1) == 0 ? 1.5 : 0.0) - 0.5 * P[t];
@@ -561,6 +564,10 @@ __global__ void k_newton_schulz(double* P, int n) {
 // ms, n = 120 4.6 / 5.2 -> 2.7 / 2.9, n = 192 9.7 / 10.3 -> 4.3 / 4.6; n = 378
 // (FP32 start without the refinements before) 16.5 / 15.1 -> 14.4 / 10.9.
 // ws: start32_ws_doubles(m, n) doubles, ws32: m n + n^2 floats.
+bool jacobi32_small_fits(const itg_handle* h, int64_t m, int64_t n);
+int jacobi32_small(itg_handle* h, const double* W, int64_t m, int64_t n, double scale, float tol, float amin,
+                   float amin_conv, int max_sweeps, double* V);
+
 int64_t start32_ws_doubles(int64_t m, int64_t n) { return 3 * n * n + m * n + 2 * n; }
 
 int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, double fro, double* ws, float* ws32,
@@ -568,25 +575,29 @@ int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, do
   // a power of two: A's squares then stay in range, and scaling it is exact
   const int ex = std::ilogb(fro);
   const double scale = std::ldexp(1.0, ex < -1000 ? 1000 : -ex);
-  float* W32 = ws32;
-  float* V32 = ws32 + m * n;
-  k_to_float<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m * n, scale, W32);
-  k_identity32<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>((int)n, V32);
-  ITG_CHECK_LAUNCH(h);
   const double f = fro * scale;  // in [1, 2)
-  int sweeps = 0;
   // columns below 1e-15 of the norm are left alone (their squares leave FP32's
   // range), those below 1e-7 do not keep the sweeps running
-  const int st = itg::jacobi_blocked<float>(h, W32, m, (int)n, V32, 1e-5f, (float)(1e-30 * f * f), 30, flag, &sweeps,
-                                            (float)(1e-14 * f * f));
-  if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
+  const float amin = (float)(1e-30 * f * f), amin_conv = (float)(1e-14 * f * f);
   double* P = ws;
   double* M = P + n * n;
   double* Y = M + n * n;
   double* A = Y + n * n;
   double* diag = A + m * n;
   double* rows = diag + n;
-  k_to_double<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(V32, n * n, Y);
+  if (jacobi32_small_fits(h, m, n)) {
+    ITG_TRY(jacobi32_small(h, W, m, n, scale, 1e-5f, amin, amin_conv, 30, Y));
+  } else {
+    float* W32 = ws32;
+    float* V32 = ws32 + m * n;
+    int sweeps = 0;
+    k_to_float<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m * n, scale, W32);
+    k_identity32<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>((int)n, V32);
+    ITG_CHECK_LAUNCH(h);
+    const int st = itg::jacobi_blocked<float>(h, W32, m, (int)n, V32, 1e-5f, amin, 30, flag, &sweeps, amin_conv);
+    if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
+    k_to_double<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(V32, n * n, Y);
+  }
   k_copy_scaled<<<itg_blocks_for(m * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(W, m * n, scale, A);
   ITG_CHECK_LAUNCH(h);
   // heuristic tiles: timing the variants of each new shape would cost more than the products
@@ -597,19 +608,18 @@ int jacobi_start32(itg_handle* h, double* W, int64_t m, int64_t n, double* V, do
     ~NoTune() { h->autotune = was; }
   } no_tune(h);
   const int gb = itg_blocks_for(n * n, 256, h->num_sms * 16);
+  const bool overlap = itg_small_grid(h, gb);
   auto newton_schulz = [&](const double* X, double* Q, double* out) -> int {  // out = X (3 I - X^T X) / 2
     ITG_TRY(gemm(h, true, n, n, n, 1.0, X, X, 0.0, Q, ITG_PREC_FP64));
-    k_newton_schulz<<<gb, 256, 0, h->stream>>>(Q, (int)n);
-    ITG_CHECK_LAUNCH(h);
+    ITG_TRY(itg_launch_after(h, overlap, dim3(gb), 256, 0, k_newton_schulz, Q, (int)n));
     return gemm(h, false, n, n, n, 1.0, X, Q, 0.0, out, ITG_PREC_FP64);
   };
   ITG_TRY(newton_schulz(Y, P, V));
   for (int it = 0; it < 2; ++it) {
     ITG_TRY(gemm(h, false, m, n, n, 1.0, A, V, 0.0, W, ITG_PREC_FP64));
     ITG_TRY(gemm(h, true, n, n, m, 1.0, W, W, 0.0, P, ITG_PREC_FP64));
-    k_generator_rows<<<(int)n, 128, 0, h->stream>>>(P, (int)n, diag, rows);
-    k_generator<<<gb, 256, 0, h->stream>>>(P, (int)n, diag, rows, Y, M);
-    ITG_CHECK_LAUNCH(h);
+    ITG_TRY(itg_launch_after(h, overlap, dim3((unsigned)n), 128, 0, k_generator_rows, P, (int)n, diag, rows));
+    ITG_TRY(itg_launch_after(h, overlap, dim3(gb), 256, 0, k_generator, P, (int)n, diag, rows, Y, M));
     ITG_TRY(gemm(h, false, n, n, n, 0.5, Y, Y, 1.0, M, ITG_PREC_FP64));
     ITG_TRY(gemm(h, false, n, n, n, 1.0, V, M, 0.0, P, ITG_PREC_FP64));
     ITG_TRY(newton_schulz(P, Y, V));
