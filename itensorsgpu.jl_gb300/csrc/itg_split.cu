@@ -965,10 +965,11 @@ __device__ __forceinline__ uint4 pack_digits8(const unsigned long long (&w)[8], 
 // row of T1 (coalesced across the CTA per c), forms the row exponent and the
 // 6 balanced digits of each element, and writes them K-major with the
 // 128-byte swizzle into shared memory, two slices per 128-byte row (slice p
-// at k offset 32 (p % 2) of tile p / 2); Weff's column digits are written the
-// same way once per CTA.  One thread issues the 21 digit products (one or two
-// K = 16 steps each) into six TMEM level accumulators of 16 columns, in two
-// passes for nj > 16 (the second beside the conversion of the first); one
+// at k offset 32 (p % 2) of tile p / 2); Weff's column digits once per CTA, a
+// row each digit and column.  Warp 0 issues the digit products into six TMEM
+// level accumulators of 16 columns, in two passes for nj > 16 (the second beside
+// the conversion of the first): digit p of A with digits 0 .. 5 - p of B is one
+// product of 16 (6 - p) columns, six (or twelve, K = 16 each) instead of 21; one
 // group per level suffices because sum_{p+q=L} nc |a_p| |b_q| <= 32 (2 * 2^15
 // + 4 * 2^14) = 2^22 keeps every FP32 partial sum an exact integer.  Each thread then reads
 // its row's level sums, forms the int64 fixed-point value and converts it to
@@ -979,7 +980,9 @@ __device__ __forceinline__ uint4 pack_digits8(const unsigned long long (&w)[8], 
 // of an SM overlap theirs.  At chi = 1024 (2^20 rows, nc = nj = 20; its reads and
 // writes take 50 us at the measured HBM rate) 379 -> 255 us: digits as one biased
 // word (33 instead of 65 instructions an element), level sums combined in
-// pairs in 32 bits, 128 instead of 256 TMEM columns (two CTAs an SM before).
+// pairs in 32 bits, 128 instead of 256 TMEM columns (two CTAs an SM before); then
+// -> 188 us: a quarter of the products to issue (42 took 1.3 us a pass), and the
+// passes one loop (a fifth of the warps' stalls waited for instructions).
 constexpr int MID_ROWS = 128;
 constexpr int MID_THREADS = 128;
 constexpr int MID_KSLICE = 32;  // padded K per slice (nc <= 32)
@@ -989,12 +992,11 @@ constexpr int MID_NTILE = (S_SLICES + 1) / 2;  // 3 tiles hold the 6 slices
 constexpr uint32_t MID_TMEM_COLS = 128;        // six level accumulators of 16 columns
 
 // NPASS: passes over 16 output columns.
-template <int NPASS>
+constexpr int MID_B_TILE = S_SLICES * 16 * 128;  // bytes: a row (128 B, 32 k of each pass) a digit and column
 struct MidSmem {
-  static constexpr int B_TILE = NPASS * 16 * 128;
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = MID_NTILE * MID_A_TILE;
-  static constexpr int TOTAL = 1024 /*align slack*/ + B_OFF + MID_NTILE * B_TILE + 256;
+  static constexpr int TOTAL = 1024 /*align slack*/ + B_OFF + MID_B_TILE + 256;
 };
 
 // byte offset of element (row i, k) of a K-major 128-byte-swizzled tile
@@ -1020,6 +1022,21 @@ __device__ __forceinline__ void digits8(uint8_t* tiles, int tile_bytes, int i, i
   *(uint4*)(tiles + 2 * tile_bytes + odd) = pack_digits8<5>(w, sg);
 }
 
+// The same of a column of B: digit q in row 16 q + i, at k offset c0.
+__device__ __forceinline__ void digits8_rows(uint8_t* tile, int i, int c0, const double* x, int ef) {
+  unsigned long long w[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = digit_word(x[e], ef);
+  const uint32_t sg[4] = {digit_signs(x[0], x[1]), digit_signs(x[2], x[3]), digit_signs(x[4], x[5]),
+                          digit_signs(x[6], x[7])};
+  *(uint4*)(tile + sw128_off(i, c0)) = pack_digits8<0>(w, sg);
+  *(uint4*)(tile + sw128_off(16 + i, c0)) = pack_digits8<1>(w, sg);
+  *(uint4*)(tile + sw128_off(32 + i, c0)) = pack_digits8<2>(w, sg);
+  *(uint4*)(tile + sw128_off(48 + i, c0)) = pack_digits8<3>(w, sg);
+  *(uint4*)(tile + sw128_off(64 + i, c0)) = pack_digits8<4>(w, sg);
+  *(uint4*)(tile + sw128_off(80 + i, c0)) = pack_digits8<5>(w, sg);
+}
+
 template <int NPASS>
 __global__ void __launch_bounds__(MID_THREADS, 3)
 k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff, double* __restrict__ T3,
@@ -1028,9 +1045,9 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
   constexpr int NJP = 16 * NPASS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = base + MidSmem<NPASS>::A_OFF;
-  uint8_t* sB = base + MidSmem<NPASS>::B_OFF;
-  uint8_t* tail = sB + MID_NTILE * MidSmem<NPASS>::B_TILE;
+  uint8_t* sA = base + MidSmem::A_OFF;
+  uint8_t* sB = base + MidSmem::B_OFF;
+  uint8_t* tail = sB + MID_B_TILE;
   uint64_t* done = (uint64_t*)tail;
   uint32_t* tmem_slot = (uint32_t*)(tail + 8);
   int* fB = (int*)(tail + 16);  // [NJP] column exponent fields of Weff
@@ -1075,7 +1092,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
         const int c = cg * 8 + e;
         w[e] = (j < nj && c < nc) ? Weff[c + (int64_t)nc * j] : 0.0;
       }
-      digits8(sB, MidSmem<NPASS>::B_TILE, j, cg * 8, w, ef);
+      digits8_rows(sB, j & 15, MID_KSLICE * (j >> 4) + cg * 8, w, ef);
     }
   }
   tc_fence_before();
@@ -1085,21 +1102,22 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
   const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
   const int ksteps = nc > 16 ? 2 : 1;
   const int64_t nblk = (R + MID_ROWS - 1) / MID_ROWS;
-  // the 21 digit products of output columns 16 h .. 16 h + 15 (one thread)
+  // The 21 digit products of output columns 16 h .. 16 h + 15 (warp 0): digit p
+  // of A meets digits 0 .. 5 - p of B, whose rows and whose levels' columns lie
+  // side by side, in one product of 16 (6 - p) columns.
   auto issue = [&](int h) {
-    constexpr uint32_t idesc = idesc_bf16(MID_ROWS, 16);
-    for (int L = 0; L < S; ++L) {
-      for (int p = 0; p <= L; ++p) {
-        const int q = L - p;
-        const uint64_t ad = sdesc_sw128(smem_u32(sA + (p >> 1) * MID_A_TILE));
-        const uint64_t bd = sdesc_sw128(smem_u32(sB + (q >> 1) * MidSmem<NPASS>::B_TILE + h * 16 * 128));
-        for (int s = 0; s < ksteps; ++s) {
-          const uint64_t ka = (uint64_t)(2 * (2 * (p & 1) + s)), kb = (uint64_t)(2 * (2 * (q & 1) + s));
-          tc_mma_bf16(tmem_base + (uint32_t)(L * 16), ad + ka, bd + kb, idesc, (p > 0 || s > 0) ? 1u : 0u);
-        }
+    const bool leader = elect_one();
+#pragma unroll
+    for (int p = 0; p < S; ++p) {
+      const uint32_t idesc = idesc_bf16(MID_ROWS, 16 * (S - p));
+      const uint64_t ad = sdesc_sw128(smem_u32(sA + (p >> 1) * MID_A_TILE)) + (uint64_t)(4 * (p & 1));
+      const uint64_t bd = sdesc_sw128(smem_u32(sB)) + (uint64_t)(4 * h);
+      if (leader) {
+        tc_mma_bf16(tmem_base + (uint32_t)(p * 16), ad, bd, idesc, p > 0 ? 1u : 0u);
+        if (ksteps > 1) tc_mma_bf16(tmem_base + (uint32_t)(p * 16), ad + 2, bd + 2, idesc, 1u);
       }
     }
-    tc_commit(done);
+    if (leader) tc_commit(done);
   };
   bool ok = true;
   uint32_t phase = 0;
@@ -1127,9 +1145,9 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (t == 0) issue(0);
+    if (warp == 0) issue(0);
     const int em = eA - 1022;
-#pragma unroll
+#pragma unroll 1
     for (int h = 0; h < NPASS; ++h) {
       // every thread waits (bounded) for the products, then takes its row's level sums
       ok = mbar_wait(done, phase, err, abort_flag, wait_ns);
@@ -1149,7 +1167,7 @@ k_heff_mid_split(const double* __restrict__ T1, const double* __restrict__ Weff,
       tc_fence_before();
       __syncthreads();
       tc_fence_after();
-      if (h + 1 < NPASS && t == 0) issue(h + 1);
+      if (h + 1 < NPASS && warp == 0) issue(h + 1);
       // fixed point sum_L s_L 2^(8 (5 - L)), the level sums in pairs first: each
       // is an integer of at most 2^22 in magnitude (float -> int by the
       // 1.5 * 2^23 shift), so s_L 2^8 + s_(L+1) fits in 32 bits
@@ -1508,7 +1526,7 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
     static bool attr = false;
     if (!attr) {
       ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       MidSmem<NPASS>::TOTAL));
+                                       MidSmem::TOTAL));
       ITG_CUDA(h, cudaFuncSetAttribute(k_heff_mid_split<NPASS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
       attr = true;
@@ -1516,7 +1534,7 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
     // three CTAs per SM: by shared memory (the carveout is set to its maximum)
     // and registers; TMEM (512 columns per SM) would allow four
     const int64_t g = std::min<int64_t>(grid, (int64_t)3 * h->num_sms);
-    ITG_TRY(itg_launch_after(h, !itg_capturing(h), dim3((unsigned)g), MID_THREADS, MidSmem<NPASS>::TOTAL,
+    ITG_TRY(itg_launch_after(h, !itg_capturing(h), dim3((unsigned)g), MID_THREADS, MidSmem::TOTAL,
                              k_heff_mid_split<NPASS>, T1, Weff, T3, R, nc, nj, h->wait_ns, err));
     return ITG_OK;
   };
