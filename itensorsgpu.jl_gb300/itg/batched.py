@@ -6,7 +6,7 @@ own bond dimensions and maxdim.  Every bond update runs for all instances at
 once: phi formation and environment updates as grouped contractions
 (itg_contract_grouped), the eigensolver as itg_davidson_heff2_batched (H_eff
 chain as grouped launches, segmented vector kernels), and the factorisation as
-itg_svd_trunc_batched (one CTA per instance).  Results equal looping
+itg_svd_trunc_batched (one CTA per instance) and itg_svd_absorb_batched.  Results equal looping
 itg.dmrg over the instances (same algorithm; the SVD is always FP64 Jacobi here).
 """
 from __future__ import annotations
