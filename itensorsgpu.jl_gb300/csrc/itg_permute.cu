@@ -223,6 +223,49 @@ k_perm_transpose(const double* __restrict__ A, double* B, const double* Bin, Per
   }
 }
 
+// The transpose by 32 x 32 tiles, blockIdx.y over the batches: four loads a
+// thread and eight CTAs an SM instead of eight and six.  It is the better one
+// where the scalars need FP64 instructions (they run between the loads of more
+// CTAs: 1.5 A - 0.5 B of 100 x 90 x 80 x 70 0.40 -> 0.32 ms) and where equal tiles leave
+// lanes idle that these fill (perm_tiles32).
+template <int OP>
+__global__ void __launch_bounds__(256)
+k_perm_transpose32(const double* __restrict__ A, double* B, const double* Bin, PermScalars sc, int64_t n0, int64_t nq,
+                   int64_t sqA, int64_t s0B, int64_t nbatch, RestDesc rest) {
+  constexpr int TP = 32;
+  __shared__ double tile[TP][TP + 1];
+  const int t0 = (int)((n0 + TP - 1) / TP), tq = (int)((nq + TP - 1) / TP), tiles = t0 * tq;
+  for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
+    int64_t oa, ob;
+    rest_offsets(rest, b, oa, ob);
+    for (int r = blockIdx.x; r < tiles; r += gridDim.x) {
+      const int iq = r / t0, i0 = r - iq * t0;
+      const int64_t base0 = (int64_t)i0 * TP, baseq = (int64_t)iq * TP;
+      // read along mode 0 (contiguous in A), all loads first
+      double v[TP / 8];
+#pragma unroll
+      for (int j = 0; j < TP / 8; ++j) {
+        const int64_t i = base0 + threadIdx.x, k = baseq + threadIdx.y + 8 * j;
+        v[j] = (i < n0 && k < nq) ? A[oa + i + k * sqA] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < TP / 8; ++j) tile[threadIdx.y + 8 * j][threadIdx.x] = v[j];
+      __syncthreads();
+      // write along mode q (contiguous in B)
+#pragma unroll
+      for (int j = 0; j < TP / 8; ++j) {
+        const int y = threadIdx.y + 8 * j;
+        const int64_t k = baseq + threadIdx.x, i = base0 + y;
+        if (i < n0 && k < nq) {
+          const int64_t o = ob + k + i * s0B;
+          B[o] = perm_op<OP>(sc, tile[threadIdx.x][y], perm_reads_b(OP) ? Bin[o] : 0.0);
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // Tile of the transpose: about 64 x 64, the other side longer where one mode
 // is short, and equal tiles within each mode; padded rows fit in 35 KB, so six
 // CTAs share an SM.  l0, lq: log2 of the lanes along each mode.
@@ -250,12 +293,18 @@ void perm_launch_rows(int blocks, cudaStream_t st, const double* A, double* B, c
                                                    fast_div(nseg > 1 ? 1 : (uint32_t)d0), items, rest);
 }
 
-template <int OP>
-void perm_launch_transpose(int blocks, size_t smem, cudaStream_t st, const double* A, double* B, const double* Bin,
-                           PermScalars sc, int64_t n0, int64_t nq, int64_t sqA, int64_t s0B, int e0, int eq, int l0,
-                           int lq, int64_t t0, int64_t tq, int64_t items, const RestDesc& rest) {
-  k_perm_transpose<OP><<<blocks, PERM_THREADS, smem, st>>>(A, B, Bin, sc, n0, nq, sqA, s0B, e0, eq, l0, lq, t0, tq,
-                                                           items, rest);
+// Whether 32 x 32 tiles take the transpose, by the share of working lanes against
+// theirs: for copies and sums below 0.65 (sum, 96 x 96: 0.56, 0.190 against 0.173 ms;
+// 80 x 80: 0.57, 0.206 against 0.189; but 100 x 80: 0.75, 0.304 against 0.321); with
+// general scalars up to 1.3 (100 x 80: 0.40 against 0.32 ms, 512 x 512: 1, 0.365 against
+// 0.361), above it a mode is short.
+bool perm_tiles32(int op, int64_t n0, int64_t nq, int e0, int eq, int l0, int lq) {
+  auto share = [](int64_t n, int e, int l) {
+    const int lanes = (e + (1 << l) - 1) >> l << l;
+    return (double)n / ((double)((n + e - 1) / e) * lanes);
+  };
+  const double r = share(n0, e0, l0) * share(nq, eq, lq) / (share(n0, 32, 5) * share(nq, 32, 5));
+  return r < (op == PERM_SCALE || op == PERM_AXPBY ? 1.3 : 0.65);
 }
 
 // Resolve modesB as a permutation of modesA.  perm[j] = A-position of B's mode j.
@@ -375,15 +424,24 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
     int64_t nbatch = total / (n0 * nq);
     int e0, eq, l0, lq;
     perm_tile(n0, nq, e0, eq, l0, lq);
-    const int64_t t0 = (n0 + e0 - 1) / e0, tq = (nq + eq - 1) / eq;
-    if (t0 * tq > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "permute: transpose too large");
-    const int64_t items = t0 * tq * nbatch;
-    const int blocks = (int)std::min<int64_t>(items, (int64_t)h->num_sms * 48);
-    const size_t smem = sizeof(double) * (size_t)eq * (e0 | 1);
     const int64_t sqA = d.strA[q], s0B = d.strB[0];
+    const bool small = perm_tiles32(op, n0, nq, e0, eq, l0, lq);
+    const int64_t t0 = (n0 + (small ? 32 : e0) - 1) / (small ? 32 : e0);
+    const int64_t tq = (nq + (small ? 32 : eq) - 1) / (small ? 32 : eq);
+    if (t0 * tq > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "permute: transpose too large");
     auto run = [&](auto tag) {
-      perm_launch_transpose<decltype(tag)::value>(blocks, smem, h->stream, A, B, bin, sc, n0, nq, sqA, s0B, e0, eq, l0,
-                                                  lq, t0, tq, items, rest);
+      constexpr int OP = decltype(tag)::value;
+      if (small) {
+        const int64_t want = (int64_t)h->num_sms * 32, gx = std::min<int64_t>(t0 * tq, want);
+        const int64_t gy = std::min<int64_t>(std::min<int64_t>(nbatch, std::max<int64_t>(1, want / gx)), 65535);
+        k_perm_transpose32<OP><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, h->stream>>>(A, B, bin, sc, n0, nq, sqA,
+                                                                                               s0B, nbatch, rest);
+      } else {
+        const int64_t items = t0 * tq * nbatch;
+        const int blocks = (int)std::min<int64_t>(items, (int64_t)h->num_sms * 48);
+        k_perm_transpose<OP><<<blocks, PERM_THREADS, sizeof(double) * (size_t)eq * (e0 | 1), h->stream>>>(
+            A, B, bin, sc, n0, nq, sqA, s0B, e0, eq, l0, lq, t0, tq, items, rest);
+      }
     };
     if (op == PERM_COPY) run(std::integral_constant<int, PERM_COPY>());
     else if (op == PERM_SCALE) run(std::integral_constant<int, PERM_SCALE>());
