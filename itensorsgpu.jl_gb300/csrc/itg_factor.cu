@@ -582,7 +582,7 @@ constexpr int64_t ONECTA_MAX_N = 192;
 constexpr int64_t PRECOND_MIN_N = 24;
 // From this many columns the FP64 Jacobi starts from the FP32 rotations
 // (jacobi_start32): below, its products cost what the sweeps do (n = 16 random
-// 0.59 -> 0.55 ms, sigma = exp(-32 k / n) 0.90 -> 0.91 ms).
+// 0.59 -> 0.44 ms, sigma = exp(-32 k / n) 0.90 -> 0.89 ms).
 constexpr int64_t START32_MIN_N = 16;
 // Below this many columns one CTA runs all sweeps in one launch (n = 10: 0.64
 // against 0.75 ms for the queued steps, n = 12: 0.87 against 0.82 ms).
