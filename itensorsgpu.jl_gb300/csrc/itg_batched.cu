@@ -4,6 +4,7 @@
 // per chain step for all instances) and whose vector operations are segmented
 // kernels over all instances' vectors at once.
 #include "itg_internal.cuh"
+#include "itg_rank.cuh"
 #include "itg_truncate.cuh"
 
 #include <cmath>
@@ -170,7 +171,7 @@ k_svd_batched(SvdJob* __restrict__ jobs, double tol_eps, int max_sweeps, TruncRu
     int r = 0;
     for (int i = 0; i < nn; ++i) {
       const double u = J.sig[i];
-      r += (u > v) || (u == v && i < j);
+      r += itg_rank_before(u, i, v, j);
     }
     J.order[r] = j;
     J.S[r] = v;

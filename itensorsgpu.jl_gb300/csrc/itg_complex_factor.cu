@@ -19,6 +19,7 @@
 // sigma^2) as the real path.  One launch per round-robin step; these serve
 // the complex tensors of the reference's tests, not the DMRG sweep.
 #include "itg_internal.cuh"
+#include "itg_rank.cuh"
 
 #include <cmath>
 
@@ -135,7 +136,7 @@ __global__ void k_zrank(const double* __restrict__ sig, int n, int* __restrict__
     int r = 0;
     for (int i = 0; i < n; ++i) {
       const double u = sig[i];
-      r += (u > v) || (u == v && i < j);
+      r += itg_rank_before(u, i, v, j);
     }
     order[r] = j;
     S[r] = v;
@@ -190,7 +191,7 @@ __global__ void k_zshift_rank(const double* __restrict__ sig, int n, double shif
     int r = 0;
     for (int i = 0; i < n; ++i) {
       const double u = sig[i];
-      r += (u > v) || (u == v && i < j);
+      r += itg_rank_before(u, i, v, j);
     }
     order[r] = j;
     D[r] = v - shift;

@@ -1,6 +1,7 @@
 // Factorisations: on-device truncation (K6), one-sided Jacobi SVD (K5),
 // symmetric eigendecomposition through the shifted SVD, and the thin Householder QR (K7).
 #include "itg_internal.cuh"
+#include "itg_rank.cuh"
 #include "itg_truncate.cuh"
 
 #include <cmath>
@@ -253,7 +254,7 @@ k_rank_desc(const double* __restrict__ sig, int n, double shift, int* __restrict
   int r = 0;
   for (int i = lane; i < n; i += 32) {
     const double u = sig[i];
-    r += (u > v) || (u == v && i < j);
+    r += itg_rank_before(u, i, v, j);
   }
   r = (int)__reduce_add_sync(0xffffffffu, (unsigned)r);
   if (lane == 0) {
