@@ -672,6 +672,13 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   }
   char* stage = (char*)h->stage;
   double* norm0 = (double*)(stage + (ring & ~(size_t)255));
+  // The next call writes the ring from the host, in no stream's order: whatever
+  // ends this one early (an allocation that fails between two launches), kernels
+  // that still read their instances' numbers from it are waited for.
+  struct RingInUse {
+    itg_handle* h;
+    ~RingInUse() { cudaStreamSynchronize(h->stream); }
+  } ring_in_use{h};
   size_t staged = 0;
   auto put = [&](const void* src, size_t bytes) -> const void* {
     void* at = stage + staged;
