@@ -355,6 +355,14 @@ __global__ void k_lincomb(int64_t n, double a, const double* __restrict__ x, dou
 constexpr int DV_THREADS = 256;
 constexpr int DV_BLOCKS = 512;   // blocks of the norms
 constexpr int DV_KMAX = 4;       // basis sizes with unrolled kernels
+constexpr int DV_BASIS = 32;     // largest basis
+// Doubles of the small workspace: scalars, coefficients (DV_BASIS), the projected
+// matrix; the learned preconditioner's loop lays out k^2 + 4 k + 8 of its own.
+constexpr int DV_COEF = 8, DV_G = DV_COEF + DV_BASIS;
+constexpr int64_t dv_small_doubles(int64_t k) {
+  const int64_t queued = DV_G + k * k, learned = k * k + 4 * k + 8;
+  return queued > learned ? queued : learned;
+}
 
 __device__ __forceinline__ double dv_block_sum(double v, double* sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -499,7 +507,7 @@ k_dv_gram(int64_t n, const double* __restrict__ V, const double* __restrict__ AV
 }
 
 struct DvCoef {
-  double y[32];
+  double y[DV_BASIS];
 };
 
 // X = V y, HX = AV y, Rv = HX - theta X, t = Rv / (dg - theta) (guarded; not
@@ -719,8 +727,9 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
                           unsigned* cnt, MV0&& matvec_direct, MV&& matvec, CAP&& capture, double* energy,
                           int* nmatvec, int* fallbacks) {
   // device scalars: [0..2] |Rv|, |X|, |t|; [3] |t| after orthogonalisation; [4] |psi|; then coefficients
+  // (DV_G: the k x k matrix of a basis without unrolled kernels)
   double* dsc = sm;
-  double* coef = sm + 8;
+  double* coef = sm + DV_COEF;
   double* hp = h->pinned;          // host copies: [0..2], [3], [4] as above; G from 8
   double* hG = hp + 8;
   const int nbn = itg_blocks_for(n, DV_THREADS, DV_BLOCKS);
@@ -738,7 +747,7 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
   };
   auto gram = [&](int k) -> int {
     if (k > DV_KMAX || (int64_t)k * k * chunks(k) > ITG_GEMV_MAX_PART) {
-      double* G = coef + 32;
+      double* G = sm + DV_G;
       for (int j = 0; j < k; ++j) ITG_TRY(itg_gemv_t(h, n, k, V, n, AV + (int64_t)j * n, G + (int64_t)j * k));
       ITG_CUDA(h, cudaMemcpyAsync(hG, G, sizeof(double) * k * k, cudaMemcpyDeviceToHost, h->stream));
       return ITG_OK;
@@ -885,7 +894,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
       h->slice_cache[1].valid = false;
     }
   } env_scope(h);
-  const int kmax = krylovdim < 2 ? 2 : (krylovdim > 32 ? 32 : krylovdim);
+  const int kmax = krylovdim < 2 ? 2 : (krylovdim > DV_BASIS ? DV_BASIS : krylovdim);
   if (maxiter < 1) maxiter = 1;
   const int64_t n = D.n();
   // scratch: heff work | V (n*kmax) | AV (n*kmax) | dg | X | HX | Rv | small | partials
@@ -894,7 +903,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
   size_t oH = take(heff_work_bytes(D));
   size_t oV = take(sizeof(double) * n * kmax), oAV = take(sizeof(double) * n * kmax);
   size_t oDg = take(sizeof(double) * n), oX = take(sizeof(double) * n), oHX = take(sizeof(double) * n),
-         oR = take(sizeof(double) * n), oSm = take(sizeof(double) * (kmax * kmax + 4 * kmax + 8)),
+         oR = take(sizeof(double) * n), oSm = take(sizeof(double) * dv_small_doubles(kmax)),
          oPart = take(sizeof(double) * 3 * DV_BLOCKS), oCnt = take(sizeof(unsigned) * 4);
   size_t oXg = take(h->use_graphs ? sizeof(double) * n : 0), oYg = take(h->use_graphs ? sizeof(double) * n : 0);
   size_t oFx = take(mlp ? sizeof(float) * n * 5 : 0), oFm = take(mlp ? sizeof(float) * n : 0),
