@@ -251,8 +251,11 @@ ITG_API int itg_set_wait_limit_ns(itg_handle* h, uint64_t ns);
  * the wait ran out as designed):
  *   which = 0: the cooperative Jacobi's grid barrier, on 2 blocks, counting
  *              one participant that never arrives;
- *   which = 1: the split GEMM's mbarrier wait, on a barrier nobody arrives on.
- * Takes the handle's wait limit; synchronises.  Failure-path check for
+ *   which = 1: the split GEMM's mbarrier wait, on a barrier nobody arrives on;
+ *   which = 2: the same, recorded as the split kernels record it: this call
+ *              returns ITG_OK without waiting, the next synchronising one
+ *              reports.
+ * Takes the handle's wait limit; 0 and 1 synchronise.  Failure-path check for
  * callers and tests; nothing faults, traps or hangs. */
 ITG_API int itg_wait_selftest(itg_handle* h, int which);
 /* Work partition of the split GEMM's stream-K schedule (host-only arithmetic,

@@ -272,7 +272,7 @@ extern "C" int itg_svd_trunc_batched(itg_handle* h, int count, const int64_t* m,
   const TruncRule rule = {mindim, cutoff, absoluteCutoff, doRelCutoff, legacy_gpu};
   k_svd_batched<<<count, 1024, 0, h->stream>>>(djobs, 2.220446049250313e-16, 60, rule, h->pinned);
   ITG_CHECK_LAUNCH(h);
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   for (int i = 0; i < count; ++i) {
     k[i] = (int64_t)h->pinned[3 * i];
     truncerr[i] = h->pinned[3 * i + 1];
@@ -712,7 +712,7 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
   auto ints = [&](const std::vector<int>& v) { return (const int*)put(v.data(), sizeof(int) * v.size()); };
   auto doubles = [&](const std::vector<double>& v) { return (const double*)put(v.data(), 8 * v.size()); };
   auto wait = [&]() -> int {
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     staged = 0;
     return ITG_OK;
   };
@@ -900,7 +900,7 @@ extern "C" int itg_davidson_heff2_batched(itg_handle* h, int count, const int64_
     ITG_TRY(normalise_into(fin, true));
     for (int i : fin) done[i] = 1;
   }
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   for (int i = 0; i < count; ++i) {
     energy[i] = theta[i];
     if (nmatvec) nmatvec[i] = nmv[i];

@@ -288,7 +288,7 @@ extern "C" int itg_svd_trunc_z(itg_handle* h, int64_t m, int64_t n, const double
   ITG_CHECK_LAUNCH(h);
   ITG_TRY(itg::nrm2_dev(h, 2 * mm * nn, W, red + 1000, red));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, red + 1000, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   const double fro = h->pinned[0];
   const double tol = EPS * sqrt((double)mm);
   const double amin_conv = (10.0 * EPS * fro) * (10.0 * EPS * fro);
@@ -301,7 +301,7 @@ extern "C" int itg_svd_trunc_z(itg_handle* h, int64_t m, int64_t n, const double
       k_zjacobi_step<<<np / 2, 256, 0, h->stream>>>(W, mm, (int)nn, Vw, tol, amin_conv, step, flag);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     if (hp[0] == 0) {
       sweeps = sw + 1;
       break;
@@ -322,7 +322,7 @@ extern "C" int itg_svd_trunc_z(itg_handle* h, int64_t m, int64_t n, const double
   ITG_CHECK_LAUNCH(h);
   h->last_sweeps = sweeps;
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, out3, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   if (k) *k = (int64_t)h->pinned[0];
   if (truncerr) *truncerr = h->pinned[1];
   if (docut) *docut = h->pinned[2];
@@ -364,7 +364,7 @@ extern "C" int itg_eigh_trunc_z(itg_handle* h, int64_t n, const double* A, int64
   k_zgershgorin<<<1, 1024, 0, h->stream>>>(A, lda, n, cdev);
   ITG_CHECK_LAUNCH(h);
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, cdev, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   const double shift = h->pinned[0] > 0.0 ? h->pinned[0] : 1.0;
   k_zload<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, n, n, 0, W);
   k_zshift_diag<<<itg_blocks_for(n, 256, 64), 256, 0, h->stream>>>(W, n, shift);
@@ -372,7 +372,7 @@ extern "C" int itg_eigh_trunc_z(itg_handle* h, int64_t n, const double* A, int64
   ITG_CHECK_LAUNCH(h);
   ITG_TRY(itg::nrm2_dev(h, 2 * n * n, W, red + 1000, red));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, red + 1000, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   const double fro = h->pinned[0];
   const double tol = EPS * sqrt((double)n);
   const double amin_conv = (10.0 * EPS * fro) * (10.0 * EPS * fro);
@@ -385,7 +385,7 @@ extern "C" int itg_eigh_trunc_z(itg_handle* h, int64_t n, const double* A, int64
       k_zjacobi_step<<<np / 2, 256, 0, h->stream>>>(W, n, (int)n, Vw, tol, amin_conv, step, flag);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     if (hp[0] == 0) {
       sweeps = sw + 1;
       break;
@@ -400,7 +400,7 @@ extern "C" int itg_eigh_trunc_z(itg_handle* h, int64_t n, const double* A, int64
   ITG_CHECK_LAUNCH(h);
   h->last_sweeps = sweeps;
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, out3, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   if (k) *k = (int64_t)h->pinned[0];
   if (truncerr) *truncerr = h->pinned[1];
   if (docut) *docut = h->pinned[2];

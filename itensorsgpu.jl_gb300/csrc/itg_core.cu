@@ -55,12 +55,13 @@ extern "C" int itg_create(int device, itg_handle** out) {
     delete h;
     return ITG_ERR_ALLOC;
   }
-  if (cudaMalloc((void**)&h->dev_status, 64) != cudaSuccess) {
+  if (cudaMallocHost((void**)&h->wait_status, 64) != cudaSuccess) {
+    cudaFree(h->gemv_part);
     cudaFreeHost(h->pinned);
     delete h;
     return ITG_ERR_ALLOC;
   }
-  cudaMemset(h->dev_status, 0, 64);
+  *h->wait_status = ITG_OK;
   if (const char* at = std::getenv("ITG_AUTOTUNE")) h->autotune = std::atoi(at) != 0;
   *out = h;
   return ITG_OK;
@@ -144,7 +145,7 @@ extern "C" int itg_destroy(itg_handle* h) {
   if (h->tune_buf) cudaFree(h->tune_buf);
   if (h->pinned) cudaFreeHost(h->pinned);
   if (h->stage) cudaFreeHost(h->stage);
-  if (h->dev_status) cudaFree(h->dev_status);
+  if (h->wait_status) cudaFreeHost(h->wait_status);
   if (h->gemv_part) cudaFree(h->gemv_part);
   if (h->qr_ev_ready) cudaEventDestroy(h->qr_ev_ready);
   if (h->qr_ev_done) cudaEventDestroy(h->qr_ev_done);
@@ -172,9 +173,18 @@ extern "C" int itg_set_graphs(itg_handle* h, int enable) {
   return ITG_OK;
 }
 
+int itg_wait_stream(itg_handle* h) {
+  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  volatile int* status = h->wait_status;
+  if (*status == ITG_OK) return ITG_OK;
+  *status = ITG_OK;
+  return itg_fail(h, ITG_ERR_TIMEOUT, "a wait of a split product on this handle ran out (limit %llu ns): what was computed "
+                  "since the last synchronising call is not valid", (unsigned long long)h->wait_ns);
+}
+
 extern "C" int itg_synchronize(itg_handle* h) {
   if (!h) return ITG_ERR_INVALID;
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   return ITG_OK;
 }
 
@@ -288,7 +298,7 @@ extern "C" int itg_memcpy_d2h(itg_handle* h, void* dst, const void* src, size_t 
   if (!h || (!dst && bytes) || (!src && bytes)) return ITG_ERR_INVALID;
   if (bytes == 0) return ITG_OK;
   ITG_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   return ITG_OK;
 }
 
@@ -430,7 +440,7 @@ extern "C" int itg_dot(itg_handle* h, int64_t n, const double* x, const double* 
   ITG_TRY(itg::dot_dev(h, n, x, y, part + REDUCE_BLOCKS, part));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, part + REDUCE_BLOCKS, sizeof(double),
                               cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   *result = h->pinned[0];
   return ITG_OK;
 }
@@ -442,7 +452,7 @@ extern "C" int itg_nrm2(itg_handle* h, int64_t n, const double* x, double* resul
   ITG_TRY(itg::nrm2_dev(h, n, x, part + REDUCE_BLOCKS, part));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, part + REDUCE_BLOCKS, sizeof(double),
                               cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   *result = h->pinned[0];
   return ITG_OK;
 }

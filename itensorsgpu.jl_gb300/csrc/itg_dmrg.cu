@@ -796,7 +796,7 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
   bool queued = false, restarted = false, first = true;
   for (int restart = 0;;) {
     ITG_TRY(gram(k));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     if (first && !(hp[4] > 0.0)) return itg_fail(h, ITG_ERR_INVALID, "davidson: zero start vector");
     first = false;
     if (restarted) {
@@ -816,13 +816,13 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
         ITG_CUDA(h, cudaMemcpyAsync(t, Rv, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
         ITG_TRY(launch(k_dv_norm, nbn, n, t, part, cnt + 3, dsc + 2, hp + 2));
         ITG_TRY(orthogonalise(k - 1, t));
-        ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+        ITG_TRY(itg_wait_stream(h));
         accept = hp[3] > 1e-6 * hp[2] && hp[3] > 1e-14;
         if (accept) {
           ITG_TRY(scale(dsc + 3, t, t, nullptr, nullptr));
           ITG_TRY(matvec(t, AV + (int64_t)(k - 1) * n));
           ITG_TRY(gram(k));
-          ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+          ITG_TRY(itg_wait_stream(h));
         }
       } else if (accept) {
         accept = hp[3] > 1e-14;
@@ -868,7 +868,7 @@ static int davidson_plain(itg_handle* h, int64_t n, int kmax, int maxiter, doubl
     ++k;
   }
   ITG_TRY(scale(dsc + 1, X, psi, nullptr, nullptr));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   *energy = theta;
   if (nmatvec) *nmatvec = nmv;
   if (fallbacks) *fallbacks = 0;
@@ -936,7 +936,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
     ITG_TRY(itg::nrm2_dev(h, n, x, sm + kmax * kmax + 4 * kmax, part));
     ITG_CUDA(h, cudaMemcpyAsync(hp, sm + kmax * kmax + 4 * kmax, sizeof(double),
                                 cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     out = hp[0];
     return ITG_OK;
   };
@@ -1010,7 +1010,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
         ITG_TRY(itg_gemv_t(h, n, k, V, n, AV + (int64_t)j * n, sm + (int64_t)j * k));
       }
       ITG_CUDA(h, cudaMemcpyAsync(hp, sm, sizeof(double) * k * k, cudaMemcpyDeviceToHost, h->stream));
-      ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+      ITG_TRY(itg_wait_stream(h));
       G.assign(k * k, 0.0);
       for (int i = 0; i < k; ++i)
         for (int j = 0; j < k; ++j) G[i + k * j] = 0.5 * (hp[i + k * j] + hp[j + k * i]);
@@ -1046,7 +1046,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
           k_abs_diff_sum<<<nb, 256, 0, h->stream>>>(n, dg, theta, Fp);
           ITG_CHECK_LAUNCH(h);
           ITG_CUDA(h, cudaMemcpyAsync(hp, Fp, sizeof(double) * nb, cudaMemcpyDeviceToHost, h->stream));
-          ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+          ITG_TRY(itg_wait_stream(h));
           double ds = 0.0;
           for (int q = 0; q < nb; ++q) ds += hp[q];
           ds /= (double)n;
@@ -1094,7 +1094,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
   ITG_TRY(nrm(X, xn));
   k_lincomb<<<gb, 256, 0, h->stream>>>(n, 1.0 / xn, X, 0.0, psi);
   ITG_CHECK_LAUNCH(h);
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   *energy = theta;
   if (nmatvec) *nmatvec = nmv;
   if (fallbacks) *fallbacks = nfallback;

@@ -35,7 +35,7 @@ int truncate_dev(itg_handle* h, const double* P, int64_t n, int64_t maxdim, int6
 static int read_out3(itg_handle* h, const double* out3, int64_t* n_keep, double* truncerr,
                      double* docut) {
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, out3, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   if (n_keep) *n_keep = (int64_t)h->pinned[0];
   if (truncerr) *truncerr = h->pinned[1];
   if (docut) *docut = h->pinned[2];
@@ -614,7 +614,7 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   // towards convergence, otherwise the sweeps never settle.
   ITG_TRY(itg::nrm2_dev(h, m * n, W, h->gemv_part + 1024, h->gemv_part));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, h->gemv_part + 1024, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   const double fro = h->pinned[0];
   const double amin_conv = (10.0 * 2.220446049250313e-16 * fro) * (10.0 * 2.220446049250313e-16 * fro);
   // one CTA for all sweeps: the smallest problems, and those that the
@@ -625,7 +625,7 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
     ITG_CHECK_LAUNCH(h);
     int* hp = (int*)h->pinned;
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     *sweeps_done = hp[0];
     return hp[0] >= JACOBI_MAX_SWEEPS ? ITG_ERR_NOTCONVERGED : ITG_OK;
   }
@@ -650,7 +650,7 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
       k_jacobi_step<<<np / 2, 256, 0, h->stream>>>(W, m, (int)n, V, tol, amin_conv, step, flag_dev);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag_dev, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     if (hp[0] == 0) { *sweeps_done = sweep + 1; return ITG_OK; }
   }
   *sweeps_done = JACOBI_MAX_SWEEPS;
@@ -971,7 +971,7 @@ extern "C" int itg_eigh_trunc(itg_handle* h, int64_t n, const double* A, int64_t
   k_gershgorin<<<1, 1024, 0, h->stream>>>(A, lda, n, cdev);
   ITG_CHECK_LAUNCH(h);
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, cdev, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   const double shift = h->pinned[0] > 0.0 ? h->pinned[0] : 1.0;
   k_copy_matrix<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, n, n, W, shift);
   ITG_CHECK_LAUNCH(h);

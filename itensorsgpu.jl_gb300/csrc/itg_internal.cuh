@@ -91,8 +91,10 @@ struct itg_handle {
   double* gemv_part = nullptr;
   // Persistent device buffers of the contraction plans, keyed by shape.
   std::unordered_map<std::string, std::shared_ptr<ContractPlan>> plans;
-  // Device status word for bounded waits (ITG_ERR_TIMEOUT reporting).
-  int* dev_status = nullptr;
+  // Status word of the split kernels' bounded waits, in pinned memory: a kernel
+  // whose wait runs out writes ITG_ERR_TIMEOUT there (and nothing else writes it),
+  // itg_wait_stream reports and clears it.
+  int* wait_status = nullptr;
   // Limit of every bounded device-side wait, in %globaltimer nanoseconds
   // (itg_set_wait_limit_ns).
   uint64_t wait_ns = 4000000000ull;
@@ -175,6 +177,10 @@ int itg_fail(itg_handle* h, int code, const char* fmt, ...);
   } while (0)
 
 #define ITG_CHECK_LAUNCH(h) ITG_CUDA((h), cudaGetLastError())
+
+// Waits for the handle's stream; ITG_ERR_TIMEOUT when a bounded wait of a kernel
+// before that ran out.  Every entry point that reads results back waits so.
+int itg_wait_stream(itg_handle* h);
 
 // A kernel that was started while its predecessor on the stream drains: what
 // comes before this call may overlap it, what comes after sees its results (and

@@ -837,7 +837,7 @@ int grid_barrier_selftest(itg_handle* h, int* status, int* blocks_out) {
   ITG_CHECK_LAUNCH(h);
   int* hp = (int*)h->pinned;
   ITG_CUDA(h, cudaMemcpyAsync(hp, aux, 4 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   *status = hp[2];
   *blocks_out = hp[3];
   return ITG_OK;
@@ -909,7 +909,7 @@ int jacobi_persistent(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin
   if (st != ITG_OK) return st;
   int* hp = (int*)h->pinned;
   ITG_CUDA(h, cudaMemcpyAsync(hp, aux, sizeof(int) * 4, cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   if (hp[2] != 0 || hp[3] < 0)
     return itg_fail(h, ITG_ERR_TIMEOUT, "Jacobi grid barrier timed out (n=%d)", n);
   *sweeps = hp[3] > max_sweeps ? max_sweeps : hp[3];
@@ -935,7 +935,7 @@ int jb_sweeps(itg_handle* h, int steps, int max_sweeps, int chunk, int* flag, in
       for (int step = 0; step < steps; ++step) launch(q, step, q > sw ? flag + q - 1 : nullptr, flag + q);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag + sw, sizeof(int) * (end - sw), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     for (int q = sw; q < end; ++q)
       if (hp[q - sw] == 0) {
         *sweeps = q + 1;

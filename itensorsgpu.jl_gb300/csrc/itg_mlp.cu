@@ -335,7 +335,7 @@ extern "C" int itg_mlp_get_params(itg_handle* h, void* mlp, float* host) {
   if (!h || !mlp || !host) return ITG_ERR_INVALID;
   Mlp* M = (Mlp*)mlp;
   ITG_CUDA(h, cudaMemcpyAsync(host, M->master, sizeof(float) * M->nparam, cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   return ITG_OK;
 }
 
@@ -345,7 +345,7 @@ extern "C" int itg_mlp_set_params(itg_handle* h, void* mlp, const float* host) {
   ITG_CUDA(h, cudaMemcpyAsync(M->master, host, sizeof(float) * M->nparam, cudaMemcpyHostToDevice, h->stream));
   k_to_bf16<<<64, 256, 0, h->stream>>>(M->master, M->nparam, M->w16);
   ITG_CHECK_LAUNCH(h);
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   return ITG_OK;
 }
 
@@ -403,7 +403,7 @@ extern "C" int itg_mlp_train_step(itg_handle* h, void* mlp, int64_t n, const flo
   if (loss) {
     std::vector<float> lp(ctas);
     ITG_CUDA(h, cudaMemcpyAsync(lp.data(), M->loss_part, sizeof(float) * ctas, cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     double s = 0.0;
     for (float x : lp) s += x;
     *loss = (float)(s / (double)n);

@@ -102,7 +102,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
       if (t0 == 0) {
         t0 = now;
       } else if (now - t0 > wait_ns) {
-        atomicExch(err, ITG_ERR_TIMEOUT);
+        *(volatile int*)err = ITG_ERR_TIMEOUT;
         *abort_flag = 1;
         return false;
       }
@@ -838,7 +838,7 @@ __global__ void k_mbar_selftest(int* err, uint64_t wait_ns) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const bool ok = mbar_wait(&bar, 0, err, (volatile int*)&abort_flag, wait_ns);
-    if (ok) atomicExch(err, ITG_OK);
+    if (ok) *(volatile int*)err = ITG_OK;
   }
   __syncthreads();
 }
@@ -1432,7 +1432,7 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   long long* acc = (long long*)(ws + oAcc);
   long long* tacc = (long long*)(ws + oTacc);
   int* cnt = (int*)(ws + oCnt);
-  int* err = h->dev_status;  // written only by a wait that runs out
+  int* err = h->wait_status;  // written only by a wait that runs out
   if (Mpad / 32 > 65535 || Npad / 32 > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: too many rows");
   const bool capturing = cap != cudaStreamCaptureStatusNone;
   {
@@ -1520,7 +1520,7 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
   if (nc < 1 || nj < 1 || nc > MID_KSLICE || nj > 32) return ITG_ERR_UNSUPPORTED;
   const int64_t grid = (R + MID_ROWS - 1) / MID_ROWS;
   if (grid > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "heff mid: too many rows");
-  int* err = h->dev_status;
+  int* err = h->wait_status;
   auto launch = [&](auto tag) -> int {
     constexpr int NPASS = decltype(tag)::value;
     static bool attr = false;
@@ -1612,10 +1612,15 @@ extern "C" int itg_wait_selftest(itg_handle* h, int which) {
     ITG_CHECK_LAUNCH(h);
     int* hp = (int*)h->pinned;
     ITG_CUDA(h, cudaMemcpyAsync(hp, err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     if (hp[0] == ITG_ERR_TIMEOUT)
       return itg_fail(h, ITG_ERR_TIMEOUT, "mbarrier wait ran out after %llu ns", (unsigned long long)h->wait_ns);
     return itg_fail(h, ITG_ERR_INVALID, "mbarrier self-test: the wait did not run out (%d)", hp[0]);
+  }
+  if (which == 2) {
+    split::k_mbar_selftest<<<1, 32, 0, h->stream>>>(h->wait_status, h->wait_ns);
+    ITG_CHECK_LAUNCH(h);
+    return ITG_OK;
   }
   return itg_fail(h, ITG_ERR_INVALID, "unknown self-test %d", which);
 }

@@ -329,7 +329,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
     double* red = ws + 5 * sq + ((mm * nn > sq) ? mm * nn : sq) + 64;
     ITG_TRY(itg::nrm2_dev(h, mm * nn, Awork, red + 520, red));
     ITG_CUDA(h, cudaMemcpyAsync(h->pinned, red + 520, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     fro = h->pinned[0];
   }
   const float amin = (float)(1e-14 * fro * fro);
@@ -337,7 +337,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
     k_jacobi32_onecta<<<1, 1024, 0, h->stream>>>(W32, mm, n, V32, tol32, amin, 30, flag);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     sweeps = hp[0];
   } else {
     int st = ITG_ERR_UNSUPPORTED;
@@ -355,7 +355,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
           k_jacobi32_step<<<np / 2, 256, 0, h->stream>>>(W32, mm, n, V32, tol32, amin, step, flag);
         ITG_CHECK_LAUNCH(h);
         ITG_CUDA(h, cudaMemcpyAsync(hp, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-        ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+        ITG_TRY(itg_wait_stream(h));
         if (hp[0] == 0) break;
       }
       sweeps++;
@@ -385,7 +385,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
     k_max_abs<<<1, 1024, 0, h->stream>>>(lam, n, mx);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(h->pinned, mx, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     const double lmax = h->pinned[0] > 0.0 ? h->pinned[0] : 1.0;
     // pairs closer than the current eigenvector error are treated as one
     // cluster (only their orthogonality is restored): 1e-6 relative after the
@@ -417,7 +417,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
     k_max_abs<<<1, 1024, 0, h->stream>>>(red, 512, mx + 1);
     ITG_CHECK_LAUNCH(h);
     ITG_CUDA(h, cudaMemcpyAsync(h->pinned, mx + 1, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+    ITG_TRY(itg_wait_stream(h));
     dev = h->pinned[0];
     if (!(dev > NS_TARGET) || it == NS_MAX) break;
     k_half_identity_minus<<<gb, 256, 0, h->stream>>>(P, n, Q);
@@ -433,7 +433,7 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
   k_max_abs<<<1, 1024, 0, h->stream>>>(lam, n, mx);
   ITG_CHECK_LAUNCH(h);
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, mx, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_CUDA(h, cudaStreamSynchronize(h->stream));
+  ITG_TRY(itg_wait_stream(h));
   // Safeguard: the first-order refinement needs a start close enough to the
   // eigenvectors; when it was not (X not orthonormal to 1e-12 after the
   // Newton-Schulz steps, or not finite) the caller redoes the problem with
