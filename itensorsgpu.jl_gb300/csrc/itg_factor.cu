@@ -240,14 +240,15 @@ __global__ void k_unit_cols(double* __restrict__ V, int64_t n) {
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) v[i] *= f;
 }
 
-// Stable descending rank of each value (ties by index): order[rank] = j.  A warp
+// Stable descending rank of each value (ties by index): order[rank] = j, and the
+// values themselves, v unit - shift.  A warp
 // a value (one thread a value took 56 us at n = 378 and 311 at 2048; the 2048 x
 // 2048 mixed split went from 109.5 to 108.7 ms with it).
 constexpr int RANK_THREADS = 256;
 inline int rank_blocks(int64_t n) { return (int)((n + RANK_THREADS / 32 - 1) / (RANK_THREADS / 32)); }
 __global__ void __launch_bounds__(RANK_THREADS)
-k_rank_desc(const double* __restrict__ sig, int n, double shift, int* __restrict__ order, double* __restrict__ S,
-            double* __restrict__ P, int square) {
+k_rank_desc(const double* __restrict__ sig, int n, double unit, double shift, int* __restrict__ order,
+            double* __restrict__ S, double* __restrict__ P, int square) {
   const int j = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (j >= n) return;
   const double v = sig[j];
@@ -259,7 +260,7 @@ k_rank_desc(const double* __restrict__ sig, int n, double shift, int* __restrict
   r = (int)__reduce_add_sync(0xffffffffu, (unsigned)r);
   if (lane == 0) {
     order[r] = j;
-    const double sv = v - shift;
+    const double sv = v * unit - shift;
     S[r] = sv;
     P[r] = square ? sv * sv : sv;
   }
@@ -597,12 +598,19 @@ size_t start32_bytes(const itg_handle* h, int64_t m, int64_t n) {
   return start32(h, m, n) ? itg_align256(sizeof(double) * itg::start32_ws_doubles(m, n)) + sizeof(float) * (m * n + n * n) : 0;
 }
 
+// |W|_F outside 2^+-JACOBI_RANGE: the sweeps work on squared norms and dot
+// products down to eps^2 of them, which then leave FP64's range.
+constexpr int JACOBI_RANGE = 300;
+
 // Runs Jacobi on W (m x n, m >= n) with V = I.  Returns ITG_ERR_NOTCONVERGED
 // (results still usable) when the sweep limit is hit.  flag_dev: at least
 // JACOBI_AUX_INTS device ints.
 // ws: start32_bytes(m, n).
+// *unit: W comes out divided by this power of two (1 unless its norm was out of
+// range), so the singular values are its column norms times *unit.
 int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* flag_dev, char* ws,
-               int* sweeps_done) {
+               int* sweeps_done, double* unit) {
+  *unit = 1.0;
   k_identity<<<itg_blocks_for(n * n, 256, h->num_sms * 8), 256, 0, h->stream>>>((int)n, V);
   ITG_CHECK_LAUNCH(h);
   const double tol = 2.220446049250313e-16 * sqrt((double)m);
@@ -615,7 +623,13 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   ITG_TRY(itg::nrm2_dev(h, m * n, W, h->gemv_part + 1024, h->gemv_part));
   ITG_CUDA(h, cudaMemcpyAsync(h->pinned, h->gemv_part + 1024, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   ITG_TRY(itg_wait_stream(h));
-  const double fro = h->pinned[0];
+  double fro = h->pinned[0];
+  if (std::isfinite(fro) && fro > 0.0 && std::abs(std::ilogb(fro)) > JACOBI_RANGE) {
+    const int ex = std::ilogb(fro);  // >= -538: the squares' sum is at least 2^-1074
+    *unit = std::ldexp(1.0, ex);
+    ITG_TRY(itg_scal(h, m * n, std::ldexp(1.0, -ex), W));
+    fro = std::ldexp(fro, -ex);
+  }
   const double amin_conv = (10.0 * 2.220446049250313e-16 * fro) * (10.0 * 2.220446049250313e-16 * fro);
   // one CTA for all sweeps: the smallest problems, and those that the
   // register-resident steps cannot take (a small n with very long columns) or
@@ -839,18 +853,19 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     double* lam = (double*)(base + oLam);
     double* Uw = (double*)(base + oUw);
     k_sqrt_clamp<<<itg_blocks_for(nn, 256, 64), 256, 0, h->stream>>>(lam, (int)nn, sig);
-    k_rank_desc<<<rank_blocks(nn), RANK_THREADS, 0, h->stream>>>(sig, (int)nn, 0.0, order, S, P, 1);
+    k_rank_desc<<<rank_blocks(nn), RANK_THREADS, 0, h->stream>>>(sig, (int)nn, 1.0, 0.0, order, S, P, 1);
     ITG_CHECK_LAUNCH(h);
     ITG_TRY(itg::truncate_dev(h, P, nn, maxdim, mindim, cutoff, absoluteCutoff, doRelCutoff, legacy_gpu, out3));
     if (want_other || !pre) k_gather_cols<<<g1, 256, 0, h->stream>>>(Uw, mj, order, sig, 0, (int)nn, Jl_dst, ld_l);
     k_gather_cols<<<g2, 256, 0, h->stream>>>(Vw, nn, order, sig, 0, (int)nn, Jr_dst, ld_r);
     ITG_CHECK_LAUNCH(h);
   } else {
-    st = jacobi_run(h, J, mj, nn, Vw, flag, base + oStart, &sweeps);
+    double unit = 1.0;
+    st = jacobi_run(h, J, mj, nn, Vw, flag, base + oStart, &sweeps, &unit);
     if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
     k_unit_cols<<<(unsigned)nn, 256, 0, h->stream>>>(Vw, nn);
     k_col_norms<<<(unsigned)nn, 256, 0, h->stream>>>(J, mj, sig);
-    k_rank_desc<<<rank_blocks(nn), RANK_THREADS, 0, h->stream>>>(sig, (int)nn, 0.0, order, S, P, 1);
+    k_rank_desc<<<rank_blocks(nn), RANK_THREADS, 0, h->stream>>>(sig, (int)nn, unit, 0.0, order, S, P, 1);
     ITG_CHECK_LAUNCH(h);
     ITG_TRY(itg::truncate_dev(h, P, nn, maxdim, mindim, cutoff, absoluteCutoff, doRelCutoff, legacy_gpu, out3));
     // U_J = J[:, order] / sig; V_J = Vw[:, order].
@@ -976,11 +991,12 @@ extern "C" int itg_eigh_trunc(itg_handle* h, int64_t n, const double* A, int64_t
   k_copy_matrix<<<itg_blocks_for(n * n, 256, h->num_sms * 16), 256, 0, h->stream>>>(A, lda, n, n, W, shift);
   ITG_CHECK_LAUNCH(h);
   int sweeps = 0;
-  int st = jacobi_run(h, W, n, n, Vw, flag, base + oStart, &sweeps);
+  double unit = 1.0;
+  int st = jacobi_run(h, W, n, n, Vw, flag, base + oStart, &sweeps, &unit);
   if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
   k_unit_cols<<<(unsigned)n, 256, 0, h->stream>>>(Vw, n);
   k_col_norms<<<(unsigned)n, 256, 0, h->stream>>>(W, n, sig);
-  k_rank_desc<<<rank_blocks(n), RANK_THREADS, 0, h->stream>>>(sig, (int)n, shift, order, D, P, 0);
+  k_rank_desc<<<rank_blocks(n), RANK_THREADS, 0, h->stream>>>(sig, (int)n, unit, shift, order, D, P, 0);
   ITG_CHECK_LAUNCH(h);
   ITG_TRY(itg::truncate_dev(h, P, n, maxdim, mindim, cutoff, absoluteCutoff, doRelCutoff, legacy_gpu, out3));
   dim3 g2(itg_blocks_for(n, 256, 64), (unsigned)n);

@@ -487,9 +487,10 @@ __device__ __forceinline__ bool jp_angle(float a, float b, float g, float tol, f
 
 // x 2^-(e - 1023) as a float, truncated, and a float as a double, by integer
 // instructions: an FP64 conversion occupies a quarter of an SM for 64 clocks.
+// Zero and subnormal numbers (exponent field 0, no leading one) give zero.
 __device__ __forceinline__ float jp_to_float(double x, int e) {
-  const int hi = __double2hiint(x);
-  const int ex = ((hi >> 20) & 0x7FF) - e + 127;
+  const int hi = __double2hiint(x), field = (hi >> 20) & 0x7FF;
+  const int ex = field == 0 ? 0 : field - e + 127;
   const int bits = (ex << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)__double2loint(x) >> 29);
   return ex <= 0 ? 0.f : __int_as_float((hi & 0x80000000) | (ex >= 255 ? 0x7F800000 : bits));
 }
