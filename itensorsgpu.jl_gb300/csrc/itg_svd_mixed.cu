@@ -311,7 +311,6 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
   prof_jacobi.emplace(h, ITG_KERNEL_SVD_JACOBI);
   float* W32 = ws32;
   float* V32 = ws32 + mm * nn;
-  k_to_float<<<itg_blocks_for(mm * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(Awork, mm * nn, 1.0, W32);
   k_identity32<<<itg_blocks_for(nn * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(n, V32);
   ITG_CHECK_LAUNCH(h);
   const int np = n + (n & 1);
@@ -332,6 +331,17 @@ int svd_mixed_core(itg_handle* h, const double* Awork, int64_t mm, int64_t nn, i
     ITG_TRY(itg_wait_stream(h));
     fro = h->pinned[0];
   }
+  // scaled by a power of two to a norm in [1, 2), as the columns' squares leave
+  // FP32's range first (norms below 1e-18 or above 1e19); the rotations do not
+  // depend on it, and within the range no bit does
+  double scale = 1.0;
+  if (std::isfinite(fro) && fro > 0.0) {
+    const int ex = std::ilogb(fro);
+    scale = std::ldexp(1.0, ex < -1000 ? 1000 : -ex);
+    fro *= scale;
+  }
+  k_to_float<<<itg_blocks_for(mm * nn, 256, h->num_sms * 16), 256, 0, h->stream>>>(Awork, mm * nn, scale, W32);
+  ITG_CHECK_LAUNCH(h);
   const float amin = (float)(1e-14 * fro * fro);
   if (n <= ONECTA32_MAX_N && (h->jacobi_mode != 0 || mm > 2048)) {
     k_jacobi32_onecta<<<1, 1024, 0, h->stream>>>(W32, mm, n, V32, tol32, amin, 30, flag);
