@@ -265,8 +265,7 @@ int launch_gemm_t(itg_handle* h, const ContractPlan& p, const double* A, const d
   if (gy > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "N=%lld too large", (long long)p.N);
   dim3 grid((unsigned)gx, (unsigned)gy);
   ProfScope prof(h, ITG_KERNEL_GEMM_F64);
-  const bool overlap = itg_small_grid(h, gx * gy) && !itg_capturing(h);
-  return itg_launch_after(h, overlap, grid, GTHREADS, smem, k_gemm_gather_f64<BM, BN, AK, BK>, A, B, C, p.offAm(),
+  return itg_launch_after(h, itg_small_grid(h, gx * gy), grid, GTHREADS, smem, k_gemm_gather_f64<BM, BN, AK, BK>, A, B, C, p.offAm(),
                           p.offAk(), p.offBk(), p.offBn(), p.offCm(), p.offCn(), p.M, p.N, p.K, alpha, beta);
 }
 
@@ -607,8 +606,10 @@ int time_variant(itg_handle* h, F&& launch, float& best_ms) {
   best_ms = 1e30f;
   for (int r = 0; r < 3 && st == ITG_OK; ++r) {
     cudaEventRecord(e0, h->stream);
+    h->chained = false;
     st = launch();
     cudaEventRecord(e1, h->stream);
+    h->chained = false;
     if (cudaEventSynchronize(e1) != cudaSuccess) st = itg_fail(h, ITG_ERR_CUDA, "autotune timing failed");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
@@ -836,6 +837,7 @@ extern "C" int itg_contract(itg_handle* h, int dtype, double alpha, const void* 
     return itg_fail(h, ITG_ERR_INVALID, "null dims/modes");
   if (!A || !B || !C) return itg_fail(h, ITG_ERR_INVALID, "null tensor pointer");
   if (C == A || C == B) return itg_fail(h, ITG_ERR_INVALID, "C must not alias A or B");
+  h->chained = false;
   for (int i = 0; i < rankA; ++i)
     if (dimsA[i] < 0) return itg_fail(h, ITG_ERR_SHAPE, "negative dimension");
   for (int i = 0; i < rankB; ++i)

@@ -91,12 +91,14 @@ ProfScope::ProfScope(itg_handle* hh, int k) : h(hh), kind(k) {
   if (!h->prof_on) return;
   e1 = prof_event(h);
   cudaEventRecord(e1, h->stream);
+  h->chained = false;
 }
 
 ProfScope::~ProfScope() {
   if (!e1) return;
   cudaEvent_t e2 = prof_event(h);
   cudaEventRecord(e2, h->stream);
+  h->chained = false;
   h->prof_events.push_back({kind, {e1, e2}});
 }
 
@@ -158,6 +160,7 @@ extern "C" int itg_destroy(itg_handle* h) {
 extern "C" int itg_set_stream(itg_handle* h, void* stream) {
   if (!h) return ITG_ERR_INVALID;
   h->stream = (cudaStream_t)stream;
+  h->chained = false;
   return ITG_OK;
 }
 

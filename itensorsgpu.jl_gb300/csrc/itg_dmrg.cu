@@ -86,8 +86,7 @@ k_heff_mid(const double* __restrict__ T1, const double* __restrict__ Weff, doubl
 
 int launch_heff_mid(itg_handle* h, const double* T1, const double* Weff, double* T3, int64_t R, int nc, int nj) {
   const int64_t gx = (nj + MID_J - 1) / MID_J, gy = (R + MID_R - 1) / MID_R;
-  const bool overlap = itg_small_grid(h, gx * gy) && !itg_capturing(h);
-  return itg_launch_after(h, overlap, dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535)), MID_R,
+  return itg_launch_after(h, itg_small_grid(h, gx * gy), dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535)), MID_R,
                           sizeof(double) * nc * (nj < MID_J ? nj : MID_J), k_heff_mid, T1, Weff, T3, R, nc, nj);
 }
 
@@ -961,6 +960,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
     const bool prof = h->prof_on;
     h->prof_on = false;
     h->stream = h->cap_stream;
+    h->chained = false;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal);
     int st = ITG_OK;
@@ -969,6 +969,7 @@ static int davidson_impl(itg_handle* h, int64_t chiL, int64_t chiR, int64_t d, i
       e = cudaStreamEndCapture(h->cap_stream, &graph);
     }
     h->stream = saved;
+    h->chained = false;
     h->prof_on = prof;
     if (st != ITG_OK) return st;
     if (e != cudaSuccess) return itg_fail(h, ITG_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));

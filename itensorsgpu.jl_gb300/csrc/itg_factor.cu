@@ -444,8 +444,7 @@ __global__ void __launch_bounds__(HOUSE_THREADS)
 k_house_step(double* __restrict__ A, int64_t m, int j, double* __restrict__ Vh, double* __restrict__ tau,
              double* __restrict__ rdiag) {
   __shared__ double red[HOUSE_THREADS / 16];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  itg_grid_wait();
   const double* x = A + (int64_t)j * m;
   double* col = A + (int64_t)(j + blockIdx.x) * m;
   const int t = threadIdx.x;
@@ -497,8 +496,7 @@ k_house_step_plain(double* __restrict__ A, int64_t m, int j, double* __restrict_
     __syncthreads();
     return s;
   };
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  itg_grid_wait();
   const double* x = A + (int64_t)j * m;
   const double alpha = x[j];
   double s2 = 0.0;
@@ -536,21 +534,12 @@ k_house_step_plain(double* __restrict__ A, int64_t m, int j, double* __restrict_
 
 namespace itg {
 // Steps j0 .. j0 + count - 1 on columns up to jend, on the handle's stream.
-// after_kernel: the last thing put on the stream is a kernel.
-int house_panel(itg_handle* h, bool fast, bool after_kernel, double* A, int64_t m, int64_t j0, int64_t count,
-                int64_t jend, double* Vh, double* tau, double* rdiag) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
+                double* tau, double* rdiag) {
   for (int64_t j = j0; j < j0 + count; ++j) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(jend - j));
-    cfg.blockDim = dim3(fast ? HOUSE_THREADS : 256);
-    cfg.stream = h->stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = j > j0 || after_kernel ? 1 : 0;
-    if (fast) ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step, A, m, (int)j, Vh, tau, rdiag));
-    else ITG_CUDA(h, cudaLaunchKernelEx(&cfg, k_house_step_plain, A, m, (int)j, Vh, tau, rdiag));
+    const dim3 grid((unsigned)(jend - j));
+    if (fast) ITG_TRY(itg_launch_after(h, true, grid, HOUSE_THREADS, 0, k_house_step, A, m, (int)j, Vh, tau, rdiag));
+    else ITG_TRY(itg_launch_after(h, true, grid, 256, 0, k_house_step_plain, A, m, (int)j, Vh, tau, rdiag));
   }
   return ITG_OK;
 }

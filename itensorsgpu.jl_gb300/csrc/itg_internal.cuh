@@ -71,6 +71,9 @@ struct itg_handle {
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
+  // The last thing that this library put on `stream` is one of its kernels (see
+  // itg_launch_after).  False is always safe.
+  bool chained = false;
   std::string last_error;
   // Reusable device scratch.  Operations on one handle are ordered on its
   // stream, so a buffer can be handed to the next call once the previous
@@ -168,15 +171,23 @@ int jacobi_blocked(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, i
 // Error helpers ---------------------------------------------------------------
 int itg_fail(itg_handle* h, int code, const char* fmt, ...);
 
+// Any runtime call that is checked here may put a copy, an event or a wait on
+// the stream, so it ends a chain of kernels.
 #define ITG_CUDA(h, call)                                                        \
   do {                                                                           \
     cudaError_t _e = (call);                                                     \
+    (h)->chained = false;                                                        \
     if (_e != cudaSuccess)                                                       \
       return itg_fail((h), ITG_ERR_CUDA, "%s failed: %s (%s:%d)", #call,          \
                       cudaGetErrorString(_e), __FILE__, __LINE__);               \
   } while (0)
 
-#define ITG_CHECK_LAUNCH(h) ITG_CUDA((h), cudaGetLastError())
+// Directly after a kernel launch.
+#define ITG_CHECK_LAUNCH(h)               \
+  do {                                    \
+    ITG_CUDA((h), cudaGetLastError());    \
+    (h)->chained = true;                  \
+  } while (0)
 
 // Waits for the handle's stream; ITG_ERR_TIMEOUT when a bounded wait of a kernel
 // before that ran out.  Every entry point that reads results back waits so.
@@ -190,9 +201,17 @@ __device__ __forceinline__ void itg_grid_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches a kernel that calls itg_grid_wait.  overlap: it may start early (not
-// when the last thing put on the stream is an event or a wait for one, nor
-// inside a capture).
+inline bool itg_capturing(itg_handle* h) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
+// Launches a kernel that calls itg_grid_wait.  overlap: it may start early, which
+// it then does only directly after another kernel of this library on the same
+// stream and outside a capture: the attribute loosens the order between two
+// kernels, and what it means behind a copy, an event or a wait for one, or for a
+// captured node's edges, is not left to it.  Entry points that launch through
+// here first forget the chain (the caller may have put anything on the stream).
 // Blocks that start early are placed on the SMs that drain first.  A grid of up
 // to one block an SM gains its launch (N = 20 DMRG, some 100 small kernels a
 // bond, 79 -> 68 ms); a larger one that is bound by the FP64 pipes ends up uneven (H_eff at
@@ -209,17 +228,13 @@ int itg_launch_after(itg_handle* h, bool overlap, dim3 grid, int threads, size_t
   cfg.dynamicSmemBytes = smem;
   cfg.stream = h->stream;
   cfg.attrs = &at;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cfg.numAttrs = overlap && h->chained && !itg_capturing(h) ? 1 : 0;
   ITG_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, (P)args...));
+  h->chained = true;
   return ITG_OK;
 }
 
 inline bool itg_small_grid(const itg_handle* h, int64_t blocks) { return blocks <= h->num_sms; }
-
-inline bool itg_capturing(itg_handle* h) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(h->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
-}
 
 #define ITG_TRY(expr)            \
   do {                           \

@@ -565,8 +565,7 @@ k_jacobi_reg_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, float 
   __shared__ Rot rotw[MAXW][WB];         // the current round, one copy a warp
   __shared__ unsigned rmask[NR];
   // the previous step's kernel must be done before its columns are read
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  itg_grid_wait();
   if (prev && *(const volatile int*)prev == 0) return;
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
   const int bi = jp_player(blockIdx.x, step, nbp), bj = jp_player(nbp - 1 - blockIdx.x, step, nbp);
@@ -933,8 +932,7 @@ int jb_sweeps(itg_handle* h, int steps, int max_sweeps, int chunk, int* flag, in
   for (int sw = 0; sw < max_sweeps;) {
     const int end = sw + chunk < max_sweeps ? sw + chunk : max_sweeps;
     for (int q = sw; q < end; ++q)
-      for (int step = 0; step < steps; ++step) launch(q, step, q > sw ? flag + q - 1 : nullptr, flag + q);
-    ITG_CHECK_LAUNCH(h);
+      for (int step = 0; step < steps; ++step) ITG_TRY(launch(q, step, q > sw ? flag + q - 1 : nullptr, flag + q));
     ITG_CUDA(h, cudaMemcpyAsync(hp, flag + sw, sizeof(int) * (end - sw), cudaMemcpyDeviceToHost, h->stream));
     ITG_TRY(itg_wait_stream(h));
     for (int q = sw; q < end; ++q)
@@ -959,9 +957,11 @@ int jb_run(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_co
     attr = true;
   }
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
-  return jb_sweeps(h, nbp - 1, max_sweeps, 1, flag, sweeps, [&](int, int step, const int*, int* rot) {
+  return jb_sweeps(h, nbp - 1, max_sweeps, 1, flag, sweeps, [&](int, int step, const int*, int* rot) -> int {
     k_jacobi_block_step<T, WB, JB_THREADS><<<nbp / 2, JB_THREADS, smem, h->stream>>>(
         W, m, n, V, tol, conv_tol(tol), amin, amin_conv, step, step == 0, rot);
+    ITG_CHECK_LAUNCH(h);
+    return ITG_OK;
   });
 }
 
@@ -976,23 +976,11 @@ int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_
   // about 25: FP32 takes six sweeps and more, FP64 (after the FP32 start, which
   // smaller problems do not take) mostly one
   const int chunk = sizeof(T) == 4 ? (n <= 160 ? 7 : (n <= 512 ? 4 : 1)) : (n < 16 ? 5 : 1);
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(nbp / 2));
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.stream = h->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  const dim3 grid((unsigned)(nbp / 2));
   const float tolf = (float)tol, tolc = (float)conv_tol(tol);
   return jb_sweeps(h, nbp - 1, max_sweeps, chunk, flag, sweeps, [&](int, int step, const int* prev, int* rot) {
-    if (step == 0)
-      cudaLaunchKernelEx(&cfg, k_jacobi_reg_step<T, WB, RPT, VEC, true, MAXT>, W, m, n, V, tolf, tolc, amin, amin_conv,
-                         step, prev, rot);
-    else
-      cudaLaunchKernelEx(&cfg, k_jacobi_reg_step<T, WB, RPT, VEC, false, MAXT>, W, m, n, V, tolf, tolc, amin,
-                         amin_conv, step, prev, rot);
+    auto kernel = step == 0 ? k_jacobi_reg_step<T, WB, RPT, VEC, true, MAXT> : k_jacobi_reg_step<T, WB, RPT, VEC, false, MAXT>;
+    return itg_launch_after(h, true, grid, threads, 0, kernel, W, m, n, V, tolf, tolc, amin, amin_conv, step, prev, rot);
   });
 }
 

@@ -12,9 +12,11 @@
 // Y <- Y - V (T (V^T Y)).  All of it is FP64.
 #include "itg_internal.cuh"
 
+#include <utility>
+
 namespace itg {
-int house_panel(itg_handle* h, bool fast, bool after_kernel, double* A, int64_t m, int64_t j0, int64_t count,
-                int64_t jend, double* Vh, double* tau, double* rdiag);
+int house_panel(itg_handle* h, bool fast, double* A, int64_t m, int64_t j0, int64_t count, int64_t jend, double* Vh,
+                double* tau, double* rdiag);
 }  // namespace itg
 
 namespace {
@@ -186,7 +188,7 @@ k_wy_update(const double* __restrict__ Vh, int64_t m, int64_t jb, int bw, const 
 }
 
 // Partial sums of V_p^T B into part; nchunk: how many.
-int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, int64_t jb, int bw, const double* B,
+int skinny_vt_b(itg_handle* h, const double* Vh, int64_t m, int64_t jb, int bw, const double* B,
                 int64_t ldb, int64_t b0, int64_t N, double* part, int64_t part_doubles, int* nchunk_out) {
   const int64_t K = m - jb;
   const int64_t ntile = (N + 31) / 32;
@@ -198,7 +200,7 @@ int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, i
   const int64_t kchunk = ((K + nchunk - 1) / nchunk + SK_TILE_K - 1) / SK_TILE_K * SK_TILE_K;
   nchunk = (K + kchunk - 1) / kchunk;
   const dim3 grid((unsigned)ntile, (unsigned)nchunk, 32 / SK_ROWS);
-  ITG_TRY(itg_launch_after(h, after_kernel, grid, 256, 0, k_skinny_partial, Vh, m, jb, bw, B, ldb, b0, N, kchunk,
+  ITG_TRY(itg_launch_after(h, true, grid, 256, 0, k_skinny_partial, Vh, m, jb, bw, B, ldb, b0, N, kchunk,
                            part));
   *nchunk_out = (int)nchunk;
   return ITG_OK;
@@ -207,11 +209,11 @@ int skinny_vt_b(itg_handle* h, bool after_kernel, const double* Vh, int64_t m, i
 // C(jb:m, c0 : c0 + N) -= V_p (op(T_p) (V_p^T C(jb:m, c0 : c0 + N))) on the
 // handle's current stream; Z2 holds 32 N doubles.
 template <bool TRANS>
-int wy_apply(itg_handle* h, bool after_kernel, double* C, int64_t m, int64_t jb, int bw, const double* Vh,
+int wy_apply(itg_handle* h, double* C, int64_t m, int64_t jb, int bw, const double* Vh,
              const double* Tp, int64_t c0, int64_t N, double* Z2, double* part, int64_t part_doubles) {
   if (N <= 0) return ITG_OK;
   int nchunk = 0;
-  ITG_TRY(skinny_vt_b(h, after_kernel, Vh, m, jb, bw, C, m, c0, N, part, part_doubles, &nchunk));
+  ITG_TRY(skinny_vt_b(h, Vh, m, jb, bw, C, m, c0, N, part, part_doubles, &nchunk));
   ITG_TRY(itg_launch_after(h, true, dim3((unsigned)((N + 7) / 8)), 256, 0, k_skinny_t<TRANS>, part, nchunk, bw, N, Tp,
                            Z2));
   const bool half = ((m - jb + 31) / 32) * ((N + 15) / 16) < h->num_sms;
@@ -248,12 +250,20 @@ namespace itg {
 // buffers.  Results are deterministic (the split of V^T A's K
 // range into chunks depends only on the column counts).
 namespace {
-// The handle's stream is swapped for the panel stream while this lives.
+// The handle's stream is swapped for the panel stream while this lives, and with
+// it whether the stream's last thing is a kernel (chained: the panel stream's).
 struct OnStream {
   itg_handle* h;
   cudaStream_t saved;
-  OnStream(itg_handle* hh, cudaStream_t s) : h(hh), saved(hh->stream) { h->stream = s; }
-  ~OnStream() { h->stream = saved; }
+  bool& chained;
+  OnStream(itg_handle* hh, cudaStream_t s, bool& c) : h(hh), saved(hh->stream), chained(c) {
+    h->stream = s;
+    std::swap(h->chained, chained);
+  }
+  ~OnStream() {
+    h->stream = saved;
+    std::swap(h->chained, chained);
+  }
 };
 
 int qr_lookahead_init(itg_handle* h) {
@@ -275,14 +285,15 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
   double *Zu = partp + part_doubles, *partu = Zu + (int64_t)NB * n;        // the handle's stream
   ITG_TRY(qr_lookahead_init(h));
   cudaStream_t main_stream = h->stream;
+  bool chained = false;  // of the panel stream
   // the panel stream starts after everything already queued on the handle's stream
   ITG_CUDA(h, cudaEventRecord(h->qr_ev_done, main_stream));
   {
-    OnStream on(h, h->qr_stream);
+    OnStream on(h, h->qr_stream, chained);
     ITG_CUDA(h, cudaStreamWaitEvent(h->stream, h->qr_ev_done, 0));
     if (nref > 0) {
       const int64_t w = nref < NB ? nref : NB;
-      ITG_TRY(house_panel(h, fast, false, W, m, 0, w, w, Vh, tau, rd));
+      ITG_TRY(house_panel(h, fast, W, m, 0, w, w, Vh, tau, rd));
     }
   }
   for (int64_t jb = 0, panel = 0; jb < nref; jb += NB, ++panel) {
@@ -293,25 +304,25 @@ int qr_blocked(itg_handle* h, double* W, int64_t m, int64_t n, int64_t nref, dou
     const int64_t nnext = nt > 0 && jn < nref ? ((nref - jn < NB) ? nref - jn : NB) : 0;
     const int64_t nrest = nt > 0 ? nt - nnext : 0;
     {
-      OnStream on(h, h->qr_stream);
+      OnStream on(h, h->qr_stream, chained);
       int nchunk = 0;
-      ITG_TRY(skinny_vt_b(h, true, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
+      ITG_TRY(skinny_vt_b(h, Vh, m, jb, (int)bw, Vh, m, jb, bw, partp, part_doubles, &nchunk));
       ITG_TRY(itg_launch_after(h, true, dim3(1), 256, 0, k_larft, partp, nchunk, tau + jb, (int)bw, Tp));
       if (nt <= 0) continue;
       // V_p and T_p are final: the handle's stream may update the rest
       ITG_CUDA(h, cudaEventRecord(h->qr_ev_ready, h->stream));
       // panel p + 1's columns got panel p - 1's update on the handle's stream
       if (panel > 0) ITG_CUDA(h, cudaStreamWaitEvent(h->stream, h->qr_ev_done, 0));
-      ITG_TRY(wy_apply<true>(h, false, W, m, jb, (int)bw, Vh, Tp, jn, nnext, Zp, partp, part_doubles));
+      ITG_TRY(wy_apply<true>(h, W, m, jb, (int)bw, Vh, Tp, jn, nnext, Zp, partp, part_doubles));
     }
     if (nrest > 0) {
       ITG_CUDA(h, cudaStreamWaitEvent(main_stream, h->qr_ev_ready, 0));
-      ITG_TRY(wy_apply<true>(h, false, W, m, jb, (int)bw, Vh, Tp, jn + nnext, nrest, Zu, partu, part_doubles));
+      ITG_TRY(wy_apply<true>(h, W, m, jb, (int)bw, Vh, Tp, jn + nnext, nrest, Zu, partu, part_doubles));
     }
     ITG_CUDA(h, cudaEventRecord(h->qr_ev_done, main_stream));
     if (nnext > 0) {
-      OnStream on(h, h->qr_stream);
-      ITG_TRY(house_panel(h, fast, true, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
+      OnStream on(h, h->qr_stream, chained);
+      ITG_TRY(house_panel(h, fast, W, m, jn, nnext, jn + nnext, Vh, tau, rd));
     }
   }
   // the handle's stream continues after the last panel's work
@@ -331,7 +342,7 @@ int q_apply_blocked(itg_handle* h, double* Y, int64_t m, int64_t n, int64_t ncol
   for (int64_t panel = npanel - 1; panel >= 0; --panel) {
     const int64_t jb = panel * NB;
     const int64_t bw = (n - jb < NB) ? n - jb : NB;
-    ITG_TRY(wy_apply<false>(h, panel != npanel - 1, Y, m, jb, (int)bw, Vh, Tbuf + panel * NB * NB, 0, ncols, Z2, part,
+    ITG_TRY(wy_apply<false>(h, Y, m, jb, (int)bw, Vh, Tbuf + panel * NB * NB, 0, ncols, Z2, part,
                             QR_PART_CHUNKS * 32 * ncols));
   }
   return ITG_OK;

@@ -1358,8 +1358,6 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   const bool shares = r != 0;  // the tail tiles are split between CTAs
   const size_t tile_bytes = sizeof(long long) * (size_t)BN * BM;
   // operands whose slices are kept (SliceCache): reuse on a match, else fill
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  ITG_CUDA(h, cudaStreamIsCapturing(h->stream, &cap));
   SliceCache* cache[2] = {nullptr, nullptr};
   bool hit[2] = {false, false};
   const double* srcs[2] = {A, B};
@@ -1372,7 +1370,7 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
       cache[i] = &c;
       continue;
     }
-    if (cap != cudaStreamCaptureStatusNone) continue;  // no allocation inside a capture: plain path
+    if (itg_capturing(h)) continue;  // no allocation inside a capture: plain path
     const size_t need = itg_align256(sizeof(int) * rpads[i]) + (size_t)2 * S * rpads[i] * Kpad;
     if (c.bytes < need) {
       ITG_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -1434,7 +1432,6 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   int* cnt = (int*)(ws + oCnt);
   int* err = h->wait_status;  // written only by a wait that runs out
   if (Mpad / 32 > 65535 || Npad / 32 > 65535) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: too many rows");
-  const bool capturing = cap != cudaStreamCaptureStatusNone;
   {
     ProfScope prof(h, ITG_KERNEL_SPLIT_PREP);
     PrepOp op[2] = {};
@@ -1463,9 +1460,9 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
     const int64_t sb = op[0].sblocks + op[1].sblocks;
     if (eb > INT32_MAX || sb > INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "split: problem too large");
     if (eb > 0)
-      ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)eb), 256, 0, k_split_exponents, op[0], op[1], (uint4*)tacc,
+      ITG_TRY(itg_launch_after(h, true, dim3((unsigned)eb), 256, 0, k_split_exponents, op[0], op[1], (uint4*)tacc,
                                nzero));
-    if (sb > 0) ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)sb), 256, 0, k_make_slices, op[0], op[1]));
+    if (sb > 0) ITG_TRY(itg_launch_after(h, true, dim3((unsigned)sb), 256, 0, k_make_slices, op[0], op[1]));
   }
   for (int i = 0; i < 2; ++i) {
     if (!cache[i] || hit[i]) continue;
@@ -1506,10 +1503,9 @@ int run(itg_handle* h, const ContractPlan& p, const double* A, const double* B, 
   a.err = err;
   {
     ProfScope prof(h, ITG_KERNEL_GEMM_SPLIT);
-    ITG_TRY(itg_launch_after(h, !capturing, dim3((unsigned)grid), NUM_THREADS, Smem<BN>::TOTAL, k_split_gemm<BN>, mA, mB,
+    ITG_TRY(itg_launch_after(h, true, dim3((unsigned)grid), NUM_THREADS, Smem<BN>::TOTAL, k_split_gemm<BN>, mA, mB,
                              a));
   }
-  ITG_CHECK_LAUNCH(h);
   return ITG_OK;
 }
 
@@ -1534,7 +1530,7 @@ int heff_mid_split(itg_handle* h, int64_t R, int nc, int nj, const double* T1, c
     // three CTAs per SM: by shared memory (the carveout is set to its maximum)
     // and registers; TMEM (512 columns per SM) would allow four
     const int64_t g = std::min<int64_t>(grid, (int64_t)3 * h->num_sms);
-    ITG_TRY(itg_launch_after(h, !itg_capturing(h), dim3((unsigned)g), MID_THREADS, MidSmem::TOTAL,
+    ITG_TRY(itg_launch_after(h, true, dim3((unsigned)g), MID_THREADS, MidSmem::TOTAL,
                              k_heff_mid_split<NPASS>, T1, Weff, T3, R, nc, nj, h->wait_ns, err));
     return ITG_OK;
   };
