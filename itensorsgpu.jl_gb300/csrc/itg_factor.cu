@@ -4,6 +4,7 @@
 #include "itg_rank.cuh"
 #include "itg_truncate.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 // The walk is a chain of additions and loads: from shared memory where the
@@ -217,6 +218,35 @@ __global__ void k_col_norms(const double* __restrict__ W, int64_t m, double* __r
     double t = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
     sig[blockIdx.x] = sqrt(t);
+  }
+}
+
+// From the column norms of W, into pinned host memory: out[0] = the smallest
+// non-zero one over |W|_F (0 when there is none), out[1] = |W|_F.
+__global__ void __launch_bounds__(256)
+k_col_grading(const double* __restrict__ sig, int64_t n, double* out) {
+  __shared__ double sh[2][8];
+  double s = 0.0, least = INFINITY;
+  for (int64_t i = threadIdx.x; i < n; i += 256) {
+    const double v = sig[i];
+    s = fma(v, v, s);
+    if (v > 0.0) least = fmin(least, v);
+  }
+  s = warp_sum(s);
+  for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
+  if ((threadIdx.x & 31) == 0) {
+    sh[0][threadIdx.x >> 5] = s;
+    sh[1][threadIdx.x >> 5] = least;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      s += sh[0][w];
+      least = fmin(least, sh[1][w]);
+    }
+    const double fro = sqrt(s);
+    out[0] = least < INFINITY ? least / fro : 0.0;
+    out[1] = fro;
   }
 }
 
@@ -579,6 +609,13 @@ constexpr int64_t START32_MIN_N = 16;
 // against 0.75 ms for the queued steps, n = 12: 0.87 against 0.82 ms).
 constexpr int64_t REG_MIN_N = 12;
 
+// Columns whose norm is below this share of |W|_F are rounding noise unless W
+// came with them.
+constexpr double NOISE = 10.0 * 2.220446049250313e-16;
+// FP64 sweeps in which the columns of a graded W count towards convergence
+// whatever their size (see jacobi_run); they take three to six.
+constexpr int GRADED_SWEEPS = 10;
+
 // Workspace of jacobi_run's FP32 start, 0 where it is not taken.
 bool start32(const itg_handle* h, int64_t m, int64_t n) {
   return n >= START32_MIN_N && h->jacobi_mode == 0 && m <= 2048;
@@ -597,8 +634,11 @@ constexpr int JACOBI_RANGE = 300;
 // ws: start32_bytes(m, n).
 // *unit: W comes out divided by this power of two (1 unless its norm was out of
 // range), so the singular values are its column norms times *unit.
+// grading: what k_col_grading wrote for the matrix that the problem came with
+// (W or, before a QR, one of the same norm), or null; known: the stream has been
+// waited for since.
 int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* flag_dev, char* ws,
-               int* sweeps_done, double* unit) {
+               int* sweeps_done, double* unit, const volatile double* grading, bool known) {
   *unit = 1.0;
   k_identity<<<itg_blocks_for(n * n, 256, h->num_sms * 8), 256, 0, h->stream>>>((int)n, V);
   ITG_CHECK_LAUNCH(h);
@@ -609,17 +649,19 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   // matrices of a direct sum of two MPS): their pairs keep being rotated (so
   // that W's columns stay as orthogonal as rounding allows) but do not count
   // towards convergence, otherwise the sweeps never settle.
-  ITG_TRY(itg::nrm2_dev(h, m * n, W, h->gemv_part + 1024, h->gemv_part));
-  ITG_CUDA(h, cudaMemcpyAsync(h->pinned, h->gemv_part + 1024, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  ITG_TRY(itg_wait_stream(h));
-  double fro = h->pinned[0];
+  if (!grading) {
+    ITG_TRY(itg::nrm2_dev(h, m * n, W, h->gemv_part + 1024, h->gemv_part));
+    ITG_CUDA(h, cudaMemcpyAsync(h->pinned, h->gemv_part + 1024, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  }
+  if (!known) ITG_TRY(itg_wait_stream(h));
+  double fro = grading ? grading[1] : h->pinned[0];
   if (std::isfinite(fro) && fro > 0.0 && std::abs(std::ilogb(fro)) > JACOBI_RANGE) {
     const int ex = std::ilogb(fro);  // >= -538: the squares' sum is at least 2^-1074
     *unit = std::ldexp(1.0, ex);
     ITG_TRY(itg_scal(h, m * n, std::ldexp(1.0, -ex), W));
     fro = std::ldexp(fro, -ex);
   }
-  const double amin_conv = (10.0 * 2.220446049250313e-16 * fro) * (10.0 * 2.220446049250313e-16 * fro);
+  const double amin_conv = (NOISE * fro) * (NOISE * fro);
   // one CTA for all sweeps: the smallest problems, and those that the
   // register-resident steps cannot take (a small n with very long columns) or
   // where they are switched off
@@ -636,8 +678,21 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
     ITG_TRY(itg::jacobi_start32(h, W, m, n, V, fro, (double*)ws,
                                 (float*)(ws + itg_align256(sizeof(double) * itg::start32_ws_doubles(m, n))), flag_dev));
   if (h->jacobi_mode == 0 || h->jacobi_mode == 3) {
-    const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, JACOBI_MAX_SWEEPS, flag_dev,
+    // Small columns that W came with (a graded matrix) are not noise: one-sided
+    // rotations resolve them relative to their own size, but not in the one
+    // sweep that the FP32 start leaves to the large ones.  They count as well,
+    // in a bounded number of sweeps, as other columns of W may be noise.
+    int before = 0;
+    if (start32(h, m, n) && grading && grading[0] > 0.0 && grading[0] < NOISE) {
+      const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, GRADED_SWEEPS, flag_dev, &before, 0.0);
+      if (st != ITG_ERR_NOTCONVERGED) {
+        *sweeps_done = before;
+        return st;
+      }
+    }
+    const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, JACOBI_MAX_SWEEPS - before, flag_dev,
                                                sweeps_done, amin_conv);
+    *sweeps_done += before;
     if (st != ITG_ERR_UNSUPPORTED) return st;
   } else if (h->jacobi_mode == 2) {
     const int st = itg::jacobi_persistent<double>(h, W, m, (int)n, V, tol, 0.0, JACOBI_MAX_SWEEPS, flag_dev,
@@ -737,10 +792,15 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
   // exactly orthonormal: that side is then Q times the rotations (or the
   // refined eigenvectors), never U_J = J V_J / S, which loses orthogonality
   // in columns whose S is small or rounding noise (rank-deficient inputs)
-  const bool pre = (h->svd_qr_precond && nn > PRECOND_MIN_N) || iso != ISO_NONE;
+  bool pre = (h->svd_qr_precond && nn > PRECOND_MIN_N) || iso != ISO_NONE;
   const bool two = pre && iso == ISO_RIGHT;
+  // A graded W keeps its small singular values and their vectors accurate
+  // relative to their size in one-sided rotations of its own columns; R^T, whose
+  // rows are scaled instead, does not.  Small problems can tell (one more wait for
+  // the host) and leave out a QR that is there for speed only.
+  const bool may_skip = pre && iso == ISO_NONE && !mixed && nn <= ONECTA_MAX_N && h->jacobi_mode == 0;
   // the Jacobi problem: W itself (mj = mm rows) or J (nn x nn)
-  const int64_t mj = pre ? nn : mm;
+  int64_t mj = pre ? nn : mm;
   size_t oW = take(sizeof(double) * mm * nn), oV = take(sizeof(double) * nn * nn),
          oSig = take(sizeof(double) * nn), oP = take(sizeof(double) * nn),
          oOrd = take(sizeof(int) * nn), oOut = take(4 * sizeof(double)), oFlag = take(sizeof(int) * JACOBI_AUX_INTS);
@@ -752,7 +812,8 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     oWs = take(sizeof(double) * itg::svd_mixed_ws_doubles(mj, nn));
     oWs32 = take(sizeof(float) * (mj * nn + nn * nn));
   }
-  const size_t oStart = take(start32_bytes(h, mj, nn));
+  const size_t oStart = take(may_skip ? std::max(start32_bytes(h, mm, nn), start32_bytes(h, nn, nn))
+                                      : start32_bytes(h, mj, nn));
   size_t oTq = 0, oTq2 = 0, oQws = 0;
   if (pre) {
     oVh = take(sizeof(double) * mm * nn);
@@ -787,6 +848,22 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
   }
   int sweeps = 0;
   int st = ITG_OK;
+  // the grading of W's columns, before a QR
+  const volatile double* grading = nullptr;
+  if (!mixed && nn > 1) {
+    double* out = h->pinned + ITG_PINNED_DOUBLES - 2;
+    k_col_norms<<<(unsigned)nn, 256, 0, h->stream>>>(W, mm, sig);
+    k_col_grading<<<1, 256, 0, h->stream>>>(sig, nn, out);
+    ITG_CHECK_LAUNCH(h);
+    grading = out;
+  }
+  if (may_skip) {
+    ITG_TRY(itg_wait_stream(h));
+    if (grading[0] > 0.0 && grading[0] < NOISE) {
+      pre = false;
+      mj = mm;
+    }
+  }
   double* Uw_dst = tr ? V : U;  // rows mm
   double* Vw_dst = tr ? U : V;  // rows nn
   double* J = W;
@@ -850,7 +927,7 @@ static int svd_trunc_impl(itg_handle* h, int64_t m, int64_t n, const double* A, 
     ITG_CHECK_LAUNCH(h);
   } else {
     double unit = 1.0;
-    st = jacobi_run(h, J, mj, nn, Vw, flag, base + oStart, &sweeps, &unit);
+    st = jacobi_run(h, J, mj, nn, Vw, flag, base + oStart, &sweeps, &unit, grading, may_skip);
     if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
     k_unit_cols<<<(unsigned)nn, 256, 0, h->stream>>>(Vw, nn);
     k_col_norms<<<(unsigned)nn, 256, 0, h->stream>>>(J, mj, sig);
@@ -981,7 +1058,7 @@ extern "C" int itg_eigh_trunc(itg_handle* h, int64_t n, const double* A, int64_t
   ITG_CHECK_LAUNCH(h);
   int sweeps = 0;
   double unit = 1.0;
-  int st = jacobi_run(h, W, n, n, Vw, flag, base + oStart, &sweeps, &unit);
+  int st = jacobi_run(h, W, n, n, Vw, flag, base + oStart, &sweeps, &unit, nullptr, false);
   if (st != ITG_OK && st != ITG_ERR_NOTCONVERGED) return st;
   k_unit_cols<<<(unsigned)n, 256, 0, h->stream>>>(Vw, n);
   k_col_norms<<<(unsigned)n, 256, 0, h->stream>>>(W, n, sig);
