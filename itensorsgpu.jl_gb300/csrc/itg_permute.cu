@@ -293,18 +293,34 @@ void perm_launch_rows(int blocks, cudaStream_t st, const double* A, double* B, c
                                                    fast_div(nseg > 1 ? 1 : (uint32_t)d0), items, rest);
 }
 
-// Whether 32 x 32 tiles take the transpose, by the share of working lanes against
-// theirs: for copies and sums below 0.65 (sum, 96 x 96: 0.56, 0.190 against 0.173 ms;
-// 80 x 80: 0.57, 0.206 against 0.189; but 100 x 80: 0.75, 0.304 against 0.321); with
-// general scalars up to 1.3 (100 x 80: 0.40 against 0.32 ms, 512 x 512: 1, 0.365 against
-// 0.361), above it a mode is short.
+// Whether 32 x 32 tiles take the transpose.  Their time over that of equal tiles
+// for copy, sum and general sum of 2^24 elements, n0 x batches x nq reversed:
+//   both modes up to 32: an equal tile is then no larger than theirs, and twice as
+//     many of theirs share an SM.  2 x 2 0.66, 0.53, 0.53; 16 x 16 0.61, 0.61, 0.61;
+//     32 x 32 0.64, 0.68, 0.55; only 32 x 2 1.12 for the general sum.
+//   one of 17 to 32: half of the wide lanes' loads are idle on that side.  20 x 64
+//     0.77, 0.85, 0.76; on the side of the writes 64 x 20 0.91, 0.75, 0.58 but, for
+//     copies, 128 x 20 1.04.
+//   one of 9 to 16: where the writes or the scalars count, 12 x 80 1.02, 0.90, 0.81;
+//     16 x 48 1.01, 0.95, 0.85; 16 x 160 1.08, 0.99, 0.85; 64 x 12 1.10, 1.03, 0.95;
+//     not 128 x 12 (1.38, 1.14, 1.06).
+//   longer ones: by the share of working lanes against theirs, below 0.745 (160 x 160,
+//     0.71: 0.85, 0.92; 129 x 129, 0.69: 0.94, 0.93; 65 x 33, 0.75: 1.47, 1.31), with
+//     general scalars below 1.3 (64 x 64, 1: 0.94; 100 x 100, 1: 0.98; above it a
+//     mode is short: 128 x 8 1.70).
 bool perm_tiles32(int op, int64_t n0, int64_t nq, int e0, int eq, int l0, int lq) {
+  const bool general = op == PERM_SCALE || op == PERM_AXPBY;
+  if (n0 <= 32 && nq <= 32) return op != PERM_AXPBY || n0 < 32 || nq > 8;
+  if (n0 > 16 && n0 <= 32) return true;
+  if (nq > (op == PERM_COPY ? 24 : 16) && nq <= 32) return true;
+  if (n0 > 8 && n0 <= 16 && nq <= (op == PERM_AXPBY ? 200 : 96) && (general || (op == PERM_ADD && nq > 64))) return true;
+  if (general && nq > 8 && nq <= 16 && n0 <= 96) return true;
   auto share = [](int64_t n, int e, int l) {
     const int lanes = (e + (1 << l) - 1) >> l << l;
     return (double)n / ((double)((n + e - 1) / e) * lanes);
   };
   const double r = share(n0, e0, l0) * share(nq, eq, lq) / (share(n0, 32, 5) * share(nq, 32, 5));
-  return r < (op == PERM_SCALE || op == PERM_AXPBY ? 1.3 : 0.65);
+  return r < (general ? 1.3 : 0.745);
 }
 
 // Resolve modesB as a permutation of modesA.  perm[j] = A-position of B's mode j.
