@@ -123,8 +123,10 @@ k_perm_rows(const double* __restrict__ A, double* B, const double* Bin, PermScal
         }
       }
 #pragma unroll
-      for (int u = 0; u < PERM_FLIGHT; ++u)
+      for (int u = 0; u < PERM_FLIGHT; ++u) {
+        if (e0 - (int)threadIdx.x + u * PERM_THREADS >= total) break;  // the block's: no products for nobody
         if (o[u] >= 0) B[o[u]] = perm_op<OP>(sc, v[u], perm_reads_b(OP) ? w[u] : 0.0);
+      }
     }
   }
 }
@@ -303,24 +305,38 @@ void perm_launch_rows(int blocks, cudaStream_t st, const double* A, double* B, c
 //     copies, 128 x 20 1.04.
 //   one of 9 to 16: where the writes or the scalars count, 12 x 80 1.02, 0.90, 0.81;
 //     16 x 48 1.01, 0.95, 0.85; 16 x 160 1.08, 0.99, 0.85; 64 x 12 1.10, 1.03, 0.95;
-//     not 128 x 12 (1.38, 1.14, 1.06).
+//     128 x 12 1.38, 1.14, 1.06 (0.85 of 2^20 elements).
 //   longer ones: by the share of working lanes against theirs, below 0.745 (160 x 160,
-//     0.71: 0.85, 0.92; 129 x 129, 0.69: 0.94, 0.93; 65 x 33, 0.75: 1.47, 1.31), with
-//     general scalars below 1.3 (64 x 64, 1: 0.94; 100 x 100, 1: 0.98; above it a
-//     mode is short: 128 x 8 1.70).
+//     0.71: 0.85, 0.92; 129 x 129, 0.69: 0.94, 0.93; 65 x 33, 0.75: 1.47, 1.31) or,
+//     where theirs are full, 0.8 (128 x 96, 0.75: 0.91, 0.94; but 64 x 160, 0.84: 0.94,
+//     and 1.13 of 2^22 elements), with general scalars below 1.3 (64 x 64, 1: 0.94; 100 x 100, 1: 0.98; above
+//     it a mode is short: 128 x 8 1.70).
 bool perm_tiles32(int op, int64_t n0, int64_t nq, int e0, int eq, int l0, int lq) {
   const bool general = op == PERM_SCALE || op == PERM_AXPBY;
   if (n0 <= 32 && nq <= 32) return op != PERM_AXPBY || n0 < 32 || nq > 8;
   if (n0 > 16 && n0 <= 32) return true;
   if (nq > (op == PERM_COPY ? 24 : 16) && nq <= 32) return true;
-  if (n0 > 8 && n0 <= 16 && nq <= (op == PERM_AXPBY ? 200 : 96) && (general || (op == PERM_ADD && nq > 64))) return true;
-  if (general && nq > 8 && nq <= 16 && n0 <= 96) return true;
+  if (n0 > 8 && n0 <= 16 && (op == PERM_AXPBY || (nq <= 96 && (general || (op == PERM_ADD && nq > 64))))) return true;
+  if (general && nq > 8 && nq <= 16) return true;
   auto share = [](int64_t n, int e, int l) {
     const int lanes = (e + (1 << l) - 1) >> l << l;
     return (double)n / ((double)((n + e - 1) / e) * lanes);
   };
-  const double r = share(n0, e0, l0) * share(nq, eq, lq) / (share(n0, 32, 5) * share(nq, 32, 5));
-  return r < (general ? 1.3 : 0.745);
+  const double theirs = share(n0, 32, 5) * share(nq, 32, 5), r = share(n0, e0, l0) * share(nq, eq, lq) / theirs;
+  return r < (general ? 1.3 : (theirs > 0.95 ? 0.8 : 0.745));
+}
+
+// Whether 32 x 32 tiles take a transpose that is too small to fill the GPU.  As long
+// as the equal tiles fit on it at once (four to an SM) their number does not count,
+// but the rounds of loads of one of them, about 0.3 us each for a copy and 0.4 to 0.5
+// with Bin, beside 1.9 us; the 32 x 32 ones take one round each, and eight share an SM
+// (2^16 elements, 16 x 16 x 256, eight rounds: copy 4.7 -> 2.1 us, sum 6.5 -> 2.5;
+// 1000 x 2: 7.0 -> 1.8; but 2^18, 256 x 512 x 2, six rounds: 4.4 against 10.7 us).
+bool perm_few_tiles(int sms, int op, int64_t n0, int64_t nq, int64_t nbatch, int e0, int eq, int l0, int lq) {
+  auto up = [](int64_t n, int64_t d) { return (n + d - 1) / d; };
+  const int64_t equal = up(n0, e0) * up(nq, eq) * nbatch, by32 = up(n0, 32) * up(nq, 32) * nbatch;
+  const int64_t rounds = up(e0, 2 << l0) * up(eq, 4 * (PERM_THREADS >> l0)) + up(eq, 2 << lq) * up(e0, 4 * (PERM_THREADS >> lq));
+  return equal <= 4 * (int64_t)sms && (double)by32 <= sms * (0.6 + (op == PERM_COPY ? 1.0 : 1.3) * rounds);
 }
 
 // Resolve modesB as a permutation of modesA.  perm[j] = A-position of B's mode j.
@@ -405,9 +421,12 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
       rest.n++;
     }
     const int64_t d0 = d.dims[0], nrows = total / d0;
-    // short rows share an item, long ones are cut into segments
-    const int64_t seg = PERM_ITEM, nseg = d0 > 2 * PERM_ITEM ? (d0 + seg - 1) / seg : 1;
-    int64_t rows = nseg > 1 ? 1 : std::min<int64_t>(std::max<int64_t>(1, PERM_ITEM / d0), PERM_ROWS);
+    // short rows share an item, long ones are cut into segments; smaller items
+    // where those of PERM_ITEM would leave SMs idle (24 x 96 x 3, a copy 3.7 -> 2.1 us)
+    const int64_t share = (total + 4 * h->num_sms - 1) / (4 * h->num_sms);
+    const int64_t seg = std::min<int64_t>(PERM_ITEM, (share + PERM_THREADS - 1) / PERM_THREADS * PERM_THREADS);
+    const int64_t nseg = d0 > 2 * seg ? (d0 + seg - 1) / seg : 1;
+    int64_t rows = nseg > 1 ? 1 : std::min<int64_t>(std::max<int64_t>(1, seg / d0), PERM_ROWS);
     const int64_t items = nseg > 1 ? nrows * nseg : (nrows + rows - 1) / rows;
     const int blocks = (int)std::min<int64_t>(items, (int64_t)h->num_sms * 64);
     auto run = [&](auto tag) {
@@ -441,7 +460,8 @@ static int permute_axpby(itg_handle* h, double alpha, const double* A, int rank,
     int e0, eq, l0, lq;
     perm_tile(n0, nq, e0, eq, l0, lq);
     const int64_t sqA = d.strA[q], s0B = d.strB[0];
-    const bool small = perm_tiles32(op, n0, nq, e0, eq, l0, lq);
+    const bool small = perm_few_tiles(h->num_sms, op, n0, nq, nbatch, e0, eq, l0, lq) ||
+                       perm_tiles32(op, n0, nq, e0, eq, l0, lq);
     const int64_t t0 = (n0 + (small ? 32 : e0) - 1) / (small ? 32 : e0);
     const int64_t tq = (nq + (small ? 32 : eq) - 1) / (small ? 32 : eq);
     if (t0 * tq > (int64_t)INT32_MAX) return itg_fail(h, ITG_ERR_UNSUPPORTED, "permute: transpose too large");
