@@ -837,6 +837,9 @@ extern "C" int itg_contract(itg_handle* h, int dtype, double alpha, const void* 
     return itg_fail(h, ITG_ERR_INVALID, "null dims/modes");
   if (!A || !B || !C) return itg_fail(h, ITG_ERR_INVALID, "null tensor pointer");
   if (C == A || C == B) return itg_fail(h, ITG_ERR_INVALID, "C must not alias A or B");
+  // the caller may have put anything on the stream (right behind another product
+  // this costs the early launch: 16 x 16 x 32 2.9 -> 5.2 us on the device, which the
+  // host's share of a call hides)
   h->chained = false;
   for (int i = 0; i < rankA; ++i)
     if (dimsA[i] < 0) return itg_fail(h, ITG_ERR_SHAPE, "negative dimension");

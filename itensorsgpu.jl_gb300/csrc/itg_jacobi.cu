@@ -973,8 +973,8 @@ int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
   const int threads = (int)((m + RPT - 1) / RPT + 31) / 32 * 32;
   // a queued step costs about 1 us when it has nothing to do, a look at the flags
-  // about 25: FP32 takes six sweeps and more, FP64 (after the FP32 start, which
-  // smaller problems do not take) mostly one
+  // about 25: FP32 takes seven sweeps and more (all seven are queued where they are
+  // cheap), FP64 (after the FP32 start, which smaller problems do not take) mostly one
   const int chunk = sizeof(T) == 4 ? (n <= 160 ? 7 : (n <= 512 ? 4 : 1)) : (n < 16 ? 5 : 1);
   const dim3 grid((unsigned)(nbp / 2));
   const float tolf = (float)tol, tolc = (float)conv_tol(tol);

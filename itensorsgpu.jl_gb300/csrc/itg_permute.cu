@@ -8,9 +8,9 @@
 //                 one per CTA.
 //   * transpose — different fastest modes: tiles staged through shared memory
 //                 so that reads of A and writes of B are both coalesced.
-// Both walk items of about 4096 elements by a linear index whose quotient is a
-// multiply, so that no lane idles on a ragged edge, with eight loads of every
-// thread in flight.
+// Both take items of about 4096 elements (fewer where there are few) with eight
+// loads of every thread in flight, or the transpose 32 x 32 tiles with four
+// (perm_tiles32, perm_few_tiles).
 #include "itg_internal.cuh"
 
 #include <algorithm>
@@ -226,10 +226,11 @@ k_perm_transpose(const double* __restrict__ A, double* B, const double* Bin, Per
 }
 
 // The transpose by 32 x 32 tiles, blockIdx.y over the batches: four loads a
-// thread and eight CTAs an SM instead of eight and six.  It is the better one
+// thread and eight CTAs an SM instead of eight and four.  It is the better one
 // where the scalars need FP64 instructions (they run between the loads of more
-// CTAs: 1.5 A - 0.5 B of 100 x 90 x 80 x 70 0.40 -> 0.32 ms) and where equal tiles leave
-// lanes idle that these fill (perm_tiles32).
+// CTAs: 1.5 A - 0.5 B of 100 x 90 x 80 x 70 0.40 -> 0.32 ms), where modes are short or
+// equal tiles leave lanes idle that these fill (perm_tiles32), and where there are
+// few tiles at all (perm_few_tiles).
 template <int OP>
 __global__ void __launch_bounds__(256)
 k_perm_transpose32(const double* __restrict__ A, double* B, const double* Bin, PermScalars sc, int64_t n0, int64_t nq,
@@ -269,8 +270,8 @@ k_perm_transpose32(const double* __restrict__ A, double* B, const double* Bin, P
 }
 
 // Tile of the transpose: about 64 x 64, the other side longer where one mode
-// is short, and equal tiles within each mode; padded rows fit in 35 KB, so six
-// CTAs share an SM.  l0, lq: log2 of the lanes along each mode.
+// is short, and equal tiles within each mode; padded rows fit in 35 KB (of the
+// four CTAs of an SM 140).  l0, lq: log2 of the lanes along each mode.
 void perm_tile(int64_t n0, int64_t nq, int& e0, int& eq, int& l0, int& lq) {
   auto even = [](int64_t n, int64_t cap) { return (int)((n + (n + cap - 1) / cap - 1) / ((n + cap - 1) / cap)); };
   int64_t c0 = 64, cq = 64;

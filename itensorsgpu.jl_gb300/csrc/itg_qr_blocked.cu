@@ -1,5 +1,5 @@
 // Blocked Householder QR and the application of its Q, with the trailing
-// updates as matrix products through the contraction engine (compact WY form
+// updates as matrix products by kernels of their own (compact WY form
 // of Schreiber & Van Loan, "A storage-efficient WY representation for
 // products of Householder transformations", SIAM J. Sci. Stat. Comput. 10
 // (1989); the T recurrence is LAPACK's larft, restated).

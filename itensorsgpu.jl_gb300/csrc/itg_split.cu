@@ -240,8 +240,8 @@ __host__ __device__ __forceinline__ int digit_log2(int p) { return p == 0 ? 8 : 
 // (level L, pair p, k-block kb) in level-major order; a group is a run of
 // items of one level whose summed |product| bound stays <= 2^24.  It is walked
 // in runs of k-blocks of one pair inside one group: the two roles that issue an
-// item are one thread each, and stepping the schedule item by item cost them
-// 640 clocks of an item's 900 (its four products take 512).
+// item are one warp each with one lane that issues, and stepping the schedule item
+// by item took 640 clocks of an item's 900 (its four products take 512).
 constexpr int GROUP_LOG2 = 24, BK_LOG2 = 6;
 static_assert(BK == 1 << BK_LOG2, "");
 struct Sched {
@@ -429,8 +429,8 @@ __device__ __forceinline__ void load_acc16(uint32_t lane_base, const long long* 
 // last one to arrive converts.  Nobody waits for anybody else.
 //
 // What bounds it: per item of four products, first the issuing warp, not the
-// copies (without any loads the time was the same): stepping the schedule, its
-// operands moved to uniform registers inside a one-lane branch and a fence took
+// copies (without any loads the time was the same): stepping the schedule,
+// issuing from a branch for one lane and a fence took
 // 900 clocks where the products take 512 (BN = 256) or 256.  Runs of k-blocks
 // (Sched), warp-wide loops with one elected lane and two items a stage
 // (BN = 128) brought an item from 0.49 to 0.39 us (256) and 0.23 (128), the two
@@ -497,9 +497,9 @@ k_split_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ C
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    // The whole warp walks the schedule and one lane issues (as below): inside
-    // a branch for one lane every operand of a copy or product would have to be
-    // moved to the uniform registers again.
+    // The whole warp walks the schedule and one lane issues (as below): the
+    // four products of an item took 316 clocks to issue from a loop that was
+    // inside a branch for one lane.
     const bool leader = elect_one();
     int it = 0, s = 0;
     uint32_t ph = 1;  // parity of the stage's last release (none before the first round)
