@@ -680,10 +680,11 @@ int jacobi_run(itg_handle* h, double* W, int64_t m, int64_t n, double* V, int* f
   if (h->jacobi_mode == 0 || h->jacobi_mode == 3) {
     // Small columns that W came with (a graded matrix) are not noise: one-sided
     // rotations resolve them relative to their own size, but not in the one
-    // sweep that the FP32 start leaves to the large ones.  They count as well,
-    // in a bounded number of sweeps, as other columns of W may be noise.
+    // sweep that the FP32 start leaves to the large ones.  They count as well
+    // (amin_conv 0: by the steps that tell pairs of any ratio), in a bounded
+    // number of sweeps, as other columns of W may be noise.
     int before = 0;
-    if (start32(h, m, n) && grading && grading[0] > 0.0 && grading[0] < NOISE) {
+    if (h->jacobi_mode == 0 && m <= 2048 && grading && grading[0] > 0.0 && grading[0] < NOISE) {
       const int st = itg::jacobi_blocked<double>(h, W, m, (int)n, V, tol, 0.0, GRADED_SWEEPS, flag_dev, &before, 0.0);
       if (st != ITG_ERR_NOTCONVERGED) {
         *sweeps_done = before;

@@ -464,11 +464,13 @@ __device__ __forceinline__ T jp_transpose_sum(T (&v)[NV], int lane) {
 //
 // jp_angle: the rotation of a pair from its squared norms and dot product;
 // true when the pair is rotated.  t = tan(theta), for the norms' update; major:
-// it counts against convergence.
+// it counts against convergence.  FAR (FP64): the pair's norms may be any factor
+// apart, see below.
 __device__ __forceinline__ float jp_sqrt1p2(float x) {  // sqrt(1 + x^2), a few ulp
   const float y = fmaf(x, x, 1.f);
   return y * rsqrtf(y);
 }
+template <bool FAR>
 __device__ __forceinline__ bool jp_angle(float a, float b, float g, float tol, float tol_conv, float amin,
                                          float amin_conv, float& t, float& u, float& s, bool& major) {
   const float cosine = fabsf(g) * rsqrtf(a) * rsqrtf(b);  // NaN for a zero column
@@ -501,17 +503,26 @@ __device__ __forceinline__ double jp_to_double(float x) {  // normal numbers; be
 __device__ __forceinline__ bool jp_less(double x, double y) {  // x < y for non-negative x and y
   return __double_as_longlong(x) < __double_as_longlong(y);
 }
+template <bool FAR>
 __device__ __forceinline__ bool jp_angle(double a, double b, double g, float tol, float tol_conv, double amin,
                                          double amin_conv, double& t, double& u, double& s, bool& major) {
-  // scaled by a power of two so that max(a, b) is in [1, 2): FP32 then spans
-  // norm ratios to 1e-19
+  // scaled by a power of two so that max(a, b) is in [1, 2)
   const int ea = (__double2hiint(a) >> 20) & 0x7FF, eb = (__double2hiint(b) >> 20) & 0x7FF;
   const int e = ea > eb ? ea : eb;
   const double d = b - a;
   const float fg = jp_to_float(g, e), fa = jp_to_float(a, e), fb = jp_to_float(b, e), fd = jp_to_float(d, e);
-  const float cosine = fabsf(fg) * rsqrtf(fa) * rsqrtf(fb);
-  major = jp_less(amin_conv, a) && jp_less(amin_conv, b) && cosine > tol_conv;
-  const bool rot = jp_less(amin, a) && jp_less(amin, b) && cosine > tol;
+  float cosine = fabsf(fg) * rsqrtf(fa) * rsqrtf(fb);
+  // Norms more than 2^55 apart (a graded matrix): the squares and g leave FP32's
+  // range, so the cosine takes each number by its own exponent; the angle is g / d
+  // to the last bit.  (In every sweep it would cost 1 to 2 % of an SVD.)
+  const int lo = ea < eb ? ea : eb;
+  const bool far = FAR && lo + 110 < e;
+  if (far)
+    cosine = fabsf(jp_to_float(g, (ea + eb) >> 1)) * rsqrtf(jp_to_float(a, ea)) * rsqrtf(jp_to_float(b, eb)) *
+             ((ea + eb) & 1 ? 0.70710678f : 1.f);
+  major = (!FAR || lo > 0) && jp_less(amin_conv, a) && jp_less(amin_conv, b) && cosine > tol_conv;
+  // (a column with NaN or infinity is left alone)
+  const bool rot = e < 2047 && jp_less(amin, a) && jp_less(amin, b) && cosine > tol;
   const float zeta = __fdividef(fd, 2.f * fg);
   const float az = fabsf(zeta);
   const float tf = copysignf(__fdividef(az > 1e9f ? 0.5f : 1.f, az > 1e9f ? az : az + jp_sqrt1p2(az)), zeta);
@@ -535,6 +546,12 @@ __device__ __forceinline__ bool jp_angle(double a, double b, double g, float tol
   const double s0 = (u + u) * r;
   const double er = fma(-x, r, 1.0);
   s = fma(s0, fma(er, er, er), s0);
+  if (far) {
+    const double p = __hiloint2double((2046 - ((__double2hiint(d) >> 20) & 0x7FF)) << 20, 0), dm = d * p;
+    const double r0 = jp_to_double(__fdividef(1.f, jp_to_float(dm, 1023)));
+    t = s = g * p * fma(r0, fma(-dm, r0, 1.0), r0);
+    u = 0.5 * t;
+  }
   if (!rot) t = u = s = 0.0;
   return rot;
 }
@@ -549,7 +566,7 @@ constexpr int64_t JR_MAX_M = 2048;  // rows held in registers: 8 for each of 256
 
 // `prev`: nullptr, or the rotated flag of the sweep before (the step does
 // nothing when that sweep had converged; lets several sweeps be queued).
-template <class T, int WB, int RPT, bool VEC, bool FIRST, int MAXT>
+template <class T, int WB, int RPT, bool VEC, bool FIRST, int MAXT, bool FAR>
 __global__ void __launch_bounds__(MAXT)
 k_jacobi_reg_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, float tol, float tol_conv, T amin,
                   T amin_conv, int step, const int* prev, int* rotated) {
@@ -696,7 +713,7 @@ k_jacobi_reg_step(T* __restrict__ W, int64_t m, int n, T* __restrict__ V, float 
     const T a = __shfl_sync(0xffffffffu, norm, pr), b = __shfl_sync(0xffffffffu, norm, partner(pr));
     T tt, u, s;
     bool major;
-    const bool rot = jp_angle(a, b, g, tol, tol_conv, amin, amin_conv, tt, u, s, major);
+    const bool rot = jp_angle<FAR>(a, b, g, tol, tol_conv, amin, amin_conv, tt, u, s, major);
     const T an = a - tt * g, bn = b + tt * g;
     const unsigned mask = __ballot_sync(0xffffffffu, rot) & ((1u << WB) - 1u);
     any_major |= __ballot_sync(0xffffffffu, rot && major);
@@ -793,7 +810,7 @@ k_jacobi32_small(const double* __restrict__ W, int m, int n, double scale, float
         g = __shfl_sync(0xffffffffu, d, 16);
         float tt, u, s;
         bool major;
-        if (jp_angle(a, b, g, tol, tol, amin, amin_conv, tt, u, s, major)) {
+        if (jp_angle<false>(a, b, g, tol, tol, amin, amin_conv, tt, u, s, major)) {
 #pragma unroll
           for (int k = 0; k < RPT; ++k) {
             wp[32 * k] = fmaf(-s, fmaf(u, x[k], y[k]), x[k]);
@@ -967,7 +984,7 @@ int jb_run(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_co
 
 // Register-resident steps (m <= JR_MAX_M), each launched so that it may start
 // while its predecessor drains (it waits for its results itself).
-template <class T, int WB, int RPT, bool VEC, int MAXT>
+template <class T, int WB, int RPT, bool VEC, int MAXT, bool FAR = false>
 int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_conv, int max_sweeps, int* flag,
              int* sweeps) {
   const int nb = (n + WB - 1) / WB, nbp = nb + (nb & 1);
@@ -979,7 +996,8 @@ int jr_run_t(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_
   const dim3 grid((unsigned)(nbp / 2));
   const float tolf = (float)tol, tolc = (float)conv_tol(tol);
   return jb_sweeps(h, nbp - 1, max_sweeps, chunk, flag, sweeps, [&](int, int step, const int* prev, int* rot) {
-    auto kernel = step == 0 ? k_jacobi_reg_step<T, WB, RPT, VEC, true, MAXT> : k_jacobi_reg_step<T, WB, RPT, VEC, false, MAXT>;
+    auto kernel = step == 0 ? k_jacobi_reg_step<T, WB, RPT, VEC, true, MAXT, FAR>
+                            : k_jacobi_reg_step<T, WB, RPT, VEC, false, MAXT, FAR>;
     return itg_launch_after(h, true, grid, threads, 0, kernel, W, m, n, V, tolf, tolc, amin, amin_conv, step, prev, rot);
   });
 }
@@ -1006,10 +1024,16 @@ int jr_run(itg_handle* h, T* W, int64_t m, int n, T* V, T tol, T amin, T amin_co
     if (vec) return jr_run_t<T, 8, 8, true, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
     return jr_run_t<T, 8, 8, false, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
   } else {
-    if (m <= 128) return jr_run_t<T, 4, 1, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
-    if (m <= 256) return jr_run_t<T, 4, 2, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
-    if (m <= 512) return jr_run_t<T, 4, 4, false, 128>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
-    return jr_run_t<T, 4, 8, false, 256>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    auto run = [&](auto far) {
+      constexpr bool F = decltype(far)::value;
+      if (m <= 128) return jr_run_t<T, 4, 1, false, 128, F>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+      if (m <= 256) return jr_run_t<T, 4, 2, false, 128, F>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+      if (m <= 512) return jr_run_t<T, 4, 4, false, 128, F>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+      return jr_run_t<T, 4, 8, false, 256, F>(h, W, m, n, V, tol, amin, amin_conv, max_sweeps, flag, sweeps);
+    };
+    // columns of any size count: a graded matrix
+    if (amin_conv == T(0)) return run(std::true_type());
+    return run(std::false_type());
   }
 }
 

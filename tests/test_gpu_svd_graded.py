@@ -45,3 +45,28 @@ def test_values_of_a_graded_matrix(gpu, n, p, order):
     U, S, V, _ = gpu.svd(gpu.cuITensor(A, i, j), i, mindim=n)
     rel = np.abs(S.store.data.cpu().numpy() / ref - 1)
     assert rel.max() <= 100 * 4 * n * EPS
+
+
+@pytest.mark.parametrize("n,p,order", [(16, 40, "down"), (24, 60, "mixed"), (44, 40, "up"), (97, 60, "down"),
+                                       (150, 40, "mixed")])
+def test_sizes_beyond_fp32(gpu, n, p, order):
+    """Squared norms further apart than FP32's range: the sweeps must still see which pairs are orthogonal, and end."""
+    test_factors_of_a_graded_matrix(gpu, n, p, False, order)
+
+
+@pytest.mark.parametrize("n,tiny", [(14, 1e-25), (24, 1e-18), (48, 1e-18), (96, 1e-25), (192, 1e-18)])
+def test_one_small_column(gpu, n, tiny):
+    """A single column far below the others: a few sweeps more than without it, not as many as are allowed."""
+    import ctypes as C
+    from itg import _lib
+    A = np.random.default_rng(n).standard_normal((n, n))
+    A[:, 3] *= tiny
+    i, j = gpu.Index(n), gpu.Index(n)
+    U, S, V, _ = gpu.svd(gpu.cuITensor(A, i, j), i, mindim=n)
+    sweeps = C.c_int()
+    _lib.handle(0).call("itg_svd_info", C.byref(sweeps), None, None)
+    assert sweeps.value <= 8
+    tol = 4 * n * EPS
+    u, s, v = U.array(), S.store.data.cpu().numpy(), V.array()
+    assert max(np.abs(q.T @ q - np.eye(n)).max() for q in (u, v)) <= tol
+    assert np.linalg.norm((u * s) @ v.T - A) <= tol * np.linalg.norm(A)
