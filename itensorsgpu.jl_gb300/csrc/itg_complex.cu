@@ -213,6 +213,7 @@ extern "C" int itg_contract_z(itg_handle* h, int dtypeA, int dtypeB, const doubl
     if (dimsB[i] < 0) return itg_fail(h, ITG_ERR_SHAPE, "negative dimension");
   for (int i = 0; i < rankC; ++i)
     if (dimsC[i] < 0) return itg_fail(h, ITG_ERR_SHAPE, "negative dimension");
+  h->chained = false;  // a product with a real operand is this call's first launch (as in itg_contract)
   return itg::contract_z(h, dtypeA, dtypeB, alpha[0], alpha[1], (const double*)A, rankA, dimsA, modesA,
                          (const double*)B, rankB, dimsB, modesB, beta[0], beta[1], (double*)C, rankC, dimsC, modesC,
                          precision);

@@ -117,3 +117,44 @@ def test_products_in_a_capture(gpu, h):
     chain(direct)
     h.call("itg_synchronize")
     assert all(torch.equal(a, b) for a, b in zip(outs, direct))
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "split"])
+def test_mixed_product_behind_another_streams_event(gpu, h, prec):
+    """real x complex, whose first launch is the product itself: both operands come from a second stream."""
+    import torch
+    from itg import _lib
+    rng = np.random.default_rng(6)
+    reals = [rng.standard_normal((N, N)) for _ in range(4)]
+    cplx = [rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N)) for _ in range(4)]
+    dev = lambda x: torch.from_numpy(x.ravel(order="F").copy()).cuda()
+    dr, dc = [dev(x) for x in reals], [dev(x) for x in cplx]
+    big = torch.empty(1 << 26, dtype=torch.float64, device="cuda")
+    A, B = torch.zeros_like(dr[0]), torch.zeros_like(dc[0])
+    got = [torch.empty_like(B) for _ in dr]
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    h.call("itg_set_stream", C.c_void_p(s1.cuda_stream))
+    d, m = _lib.i64arr([N, N]), _lib.i32arr
+    one, zero = (C.c_double * 2)(1.0, 0.0), (C.c_double * 2)(0.0, 0.0)
+
+    def mul(out):
+        h.call("itg_contract_z", 0, 1, one, _p(A), 2, d, m([1, 2]), _p(B), 2, d, m([2, 3]), zero, _p(out), 2, d,
+               m([1, 3]), prec)
+    torch.cuda.synchronize()
+    mul(got[0])                             # plans, tuning
+    torch.cuda.synchronize()
+    for x, z, g in zip(dr, dc, got):
+        with torch.cuda.stream(s2):
+            s2.wait_stream(s1)
+            big.fill_(1.0)
+            A.copy_(x)
+            B.copy_(z)
+            ev = s2.record_event()
+        s1.wait_event(ev)                   # the last thing that the library put on s1 is a product
+        mul(g)
+    torch.cuda.synchronize()
+    for x, z, g in zip(reals, cplx, got):
+        ref = x @ z
+        # N eps |x| |z|, with |x| |z| ~ sqrt(N) |x z|, is 2e-13
+        got_xz = g.cpu().numpy().reshape(N, N, order="F")
+        assert np.linalg.norm(got_xz - ref) <= 1e-12 * np.linalg.norm(ref)
